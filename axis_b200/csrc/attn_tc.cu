@@ -41,24 +41,6 @@ struct FwdSmem {
     static constexpr int Q = 0, K0 = 16384, V0 = K0 + 2 * 16384, BARS = V0 + 2 * 16384, TOTAL = BARS + 128 + 1024;
 };
 
-// Issue forms for a converged warp: every lane executes the surrounding code (so addresses and descriptors stay
-// warp-uniform and cheap to form) and the elected lane issues.  Measured on B200: a 128 x 64 x 16 MMA with A in
-// TMEM issues every 32.6 cycles this way (its 32 cycles of math) against 45-50 from a lone thread in a divergent branch.
-__device__ __forceinline__ void mma_ts_e(uint32_t d, uint32_t a, uint64_t bd, uint32_t id, uint32_t acc) {
-    asm volatile("{\n\t.reg .pred p, q;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-                 ::"r"(d), "r"(a), "l"(bd), "r"(id), "r"(acc) : "memory");
-}
-__device__ __forceinline__ void mma_ss_e(uint32_t d, uint64_t ad, uint64_t bd, uint32_t id, uint32_t acc) {
-    asm volatile("{\n\t.reg .pred p, q;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                 ::"r"(d), "l"(ad), "l"(bd), "r"(id), "r"(acc) : "memory");
-}
-__device__ __forceinline__ void commit_e(uint32_t bar) {
-    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
-                 "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar) : "memory");
-}
-
 // Forward CTA: 128 queries of one head; four softmax warps (a thread owns a query row) and one control warp that
 // loads by TMA and issues the MMAs.  TMEM (256 columns, two CTAs per SM): S 0..127, P 128..191 (packed bf16),
 // O 192..255.  P has columns of its own, so S(j+1) = Q K(j+1)^T is issued as soon as the softmax threads have read
@@ -346,11 +328,6 @@ struct BwdSmem {
 };
 static_assert(BwdSmem::TOTAL <= 227 * 1024, "backward shared memory exceeds the per-CTA limit");
 static_assert(BwdSmem::DO0 % 1024 == 0 && BwdSmem::DS0 % 1024 == 0 && BwdSmem::DQ % 1024 == 0, "swizzled tiles need 1024-byte alignment");
-
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* r) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
-}
 
 #ifdef AXENG_PROF
 // instrumented builds only: per-CTA cycle counters (16 long long per CTA), see the host launcher

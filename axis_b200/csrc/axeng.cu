@@ -113,7 +113,7 @@ API int eng_init(void) {
     if (cudaMalloc(&G.d_status, 64)) { set_err("status alloc failed"); return 3; }
     cudaMemset(G.d_status, 0, 64);
     if (ax_gemm_tc_init()) { set_err("tensor-core GEMM init failed: %s", cudaGetErrorString(cudaGetLastError())); return 4; }
-    if (ax_attn_mma_init() || ax_attn_tc_init()) { set_err("tensor-core attention init failed: %s", cudaGetErrorString(cudaGetLastError())); return 4; }
+    if (ax_attn_mma_init() || ax_attn_tc_init() || ax_attn_tcs_init()) { set_err("tensor-core attention init failed: %s", cudaGetErrorString(cudaGetLastError())); return 4; }
     memset(G.prof_ms, 0, sizeof(G.prof_ms));
     memset(G.prof_calls, 0, sizeof(G.prof_calls));
     G.inited = true; G.rank = 0; G.world = 1; G.fallback = 0;
@@ -878,6 +878,7 @@ static int exec_op(const EngOp* op) {
             G.launches++;
             if (dt == 1 && !(G.fallback & 2)) {
                 int rc = ax_attn_fwd_tc(BUFP(op->a), BUFP(op->b), BUFP(op->d), BUFP(op->c), (float*)BUFP(op->sa), s, G.d_status, st);
+                if (rc < 0) rc = ax_attn_fwd_tcs(BUFP(op->a), BUFP(op->b), BUFP(op->d), BUFP(op->c), (float*)BUFP(op->sa), s, G.d_status, st);
                 if (rc < 0) rc = ax_attn_fwd_mma(BUFP(op->a), BUFP(op->b), BUFP(op->d), BUFP(op->c), (float*)BUFP(op->sa), s, st);
                 if (rc >= 0) return rc;
             }
@@ -923,8 +924,12 @@ static int exec_op(const EngOp* op) {
                 if (rc) return rc;
                 rc = -1;
                 for (int fuse = rc_ != nullptr; rc < 0 && fuse >= 0 && dt == 1 && !(G.fallback & 2); fuse--) {
-                    rc = ax_attn_bwd_mma(BUFP(op->a), BUFP(op->b), BUFP(op->d), BUFP(op->c), (const float*)BUFP(op->sa), (const float*)BUFP(op->oc),
-                                         BUFP(op->tb), BUFP(op->sc), BUFP(op->oa), s, fuse ? rc_ : nullptr, fuse ? rs_ : nullptr, st);
+                    const float* cs = fuse ? rc_ : nullptr; const float* sn = fuse ? rs_ : nullptr;
+                    rc = ax_attn_bwd_tcs(BUFP(op->a), BUFP(op->b), BUFP(op->d), BUFP(op->c), (const float*)BUFP(op->sa), (const float*)BUFP(op->oc),
+                                         BUFP(op->tb), BUFP(op->sc), BUFP(op->oa), s, cs, sn, G.d_status, st);
+                    if (rc < 0)
+                        rc = ax_attn_bwd_mma(BUFP(op->a), BUFP(op->b), BUFP(op->d), BUFP(op->c), (const float*)BUFP(op->sa), (const float*)BUFP(op->oc),
+                                             BUFP(op->tb), BUFP(op->sc), BUFP(op->oa), s, cs, sn, st);
                     rotated = rc == 0 && fuse;
                 }
                 if (rc < 0)

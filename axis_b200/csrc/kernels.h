@@ -143,6 +143,12 @@ int ax_lora_proj(int count, int tb, const void* const* X, const void* const* W, 
 int ax_lora_grad(int count, const void* const* X, const void* const* S, float* const* out, const int* F, const int* layout,
                  int N, int R, float alpha, float* ws, size_t ws_bytes, cudaStream_t st);
 
+// attn_tcs.cu — the same on tcgen05 for head dims above 32 up to 64 (rope_cos / rope_sin for 64), a positive scale and enough work to
+// fill the GPU. -1 when not served.
+int ax_attn_tcs_init(void);
+int ax_attn_fwd_tcs(const void* q, const void* k, const void* v, void* o, float* lse, const AttnShape& s, int* status, cudaStream_t st);
+int ax_attn_bwd_tcs(const void* q, const void* k, const void* v, const void* dO, const float* lse, const float* Dv, void* dq, void* dk, void* dv,
+                    const AttnShape& s, const float* rope_cos, const float* rope_sin, int* status, cudaStream_t st);
 // attn_mma.cu — mma.sync attention with P and dS held to 16 bits and a sign (bf16 [B,T,H,DH], DH a multiple of 8 up to 128, any T),
 // the same bits on every run. -1 when not served.  Dv as ax_attn_bwd_simt; rope_cos / rope_sin as ax_attn_bwd_tc, for DH 32, 64, 128.
 int ax_attn_mma_init(void);

@@ -278,6 +278,25 @@ def test_attention_of_other_shapes_keeps_fp32_probabilities(eng, B, H, KV, T, DH
         assert err(runs[0][n]) <= 1.01 * err(general[n]), (n, err(runs[0][n]), err(general[n]))
 
 
+@pytest.mark.parametrize("B,H,KV,T,DH,gain", [
+    (40, 8, 4, 3, 64, 1), (20, 16, 8, 64, 48, 1), (20, 16, 8, 65, 64, 1),       # one tile: a piece of a step, one step, two
+    (4, 12, 4, 129, 64, 1), (2, 16, 2, 500, 56, 1),                             # dK / dV over clusters of two and four, some CTAs with no step
+    (1, 10, 5, 1000, 64, 6), (1, 8, 8, 1300, 40, 1)])                           # scores that move the running maximum; a narrow head
+def test_attention_with_split_probabilities_on_tcgen05(eng, B, H, KV, T, DH, gain):
+    """The shapes of the test above that fill the GPU, on the tcgen05 kernels, with the same bound against float64 and on every run;
+    gain spreads the scores, so that rows of the forward rescale."""
+    rng = np.random.default_rng(T + DH)
+    q, k, v, do = make(rng, B, H, KV, T, DH, 1)
+    scale = gain / np.sqrt(DH)
+    runs = run_bf16_attention(eng, q, k, v, do, scale, 0, times=3)
+    assert eng.last_variant() == 0x81
+    general = run_bf16_attention(eng, q, k, v, do, scale, 2)[0]
+    for n, exact in attention_f64(q, k, v, do, scale).items():
+        assert all(np.array_equal(runs[0][n], r[n]) for r in runs[1:]), n
+        err = lambda bits: float(np.linalg.norm(E.bf16_bits_to_f32(bits).transpose(0, 2, 1, 3) - exact) / np.linalg.norm(exact))
+        assert err(runs[0][n]) <= 1.01 * err(general[n]), (n, err(runs[0][n]), err(general[n]))
+
+
 @pytest.mark.parametrize("scale", [-0.25, 0.0])
 @pytest.mark.parametrize("B,H,KV,T,DH", [(1, 4, 2, 256, 64), (1, 2, 1, 256, 128), (1, 4, 2, 200, 64), (1, 2, 2, 72, 32)])
 def test_attention_with_a_scale_that_is_not_positive(eng, B, H, KV, T, DH, scale):
