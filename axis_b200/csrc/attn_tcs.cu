@@ -17,8 +17,8 @@
 //
 // Bound by the softmax warps: the schedulers issue in 37 % (forward) and 46 % (dK / dV) of the cycles, the XU pipe (exponentials) is busy
 // 37 % and 23 %; what is left of a step is the round trip MMA -> TMEM load -> MMA, which two CTAs or two groups cover in part.
-// Forward / backward with the row dots in us, mma.sync -> here (one cold launch each): B3 H24 KV8 T1000 DH64 70 / 203 -> 36 / 112,
-// B4 H24 KV8 T500 DH64 33 / 102 -> 22 / 64, B1 H12 KV4 T2500 DH64 88 / 225 -> 46 / 141, B8 H24 KV8 T320 DH64 29 / 85 -> 25 / 58.
+// Forward / backward with the row dots in us, mma.sync -> here (one cold launch each): B3 H24 KV8 T1000 DH64 70 / 203 -> 36 / 106,
+// B4 H24 KV8 T500 DH64 33 / 102 -> 22 / 60, B1 H12 KV4 T2500 DH64 88 / 225 -> 46 / 137, B8 H24 KV8 T320 DH64 29 / 85 -> 25 / 52.
 #include "common.cuh"
 #include "kernels.h"
 #include "tc_common.cuh"

@@ -431,7 +431,29 @@ int ax_silu_bwd(int dt, const void* g, const void* u, const void* grad, void* dg
     return 0;
 }
 
-// ── row dot: c[r] = sum_d a[r,d] * b[r,d], one warp per row ────────────────
+// ── row dot: c[r] = sum_d a[r,d] * b[r,d] ──────────────────────────────────
+// G lanes share a row, one 16-byte piece of each operand per lane
+template <typename T, int G>
+__global__ void k_rowdot_vec(const T* __restrict__ a, const T* __restrict__ b, float* __restrict__ c, long long rows, int dim) {
+    pdl_enter();
+    constexpr int V = 16 / sizeof(T);
+    const int per = blockDim.x / G, sub = threadIdx.x % G;
+    for (long long r0 = (long long)blockIdx.x * per; r0 < rows; r0 += (long long)gridDim.x * per) {      // whole warps stay: the shuffles see 32 lanes
+        const long long r = r0 + threadIdx.x / G;
+        float acc = 0.f;
+        if (r < rows && sub * V < dim) {
+            float x[V], y[V];
+            Vec<T>::ld(a + r * dim + sub * V, x);
+            Vec<T>::ld(b + r * dim + sub * V, y);
+#pragma unroll
+            for (int q = 0; q < V; q++) acc += x[q] * y[q];
+        }
+#pragma unroll
+        for (int o = G / 2; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (sub == 0 && r < rows) c[r] = acc;
+    }
+}
+// any width: one warp per row
 template <typename T>
 __global__ void k_rowdot(const T* a, const T* b, float* c, long long rows, int dim) {
     const int lane = threadIdx.x & 31;
@@ -445,6 +467,16 @@ __global__ void k_rowdot(const T* a, const T* b, float* c, long long rows, int d
 }
 int ax_rowdot(int dt, const void* a, const void* b, float* c, long long rows, int dim, cudaStream_t st) {
     if (rows <= 0) return 0;
+    // rows of whole 16-byte pieces, up to a warp of them (head dims): 2000 x 24 rows of 64 bf16 in a step, 8.1 us with a warp to a row, 3.4 us here
+    const int V = dt >= 1 ? 8 : 4, pieces = dim / V;
+    if (dim % V == 0 && pieces >= 1 && pieces <= 32 && aligned16(a) && aligned16(b)) {
+        const int G = pieces <= 4 ? 4 : pieces <= 8 ? 8 : pieces <= 16 ? 16 : 32;
+        auto go = [&](auto kern, auto* x, auto* y) { return ax_launch_chain(kern, dim3(ew_grid(rows * G, T256)), dim3(T256), 0, st, x, y, c, rows, dim) == cudaSuccess ? 0 : 3; };
+        const bf16 *ab = (const bf16*)a, *bb = (const bf16*)b;
+        const float *af = (const float*)a, *bf = (const float*)b;
+        if (dt >= 1) return G == 4 ? go(k_rowdot_vec<bf16, 4>, ab, bb) : G == 8 ? go(k_rowdot_vec<bf16, 8>, ab, bb) : G == 16 ? go(k_rowdot_vec<bf16, 16>, ab, bb) : go(k_rowdot_vec<bf16, 32>, ab, bb);
+        return G == 4 ? go(k_rowdot_vec<float, 4>, af, bf) : G == 8 ? go(k_rowdot_vec<float, 8>, af, bf) : G == 16 ? go(k_rowdot_vec<float, 16>, af, bf) : go(k_rowdot_vec<float, 32>, af, bf);
+    }
     if (dt >= 1) k_rowdot<bf16><<<ew_grid(rows * 32, T256), T256, 0, st>>>((const bf16*)a, (const bf16*)b, c, rows, dim);
     else k_rowdot<float><<<ew_grid(rows * 32, T256), T256, 0, st>>>((const float*)a, (const float*)b, c, rows, dim);
     return 0;
