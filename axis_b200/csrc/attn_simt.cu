@@ -11,7 +11,7 @@
 // of a lane go back to the warp as one 16-byte piece.  Tiles of the walked operand
 // are double-buffered (cp.async for fp32), so the next tile's load runs under
 // this one's arithmetic.  B2 H8 KV4 T256 DH32 fp32, one cold launch: forward 64 -> 23 us,
-// dQ 65 -> 23 us, dK/dV 115 -> 54 us against one row per warp and scalar reads.
+// dQ 65 -> 23 us, dK/dV 115 -> 54 us against one row per warp and scalar reads; with the walk cut over clusters 21, 17 and 22.
 #include <initializer_list>
 
 #include "common.cuh"
@@ -97,10 +97,22 @@ __device__ __forceinline__ void attn_axpy(float (&acc)[AR][NJ], const float* w, 
     }
 }
 
+// Where rows are few, a cluster of S CTAs takes the tiles that a block of rows walks in turn, and the sums meet through distributed
+// shared memory: a unit is a warp's row of accumulators, [unit][i][thread], and each CTA finishes 1 / S of the units, in rank order.
+__device__ __forceinline__ void attn_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float attn_peer(const float* p, int rank) {
+    float x;
+    asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %1, %2;\n\tld.shared::cluster.f32 %0, [ra];\n\t}"
+                 : "=f"(x) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank) : "memory");
+    return x;
+}
+
 template <typename T, int NJ>
 __global__ void __launch_bounds__(ATH)
 k_attn_fwd_simt(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, T* __restrict__ o,
-                float* __restrict__ lse, AttnShape s, int vec) {
+                float* __restrict__ lse, AttnShape s, int vec, int S) {
     extern __shared__ __align__(16) float smem[];
     const int DH = s.DH, LD = attn_ld(DH), q4 = (DH + 3) / 4, TILE = AKT * LD;
     float* Ks = smem;                    // two tiles each
@@ -109,12 +121,16 @@ k_attn_fwd_simt(const T* __restrict__ q, const T* __restrict__ k, const T* __res
     float* Ps = Qs + TILE;               // [warp][key][AR]
     const int b = blockIdx.z, h = blockIdx.y, g = h / (s.H / s.KV);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r0 = (gridDim.x - 1 - blockIdx.x) * ABLK, t0 = r0 + warp * AR;      // the longest rows first
+    const int part = blockIdx.x % S, r0 = (gridDim.x / S - 1 - blockIdx.x / S) * ABLK, t0 = r0 + warp * AR;      // the longest rows first
     const T* kbase = k + b * s.kb + g * s.kh;
     const T* vbase = v + b * s.kb + g * s.kh;
+    const int ntiles = min(r0 + ABLK - 1, s.T - 1) / AKT + 1;
+    pdl_enter();
     attn_tile(Qs, q + b * s.qb + h * s.qh, s.qt, r0, s.T, DH, LD, vec);
-    attn_tile(Ks, kbase, s.kt, 0, s.T, DH, LD, vec);
-    attn_tile(Vs, vbase, s.kt, 0, s.T, DH, LD, vec);
+    if (part < ntiles) {
+        attn_tile(Ks, kbase, s.kt, part * AKT, s.T, DH, LD, vec);
+        attn_tile(Vs, vbase, s.kt, part * AKT, s.T, DH, LD, vec);
+    }
     attn_commit();
     float m[AR], l[AR], acc[AR][NJ];     // l: this lane's share of the row sum
 #pragma unroll
@@ -125,14 +141,13 @@ k_attn_fwd_simt(const T* __restrict__ q, const T* __restrict__ k, const T* __res
     }
     const float* myQ = Qs + warp * AR * LD;
     float* myP = Ps + warp * AKT * AR;
-    const int ntiles = min(r0 + ABLK - 1, s.T - 1) / AKT + 1;
-    for (int kt = 0; kt < ntiles; kt++) {
+    for (int kt = part, cur = 0; kt < ntiles; kt += S, cur ^= 1) {
         attn_wait();
         __syncthreads();
-        const int cur = kt & 1, nxt = cur ^ 1;
-        if (kt + 1 < ntiles) {
-            attn_tile(Ks + nxt * TILE, kbase, s.kt, (kt + 1) * AKT, s.T, DH, LD, vec);
-            attn_tile(Vs + nxt * TILE, vbase, s.kt, (kt + 1) * AKT, s.T, DH, LD, vec);
+        const int nxt = cur ^ 1;
+        if (kt + S < ntiles) {
+            attn_tile(Ks + nxt * TILE, kbase, s.kt, (kt + S) * AKT, s.T, DH, LD, vec);
+            attn_tile(Vs + nxt * TILE, vbase, s.kt, (kt + S) * AKT, s.T, DH, LD, vec);
         }
         attn_commit();
         if (kt * AKT > t0 + AR - 1) continue;
@@ -156,6 +171,42 @@ k_attn_fwd_simt(const T* __restrict__ q, const T* __restrict__ k, const T* __res
         attn_axpy<NJ>(acc, myP, Vs + cur * TILE, LD, DH, lane);
         __syncwarp();
     }
+    if (S > 1) {                         // merge: sums at the largest of the ranks' maxima
+        attn_wait();
+        __syncthreads();
+        float* acc_x = smem + threadIdx.x;
+        float* ml_x = smem + AR * NJ * ATH + warp * AR * 2;
+#pragma unroll
+        for (int r = 0; r < AR; r++) {
+            const float ls = warp_sum(l[r]);
+            if (lane == 0) { ml_x[r * 2] = m[r]; ml_x[r * 2 + 1] = ls; }
+#pragma unroll
+            for (int i = 0; i < NJ; i++) acc_x[(r * NJ + i) * ATH] = acc[r][i];
+        }
+        attn_cluster_sync();
+        for (int r = part * AR / S; r < (part + 1) * AR / S; r++) {
+            const int t = t0 + r;
+            if (t >= s.T) continue;
+            float mx = -3.0e38f, ls = 0.f, a[NJ];
+            for (int q = 0; q < S; q++) mx = fmaxf(mx, attn_peer(ml_x + r * 2, q));
+#pragma unroll
+            for (int i = 0; i < NJ; i++) a[i] = 0.f;
+            for (int q = 0; q < S; q++) {
+                const float f = expf(attn_peer(ml_x + r * 2, q) - mx);
+                ls += attn_peer(ml_x + r * 2 + 1, q) * f;
+#pragma unroll
+                for (int i = 0; i < NJ; i++) a[i] += attn_peer(acc_x + (r * NJ + i) * ATH, q) * f;
+            }
+            T* orow = o + b * s.qb + h * s.qh + (long long)t * s.qt;
+            const float il = 1.f / ls;
+#pragma unroll
+            for (int i = 0; i < NJ; i++)
+                if (lane + 32 * i < DH) stf(orow, lane + 32 * i, a[i] * il);
+            if (lse && lane == 0) lse[((long long)b * s.H + h) * s.T + t] = mx + logf(ls);
+        }
+        attn_cluster_sync();             // peers have read
+        return;
+    }
 #pragma unroll
     for (int r = 0; r < AR; r++) {
         const int t = t0 + r;
@@ -177,7 +228,7 @@ template <typename T, typename TO, int NJ>
 __global__ void __launch_bounds__(ATH)
 k_attn_bwd_dq_simt(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
                    const T* __restrict__ dO, const float* __restrict__ lse, const float* __restrict__ Dv,
-                   TO* __restrict__ dq, AttnShape s, int vec) {
+                   TO* __restrict__ dq, AttnShape s, int vec, int S) {
     extern __shared__ __align__(16) float smem[];
     const int DH = s.DH, LD = attn_ld(DH), q4 = (DH + 3) / 4, TILE = AKT * LD;
     float* Ks = smem;
@@ -187,13 +238,17 @@ k_attn_bwd_dq_simt(const T* __restrict__ q, const T* __restrict__ k, const T* __
     float* Ps = Gs + TILE;
     const int b = blockIdx.z, h = blockIdx.y, g = h / (s.H / s.KV);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r0 = (gridDim.x - 1 - blockIdx.x) * ABLK, t0 = r0 + warp * AR;
+    const int part = blockIdx.x % S, r0 = (gridDim.x / S - 1 - blockIdx.x / S) * ABLK, t0 = r0 + warp * AR;
     const T* kbase = k + b * s.kb + g * s.kh;
     const T* vbase = v + b * s.kb + g * s.kh;
+    pdl_enter();
     attn_tile(Qs, q + b * s.qb + h * s.qh, s.qt, r0, s.T, DH, LD, vec);
     attn_tile(Gs, dO + b * s.qb + h * s.qh, s.qt, r0, s.T, DH, LD, vec);
-    attn_tile(Ks, kbase, s.kt, 0, s.T, DH, LD, vec);
-    attn_tile(Vs, vbase, s.kt, 0, s.T, DH, LD, vec);
+    const int ntiles = min(r0 + ABLK - 1, s.T - 1) / AKT + 1;
+    if (part < ntiles) {
+        attn_tile(Ks, kbase, s.kt, part * AKT, s.T, DH, LD, vec);
+        attn_tile(Vs, vbase, s.kt, part * AKT, s.T, DH, LD, vec);
+    }
     attn_commit();
     float L[AR], Dr[AR], acc[AR][NJ];
 #pragma unroll
@@ -207,14 +262,13 @@ k_attn_bwd_dq_simt(const T* __restrict__ q, const T* __restrict__ k, const T* __
     const float* myQ = Qs + warp * AR * LD;
     const float* myG = Gs + warp * AR * LD;
     float* myP = Ps + warp * AKT * AR;
-    const int ntiles = min(r0 + ABLK - 1, s.T - 1) / AKT + 1;
-    for (int kt = 0; kt < ntiles; kt++) {
+    for (int kt = part, cur = 0; kt < ntiles; kt += S, cur ^= 1) {
         attn_wait();
         __syncthreads();
-        const int cur = kt & 1, nxt = cur ^ 1;
-        if (kt + 1 < ntiles) {
-            attn_tile(Ks + nxt * TILE, kbase, s.kt, (kt + 1) * AKT, s.T, DH, LD, vec);
-            attn_tile(Vs + nxt * TILE, vbase, s.kt, (kt + 1) * AKT, s.T, DH, LD, vec);
+        const int nxt = cur ^ 1;
+        if (kt + S < ntiles) {
+            attn_tile(Ks + nxt * TILE, kbase, s.kt, (kt + S) * AKT, s.T, DH, LD, vec);
+            attn_tile(Vs + nxt * TILE, vbase, s.kt, (kt + S) * AKT, s.T, DH, LD, vec);
         }
         attn_commit();
         if (kt * AKT > t0 + AR - 1) continue;
@@ -229,6 +283,29 @@ k_attn_bwd_dq_simt(const T* __restrict__ q, const T* __restrict__ k, const T* __
         __syncwarp();
         attn_axpy<NJ>(acc, myP, Ks + cur * TILE, LD, DH, lane);
         __syncwarp();
+    }
+    if (S > 1) {
+        attn_wait();
+        __syncthreads();
+        float* acc_x = smem + threadIdx.x;
+#pragma unroll
+        for (int r = 0; r < AR; r++)
+#pragma unroll
+            for (int i = 0; i < NJ; i++) acc_x[(r * NJ + i) * ATH] = acc[r][i];
+        attn_cluster_sync();
+        for (int r = part * AR / S; r < (part + 1) * AR / S; r++) {
+            const int t = t0 + r;
+            if (t >= s.T) continue;
+            const long long roff = b * s.qb + h * s.qh + (long long)t * s.qt;
+#pragma unroll
+            for (int i = 0; i < NJ; i++) {
+                float a = 0.f;
+                for (int q = 0; q < S; q++) a += attn_peer(acc_x + (r * NJ + i) * ATH, q);
+                if (lane + 32 * i < DH) stf(dq, roff + lane + 32 * i, a);
+            }
+        }
+        attn_cluster_sync();             // peers have read
+        return;
     }
 #pragma unroll
     for (int r = 0; r < AR; r++) {
@@ -249,7 +326,7 @@ template <typename T, typename TO, int NJ>
 __global__ void __launch_bounds__(ATH)
 k_attn_bwd_dkv_simt(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
                     const T* __restrict__ dO, const float* __restrict__ lse, const float* __restrict__ Dv,
-                    TO* __restrict__ dk, TO* __restrict__ dv, AttnShape s, int vec) {
+                    TO* __restrict__ dk, TO* __restrict__ dv, AttnShape s, int vec, int S) {
     extern __shared__ __align__(16) float smem[];
     const int DH = s.DH, LD = attn_ld(DH), q4 = (DH + 3) / 4, TILE = AKT * LD;
     float* Qs = smem;                    // two tiles each
@@ -259,17 +336,18 @@ k_attn_bwd_dkv_simt(const T* __restrict__ q, const T* __restrict__ k, const T* _
     float* Ps = Vr + TILE;               // [warp][query][AR]
     const int b = blockIdx.z, g = blockIdx.y, rep = s.H / s.KV;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r0 = blockIdx.x * ABLK, j0 = r0 + warp * AR;       // the first key rows meet the most queries
+    const int part = blockIdx.x % S, r0 = blockIdx.x / S * ABLK, j0 = r0 + warp * AR;       // the first key rows meet the most queries
     const int qt0 = r0 / AKT, nq = (s.T + AKT - 1) / AKT - qt0, n_it = rep * nq;
+    pdl_enter();
     attn_tile(Kr, k + b * s.kb + g * s.kh, s.kt, r0, s.T, DH, LD, vec);
     attn_tile(Vr, v + b * s.kb + g * s.kh, s.kt, r0, s.T, DH, LD, vec);
-    auto load = [&](int it) {
+    auto load = [&](int it, int cur) {
         const long long hb = b * s.qb + (long long)(g * rep + it / nq) * s.qh;
         const int t = (qt0 + it % nq) * AKT;
-        attn_tile(Qs + (it & 1) * TILE, q + hb, s.qt, t, s.T, DH, LD, vec);
-        attn_tile(Gs + (it & 1) * TILE, dO + hb, s.qt, t, s.T, DH, LD, vec);
+        attn_tile(Qs + cur * TILE, q + hb, s.qt, t, s.T, DH, LD, vec);
+        attn_tile(Gs + cur * TILE, dO + hb, s.qt, t, s.T, DH, LD, vec);
     };
-    load(0);
+    if (part < n_it) load(part, 0);
     attn_commit();
     float ak[AR][NJ], av[AR][NJ];
 #pragma unroll
@@ -279,17 +357,17 @@ k_attn_bwd_dkv_simt(const T* __restrict__ q, const T* __restrict__ k, const T* _
     const float* myK = Kr + warp * AR * LD;
     const float* myV = Vr + warp * AR * LD;
     float* myP = Ps + warp * AKT * AR;
-    for (int it = 0; it < n_it; it++) {
+    for (int it = part, cur = 0; it < n_it; it += S, cur ^= 1) {
         const int h = g * rep + it / nq, t = (qt0 + it % nq) * AKT + lane;
         const bool live = t < s.T;
         const float L = live ? lse[((long long)b * s.H + h) * s.T + t] : 0.f;
         const float Dr = live ? Dv[b * s.db + h * s.dh_ + (long long)t * s.dtk] : 0.f;
         attn_wait();
         __syncthreads();
-        if (it + 1 < n_it) load(it + 1);
+        if (it + S < n_it) load(it + S, cur ^ 1);
         attn_commit();
-        const float* Qt = Qs + (it & 1) * TILE;
-        const float* Gt = Gs + (it & 1) * TILE;
+        const float* Qt = Qs + cur * TILE;
+        const float* Gt = Gs + cur * TILE;
         float sc[AR], dp[AR], p[AR], ds[AR];
         attn_dot(myK, Qt + lane * LD, LD, q4, sc);
         attn_dot(myV, Gt + lane * LD, LD, q4, dp);
@@ -306,6 +384,29 @@ k_attn_bwd_dkv_simt(const T* __restrict__ q, const T* __restrict__ k, const T* _
         __syncwarp();
         attn_axpy<NJ>(ak, myP, Qt, LD, DH, lane);
         __syncwarp();
+    }
+    if (S > 1) {                         // units: dK rows, then dV rows
+        attn_wait();
+        __syncthreads();
+        float* acc_x = smem + threadIdx.x;
+#pragma unroll
+        for (int r = 0; r < AR; r++)
+#pragma unroll
+            for (int i = 0; i < NJ; i++) { acc_x[(r * NJ + i) * ATH] = ak[r][i]; acc_x[((AR + r) * NJ + i) * ATH] = av[r][i]; }
+        attn_cluster_sync();
+        for (int u = part * 2 * AR / S; u < (part + 1) * 2 * AR / S; u++) {
+            const int j = j0 + u % AR;
+            if (j >= s.T) continue;
+            const long long koff = b * s.kb + g * s.kh + (long long)j * s.kt;
+#pragma unroll
+            for (int i = 0; i < NJ; i++) {
+                float a = 0.f;
+                for (int q = 0; q < S; q++) a += attn_peer(acc_x + (u * NJ + i) * ATH, q);
+                if (lane + 32 * i < DH) stf(u < AR ? dk : dv, koff + lane + 32 * i, a);
+            }
+        }
+        attn_cluster_sync();             // peers have read
+        return;
     }
 #pragma unroll
     for (int r = 0; r < AR; r++) {
@@ -334,13 +435,34 @@ static int attn_vec(int dt, const AttnShape& s, std::initializer_list<const void
     return ok;
 }
 
+// CTAs that share a block's walk of `chain` tiles: doubled up to four CTAs per SM and while each keeps half of `least` tiles.  fp32, forward / backward in us with 1 / 2 / 4 / (dK / dV) 8: B2 H8 KV4 T256 DH32 27, 21, 21 /
+// 87, 79, 59, 47; B2 H4 KV2 T200 DH64 33, 24, 19 / 111, 73, 55, 44; B1 H8 KV8 T512 DH64 65, 45, 37 / 229, 130, 101, 107; B4 H8 KV4 T128 DH32
+// 17, 15, 16 / 51, 49, 43, 36; B1 H4 KV1 T300 DH64 43, 28, 22 / 225, 126, 77, 56.
+static int attn_share(long long ctas, int chain, int most, int least) {
+    int S = 1;
+    while (S < most && ctas * S * 2 <= 4 * AX_SMS && chain >= least * S) S *= 2;
+    return S;
+}
+template <typename K, typename... A>
+static int attn_launch(K kern, dim3 grid, size_t smem, int S, cudaStream_t st, A... args) {
+    grid.x *= S;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = dim3(ATH); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = S; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at; cfg.numAttrs = ax_gemm_pdl() ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kern, args..., S) == cudaSuccess ? 0 : 3;
+}
+
 template <typename T, int NJ>
 static int attn_fwd_launch(const void* q, const void* k, const void* v, void* o, float* lse, const AttnShape& s, int vec, cudaStream_t st) {
     const size_t smem = attn_smem(s.DH, 5);
     if (!attn_smem_ok(smem, k_attn_fwd_simt<T, NJ>)) return 101;
     const dim3 grid((s.T + ABLK - 1) / ABLK, s.H, s.B);
-    k_attn_fwd_simt<T, NJ><<<grid, ATH, smem, st>>>((const T*)q, (const T*)k, (const T*)v, (T*)o, lse, s, vec);
-    return 0;
+    return attn_launch(k_attn_fwd_simt<T, NJ>, grid, smem, attn_share((long long)grid.x * grid.y * grid.z, grid.x, 4, 3), st, (const T*)q, (const T*)k, (const T*)v, (T*)o, lse, s, vec);
 }
 template <typename T>
 static int attn_fwd_nj(const void* q, const void* k, const void* v, void* o, float* lse, const AttnShape& s, int vec, cudaStream_t st) {
@@ -363,9 +485,10 @@ static int attn_bwd_launch(const void* q, const void* k, const void* v, const vo
     const size_t smem = attn_smem(s.DH, 6);
     if (!attn_smem_ok(smem, k_attn_bwd_dq_simt<T, TO, NJ>) || !attn_smem_ok(smem, k_attn_bwd_dkv_simt<T, TO, NJ>)) return 102;
     const dim3 g1((s.T + ABLK - 1) / ABLK, s.H, s.B), g2((s.T + ABLK - 1) / ABLK, s.KV, s.B);
-    k_attn_bwd_dq_simt<T, TO, NJ><<<g1, ATH, smem, st>>>((const T*)q, (const T*)k, (const T*)v, (const T*)dO, lse, Dv, (TO*)dq, s, vec);
-    k_attn_bwd_dkv_simt<T, TO, NJ><<<g2, ATH, smem, st>>>((const T*)q, (const T*)k, (const T*)v, (const T*)dO, lse, Dv, (TO*)dk, (TO*)dv, s, vec);
-    return 0;
+    const int rc = attn_launch(k_attn_bwd_dq_simt<T, TO, NJ>, g1, smem, attn_share((long long)g1.x * g1.y * g1.z, g1.x, 4, 3), st, (const T*)q, (const T*)k, (const T*)v,
+                               (const T*)dO, lse, Dv, (TO*)dq, s, vec);
+    return rc ? rc : attn_launch(k_attn_bwd_dkv_simt<T, TO, NJ>, g2, smem, attn_share((long long)g2.x * g2.y * g2.z, g2.x * (s.H / s.KV), 8, 2), st, (const T*)q, (const T*)k,
+                                 (const T*)v, (const T*)dO, lse, Dv, (TO*)dk, (TO*)dv, s, vec);
 }
 template <typename T, typename TO>
 static int attn_bwd_nj(const void* q, const void* k, const void* v, const void* dO, const float* lse,

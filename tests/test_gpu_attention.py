@@ -278,6 +278,32 @@ def test_attention_of_other_shapes_keeps_fp32_probabilities(eng, B, H, KV, T, DH
         assert err(runs[0][n]) <= 1.01 * err(general[n]), (n, err(runs[0][n]), err(general[n]))
 
 
+@pytest.mark.parametrize("B,H,KV,T,DH", [(2, 8, 4, 256, 32), (1, 2, 1, 225, 8), (1, 4, 2, 97, 40), (1, 3, 3, 130, 128), (1, 2, 1, 64, 256), (16, 8, 8, 65, 64)])
+def test_fp32_attention_over_clusters(eng, B, H, KV, T, DH):
+    """Few rows: clusters of two to eight CTAs share a block's tiles, some of them without one (the last case has none: it fills the
+    SMs).  Sums of T products of N(0,1) numbers in fp32 in any order err by less than 2^-24 sqrt(T) a term: 2e-5 of the largest
+    result, as for one CTA; a second run gives the same bits."""
+    rng = np.random.default_rng(T + DH)
+    q, k, v, do = make(rng, B, H, KV, T, DH, 0)
+    scale = 1.0 / np.sqrt(DH)
+    t = lambda x: np.ascontiguousarray(x.transpose(0, 2, 1, 3))
+    iq, ik, iv, ido = put(eng, t(q), 0), put(eng, t(k), 0), put(eng, t(v), 0), put(eng, t(do), 0)
+    out = {n: (eng.alloc(a.size), a.shape[1]) for n, a in (("o", q), ("dq", q), ("dk", k), ("dv", k))}
+    ilse, iD = eng.alloc(B * H * T), eng.alloc(B * H * T)
+    runs = []
+    for _ in range(2):
+        eng.run([op(E.ATTN_FWD, a=iq, b=ik, d=iv, c=out["o"][0], sa=ilse, m=T, n=DH, k=KV, batch=B, tb=H, dt=0, alpha=scale),
+                 op(E.ATTN_BWD, a=iq, b=ik, d=iv, c=ido, sa=ilse, sb=out["o"][0], tb=out["dq"][0], sc=out["dk"][0], oa=out["dv"][0],
+                    ob=H, oc=iD, m=T, n=DH, k=KV, batch=B, dt=0, alpha=scale)])
+        runs.append({n: eng.download(i, (B, T, heads, DH)).transpose(0, 2, 1, 3) for n, (i, heads) in out.items()})
+    lse = eng.download(ilse, (B, H, T))
+    for n, ref in attention_f64(q, k, v, do, scale).items():
+        assert np.array_equal(runs[0][n], runs[1][n]), n
+        assert np.abs(runs[0][n] - ref).max() <= 2e-5 * np.abs(ref).max(), n
+    assert np.abs(lse - O.attention_fwd(q, k, v, scale)[1]).max() <= 2e-5
+    assert eng.device_status() == 0
+
+
 @pytest.mark.parametrize("B,H,KV,T,DH,gain", [
     (40, 8, 4, 3, 64, 1), (20, 16, 8, 64, 48, 1), (20, 16, 8, 65, 64, 1),       # one tile: a piece of a step, one step, two
     (4, 12, 4, 129, 64, 1), (2, 16, 2, 500, 56, 1),                             # dK / dV over clusters of two and four, some CTAs with no step
