@@ -57,6 +57,7 @@ struct Engine {
 };
 static Engine G;
 int ax_variant = 0;
+int ax_gemm_parts = 0;
 
 static void set_err(const char* fmt, ...) {
     va_list ap; va_start(ap, fmt);
@@ -134,6 +135,7 @@ API int eng_set_fallback(int mask) {
 }
 API long long eng_bytes_allocated(void) { return G.bytes; }
 API int eng_last_variant(void) { return ax_variant; }
+API int eng_last_gemm_parts(void) { return ax_gemm_parts; }
 API int eng_sync(void) {
     int rc = (int)cudaStreamSynchronize(G.stream);
     if (!rc) rc = (int)cudaStreamSynchronize(G.comm_stream);

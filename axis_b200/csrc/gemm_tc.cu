@@ -246,6 +246,7 @@ int ax_gemm_tma_out(void) {
     static const int on = getenv("AXENG_NO_TMA_OUT") ? 0 : 1;
     return on;
 }
+bool ax_gemm_on_side(void) { return g_side != 0; }
 float* ax_splitk_ws(size_t* bytes) { if (bytes) *bytes = SPLITK_WS_BYTES; return g_splitk_ws; }
 void ax_gemm_set_mode(int mode) { g_pair_mode = mode; }
 int ax_gemm_mode(void) { return g_pair_mode; }
@@ -359,9 +360,12 @@ int ax_gemm_tc(int out_bf16, int tb, const void* A, const void* B, void* C, cons
             if (sk > 1) cost += (2.0 * sk + 1.0) * m * n * 4.0 / 4.0e12 / 0.45e-6 + 4.0;
             if (cost < best2 - 1e-9) { best2 = cost; best2_s = sk; }
         }
+        double shared;
+        if (!g_side && ax_gemm_tc2_share((int)tiles2, kblocks, &shared) > 1 && shared * 0.70 < best2) { best2 = shared * 0.70; best2_s = 1; }
         if (g_pair_mode == 2 || best2 < best) {
+            ax_variant = 0x22 + 0x100 * best2_s;
             const int rc = ax_gemm_tc2(out_bf16, tb, A, B, C, D, m, n, k, alpha, beta, status, best2_s, st);
-            if (rc >= 0) { ax_variant = 0x22 + 0x100 * best2_s; return rc; }
+            if (rc >= 0) return rc;
         }
     }
 #define GL(BN_, AM, BMj)                                                                                       \

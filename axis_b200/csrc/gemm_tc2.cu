@@ -106,19 +106,11 @@ __device__ __forceinline__ void tc_mma_ss2_e(uint32_t d_tmem, uint64_t adesc, ui
         "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
-__device__ __forceinline__ void tc_commit2_e(uint32_t bar) {
-    const uint16_t mask = 3;
+__device__ __forceinline__ void tc_commit2_e(uint32_t bar, uint16_t mask) {
     asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
                  "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
                  ::"r"(bar), "h"(mask) : "memory");
 }
-// arrive on the barrier at this shared-memory offset in both CTAs of the pair once all prior MMAs finish
-__device__ __forceinline__ void tc_commit2(uint32_t bar) {
-    const uint16_t mask = 3;
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-                 ::"r"(bar), "h"(mask) : "memory");
-}
-
 // Grouped launch: several GEMMs of one layer run as one persistent kernel.
 //   mode 1: `count` problems share A; problem g has its own B (n[g] columns) and its own C — their column
 //           tiles form one tile space (q/k/v or gate/up projections of the same input; their weight gradients).
@@ -139,8 +131,11 @@ __device__ __forceinline__ void tc_commit2(uint32_t bar) {
 // EPI_SWB (mode 2): the sum over the K-segments is the gradient dh of h = silu(g) * u and never reaches memory; the
 //           epilogue fetches g (tmD) and u (tmC2) and writes dg (tmC) and du (tmC1).
 // Grouped launches write through TMA stores and do not split K; only mode 2 takes an addend.
+// A launch of so few tiles that pairs would be left without one takes a cluster of S pairs to a tile (S 2 or 4): each sums its part of
+// the depth, then gives the others, through distributed shared memory, their columns of its accumulator, and finishes its own.
 struct GemmGroup {
     int mode, count;
+    int S;                   // pairs that share a tile's depth (1: a pair has tiles of its own)
     int n[3];
     int kb[6];
     int m[3];
@@ -197,14 +192,16 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     const uint32_t smem_base = smem_u32(smem);
     constexpr int NH = EpiCfg<EPI>::NH, EW = EpiCfg<EPI>::EW;
-    constexpr bool swiglu = EPI == EPI_SWIGLU, swb = EPI == EPI_SWB;
+    constexpr bool swiglu = EPI == EPI_SWIGLU, swb = EPI == EPI_SWB, CAN_SHARE = !swiglu && !swb;
     const bool wide_stg = swiglu || swb || tma_out == 2;           // 64 KB of staging instead of 32, five stages
     const int nst = wide_stg ? STAGES2 - 1 : STAGES2;              // operand stages in use
     const uint32_t bar_d = smem_u32(bars + 20);                    // [EW warps][16 / EW buffers] arrival barriers of fetched pieces
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t rank = cluster_rank();                 // 0 = leader (issues the MMAs)
-    const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
+    const uint32_t crank = cluster_rank(), rank = crank & 1, lead = crank & ~1u;     // rank 0 of a pair leads it (issues the MMAs)
+    const int S = grp.S, part = crank >> 1;                // this pair's part of the depth
+    const int pair = blockIdx.x / (2 * S), npairs = gridDim.x / (2 * S);
+    const uint16_t both = 3u << lead;                      // the pair's CTAs
     const int tiles_m = (m + 2 * BM2 - 1) / (2 * BM2);
     int tiles_n = (n + BN2 - 1) / BN2, kblocks_all = (k + BK2 - 1) / BK2;
     const int kb_main = kblocks_all;                       // mode 1: k-blocks of the shared segment
@@ -242,6 +239,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
         return q;
     };
     const int kb_per = (kblocks_all + ksplit - 1) / ksplit;
+    const int kb_from = S > 1 ? kblocks_all * part / S : 0, kb_to = S > 1 ? kblocks_all * (part + 1) / S : kblocks_all;
     const int num_units = num_tiles * ksplit;
 
     if (threadIdx.x == 0) {
@@ -263,8 +261,8 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
     cluster_sync_all();                                   // peer barriers are initialised before anyone signals them
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    const uint32_t full_leader = map_to_cta(bar_full, 0);  // cluster address of the leader's full[0]
-    const uint32_t tempty_leader = map_to_cta(bar_tempty, 0);
+    const uint32_t full_leader = map_to_cta(bar_full, lead);  // cluster address of the leader's full[0]
+    const uint32_t tempty_leader = map_to_cta(bar_tempty, lead);
     // programmatic dependent launch: see the single-CTA kernel
     if (timing && threadIdx.x == 0) prof[1] = clock64();
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -278,7 +276,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
         bool ok = true;
         for (int unit = pair; unit < num_units && ok; unit += npairs) {
             const int tile = unit % num_tiles, split = unit / num_tiles;
-            const int kb0 = split * kb_per, kb1 = min(kblocks_all, kb0 + kb_per);
+            const int kb0 = kb_from + split * kb_per, kb1 = min(kb_to, kb0 + kb_per);
             int tm, tl;
             const int g = locate(tile, tm, tl);
             const int row0 = tm * 2 * BM2 + rank * BM2, col0 = swiglu ? tl * 128 : tl * BN2 + rank * 128;
@@ -294,8 +292,8 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
                     while (seg + 1 < grp.count && kl >= grp.kb[seg]) { kl = 0; seg++; }
                     pA = seg == 0 ? &tmA : seg == 1 ? &tmA1 : seg == 2 ? &tmA2 : seg == 3 ? &tmEA0 : seg == 4 ? &tmEA1 : &tmEA2;
                     pB = seg == 0 ? &tmB : seg == 1 ? &tmB1 : seg == 2 ? &tmB2 : seg == 3 ? &tmEB0 : seg == 4 ? &tmEB1 : &tmEB2;
-                } else if (grp.mode == 1 && kb == kb_main) {         // the problem's own extra segment
-                    kl = 0;
+                } else if (grp.mode == 1 && kb >= kb_main) {         // the problem's own extra segment
+                    kl = kb - kb_main;
                     pA = g == 0 ? &tmEA0 : (g == 1 ? &tmEA1 : &tmEA2);
                     pB = g == 0 ? &tmEB0 : (g == 1 ? &tmEB1 : &tmEB2);
                 }
@@ -340,7 +338,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
         bool ok = true;
         for (int unit = pair; unit < num_units && ok; unit += npairs, tcount++) {
             const int split = unit / num_tiles;
-            const int kb0 = split * kb_per, kb1 = min(kblocks_all, kb0 + kb_per);
+            const int kb0 = kb_from + split * kb_per, kb1 = min(kb_to, kb0 + kb_per);
             const int acc = tcount & 1;
             const uint32_t aph = (tcount >> 1) & 1;
             if (tcount >= 2 && !mbar_wait(bar_tempty + 8 * acc, aph ^ 1)) { ok = false; break; }
@@ -356,9 +354,9 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
                 for (int kk = 0; kk < BK2 / 16; kk++)
                     tc_mma_ss2_e(d_tmem, ((uint64_t)dhi << 32) | (a_lo + kk * a_step), ((uint64_t)dhi << 32) | (b_lo + kk * b_step),
                                  idesc, (kb != kb0) || (kk != 0));
-                tc_commit2_e(bar_empty + 8 * s);       // frees the stage in both CTAs
+                tc_commit2_e(bar_empty + 8 * s, both);       // frees the stage in both CTAs
             }
-            if (ok) tc_commit2_e(bar_tfull + 8 * acc); // accumulator ready in both CTAs
+            if (ok) tc_commit2_e(bar_tfull + 8 * acc, both); // accumulator ready in both CTAs
             if (timing && lane == 0) prof[4] = clock64();
         }
         __syncwarp();
@@ -397,14 +395,15 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
             // pieces of this tile that this warp writes: half, half + NH, ...
             const int pw = swb ? 32 : cw;
             const int npt = (tma_out && !swiglu && row0 < m_g) ? (ncols + pw - 1) / pw : 0;
-            const int npc = (npt - half + NH - 1) / NH;
+            const int j0 = S > 1 ? part * (BN2 / cw / S) : 0;   // a shared tile: this part's 256 / S columns
+            const int npc = S > 1 ? max(0, min(npt - j0, BN2 / cw / S)) : (npt - half + NH - 1) / NH;
             const uint32_t pbase = pieces;
             const bool do_rope = EPI == EPI_ROPE && ((grp.rope_mask >> g) & 1);
             const int rope_t = do_rope ? (row < m_g ? row : 0) % grp.rope_T : 0;
             // lane 0: piece i of this warp of the addend, or of g and u, -> its buffer
             auto fetch_d = [&](int i) {
                 const uint32_t bi = (pbase + i) & (nbuf - 1);
-                const int x = tn * BN2 + (half + NH * i) * pw;
+                const int x = tn * BN2 + (j0 + half + NH * i) * pw;
                 mbar_expect_tx(my_bar_d + 8 * bi, 4096);
                 tma_load_3d(stg_u32 + bi * 4096, &tmD, my_bar_d + 8 * bi, x, row0, 0);
                 if (swb) tma_load_3d(stg_u32 + bi * 4096 + 2048, &tmC2, my_bar_d + 8 * bi, x, row0, 0);
@@ -423,10 +422,47 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
 #pragma unroll
                 for (int q = 0; q < 8; q++) { rc[q] = __ldg(cr + q); rs[q] = __ldg(sr + q); }
             }
-            if (!mbar_wait(bar_tfull + 8 * acc, aph) || *abort_flag) { ok = false; break; }
+            if (!mbar_wait(bar_tfull + 8 * acc, aph) || *abort_flag) ok = false;
             tc_fence_after();
             if (timing && threadIdx.x == 64) prof[5] = clock64();
             const uint32_t taddr = tmem_base + acc * BN2 + ((uint32_t)(quad * 32) << 16);
+            const int own = 8 / S;                              // 32-column chunks of a part
+            // sums of the other parts in this CTA's operand ring: [part][lane quarter][chunk][4 columns][row], 512 bytes in a row per warp
+            auto part_at = [&](int from, int c) { return ((from - (from > part)) * 4 + quad) * own * 4096 + c * 4096 + lane * 16; };
+            if (CAN_SHARE && S > 1) {                           // one tile per cluster: every warp comes by here once
+                cluster_sync_all();                             // no ring has a reader or a writer left
+                if (ok)
+                    for (int q = 1; q < S; q++) {
+                        const int to = (part + q) & (S - 1);
+                        const uint32_t dst = map_to_cta(smem_base + ((part - (part > to)) * 4 + quad) * own * 4096 + lane * 16, to * 2 + rank);
+#pragma unroll 1
+                        for (int c = 0; c < own; c++) {
+                            uint32_t r[32];
+                            tmem_ld32(taddr + (to * own + c) * 32, r);
+                            tmem_ld_wait();
+#pragma unroll
+                            for (int z = 0; z < 8; z++)
+                                asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + c * 4096 + z * 512), "r"(r[z * 4]), "r"(r[z * 4 + 1]),
+                                             "r"(r[z * 4 + 2]), "r"(r[z * 4 + 3]) : "memory");
+                        }
+                    }
+                cluster_sync_all();
+            }
+            if (!ok) break;
+            auto part_add = [&](int c, uint32_t* r) {            // chunk c of this part, the parts in order behind the own sum
+                if (!CAN_SHARE || S == 1) return;
+                for (int from = 0; from < S; from++) {
+                    if (from == part) continue;
+#pragma unroll
+                    for (int z = 0; z < 8; z++) {
+                        const float4 v = *reinterpret_cast<const float4*>(smem + part_at(from, c) + z * 512);
+                        r[z * 4] = __float_as_uint(__uint_as_float(r[z * 4]) + v.x);
+                        r[z * 4 + 1] = __float_as_uint(__uint_as_float(r[z * 4 + 1]) + v.y);
+                        r[z * 4 + 2] = __float_as_uint(__uint_as_float(r[z * 4 + 2]) + v.z);
+                        r[z * 4 + 3] = __float_as_uint(__uint_as_float(r[z * 4 + 3]) + v.w);
+                    }
+                }
+            };
             if constexpr (swiglu) {
                 // accumulator columns 0..127: gate, 128..255: up (same output columns tl*128 ..); per 64-column piece
                 // three staged outputs g, u, h, each stored by its own bulk group so that the buffers rotate freely.
@@ -530,7 +566,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
             } else if (tma_out) {
 #pragma unroll 1
                 for (int j = 0; j < npc && ok; j++) {
-                    const int c = j * cw;
+                    const int c = (j0 + j) * cw, cp = j * (cw / 32);     // first column; first chunk of the part
                     const uint32_t bi = pieces & (nbuf - 1);
                     uint8_t* buf = stg + bi * 4096 + lane * 128;
                     if (lane == 0) bulk_wait_read_le1();        // all but the latest store have read their buffers
@@ -543,6 +579,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
                     uint32_t r[32];
                     tmem_ld32(taddr + c, r);
                     tmem_ld_wait();
+                    part_add(cp, r);
                     if (f32_out) {
 #pragma unroll
                         for (int q = 0; q < 8; q++) {
@@ -560,6 +597,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
                         uint32_t r2[32];
                         tmem_ld32(taddr + c + 32, r2);
                         tmem_ld_wait();
+                        part_add(cp + 1, r2);
 #pragma unroll
                         for (int q = 0; q < 4; q++) {
                             const float4 c0 = rc[2 * q], c1 = rc[2 * q + 1], s0 = rs[2 * q], s1 = rs[2 * q + 1];
@@ -581,7 +619,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
                     } else {
 #pragma unroll
                         for (int half = 0; half < 2; half++) {
-                            if (half) { tmem_ld32(taddr + c + 32, r); tmem_ld_wait(); }
+                            if (half) { tmem_ld32(taddr + c + 32, r); tmem_ld_wait(); part_add(cp + 1, r); }
 #pragma unroll
                             for (int q = 0; q < 4; q++) {
                                 uint4* slot = reinterpret_cast<uint4*>(buf + (((half * 4 + q) ^ (lane & 7)) << 4));
@@ -636,6 +674,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
         if (tma_out && lane == 0) bulk_wait_read_all();       // staging stays valid until the last store has read it
         if (!ok && lane == 0) { *abort_flag = 1; atomicExch(status, STAT_GEMM2 | 3); }
     }
+    if (CAN_SHARE && S > 1 && warp < 2) { __syncwarp(); cluster_sync_all(); cluster_sync_all(); }      // the two of the epilogue
     tc_fence_before();
     __syncthreads();
     __syncwarp();
@@ -649,28 +688,31 @@ extern float* ax_splitk_ws(size_t* bytes);
 extern int ax_gemm_pdl(void);
 extern int ax_gemm_mode(void);
 extern int ax_gemm_tma_out(void);
+extern bool ax_gemm_on_side(void);
 template <typename TO>
 void ax_splitk_reduce_launch(const float* ws, int ksplit, TO* C, const TO* D, long long mn, float alpha, float beta, cudaStream_t st);
 
-template <int A_MN, int B_MN, typename TO, int EPI = EPI_PLAIN>
-static int pairs_for() {
-    static int g_pairs = 0;            // max co-resident pairs of this kernel (0 = unknown)
-    if (g_pairs == 0) {
+// co-resident clusters of S pairs of this kernel (0: none)
+template <int A_MN, int B_MN, typename TO, int EPI = EPI_PLAIN, int S = 1>
+static int clusters_for() {
+    static int g_max = -1;
+    if (g_max < 0) {
         cudaFuncSetAttribute(k_gemm_tc2<A_MN, B_MN, TO, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM2);
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(2 * AX_SMS, 1, 1);
+        cfg.gridDim = dim3(AX_SMS / (2 * S) * 2 * S, 1, 1);
         cfg.blockDim = dim3(EpiCfg<EPI>::THREADS, 1, 1);
         cfg.dynamicSmemBytes = SMEM2;
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+        at[0].val.clusterDim.x = 2 * S; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
         cfg.attrs = at; cfg.numAttrs = 1;
         int nc = 0;
-        if (cudaOccupancyMaxActiveClusters(&nc, k_gemm_tc2<A_MN, B_MN, TO, EPI>, &cfg) != cudaSuccess || nc < 1) { cudaGetLastError(); nc = -1; }
-        g_pairs = nc;
+        if (cudaOccupancyMaxActiveClusters(&nc, k_gemm_tc2<A_MN, B_MN, TO, EPI>, &cfg) != cudaSuccess || nc < 1) { cudaGetLastError(); nc = 0; }
+        g_max = nc;
     }
-    return g_pairs;
+    return g_max;
 }
+static int g_share_max[2] = {0, 0};      // the least of that over the kernels that share a tile, for 2 and 4 pairs
 
 // operand / output tensor maps of one problem
 template <int A_MN> static int map_a(CUtensorMap* t, const void* A, int m, int k) {
@@ -699,6 +741,22 @@ static int map_c(CUtensorMap* t, void* base, int m, int n, int nz, int osz, bool
                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? 0 : 2;
 }
 
+// Pairs to a tile (GemmGroup::S) for a launch of `tiles` tiles of kb k-blocks (0.3 us each); *cost: the launch in k-blocks.  33 clusters of
+// two pairs and 15 of four fit the GPU; two cluster barriers and the exchange of 64 or 96 KB per CTA cost what 8 and 12 k-blocks do.
+// us with 1 / 2 / 4 pairs, tiles x k-blocks: 24 x 88 37.6 / 25.9, 24 x 44 with addend 21.8 / 17.4, 24 x 32 18.3 / 15.6, 20 x 24 13.3 / 13.2,
+// 24 x 16 10.8 / 11.5 (there 16-deep products stay whole), 12 x 64 28.4 / 20.3 / 16.2, 12 x 32 17.8 / 14.2 / 13.1, 12 x 20 13.5 / 12.0 / 12.1, 12 x 12 9.5 / 9.8 / 10.8.
+int ax_gemm_tc2_share(int tiles, int kb, double* cost) {
+    int S = 1;
+    double best = kb;
+    for (int i = 0; i < 2; i++) {
+        const int q = 2 << i;
+        const double c = (double)((kb + q - 1) / q) + (i ? 12 : 8);
+        if (tiles <= g_share_max[i] && c < best) { S = q; best = c; }
+    }
+    if (cost) *cost = best;
+    return S;
+}
+
 struct SwbArgs { const void* g; const void* u; void* du; };    // SwiGLU backward in the epilogue (C = dg)
 
 // One launch.  grp.mode 0: the plain GEMM (A, B, C, D are element 0 of the arrays).  Grouped modes: see GemmGroup;
@@ -709,7 +767,7 @@ template <int A_MN, int B_MN, typename TO, int EPI = EPI_PLAIN>
 static int gemm2_launch(int mode, int count, const void* const* A, const void* const* B, void* const* C, const void* D,
                         const int* mv, const int* nv, const int* kv, float alpha, float beta, int* status, int ksplit, cudaStream_t st,
                         const void* const* XA = nullptr, const void* const* XB = nullptr, int xk = 0, const SwbArgs* swb = nullptr) {
-    const int maxp = pairs_for<A_MN, B_MN, TO, EPI>();
+    const int maxp = clusters_for<A_MN, B_MN, TO, EPI>();
     if (maxp < 1) return -1;
     const int m = mv[0], n = nv[0], k = kv[0];
     GemmGroup grp = {};
@@ -767,6 +825,15 @@ static int gemm2_launch(int mode, int count, const void* const* A, const void* c
     }
     const bool per_problem_c = mode == 1 || mode == 3;
     // output through TMA tile stores when the destination allows it: 1 = no addend to read, 2 = addend by TMA too
+    int units = ((m + 255) / 256) * tiles_n;
+    if (mode == 3) { units = 0; for (int g = 0; g < count; g++) units += ((mv[g] + 255) / 256) * ((nv[g] + 255) / 256); }
+    if (mode == 4) units = ((m + 255) / 256) * ((n + 127) / 128);
+    int kb = (k + BK2 - 1) / BK2 + grp.xkb;
+    if (mode == 2) { kb = 0; for (int g = 0; g < count; g++) kb += grp.kb[g]; }
+    // (not beside the main chain, whose kernels fill the SMs and where a cluster waits for four or eight free ones in one place: a step of
+    // 2 x 1536 tokens at D 1024 took 3522 us with the weight gradients shared, 3506 without)
+    grp.S = (EPI == EPI_PLAIN || EPI == EPI_ROPE) && ksplit == 1 && !ax_gemm_on_side() ? ax_gemm_tc2_share(units, kb, nullptr) : 1;
+    units *= ksplit;
     const int osz = ksplit > 1 ? 4 : (int)sizeof(TO);
     const bool has_d = D != nullptr && beta != 0.f && ksplit == 1;
     int tma_out = 0;
@@ -774,6 +841,7 @@ static int gemm2_launch(int mode, int count, const void* const* A, const void* c
     for (int g = 0; g < (per_problem_c ? count : (mode == 4 ? 3 : 1)); g++)
         c_ok = c_ok && ((uintptr_t)C[g] & 15) == 0 && ((long long)nv[per_problem_c ? g : 0] * osz) % 16 == 0;
     if (c_ok && (!has_d || ((uintptr_t)D & 15) == 0)) tma_out = has_d ? 2 : 1;
+    if (!tma_out) grp.S = 1;                 // (threads that store their rows write whole tiles)
     // grouped launches need the TMA-store epilogue; only the K-segment form takes an addend
     if (mode != 0 && (ksplit != 1 || !(tma_out == 1 || (tma_out == 2 && mode == 2)))) return -1;
     if (grp.rope_mask && tma_out != 1) return -1;
@@ -806,20 +874,18 @@ static int gemm2_launch(int mode, int count, const void* const* A, const void* c
         if (mode == 0 || g >= count) tmB[g] = tmB[0];
         if (mode != 4 && !swb && (!per_problem_c || g >= count || !tma_out)) tmC[g] = tmC[0];
     }
-    int units = ((m + 255) / 256) * tiles_n * ksplit;
-    if (mode == 3) { units = 0; for (int g = 0; g < count; g++) units += ((mv[g] + 255) / 256) * ((nv[g] + 255) / 256); }
-    if (mode == 4) units = ((m + 255) / 256) * ((n + 127) / 128);
     const int pairs = units < maxp ? units : maxp;
+    ax_gemm_parts = grp.S;
     size_t wsb = 0;
     float* ws = ax_splitk_ws(&wsb);
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * pairs, 1, 1);
+    cfg.gridDim = dim3(2 * pairs * grp.S, 1, 1);
     cfg.blockDim = dim3(EpiCfg<EPI>::THREADS, 1, 1);
     cfg.dynamicSmemBytes = SMEM2;
     cfg.stream = st;
     cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    at[0].val.clusterDim.x = 2 * grp.S; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
     at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at; cfg.numAttrs = ax_gemm_pdl() ? 2 : 1;
@@ -848,9 +914,17 @@ static int gemm2_launch(int mode, int count, const void* const* A, const void* c
 // Resolve the co-resident pair count of every variant up front (not while a graph is being captured).
 int ax_gemm_tc2_init(void) {
     int worst = 1 << 30;
-    int v[9] = {pairs_for<0, 1, bf16>(), pairs_for<0, 1, float>(), pairs_for<0, 0, bf16>(), pairs_for<0, 0, float>(),
-                pairs_for<1, 1, bf16>(), pairs_for<1, 1, float>(), pairs_for<0, 1, bf16, EPI_ROPE>(),
-                pairs_for<0, 1, bf16, EPI_SWIGLU>(), pairs_for<0, 0, bf16, EPI_SWB>()};
+#define ALL_KERNELS(S) clusters_for<0, 1, bf16, EPI_PLAIN, S>(), clusters_for<0, 1, float, EPI_PLAIN, S>(), clusters_for<0, 0, bf16, EPI_PLAIN, S>(),      \
+                       clusters_for<0, 0, float, EPI_PLAIN, S>(), clusters_for<1, 1, bf16, EPI_PLAIN, S>(), clusters_for<1, 1, float, EPI_PLAIN, S>(), \
+                       clusters_for<0, 1, bf16, EPI_ROPE, S>()
+    const int v[9] = {ALL_KERNELS(1), clusters_for<0, 1, bf16, EPI_SWIGLU>(), clusters_for<0, 0, bf16, EPI_SWB>()};
+    const int v2[7] = {ALL_KERNELS(2)}, v4[7] = {ALL_KERNELS(4)};
+#undef ALL_KERNELS
+    g_share_max[0] = g_share_max[1] = AX_SMS;
+    for (int i = 0; i < 7; i++) {
+        g_share_max[0] = v2[i] < g_share_max[0] ? v2[i] : g_share_max[0];
+        g_share_max[1] = v4[i] < g_share_max[1] ? v4[i] : g_share_max[1];
+    }
     for (int i = 0; i < 9; i++) worst = v[i] < worst ? v[i] : worst;
     return worst;      // pairs that can run together (<= 0: the paired kernel is unavailable)
 }

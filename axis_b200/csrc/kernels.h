@@ -15,6 +15,7 @@
 //   0x25 / 0x28 SwiGLU inside a projection pair with adapters on the same two,
 //   0x70 embedding scatter by scanning the ids, 0x71 by occurrence lists, 0x72 scale and add as one pass
 extern int ax_variant;
+extern int ax_gemm_parts;     // see eng_last_gemm_parts
 
 // elementwise.cu
 int ax_binary(int which, int dt, const void* a, const void* b, void* c, long long n, cudaStream_t st); // 0 add 1 mul 2 silu_mul
@@ -90,6 +91,7 @@ int ax_gemm_tc(int out_bf16, int tb, const void* A, const void* B, void* C, cons
 
 // gemm_tc2.cu — paired-CTA (cta_group::2) variant, 256 x 256 tile per two SMs
 int ax_gemm_tc2_init(void);
+int ax_gemm_tc2_share(int tiles, int kb, double* cost);
 int ax_gemm_tc2(int out_bf16, int tb, const void* A, const void* B, void* C, const void* D,
                 int m, int n, int k, float alpha, float beta, int* status, int ksplit, cudaStream_t st);
 void ax_gemm_set_mode(int mode);      // 0 auto, 1 single-CTA only, 2 paired whenever possible

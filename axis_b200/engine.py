@@ -359,6 +359,10 @@ class Engine:
         """Code of the kernel variant the last GEMM / cross-entropy op ran on (include/axeng.h)."""
         return int(self.lib.eng_last_variant())
 
+    def last_gemm_parts(self) -> int:
+        """Pairs of CTAs that shared a tile's depth in the last paired-CTA launch (include/axeng.h)."""
+        return int(self.lib.eng_last_gemm_parts())
+
     def bytes_allocated(self) -> int:
         return int(self.lib.eng_bytes_allocated())
 

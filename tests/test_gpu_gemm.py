@@ -849,3 +849,48 @@ def test_swiglu_of_gates_near_the_end_of_the_fp32_range(eng, mask):
         got = eng.download_bf16(o, (m, n))
         assert np.all(np.abs(got - ref) <= np.where(g < -89, 1e-36, (2.0 ** -8 + 2.0 ** -15) * np.abs(ref)))
     assert eng.device_status() == 0
+
+
+@pytest.mark.parametrize("tb", [0, 1, 2])
+@pytest.mark.parametrize("dt,addend", [(1, False), (1, True), (2, False)])
+@pytest.mark.parametrize("m,n,k,parts", [(1288, 776, 2064, 2), (1032, 1032, 1352, 2), (520, 776, 1352, 4), (520, 264, 2104, 4), (1544, 1024, 1408, 2)])
+def test_tile_depth_shared_over_a_cluster(eng, tb, dt, addend, m, n, k, parts):
+    """Few tiles: two or four pairs of CTAs share a tile's depth (uneven parts, ragged last rows, columns and depth; column parts that
+    do not exist).  The parts' sums meet in fp32 in a fixed order: the limits of one pair, and the same bits on every run."""
+    rng = np.random.default_rng(m + n + k + tb)
+    kw = dict(beta=-2.0, addend=True) if addend else dict(alpha=0.5)
+    got, ref = run_gemm(eng, rng, m, n, k, tb, dt, fallback=8, **kw)
+    assert eng.last_gemm_parts() == parts
+    check(got, ref, dt == 1, k)
+    again, _ = run_gemm(eng, np.random.default_rng(m + n + k + tb), m, n, k, tb, dt, fallback=8, **kw)
+    assert np.array_equal(got, again)
+    assert eng.device_status() == 0
+
+
+@pytest.mark.parametrize("m,k,ns,r,parts", [(1032, 1352, (512, 264, 136), 16, 2), (520, 1800, (264, 136, 72), 8, 4)])
+def test_grouped_tiles_shared_over_a_cluster(eng, m, k, ns, r, parts):
+    """The same for groups: one input and several outputs with a low-rank term each, and one output summed over K-segments."""
+    rng = np.random.default_rng(m + k)
+    mk = lambda *sh: bf(rng.standard_normal(sh).astype(np.float32))
+    A, Bs, XA, XB = mk(m, k), [mk(k, n) for n in ns], [mk(m, r) for _ in ns], [mk(r, n) for n in ns]
+    up = lambda a: put(eng, a, 1)
+    ic = [eng.alloc(m * n, 2) for n in ns]
+    ia, ib, xa, xb = up(A), [up(b) for b in Bs], [up(a) for a in XA], [up(b) for b in XB]
+    eng.set_fallback(8)
+    eng.run([op(E.GEMM_XSEG, a=xa[0], b=xa[1], d=xa[2], sa=xb[0], sb=xb[1], sc=xb[2], k=r, batch=3),
+             op(E.GEMM_GROUP, a=ia, b=ib[0], sa=ib[1], sb=ib[2], c=ic[0], d=ic[1], sc=ic[2], m=m, k=k, n=ns[0], oa=ns[1], ob=ns[2],
+                batch=3, oc=1, dt=1)])
+    assert eng.last_gemm_parts() == parts
+    for g, n in enumerate(ns):
+        check(eng.download_bf16(ic[g], (m, n)), A @ Bs[g] + XA[g] @ XB[g], True, k + r)
+    n, ks = 520, (k, 72, 200)
+    As, Bt, D = [A, mk(m, 72), mk(m, 200)], [mk(n, q) for q in ks], mk(m, n)
+    idd, c = up(D), eng.alloc(m * n, 2)
+    ia, ib = [up(a) for a in As], [up(b) for b in Bt]
+    eng.run([op(E.GEMM_XSEG, a=0, b=0, d=0, sa=0, sb=0, sc=0, k=0, batch=0, c=idd, beta=1.0),
+             op(E.GEMM_GROUP, c=c, a=ia[0], sa=ia[1], sb=ia[2], b=ib[0], d=ib[1], sc=ib[2], m=m, n=n, k=ks[0], oa=ks[1], ob=ks[2], batch=3,
+                oc=2, tb=1, dt=1)])
+    eng.set_fallback(0)
+    assert eng.last_gemm_parts() == 4
+    check(eng.download_bf16(c, (m, n)), sum(a @ b.T for a, b in zip(As, Bt)) + D, True, sum(ks))
+    assert eng.device_status() == 0
