@@ -746,30 +746,37 @@ class CompiledTransformer:
         # contributes: norm weight gradients, the embedding scatter), so the pass over the gradient arena that the clip
         # needs runs under the backward instead of between it and AdamW.  The inline plan takes the same per-bucket
         # sums on the main chain, so both plans add the same numbers in the same order.
-        def plan_with_bucket_norms():
+        # Gradient accumulation passes over the arena in the same way (step_accumulate).
+        def plan_with_bucket_ops(bucket_ops):
             merged, last, e = [], 0, ev[0]
             for b in range(nb):
                 cut = marks.get(b, last)
                 merged += plan[last:cut]
                 last = cut
-                st, ln = self._groups[0][b]
-                gn = op(GNORM_FLAT, a=self.a_grad, c=self.b_partials, d=self.b_sumsq, ob=b, m=ln // CHUNK,
-                        oa=st // CHUNK, tb=(self.b_t if b == 0 else 0))
                 if side_dw:
                     e += 2
-                    merged += [op(EVENT, tb=1, sa=0, oa=e - 1), op(EVENT, tb=2, sa=2, oa=e - 1), op(STREAM, tb=2), gn,
-                               op(EVENT, tb=1, sa=2, oa=e), op(STREAM, tb=0)]
+                    merged += [op(EVENT, tb=1, sa=0, oa=e - 1), op(EVENT, tb=2, sa=2, oa=e - 1), op(STREAM, tb=2)] + bucket_ops(b) + \
+                              [op(EVENT, tb=1, sa=2, oa=e), op(STREAM, tb=0)]
                 else:
-                    merged += [gn]
-            merged += plan[last:] + ([op(EVENT, tb=2, sa=0, oa=e)] if side_dw else [])
+                    merged += bucket_ops(b)
+            return merged + plan[last:] + ([op(EVENT, tb=2, sa=0, oa=e)] if side_dw else [])
+
+        def bucket_norm(b):
+            st, ln = self._groups[0][b]
+            return [op(GNORM_FLAT, a=self.a_grad, c=self.b_partials, d=self.b_sumsq, ob=b, m=ln // CHUNK,
+                       oa=st // CHUNK, tb=(self.b_t if b == 0 else 0))]
+
+        def update_of_bucket_norms():
             s0, sl = my_seg
-            return merged + [op(ADAMW_FLAT, a=self.a_master, b=self.a_grad, c=self.a_m, d=self.a_v,
-                                m=sl // CHUNK, k=s0 // CHUNK, sa=(self.a_mirror if hf else 0), sb=self.b_lr,
-                                tb=self.b_t, sc=self.b_wdflag, oa=self.b_sumsq, ob=nb, oc=self.b_gnorm,
-                                alpha=float(max_grad_norm or 0.0), beta=self.wd, gamma=adam_eps)]
+            return [op(ADAMW_FLAT, a=self.a_master, b=self.a_grad, c=self.a_m, d=self.a_v,
+                       m=sl // CHUNK, k=s0 // CHUNK, sa=(self.a_mirror if hf else 0), sb=self.b_lr,
+                       tb=self.b_t, sc=self.b_wdflag, oa=self.b_sumsq, ob=nb, oc=self.b_gnorm,
+                       alpha=float(self.max_grad_norm or 0.0), beta=self.wd, gamma=adam_eps)]
+        self._plan_with_bucket_ops, self._bucket_norm, self._update_of_bucket_norms = plan_with_bucket_ops, bucket_norm, update_of_bucket_norms
+        self._n_buckets = nb
         self.bucket_norms = bool(cw == 1 and not zero and nb <= 64 and all(self._groups[0][b][1] > 0 for b in range(nb)))
         if self.bucket_norms:
-            self.plan_step = plan_with_bucket_norms()
+            self.plan_step = plan_with_bucket_ops(bucket_norm) + update_of_bucket_norms()
         else:
             self.plan_step = gather_ops() + self._plan_fb_sync + opt_ops(max_grad_norm)
         self._plan_noclip = None
@@ -866,11 +873,21 @@ class CompiledTransformer:
             self.a_gacc = self.eng.alloc_zero(self._P_total * 4)
             lim = 1 << 30                     # element counts of flat ops stay inside int32
 
-            def flat(kind, **kw):
+            seen = {}
+
+            def window(buf, o, ln):
+                if ln == self._P_total:
+                    return buf
+                if (buf, o, ln) not in seen:
+                    seen[(buf, o, ln)] = self.eng.view(buf, o * 4, ln * 4)
+                return seen[(buf, o, ln)]
+
+            def flat(kind, start=0, count=None, **kw):
                 out = []
-                for o in range(0, self._P_total, lim):
-                    ln = min(lim, self._P_total - o)
-                    v = {k_: (self.eng.view(b_, o * 4, ln * 4) if o or ln < self._P_total else b_) for k_, b_ in kw["bufs"].items()}
+                end = start + (self._P_total if count is None else count)
+                for o in range(start, end, lim):
+                    ln = min(lim, end - o)
+                    v = {k_: window(b_, o, ln) for k_, b_ in kw["bufs"].items()}
                     out.append(op(kind, n=ln, dt=0, alpha=kw.get("alpha", 0.0), oa=kw.get("oa", 0), **v))
                 return out
             self._acc_flat = flat
@@ -880,17 +897,30 @@ class CompiledTransformer:
             # and the add behind a later micro-batch are one pass over memory in the library (oa = 1: nobody else reads
             # the scaled gradients)
             inv = 1.0 / n
-            first = self._gather_ops() + self.plan_fb
-            if n > 1:
-                first = first + self._acc_flat(SCALE, bufs=dict(a=self.a_grad, c=self.a_gacc), alpha=inv)
 
-            def add_to(dst):
-                sc = self._acc_flat(SCALE, bufs=dict(a=self.a_grad, c=self.a_grad), alpha=inv, oa=1)
-                ad = self._acc_flat(ADD, bufs=dict(a=self.a_gacc, b=self.a_grad, c=dst))
+            def keep(*seg):
+                return self._acc_flat(SCALE, *seg, bufs=dict(a=self.a_grad, c=self.a_gacc), alpha=inv) if n > 1 else []
+
+            def add_to(dst, *seg):
+                sc = self._acc_flat(SCALE, *seg, bufs=dict(a=self.a_grad, c=self.a_grad), alpha=inv, oa=1)
+                ad = self._acc_flat(ADD, *seg, bufs=dict(a=self.a_gacc, b=self.a_grad, c=dst))
                 return [o for pair in zip(sc, ad) for o in pair]
-            nxt = self.plan_fb + add_to(self.a_gacc)
-            last = self.plan_fb + add_to(self.a_grad)
-            self._acc_plans[n] = (first, nxt, last, self.plan_ar + self._opt_ops(self.max_grad_norm))
+            if self.bucket_norms:
+                # one GPU: a bucket's pass runs as soon as its gradients are complete, beside the backward where the weight gradients are, and
+                # the last one's is followed by the bucket's norm
+                seg = lambda b: self._groups[0][b]
+                tail = lambda b: add_to(self.a_grad, *seg(b)) if n > 1 else []
+                first = self._plan_with_bucket_ops(lambda b: keep(*seg(b)))
+                nxt = self._plan_with_bucket_ops(lambda b: add_to(self.a_gacc, *seg(b)))
+                last = self._plan_with_bucket_ops(lambda b: tail(b) + self._bucket_norm(b))
+                opt = self._update_of_bucket_norms()
+            else:
+                first = self._gather_ops() + self.plan_fb + keep()
+                nxt, last = self.plan_fb + add_to(self.a_gacc), self.plan_fb + add_to(self.a_grad)
+                opt = self.plan_ar + self._opt_ops(self.max_grad_norm)
+            if n == 1:
+                first = last if self.bucket_norms else first
+            self._acc_plans[n] = (first, nxt, last, opt)
         first, nxt, last, opt = self._acc_plans[n]
         # the host queues the micro-batches without waiting for their losses, which come back through the read-back ring; the last
         # one is read behind the update, which does not touch it, so that the call returns when the step is done

@@ -27,9 +27,9 @@
 #define XT 128                 // queries / keys per tile
 #define XD 64                  // columns of a tile (narrower heads are zero-filled)
 #define XQ 64                  // keys (dQ) or queries (dK / dV) per step
-#define STAT_XFWD 0x500
-#define STAT_XDQ 0x600
-#define STAT_XDKV 0x700
+#define STAT_XFWD 0x900
+#define STAT_XDQ 0xa00
+#define STAT_XDKV 0xb00
 
 // two numbers each as the sum of two bf16 ones
 __device__ __forceinline__ void split_bf16(float x, float y, uint32_t& hi, uint32_t& lo) {

@@ -518,3 +518,33 @@ def test_cross_entropy_zeroes_the_pad_columns_in_every_form(eng, dt, V, ld, off)
     if ld % (8 if dt else 4) or off:
         assert np.array_equal(got[:, end:], logits[:, end:])
     assert abs(eng.download(iloss, 1)[0] - loss) <= 1e-5 * abs(loss)
+
+
+@pytest.mark.parametrize("V,ld,N", [(2048, 2048, 900), (8200, 8208, 700), (32001, 32008, 450), (50000, 50000, 301)])
+def test_cross_entropy_rows_that_travel_ahead(eng, V, ld, N):
+    """More rows than blocks, so that every block fetches ahead of itself, with rows without a loss in between, in runs and at both ends.
+    An entry is within its rounding to bf16 (2^-8) and, where exponentials are kept as fp16, within 2^-11 of it and 2^-24 of the
+    row's largest."""
+    rng = np.random.default_rng(V + N)
+    logits = rnd(rng, (N, ld), 1)
+    tgt = rng.integers(0, V, N)
+    tgt[rng.random(N) < 0.3] = -1
+    tgt[:3] = tgt[200:280] = tgt[-2:] = -1
+    il, itg, iloss, iden, iscr = put(eng, logits, 1), eng.alloc(N), eng.alloc(1), eng.alloc(1), eng.alloc(N + 8)
+    eng.upload_tokens(itg, tgt, V)
+    eng.run([op(E.CE_FUSED, a=il, b=itg, c=il, d=iloss, sa=iden, sb=iscr, m=N, n=V, k=ld, dt=1)])
+    assert eng.last_variant() == 0x11
+    got = get(eng, il, (N, ld), 1)
+    live = tgt >= 0
+    assert not got[~live][:, :V].any()
+    z = logits[live][:, :V].astype(np.float64)
+    p = np.exp(z - z.max(-1, keepdims=True))
+    p /= p.sum(-1, keepdims=True)
+    cnt = int(live.sum())
+    loss = float(np.mean(-np.log(p[np.arange(cnt), tgt[live]])))
+    g = p.copy()
+    g[np.arange(cnt), tgt[live]] -= 1.0
+    err = np.abs(got[live][:, :V].astype(np.float64) * cnt - g)
+    assert (err <= np.abs(g) * 1.05 * 2.0 ** -8 + p * 2.0 ** -11 + p.max(-1, keepdims=True) * 2.0 ** -24).all()
+    assert abs(eng.download(iloss, 1)[0] - loss) <= 1e-5 * abs(loss)
+    assert eng.device_status() == 0
