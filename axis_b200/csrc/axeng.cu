@@ -1045,7 +1045,8 @@ static int exec_op(const EngOp* op) {
 //   oa = 1) dg and du leave the product's epilogue and dh is not written.  Waits of the main stream may stand between
 //   the two (they guard dg and du); they are queued first.
 //   GEMM_GROUP mode 1 of two outputs with a low-rank term each, then SILU_MUL of the two: the group runs as mode 4.
-//   SCALE of g in place (oa = 1: only the next op reads the result), then ADD of it: c = a + alpha * g in one pass.
+//   SCALE of g in place (oa = 1: only the next op reads the result), then ADD of it: c = a + alpha * g in one pass; GNORM_FLAT of c behind them
+//   joins it.
 // The products are served by the paired-CTA kernel from 256 rows and columns (one tile) on: below, and in every form that it refuses, the ops
 // run one by one.  Returns 0 (done up to *last), -1 (nothing done) or an error.
 static int run_fused(const EngOp* ops, int n_ops, int i, int* last) {
@@ -1058,6 +1059,15 @@ static int run_fused(const EngOp* ops, int n_ops, int i, int* last) {
         const char* g = (const char*)BUFP(op->a); const char* x = (const char*)BUFP(s->a); const char* c = (const char*)BUFP(s->c);
         if (BUFP(op->c) != g || BUFP(s->b) != g || !(x + b <= g || g + b <= x) || !(c == g || c == x || ((c + b <= g || g + b <= c) && (c + b <= x || x + b <= c))))
             return -1;
+        // and GNORM_FLAT of just that range behind them: in the same pass
+        const EngOp* q = i + 2 < n_ops ? &ops[i + 2] : nullptr;
+        const long long off = q ? (long long)q->oa * AX_ADAMW_CHUNK : 0, np = (n + AX_GNORM_CHUNK - 1) / AX_GNORM_CHUNK;
+        if (q && q->kind == ENG_GNORM_FLAT && q->oa >= 0 && q->ob >= 0 && (long long)q->m * AX_ADAMW_CHUNK == n && have(q->a, (off + n) * 4) && have(q->c, np * 4) &&
+            have(q->d, ((long long)q->ob + 1) * 4) && (q->tb <= 0 || have(q->tb, 4)) && (const char*)BUFP(q->a) + off * 4 == c) {
+            const int rc = ax_add_scaled_norm((const float*)x, (const float*)g, (float*)BUFP(s->c), op->alpha, (float*)BUFP(q->c), n,
+                                              q->tb > 0 ? (float*)BUFP(q->tb) : nullptr, (float*)BUFP(q->d) + q->ob, G.cur);
+            if (rc >= 0) { G.launches += 2; ax_variant = 0x73; *last = i + 2; return rc; }
+        }
         G.launches++;
         ax_variant = 0x72;
         *last = i + 1;

@@ -73,6 +73,8 @@ int ax_tick(float* t, cudaStream_t st);
 // partials[i] = sum of squares of chunk i (fixed in-chunk order); tick (may be null) += 1;
 // out (may be null) = sum of the partials in a fixed order.
 int ax_gnorm_flat(const float* g, float* partials, long long n, float* tick, float* out, cudaStream_t st);
+// c = a + alpha * b and the norm of c as ax_gnorm_flat leaves it, in one pass; -1 when not served (unaligned).
+int ax_add_scaled_norm(const float* a, const float* b, float* c, float alpha, float* partials, long long n, float* tick, float* out, cudaStream_t st);
 // One pass: scale = clip(sum(partials[0..np)) ), AdamW on n elements; wdflag[i] per AX_ADAMW_CHUNK.
 int ax_adamw_flat(float* p, const float* g, float* m, float* v, void* pbf, const unsigned char* wdflag,
                   const float* tbuf, const float* lrbuf, const float* partials, int np, float* gnorm_out,

@@ -153,6 +153,46 @@ int ax_gnorm_flat(const float* g, float* partials, long long n, float* tick, flo
     return 0;
 }
 
+// c = a + alpha * b (product and sum rounded one after the other) and the norm of c in the same pass: the last micro-batch of an
+// accumulation, 12 bytes an element instead of 16; the chunks' sums are those of k_gnorm_flat, bit for bit.  c may be a or b.
+__global__ void k_add_scaled_norm(const float* a, const float* b, float* c, float alpha, float* __restrict__ partials, long long n, float* tick) {
+    __shared__ float sh[40];
+    const long long nchunks = (n + AX_GNORM_CHUNK - 1) / AX_GNORM_CHUNK;
+    if (tick && blockIdx.x == 0 && threadIdx.x == 0) tick[0] += 1.f;
+    for (long long ch = blockIdx.x; ch < nchunks; ch += gridDim.x) {
+        const long long base = ch * AX_GNORM_CHUNK;
+        float s = 0.f;
+#pragma unroll
+        for (int it = 0; it < AX_GNORM_CHUNK / (256 * 4); it++) {
+            const long long i = base + (long long)(it * 256 + threadIdx.x) * 4;
+            if (i + 3 < n) {
+                const float4 x = *reinterpret_cast<const float4*>(a + i), y = *reinterpret_cast<const float4*>(b + i);
+                const float4 z = make_float4(__fadd_rn(x.x, __fmul_rn(alpha, y.x)), __fadd_rn(x.y, __fmul_rn(alpha, y.y)),
+                                             __fadd_rn(x.z, __fmul_rn(alpha, y.z)), __fadd_rn(x.w, __fmul_rn(alpha, y.w)));
+                *reinterpret_cast<float4*>(c + i) = z;
+                s += z.x * z.x; s += z.y * z.y; s += z.z * z.z; s += z.w * z.w;
+            } else {
+                for (long long j = i; j < n && j < i + 4; j++) {
+                    const float z = __fadd_rn(a[j], __fmul_rn(alpha, b[j]));
+                    c[j] = z;
+                    s += z * z;
+                }
+            }
+        }
+        s = block_sum(s, sh);
+        if (threadIdx.x == 0) partials[ch] = s;
+        __syncthreads();
+    }
+}
+int ax_add_scaled_norm(const float* a, const float* b, float* c, float alpha, float* partials, long long n, float* tick, float* out, cudaStream_t st) {
+    if (n <= 0 || !aligned16(a) || !aligned16(b) || !aligned16(c)) return -1;
+    const long long nchunks = (n + AX_GNORM_CHUNK - 1) / AX_GNORM_CHUNK;
+    const int grid = (int)(nchunks < AX_SMS * 8 ? nchunks : AX_SMS * 8);
+    k_add_scaled_norm<<<grid, 256, 0, st>>>(a, b, c, alpha, partials, n, tick);
+    k_sum_partials<<<1, 1024, 0, st>>>(partials, nchunks, out);
+    return 0;
+}
+
 // Every block first adds the np partials in index order (same value in every
 // block), derives the clip factor, then updates its slice.  wdflag has one
 // byte per AX_ADAMW_CHUNK elements: 1 = apply weight decay (tensors with two

@@ -548,3 +548,27 @@ def test_cross_entropy_rows_that_travel_ahead(eng, V, ld, N):
     assert (err <= np.abs(g) * 1.05 * 2.0 ** -8 + p * 2.0 ** -11 + p.max(-1, keepdims=True) * 2.0 ** -24).all()
     assert abs(eng.download(iloss, 1)[0] - loss) <= 1e-5 * abs(loss)
     assert eng.device_status() == 0
+
+
+@pytest.mark.parametrize("n,into", [(1024, "a"), (8192 * 3, "b"), (8192 * 5 + 3072, "other")])
+def test_scale_add_and_norm_in_one_pass(eng, n, into):
+    """SCALE in place with oa = 1, ADD of the result and GNORM_FLAT of the sum (one chunk, whole ones, a part of one) leave the bits of the
+    three ops run alone, and tick the step counter once; a norm of another range stays an op of its own."""
+    rng = np.random.default_rng(n)
+    a, g = rng.standard_normal(n).astype(np.float32), rng.standard_normal(n).astype(np.float32)
+    res = []
+    for hint, m, want in ((1, n // 1024, 2), (0, n // 1024, 4), (1, n // 1024 - 1, 3)):
+        if m < 1:
+            continue
+        ia, ig, tick = put(eng, a), put(eng, g), put(eng, np.zeros(1, np.float32))
+        c = {"a": ia, "b": ig, "other": eng.alloc(n)}[into]
+        parts, out = eng.alloc(n // 8192 + 1), put(eng, np.zeros(3, np.float32))
+        eng.launch_count(reset=True)
+        eng.run([op(E.SCALE, a=ig, c=ig, n=n, alpha=1.0 / 3.0, oa=hint), op(E.ADD, a=ia, b=ig, c=c, n=n),
+                 op(E.GNORM_FLAT, a=c, c=parts, d=out, ob=1, m=m, oa=0, tb=tick)])
+        assert eng.launch_count() == want
+        got = eng.download(out, (3,))
+        assert got[0] == got[2] == 0 and eng.download(tick, (1,))[0] == 1
+        res.append((eng.download(c, (n,)), got[1] if m == n // 1024 else None))
+    assert all(np.array_equal(res[0][0], r[0]) for r in res[1:]) and res[0][1] == res[1][1]
+    assert abs(res[0][1] - float((res[0][0].astype(np.float64) ** 2).sum())) <= 1e-5 * res[0][1]
