@@ -15,7 +15,7 @@
 // half empty for heads up to 32.  Bound by issue and by MMA latency: the MMA pipe (555 TFLOP/s by itself) is busy 44 / 56 / 50 % of the active cycles in
 // the forward, dQ and dK / dV kernels (B3 H24 KV8 T1000 DH64), and the schedulers issue in half of all cycles (exponentials, splits,
 // operand reads).  Times in us, forward / backward with the row dots,
-// CUDA cores -> here (for comparison: tcgen05 with 8-bit P and dS):
+// CUDA cores -> here (for comparison: tcgen05 with 8-bit P and dS; the first two and their like now run on attn_tcs.cu):
 //   B3 H24 KV8 T1000 DH64    628 / 2080 ->  70 / 203   (31 / 77)      B4 H24 KV8 T500 DH64   247 / 790 ->  33 / 102   (21 / 51)
 //   B2 H16 KV16 T1500 DH128 1439 / 3580 -> 122 / 347   (39 / 118)     B2 H8 KV4 T256 DH32    31.6 / 95 -> 11.2 / 22   (10.4 / 28)
 #include "common.cuh"
