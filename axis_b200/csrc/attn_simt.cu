@@ -421,8 +421,16 @@ k_attn_bwd_dkv_simt(const T* __restrict__ q, const T* __restrict__ k, const T* _
     }
 }
 
-// dynamic shared memory of a kernel that keeps `tiles` tiles and the warps' exchange area
-static size_t attn_smem(int DH, int tiles) { return ((size_t)tiles * AKT * attn_ld(DH) + AW * AKT * AR) * 4; }
+// Dynamic shared memory in bytes: the tiles and the warps' exchange area, or, where that is more (dK / dV of head dims up to 4), what
+// the merge of a cluster puts in their place.
+enum { ATTN_FWD, ATTN_DQ, ATTN_DKV };
+static size_t attn_smem(int which, int DH) {
+    const int nj = DH <= 32 ? 1 : DH <= 64 ? 2 : DH <= 128 ? 4 : 8;                          // columns of a row per lane
+    const size_t walk = (size_t)(which == ATTN_FWD ? 5 : 6) * AKT * attn_ld(DH) + AW * AKT * AR;
+    const size_t merge = (size_t)(which == ATTN_DKV ? 2 : 1) * AR * nj * ATH + (which == ATTN_FWD ? AW * AR * 2 : 0);
+    return (walk > merge ? walk : merge) * 4;
+}
+long long ax_attn_simt_smem(int which, int DH) { return (long long)attn_smem(which, DH); }
 template <typename K> static bool attn_smem_ok(size_t bytes, K kern) {
     if (bytes > 227 * 1024) return false;
     return bytes <= 48 * 1024 || cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
@@ -459,7 +467,7 @@ static int attn_launch(K kern, dim3 grid, size_t smem, int S, cudaStream_t st, A
 
 template <typename T, int NJ>
 static int attn_fwd_launch(const void* q, const void* k, const void* v, void* o, float* lse, const AttnShape& s, int vec, cudaStream_t st) {
-    const size_t smem = attn_smem(s.DH, 5);
+    const size_t smem = attn_smem(ATTN_FWD, s.DH);
     if (!attn_smem_ok(smem, k_attn_fwd_simt<T, NJ>)) return 101;
     const dim3 grid((s.T + ABLK - 1) / ABLK, s.H, s.B);
     return attn_launch(k_attn_fwd_simt<T, NJ>, grid, smem, attn_share((long long)grid.x * grid.y * grid.z, grid.x, 4, 3), st, (const T*)q, (const T*)k, (const T*)v, (T*)o, lse, s, vec);
@@ -482,12 +490,12 @@ int ax_attn_fwd_simt(int dt, const void* q, const void* k, const void* v, void* 
 template <typename T, typename TO, int NJ>
 static int attn_bwd_launch(const void* q, const void* k, const void* v, const void* dO, const float* lse,
                            const float* Dv, void* dq, void* dk, void* dv, const AttnShape& s, int vec, cudaStream_t st) {
-    const size_t smem = attn_smem(s.DH, 6);
-    if (!attn_smem_ok(smem, k_attn_bwd_dq_simt<T, TO, NJ>) || !attn_smem_ok(smem, k_attn_bwd_dkv_simt<T, TO, NJ>)) return 102;
+    const size_t smem_q = attn_smem(ATTN_DQ, s.DH), smem_kv = attn_smem(ATTN_DKV, s.DH);
+    if (!attn_smem_ok(smem_q, k_attn_bwd_dq_simt<T, TO, NJ>) || !attn_smem_ok(smem_kv, k_attn_bwd_dkv_simt<T, TO, NJ>)) return 102;
     const dim3 g1((s.T + ABLK - 1) / ABLK, s.H, s.B), g2((s.T + ABLK - 1) / ABLK, s.KV, s.B);
-    const int rc = attn_launch(k_attn_bwd_dq_simt<T, TO, NJ>, g1, smem, attn_share((long long)g1.x * g1.y * g1.z, g1.x, 4, 3), st, (const T*)q, (const T*)k, (const T*)v,
+    const int rc = attn_launch(k_attn_bwd_dq_simt<T, TO, NJ>, g1, smem_q, attn_share((long long)g1.x * g1.y * g1.z, g1.x, 4, 3), st, (const T*)q, (const T*)k, (const T*)v,
                                (const T*)dO, lse, Dv, (TO*)dq, s, vec);
-    return rc ? rc : attn_launch(k_attn_bwd_dkv_simt<T, TO, NJ>, g2, smem, attn_share((long long)g2.x * g2.y * g2.z, g2.x * (s.H / s.KV), 8, 2), st, (const T*)q, (const T*)k,
+    return rc ? rc : attn_launch(k_attn_bwd_dkv_simt<T, TO, NJ>, g2, smem_kv, attn_share((long long)g2.x * g2.y * g2.z, g2.x * (s.H / s.KV), 8, 2), st, (const T*)q, (const T*)k,
                                  (const T*)v, (const T*)dO, lse, Dv, (TO*)dk, (TO*)dv, s, vec);
 }
 template <typename T, typename TO>

@@ -136,6 +136,7 @@ API int eng_set_fallback(int mask) {
 API long long eng_bytes_allocated(void) { return G.bytes; }
 API int eng_last_variant(void) { return ax_variant; }
 API int eng_last_gemm_parts(void) { return ax_gemm_parts; }
+API long long eng_attn_smem(int which, int head_dim) { return which < 0 || which > 2 || head_dim < 1 || head_dim > 256 ? -1 : ax_attn_simt_smem(which, head_dim); }
 API int eng_sync(void) {
     int rc = (int)cudaStreamSynchronize(G.stream);
     if (!rc) rc = (int)cudaStreamSynchronize(G.comm_stream);

@@ -113,6 +113,7 @@ int ax_attn_fwd_simt(int dt, const void* q, const void* k, const void* v, void* 
 int ax_attn_bwd_simt(int dt, int out_dt, const void* q, const void* k, const void* v, const void* dO,
                      const float* lse, const float* Dv, void* dq, void* dk, void* dv,
                      const AttnShape& s, cudaStream_t st);
+long long ax_attn_simt_smem(int which, int DH);      // see eng_attn_smem
 
 // gemm_tc2.cu — grouped launch of the paired-CTA GEMM (mode 1: shared A, per-problem B/C/n; mode 2: one C summed
 // over per-segment A/B/k; mode 3: independent problems A/B/C/m/n of one depth k).  -1 when not served.

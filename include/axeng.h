@@ -169,6 +169,9 @@ long long eng_bytes_allocated(void);
 int eng_last_variant(void);
 /* Pairs of CTAs that shared the depth of a tile in the last paired-CTA tcgen05 launch: 1, 2 or 4. */
 int eng_last_gemm_parts(void);
+/* Dynamic shared memory in bytes of the general attention kernels, 0 forward, 1 dQ, 2 dK / dV, for a head dim of 1 to 256
+ * (else -1): host arithmetic that needs no GPU. */
+long long eng_attn_smem(int which, int head_dim);
 
 /* Fused RMSNorm backward that allocates nothing (no counterpart in the
  * reference).  dx = (res ? res : 0) + d(rmsnorm)/dx, dw = sum over rows of

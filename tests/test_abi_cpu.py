@@ -69,3 +69,16 @@ def test_no_device_means_loud_failure(lib):
     assert b"CUDA" in lib.eng_last_error()
     with pytest.raises(RuntimeError, match="engine init failed"):
         E.Engine()
+
+
+def test_general_attention_allocates_what_its_cluster_merge_writes(lib):
+    """A merge of attn_simt.cu lays out 4 rows x 32-column pieces x 256 threads of fp32 sums in a CTA's dynamic shared memory, and the
+    forward a maximum and a sum for each of its 32 rows behind them, dK / dV two such arrays; the launch allocates no less."""
+    f = lib.eng_attn_smem
+    f.restype = ctypes.c_longlong
+    for dh in range(1, 257):
+        pieces = 1 if dh <= 32 else 2 if dh <= 64 else 4 if dh <= 128 else 8
+        sums = 4 * pieces * 256 * 4
+        for which, need in ((0, sums + 32 * 2 * 4), (1, sums), (2, 2 * sums)):
+            assert need <= f(which, dh) <= 227 * 1024, (which, dh)
+    assert f(0, 0) == f(2, 257) == f(3, 64) == -1

@@ -278,7 +278,8 @@ def test_attention_of_other_shapes_keeps_fp32_probabilities(eng, B, H, KV, T, DH
         assert err(runs[0][n]) <= 1.01 * err(general[n]), (n, err(runs[0][n]), err(general[n]))
 
 
-@pytest.mark.parametrize("B,H,KV,T,DH", [(2, 8, 4, 256, 32), (1, 2, 1, 225, 8), (1, 4, 2, 97, 40), (1, 3, 3, 130, 128), (1, 2, 1, 64, 256), (16, 8, 8, 65, 64)])
+@pytest.mark.parametrize("B,H,KV,T,DH", [(2, 8, 4, 256, 32), (1, 2, 1, 225, 8), (1, 4, 2, 97, 40), (1, 3, 3, 130, 128), (1, 2, 1, 64, 256), (16, 8, 8, 65, 64),
+                                             (1, 4, 1, 33, 1), (2, 2, 2, 40, 2), (1, 8, 4, 150, 4), (1, 8, 1, 96, 256)])
 def test_fp32_attention_over_clusters(eng, B, H, KV, T, DH):
     """Few rows: clusters of two to eight CTAs share a block's tiles, some of them without one (the last case has none: it fills the
     SMs).  Sums of T products of N(0,1) numbers in fp32 in any order err by less than 2^-24 sqrt(T) a term: 2e-5 of the largest

@@ -191,6 +191,15 @@ def test_shape_fuzz(dtype, V, B, T, D, H, KV, MLP, L, tied):
     assert worst[0] <= lim_g, worst
 
 
+@pytest.mark.parametrize("V,B,T,D,H,KV,MLP,L,tied", [
+    (96, 2, 40, 32, 8, 4, 64, 1, True),        # head_dim 4
+    (64, 1, 70, 16, 8, 8, 48, 2, False),       # head_dim 2
+])
+def test_heads_narrower_than_a_warps_piece(V, B, T, D, H, KV, MLP, L, tied):
+    """Tiles of so few columns are smaller than the sums that a cluster of the fp32 dK / dV kernel merges."""
+    test_shape_fuzz("fp32", V, B, T, D, H, KV, MLP, L, tied)
+
+
 def test_lora_bf16_and_prompt_masking():
     """Frozen base + rank-8 adapters on all seven projections; first 40 % of targets masked."""
     cfg = dict(vocab_size=256, dim=128, n_layers=2, n_heads=4, n_kv_heads=2, mlp_hidden=256, tie_embeddings=True)
