@@ -675,16 +675,27 @@ static int map_rows(CUtensorMap* m, const void* base, const AttnShape& s, int he
     uint32_t box[4] = {XD, 1, (uint32_t)rows, 1};
     return tc_make_tmap_bf16(m, base, 4, dims, strides, box, true);
 }
-// Where the line to attn_mma.cu lies (us there / here, cold): its 64-row tiles and lower set-up win while the SMs are not full.
-// Forward: 4 heads T100 9.7 / 10.3, 192 heads T64 10.0 / 12.0, 8 heads T200 12.9 / 12.1, 512 heads T70 21.1 / 17.0.
-// Backward, by its 128 x 64 steps: 48 (8 heads T200) 23.5 / 27.7, 72 (8 heads T320) 26.0 / 25.7, 108 (12 heads T300) 29.7 / 33.6,
+// Where the line to attn_mma.cu lies.  Its 64-row tiles and lower set-up win where 128-row tiles are half empty or the SMs are not full.
+// Forward, us there / here (row after row of launches, heads = batch x heads): T64 384 heads 5.2 / 9.2, T20 960 heads 10.2 / 17.6, so up to 64
+// rows never here; T100 296 heads 9.6 / 6.2 (cold 16.3 / 13.3, but 192 heads 12.4 / 12.4 and 96 heads 10.5 / 10.8), 384 heads 10.8 / 10.0;
+// T129 64 heads 9.4 / 7.6, 148 heads 9.9 / 7.7, 168 heads 9.8 / 11.3, 225 heads 12.2 / 12.2, 256 heads 13.4 / 12.7, 300 heads 15.1 / 16.0, 608 heads
+// 28.3 / 27.7: two of its tiles against three there, and a last wave of CTAs (two to an SM) that is less than half full tips it;
+// T193 168 heads 14.4 / 11.2.
+static bool forward_here(const AttnShape& s) {
+    const long long ctas = (long long)s.B * s.H * ((s.T + XT - 1) / XT), wave = 2 * AX_SMS, last = ctas % wave;
+    if (s.T <= 64) return false;
+    if (s.T <= XT) return ctas > wave;
+    return s.T > 192 || ctas <= wave || ctas > 4 * wave || last == 0 || last >= wave / 2;
+}
+// Backward, by its 128 x 64 steps (us there / here, cold): 48 (8 heads T200) 23.5 / 27.7, 72 (8 heads T320) 26.0 / 25.7, 108 (12 heads T300) 29.7 / 33.6,
 // 192 (192 heads T64) 25.6 / 23.3, 320 (16 heads T500) 41.8 / 39.9.
 static long long steps(const AttnShape& s) {
     const long long tiles = (s.T + XT - 1) / XT, nq = (s.T + XQ - 1) / XQ;
     return s.B * s.H * (tiles * nq - tiles * (tiles - 1));
 }
+int ax_attn_tcs_route(int backward, const AttnShape& s) { return served(s) && (backward ? steps(s) > AX_SMS : forward_here(s)); }
 int ax_attn_fwd_tcs(const void* q, const void* k, const void* v, void* o, float* lse, const AttnShape& s, int* status, cudaStream_t st) {
-    if (!served(s) || (s.T <= XT && s.B * s.H <= 2 * AX_SMS) || !lse || !aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(o)) return -1;
+    if (!ax_attn_tcs_route(0, s) || !lse || !aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(o)) return -1;
     CUtensorMap tq, tk, tv;
     if (map_rows(&tq, q, s, s.H, XT) || map_rows(&tk, k, s, s.KV, XT) || map_rows(&tv, v, s, s.KV, XT)) return 2;
     const dim3 grid((s.T + XT - 1) / XT * s.H * s.B);
@@ -694,7 +705,7 @@ int ax_attn_fwd_tcs(const void* q, const void* k, const void* v, void* o, float*
 int ax_attn_bwd_tcs(const void* q, const void* k, const void* v, const void* dO, const float* lse, const float* Dv, void* dq, void* dk, void* dv,
                     const AttnShape& s, const float* rope_cos, const float* rope_sin, int* status, cudaStream_t st) {
     if (rope_cos && (s.DH != XD || !rope_sin || !aligned16(rope_cos) || !aligned16(rope_sin))) return -1;
-    if (!served(s) || steps(s) <= AX_SMS || !lse || !aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(dO) || !aligned16(dq) || !aligned16(dk) || !aligned16(dv)) return -1;
+    if (!ax_attn_tcs_route(1, s) || !lse || !aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(dO) || !aligned16(dq) || !aligned16(dk) || !aligned16(dv)) return -1;
     CUtensorMap q128, g128, k64, v64, q64, g64, k128, v128;
     if (map_rows(&q128, q, s, s.H, XT) || map_rows(&g128, dO, s, s.H, XT) || map_rows(&k64, k, s, s.KV, XQ) || map_rows(&v64, v, s, s.KV, XQ) ||
         map_rows(&q64, q, s, s.H, XQ) || map_rows(&g64, dO, s, s.H, XQ) || map_rows(&k128, k, s, s.KV, XT) || map_rows(&v128, v, s, s.KV, XT)) return 2;

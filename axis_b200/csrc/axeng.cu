@@ -610,6 +610,10 @@ static AttnShape shape_bthd(int B, int H, int KV, int T, int DH, float scale) {
     s.db = (long long)T * H; s.dh_ = 1; s.dtk = H;
     return s;
 }
+API int eng_attn_route(int backward, int B, int H, int KV, int T, int head_dim) {
+    if (B < 1 || H < 1 || KV < 1 || T < 1 || head_dim < 1) return 0;
+    return ax_attn_tcs_route(backward, shape_bthd(B, H, KV, T, head_dim, 1.f));
+}
 
 // rows of an embedding table (or of its gradient) that fit the buffer: ids are checked against it on the device
 static int table_rows(int idx, int dim, long long elsize) {

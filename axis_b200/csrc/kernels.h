@@ -151,6 +151,7 @@ int ax_lora_grad(int count, const void* const* X, const void* const* S, float* c
 // attn_tcs.cu — the same on tcgen05 for head dims above 32 up to 64 (rope_cos / rope_sin for 64), a positive scale and enough work to
 // fill the GPU. -1 when not served.
 int ax_attn_tcs_init(void);
+int ax_attn_tcs_route(int backward, const AttnShape& s);      // see eng_attn_route
 int ax_attn_fwd_tcs(const void* q, const void* k, const void* v, void* o, float* lse, const AttnShape& s, int* status, cudaStream_t st);
 int ax_attn_bwd_tcs(const void* q, const void* k, const void* v, const void* dO, const float* lse, const float* Dv, void* dq, void* dk, void* dv,
                     const AttnShape& s, const float* rope_cos, const float* rope_sin, int* status, cudaStream_t st);

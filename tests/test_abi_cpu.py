@@ -82,3 +82,20 @@ def test_general_attention_allocates_what_its_cluster_merge_writes(lib):
         for which, need in ((0, sums + 32 * 2 * 4), (1, sums), (2, 2 * sums)):
             assert need <= f(which, dh) <= 227 * 1024, (which, dh)
     assert f(0, 0) == f(2, 257) == f(3, 64) == -1
+
+
+@pytest.mark.parametrize("B,H,T,DH,here", [
+    # many short sequences: a 128-row tile is half empty and takes twice as long as the 64-row tiles of mma.sync
+    (24, 16, 20, 64, 0), (24, 16, 64, 48, 0), (32, 30, 40, 64, 0), (24, 16, 65, 64, 1), (4, 24, 100, 64, 0), (18, 16, 128, 56, 0),
+    # two tiles against three of mma.sync: not with a last wave that is less than half full
+    (1, 1, 129, 64, 1), (4, 37, 129, 64, 1), (3, 50, 129, 64, 0), (7, 24, 192, 64, 0), (14, 16, 160, 64, 1), (8, 37, 129, 40, 1), (19, 32, 160, 64, 1),
+    (3, 50, 193, 64, 1), (7, 24, 1000, 64, 1),
+    (7, 24, 1000, 32, 0), (7, 24, 1000, 72, 0), (7, 24, 1000, 44, 0)])
+def test_forward_attention_goes_where_it_is_faster(lib, B, H, T, DH, here):
+    for kv in {1, H}:
+        assert lib.eng_attn_route(0, B, H, kv, T, DH) == here
+
+
+def test_attention_route_of_invalid_shapes(lib):
+    for a in ((0, 8, 4, 500, 64), (1, 0, 4, 500, 64), (1, 8, 0, 500, 64), (1, 8, 3, 500, 64), (1, 8, 4, 0, 64), (1, 8, 4, 500, 0)):
+        assert lib.eng_attn_route(0, *a) == lib.eng_attn_route(1, *a) == 0
