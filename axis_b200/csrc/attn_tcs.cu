@@ -687,13 +687,22 @@ static bool forward_here(const AttnShape& s) {
     if (s.T <= XT) return ctas > wave;
     return s.T > 192 || ctas <= wave || ctas > 4 * wave || last == 0 || last >= wave / 2;
 }
-// Backward, by its 128 x 64 steps (us there / here, cold): 48 (8 heads T200) 23.5 / 27.7, 72 (8 heads T320) 26.0 / 25.7, 108 (12 heads T300) 29.7 / 33.6,
-// 192 (192 heads T64) 25.6 / 23.3, 320 (16 heads T500) 41.8 / 39.9.
+// Backward, by its 128 x 64 steps (us there / here, row after row of launches).  Up to one step an SM never here: 48 (8 heads KV 4 T193) 18.7 / 22.7,
+// 144 (24 heads KV 8 T256) 22.7 / 26.8.  Above, a CTA of dK / dV has to have something to walk for its 512 TMEM columns: a single step each never pays
+// (kv heads as heads, up to 64 rows: 192 heads T20 12.4 / 18.6, 384 heads T64 18.5 / 27.7), two do while all of them are at work at
+// once (144 heads T65 24.1 / 16.5 and 296 heads T65 26.0 / 24.7, but 608 heads T65 45.2 / 51.1 and 384 heads T129 53.4 / 59.5).  And up to
+// two steps an SM the kernels there have SMs to spare as long as their 64-row tiles are few and the walks short: 8 heads KV 4 T500 28.8 / 30.9, 16
+// heads KV 8 T384 26.9 / 28.8, but 16 heads KV 2 T384 43.1 / 37.0, 8 heads KV 8 T640 36.9 / 32.9, 64 heads T129 24.7 / 18.6.
 static long long steps(const AttnShape& s) {
     const long long tiles = (s.T + XT - 1) / XT, nq = (s.T + XQ - 1) / XQ;
     return s.B * s.H * (tiles * nq - tiles * (tiles - 1));
 }
-int ax_attn_tcs_route(int backward, const AttnShape& s) { return served(s) && (backward ? steps(s) > AX_SMS : forward_here(s)); }
+static bool backward_here(const AttnShape& s) {
+    const long long st = steps(s), nq = (s.T + XQ - 1) / XQ, key_tiles = (long long)s.B * s.KV * ((s.T + XT - 1) / XT);
+    if (st <= AX_SMS || st <= key_tiles || (st <= 2 * key_tiles && key_tiles > 2 * AX_SMS)) return false;
+    return st > 2 * AX_SMS || (long long)s.B * s.H * nq > 128 || s.H / s.KV * nq >= 20 || nq > 8;
+}
+int ax_attn_tcs_route(int backward, const AttnShape& s) { return served(s) && (backward ? backward_here(s) : forward_here(s)); }
 int ax_attn_fwd_tcs(const void* q, const void* k, const void* v, void* o, float* lse, const AttnShape& s, int* status, cudaStream_t st) {
     if (!ax_attn_tcs_route(0, s) || !lse || !aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(o)) return -1;
     CUtensorMap tq, tk, tv;

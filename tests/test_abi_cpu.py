@@ -96,6 +96,17 @@ def test_forward_attention_goes_where_it_is_faster(lib, B, H, T, DH, here):
         assert lib.eng_attn_route(0, B, H, kv, T, DH) == here
 
 
+@pytest.mark.parametrize("B,H,KV,T,DH,here", [
+    # one step for each key tile, or two for more key tiles than run at once
+    (6, 32, 32, 20, 64, 0), (24, 16, 16, 64, 48, 0), (4, 24, 8, 64, 64, 0), (40, 8, 4, 3, 64, 1), (20, 16, 4, 64, 56, 1), (32, 30, 15, 40, 64, 0),
+    (18, 16, 16, 65, 64, 1), (8, 37, 37, 65, 40, 1), (24, 16, 16, 129, 64, 0), (24, 16, 8, 129, 64, 1), (24, 16, 16, 193, 64, 1),
+    # few steps: not with few 64-row tiles and short walks
+    (1, 8, 4, 500, 64, 0), (1, 16, 8, 384, 56, 0), (1, 8, 8, 450, 64, 0), (1, 16, 2, 384, 56, 1), (1, 8, 8, 640, 56, 1), (4, 16, 16, 129, 64, 1),
+    (4, 12, 4, 129, 64, 1), (1, 8, 4, 200, 64, 0), (1, 24, 8, 500, 64, 1), (3, 24, 8, 1000, 64, 1), (3, 24, 8, 1000, 72, 0), (3, 24, 8, 1000, 32, 0)])
+def test_backward_attention_goes_where_it_is_faster(lib, B, H, KV, T, DH, here):
+    assert lib.eng_attn_route(1, B, H, KV, T, DH) == here
+
+
 def test_attention_route_of_invalid_shapes(lib):
     for a in ((0, 8, 4, 500, 64), (1, 0, 4, 500, 64), (1, 8, 0, 500, 64), (1, 8, 3, 500, 64), (1, 8, 4, 0, 64), (1, 8, 4, 500, 0)):
         assert lib.eng_attn_route(0, *a) == lib.eng_attn_route(1, *a) == 0
