@@ -702,7 +702,25 @@ static bool backward_here(const AttnShape& s) {
     if (st <= AX_SMS || st <= key_tiles || (st <= 2 * key_tiles && key_tiles > 2 * AX_SMS)) return false;
     return st > 2 * AX_SMS || (long long)s.B * s.H * nq > 128 || s.H / s.KV * nq >= 20 || nq > 8;
 }
-int ax_attn_tcs_route(int backward, const AttnShape& s) { return served(s) && (backward ? backward_here(s) : forward_here(s)); }
+// CTAs to a key tile in the dK / dV kernel.  The first key tile walks the steps of all query tiles of the group's heads, `chain` of them; an
+// even share of all steps over the SMs is `share`.  Backward in us with S = 1 / 2 / 4 CTAs to a tile (chain / share): B2 H16 KV2 T900 (120 / 13)
+// 173 / 110 / 79, B2 H8 KV2 T500 DH48 (32 / 2) 60 / 46 / 40, B1 H12 KV4 T2500 (120 / 34) 204 / 143 / 145, B1 H32 KV8 T1400 (88 / 28) 152 / 107 / 118,
+// B4 H24 KV8 T500 (24 / 12) 65 / 67 / 96, B2 H4 KV2 T200 (8 / 0) 28 / 28 / 28; eight are no better anywhere.
+// Clusters that do not all run at once (74 of two, 33 of four fit the GPU) start late: that is no loss only where the first tile's share of
+// the walk outlasts all of it spread over those that run, with two steps for the set-up and the merge of each of four and one of each
+// of two.  1 / 2 / 4 with that many key tiles: 36 (B3 H12 KV4 T384) 35 / 33 / 41, 40 (B1 H16 KV8 T640) 45 / 37 / 45, 72 (B1 H8 KV8 T1100) 51 / 45 / 66,
+// 112 (B7 H24 KV8 T129) 31 / 38 / 58, but 40 (B1 H4 KV2 T2500) 139 / 105 / 85, 36 (B1 H8 KV4 T1100) 66 / 55 / 49, 128 (B2 H24 KV8 T900) 83 / 70 / 102.
+static int parts(const AttnShape& s) {
+    const long long nq = (s.T + XQ - 1) / XQ, chain = s.H / s.KV * nq, st = steps(s), share = st / AX_SMS, key_tiles = (long long)s.B * s.KV * ((s.T + XT - 1) / XT);
+    auto fit = [&](int n, int at_once) { return key_tiles <= at_once || at_once * chain > st + n * n / 2 * key_tiles; };
+    int S = 1;
+    while (S < 4 && chain >= 8 * S && chain > 2 * S * share && fit(2 * S, S == 1 ? AX_SMS / 2 : 33)) S *= 2;
+    return S;
+}
+int ax_attn_tcs_route(int backward, const AttnShape& s) {
+    if (!served(s)) return 0;
+    return backward ? (backward_here(s) ? parts(s) : 0) : forward_here(s);
+}
 int ax_attn_fwd_tcs(const void* q, const void* k, const void* v, void* o, float* lse, const AttnShape& s, int* status, cudaStream_t st) {
     if (!ax_attn_tcs_route(0, s) || !lse || !aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(o)) return -1;
     CUtensorMap tq, tk, tv;
@@ -721,13 +739,7 @@ int ax_attn_bwd_tcs(const void* q, const void* k, const void* v, const void* dO,
     const int tiles = (s.T + XT - 1) / XT;
     if (ax_launch_chain(k_attn_dq_tcs, dim3(tiles * s.H * s.B), dim3(XG_THREADS), XdQSmem::TOTAL, st, q128, g128, k64, v64, lse, Dv, (bf16*)dq, s,
                         rope_cos, rope_sin, status) != cudaSuccess) return 3;
-    // dK / dV: the first key tile walks the steps of all query tiles of the group's heads, `chain` of them; an even share of all steps over the
-    // SMs is `share`.  Backward in us with S = 1 / 2 / 4 CTAs to a tile (chain / share): B2 H16 KV2 T900 (120 / 13) 173 / 110 / 79,
-    // B2 H8 KV2 T500 DH48 (32 / 2) 60 / 46 / 40, B1 H12 KV4 T2500 (120 / 34) 204 / 143 / 145, B1 H32 KV8 T1400 (88 / 28) 152 / 107 / 118,
-    // B4 H24 KV8 T500 (24 / 12) 65 / 67 / 96, B2 H4 KV2 T200 (8 / 0) 28 / 28 / 28; eight are no better anywhere.
-    const long long nq = (s.T + XQ - 1) / XQ, chain = s.H / s.KV * nq, share = steps(s) / AX_SMS;
-    int S = 1;
-    while (S < 4 && chain >= 8 * S && chain > 2 * S * share) S *= 2;
+    const int S = parts(s);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(tiles * s.KV * s.B * S); cfg.blockDim = dim3(XK_THREADS); cfg.dynamicSmemBytes = XdKVSmem::TOTAL; cfg.stream = st;
     cudaLaunchAttribute at[2];

@@ -170,7 +170,8 @@ int eng_last_variant(void);
 /* Pairs of CTAs that shared the depth of a tile in the last paired-CTA tcgen05 launch: 1, 2 or 4. */
 int eng_last_gemm_parts(void);
 /* Whether bf16 attention of this shape, in the layout of ENG_ATTN_FWD / ENG_ATTN_BWD and with aligned buffers, runs on the tcgen05
- * kernels with split probabilities once the whole-tile kernels have refused it (1) or not (0): host arithmetic that needs no GPU. */
+ * kernels with split probabilities once the whole-tile kernels have refused it (for the backward the number of CTAs that share a key tile,
+ * 1, 2 or 4) or not (0): host arithmetic that needs no GPU. */
 int eng_attn_route(int backward, int B, int H, int KV, int T, int head_dim);
 /* Dynamic shared memory in bytes of the general attention kernels, 0 forward, 1 dQ, 2 dK / dV, for a head dim of 1 to 256
  * (else -1): host arithmetic that needs no GPU. */
