@@ -361,7 +361,7 @@ int ax_gemm_tc(int out_bf16, int tb, const void* A, const void* B, void* C, cons
             if (cost < best2 - 1e-9) { best2 = cost; best2_s = sk; }
         }
         double shared;
-        if (!g_side && ax_gemm_tc2_share((int)tiles2, kblocks, &shared) > 1 && shared * 0.70 < best2) { best2 = shared * 0.70; best2_s = 1; }
+        if (!g_side && ax_gemm_tc2_by_tma(C, beta != 0.f ? D : nullptr, n, out_bf16 ? 2 : 4) && ax_gemm_tc2_share((int)tiles2, kblocks, &shared) > 1 && shared * 0.70 < best2) { best2 = shared * 0.70; best2_s = 1; }
         if (g_pair_mode == 2 || best2 < best) {
             ax_variant = 0x22 + 0x100 * best2_s;
             const int rc = ax_gemm_tc2(out_bf16, tb, A, B, C, D, m, n, k, alpha, beta, status, best2_s, st);

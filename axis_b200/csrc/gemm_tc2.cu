@@ -757,6 +757,11 @@ int ax_gemm_tc2_share(int tiles, int kb, double* cost) {
     return S;
 }
 
+// whether an output of n columns of osz bytes, and its addend if there is one, go by TMA (a shared tile needs that)
+bool ax_gemm_tc2_by_tma(const void* C, const void* D, long long n, int osz) {
+    return ax_gemm_tma_out() && ((uintptr_t)C & 15) == 0 && ((uintptr_t)D & 15) == 0 && n * osz % 16 == 0;
+}
+
 struct SwbArgs { const void* g; const void* u; void* du; };    // SwiGLU backward in the epilogue (C = dg)
 
 // One launch.  grp.mode 0: the plain GEMM (A, B, C, D are element 0 of the arrays).  Grouped modes: see GemmGroup;
@@ -837,10 +842,10 @@ static int gemm2_launch(int mode, int count, const void* const* A, const void* c
     const int osz = ksplit > 1 ? 4 : (int)sizeof(TO);
     const bool has_d = D != nullptr && beta != 0.f && ksplit == 1;
     int tma_out = 0;
-    bool c_ok = ax_gemm_tma_out() != 0;
+    bool c_ok = true;
     for (int g = 0; g < (per_problem_c ? count : (mode == 4 ? 3 : 1)); g++)
-        c_ok = c_ok && ((uintptr_t)C[g] & 15) == 0 && ((long long)nv[per_problem_c ? g : 0] * osz) % 16 == 0;
-    if (c_ok && (!has_d || ((uintptr_t)D & 15) == 0)) tma_out = has_d ? 2 : 1;
+        c_ok = c_ok && ax_gemm_tc2_by_tma(C[g], has_d ? D : nullptr, nv[per_problem_c ? g : 0], osz);
+    if (c_ok) tma_out = has_d ? 2 : 1;
     if (!tma_out) grp.S = 1;                 // (threads that store their rows write whole tiles)
     // grouped launches need the TMA-store epilogue; only the K-segment form takes an addend
     if (mode != 0 && (ksplit != 1 || !(tma_out == 1 || (tma_out == 2 && mode == 2)))) return -1;

@@ -94,6 +94,7 @@ int ax_gemm_tc(int out_bf16, int tb, const void* A, const void* B, void* C, cons
 // gemm_tc2.cu — paired-CTA (cta_group::2) variant, 256 x 256 tile per two SMs
 int ax_gemm_tc2_init(void);
 int ax_gemm_tc2_share(int tiles, int kb, double* cost);
+bool ax_gemm_tc2_by_tma(const void* C, const void* D, long long n, int osz);
 int ax_gemm_tc2(int out_bf16, int tb, const void* A, const void* B, void* C, const void* D,
                 int m, int n, int k, float alpha, float beta, int* status, int ksplit, cudaStream_t st);
 void ax_gemm_set_mode(int mode);      // 0 auto, 1 single-CTA only, 2 paired whenever possible

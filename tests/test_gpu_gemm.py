@@ -867,6 +867,18 @@ def test_tile_depth_shared_over_a_cluster(eng, tb, dt, addend, m, n, k, parts):
     assert eng.device_status() == 0
 
 
+@pytest.mark.parametrize("addend", [False, True])
+@pytest.mark.parametrize("n,variant,parts", [(776, 0x122, 4), (780, 0x222, 1)])
+def test_depth_is_not_shared_for_rows_that_tma_cannot_store(eng, addend, n, variant, parts):
+    """Twelve tiles 32 k-blocks deep: four pairs to a tile where rows of C are whole 16-byte pieces, else two parts through the workspace, which
+    the cost rule takes only if it knows that the tiles will not be shared."""
+    rng = np.random.default_rng(n)
+    got, ref = run_gemm(eng, rng, 520, n, 2048, 1, 1, fallback=8, **(dict(beta=-2.0, addend=True) if addend else dict(alpha=0.5)))
+    assert (eng.last_variant(), eng.last_gemm_parts()) == (variant, parts)
+    check(got, ref, True, 2048)
+    assert eng.device_status() == 0
+
+
 @pytest.mark.parametrize("m,k,ns,r,parts", [(1032, 1352, (512, 264, 136), 16, 2), (520, 1800, (264, 136, 72), 8, 4)])
 def test_grouped_tiles_shared_over_a_cluster(eng, m, k, ns, r, parts):
     """The same for groups: one input and several outputs with a low-rank term each, and one output summed over K-segments."""
