@@ -384,7 +384,7 @@ k_attn_bwd_dkv_mma(const bf16* __restrict__ q, const bf16* __restrict__ k, const
         if (!half)                                          // a thread's own places again
 #pragma unroll
             for (int i = 0; i < DHP / 2; i++) { xch[i * MA_TH] = ak[i >> 2][i & 3]; xch[(DHP / 2 + i) * MA_TH] = av[i >> 2][i & 3]; }
-        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        cluster_sync();
         constexpr int HG = DHP / 16;                        // column groups of a half head; group f and f + HG are rotary pairs
         const uint32_t base = ma_smem(xch + half * (DHP / 2) * MA_TH);
         bf16* dst = (half ? dv : dk) + b * s.kb + g * s.kh;
@@ -417,8 +417,7 @@ k_attn_bwd_dkv_mma(const bf16* __restrict__ q, const bf16* __restrict__ k, const
                 if ((f + HG) * 8 < s.DH) *reinterpret_cast<__nv_bfloat162*>(o + HG * 8) = __floats2bfloat162_rn(y0 * fac, y1 * fac);
             }
         }
-        __syncwarp();
-        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");   // peers have read
+        cluster_sync();   // peers have read
         return;
     }
     if (half) return;

@@ -99,9 +99,6 @@ __device__ __forceinline__ void attn_axpy(float (&acc)[AR][NJ], const float* w, 
 
 // Where rows are few, a cluster of S CTAs takes the tiles that a block of rows walks in turn, and the sums meet through distributed
 // shared memory: a unit is a warp's row of accumulators, [unit][i][thread], and each CTA finishes 1 / S of the units, in rank order.
-__device__ __forceinline__ void attn_cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ float attn_peer(const float* p, int rank) {
     float x;
     asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %1, %2;\n\tld.shared::cluster.f32 %0, [ra];\n\t}"
@@ -183,7 +180,7 @@ k_attn_fwd_simt(const T* __restrict__ q, const T* __restrict__ k, const T* __res
 #pragma unroll
             for (int i = 0; i < NJ; i++) acc_x[(r * NJ + i) * ATH] = acc[r][i];
         }
-        attn_cluster_sync();
+        cluster_sync();
         for (int r = part * AR / S; r < (part + 1) * AR / S; r++) {
             const int t = t0 + r;
             if (t >= s.T) continue;
@@ -204,7 +201,7 @@ k_attn_fwd_simt(const T* __restrict__ q, const T* __restrict__ k, const T* __res
                 if (lane + 32 * i < DH) stf(orow, lane + 32 * i, a[i] * il);
             if (lse && lane == 0) lse[((long long)b * s.H + h) * s.T + t] = mx + logf(ls);
         }
-        attn_cluster_sync();             // peers have read
+        cluster_sync();             // peers have read
         return;
     }
 #pragma unroll
@@ -292,7 +289,7 @@ k_attn_bwd_dq_simt(const T* __restrict__ q, const T* __restrict__ k, const T* __
         for (int r = 0; r < AR; r++)
 #pragma unroll
             for (int i = 0; i < NJ; i++) acc_x[(r * NJ + i) * ATH] = acc[r][i];
-        attn_cluster_sync();
+        cluster_sync();
         for (int r = part * AR / S; r < (part + 1) * AR / S; r++) {
             const int t = t0 + r;
             if (t >= s.T) continue;
@@ -304,7 +301,7 @@ k_attn_bwd_dq_simt(const T* __restrict__ q, const T* __restrict__ k, const T* __
                 if (lane + 32 * i < DH) stf(dq, roff + lane + 32 * i, a);
             }
         }
-        attn_cluster_sync();             // peers have read
+        cluster_sync();             // peers have read
         return;
     }
 #pragma unroll
@@ -393,7 +390,7 @@ k_attn_bwd_dkv_simt(const T* __restrict__ q, const T* __restrict__ k, const T* _
         for (int r = 0; r < AR; r++)
 #pragma unroll
             for (int i = 0; i < NJ; i++) { acc_x[(r * NJ + i) * ATH] = ak[r][i]; acc_x[((AR + r) * NJ + i) * ATH] = av[r][i]; }
-        attn_cluster_sync();
+        cluster_sync();
         for (int u = part * 2 * AR / S; u < (part + 1) * 2 * AR / S; u++) {
             const int j = j0 + u % AR;
             if (j >= s.T) continue;
@@ -405,7 +402,7 @@ k_attn_bwd_dkv_simt(const T* __restrict__ q, const T* __restrict__ k, const T* _
                 if (lane + 32 * i < DH) stf(u < AR ? dk : dv, koff + lane + 32 * i, a);
             }
         }
-        attn_cluster_sync();             // peers have read
+        cluster_sync();             // peers have read
         return;
     }
 #pragma unroll

@@ -635,7 +635,7 @@ k_attn_dkv_tcs(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     __syncthreads();
     if (warp == XK_SM_WARPS) { __syncwarp(); tc_fence_after(); tmem_dealloc(tmem, 512); }
     if (S > 1) {
-        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        cluster_sync();
         const int rows = XT / S;
         for (int i = threadIdx.x; i < 2 * rows * 4; i += XK_THREADS) {       // eight columns and their partners
             const int m = i / (rows * 4), r = part * rows + (i >> 2) % rows, c0 = (i & 3) * 8, t = j * XT + r;
@@ -653,8 +653,7 @@ k_attn_dkv_tcs(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             store_grad8(a, a + 8, c0, m ? s.scale : 1.f, m && rope_cos ? rope_cos + (long long)t * 32 : nullptr, rope_sin + (long long)t * 32,
                         (m ? dk : dv) + (((long long)b * T + t) * KV + g) * s.DH, s.DH);
         }
-        __syncwarp();
-        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");     // peers have read
+        cluster_sync();     // peers have read
     }
 }
 

@@ -112,6 +112,13 @@ static inline int ew_grid(long long work_items, int threads) {
 }
 static inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
+// Barrier over a cluster's CTAs, with release and acquire of shared memory.  The aligned forms are undefined for a warp whose lanes have not
+// come together again behind a branch.
+__device__ __forceinline__ void cluster_sync() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // Programmatic dependent launch.  A kernel of the main chain lets its successor be scheduled early and then waits
 // itself until its predecessor in the stream has completed (nothing before this point may read what that kernel
 // wrote); without the launch attribute both instructions are no-ops.

@@ -218,7 +218,7 @@ k_gemm_f32(const float* __restrict__ A, const float* __restrict__ B, float* C, c
                 sm[o] = t;
             }
         }
-        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        cluster_sync();
     }
     // output rows: all of them, or this CTA's share of the cluster's tile
     const int rows = ksplit > 1 ? BM / ksplit : BM, rb = ksplit > 1 ? split * rows : 0;
@@ -260,7 +260,7 @@ k_gemm_f32(const float* __restrict__ A, const float* __restrict__ B, float* C, c
         }
     }
     if (ksplit > 1)                                       // nobody's shared memory goes away while a peer reads it
-        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        cluster_sync();
 }
 
 template <int BM, int BN, int BK, int KG, int TM, int TN, int ST, bool A_MN, bool B_KM, bool VEC>

@@ -50,9 +50,6 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t saddr, uint32_t rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
     return r;
 }
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
@@ -258,7 +255,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
     if (warp == 1) { tmem_alloc2(smem_u32(tmem_slot), 512); tmem_relinquish2(); }
     tc_fence_before();
     __syncthreads();
-    cluster_sync_all();                                   // peer barriers are initialised before anyone signals them
+    cluster_sync();                                   // peer barriers are initialised before anyone signals them
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t full_leader = map_to_cta(bar_full, lead);  // cluster address of the leader's full[0]
@@ -430,7 +427,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
             // sums of the other parts in this CTA's operand ring: [part][lane quarter][chunk][4 columns][row], 512 bytes in a row per warp
             auto part_at = [&](int from, int c) { return ((from - (from > part)) * 4 + quad) * own * 4096 + c * 4096 + lane * 16; };
             if (CAN_SHARE && S > 1) {                           // one tile per cluster: every warp comes by here once
-                cluster_sync_all();                             // no ring has a reader or a writer left
+                cluster_sync();                             // no ring has a reader or a writer left
                 if (ok)
                     for (int q = 1; q < S; q++) {
                         const int to = (part + q) & (S - 1);
@@ -446,7 +443,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
                                              "r"(r[z * 4 + 2]), "r"(r[z * 4 + 3]) : "memory");
                         }
                     }
-                cluster_sync_all();
+                cluster_sync();
             }
             if (!ok) break;
             auto part_add = [&](int c, uint32_t* r) {            // chunk c of this part, the parts in order behind the own sum
@@ -674,11 +671,10 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
         if (tma_out && lane == 0) bulk_wait_read_all();       // staging stays valid until the last store has read it
         if (!ok && lane == 0) { *abort_flag = 1; atomicExch(status, STAT_GEMM2 | 3); }
     }
-    if (CAN_SHARE && S > 1 && warp < 2) { __syncwarp(); cluster_sync_all(); cluster_sync_all(); }      // the two of the epilogue
+    if (CAN_SHARE && S > 1 && warp < 2) { cluster_sync(); cluster_sync(); }      // the two of the epilogue
     tc_fence_before();
     __syncthreads();
-    __syncwarp();
-    cluster_sync_all();                                    // nobody frees TMEM while the peer may still use the pair
+    cluster_sync();                                    // nobody frees TMEM while the peer may still use the pair
     if (warp == 1) { __syncwarp(); tc_fence_after(); tmem_dealloc2(tmem_base, 512); }
     if (timing && threadIdx.x == 0) prof[7] = clock64();
 }

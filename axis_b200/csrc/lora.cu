@@ -345,7 +345,7 @@ __global__ void __launch_bounds__(256) k_lora_proj(const LoraProjArgs a) {
     // the cluster's parts: every CTA leaves its sum, then finishes 1 / S of the rows from all CTAs' sums, in part order
     float* mine = red + 4 * LP_TOK * R;
     for (int i = tid; i < LP_TOK * R / 2; i += 256) *reinterpret_cast<float2*>(mine + i * 2) = quarters((i * 2) / R, (i * 2) % R);
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    cluster_sync();
     const int rows = LP_TOK / a.S;
     for (int i = tid; i < rows * R / 2; i += 256) {
         const int r = part * rows + (i * 2) / R, c = (i * 2) % R;
@@ -359,7 +359,7 @@ __global__ void __launch_bounds__(256) k_lora_proj(const LoraProjArgs a) {
         }
         if (t0 + r < a.N) *reinterpret_cast<__nv_bfloat162*>(P.out + (long long)(t0 + r) * R + c) = __floats2bfloat162_rn(a.alpha * s.x, a.alpha * s.y);
     }
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");   // peers have read
+    cluster_sync();   // peers have read
 }
 
 template <int NT, int TB> static size_t lora_proj_smem() {

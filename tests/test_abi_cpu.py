@@ -118,3 +118,15 @@ def test_ctas_to_a_key_tile_of_the_attention_backward(lib, B, H, KV, T, parts):
 def test_attention_route_of_invalid_shapes(lib):
     for a in ((0, 8, 4, 500, 64), (1, 0, 4, 500, 64), (1, 8, 0, 500, 64), (1, 8, 3, 500, 64), (1, 8, 4, 0, 64), (1, 8, 4, 500, 0)):
         assert lib.eng_attn_route(0, *a) == lib.eng_attn_route(1, *a) == 0
+
+
+def test_cluster_barriers_are_met_by_converged_warps():
+    """The aligned forms of the cluster barrier stand in one helper only, behind a __syncwarp(): lanes may come to them from a branch."""
+    csrc = os.path.join(ROOT, "axis_b200", "csrc")
+    found = []
+    for f in sorted(os.listdir(csrc)):
+        src = open(os.path.join(csrc, f)).read()
+        found += [f] * src.count("barrier.cluster.arrive")
+        if f == "common.cuh":
+            assert re.search(r"void cluster_sync\(\) \{\s*__syncwarp\(\);\s*asm volatile\(\"barrier\.cluster\.arrive\.release\.aligned;", src)
+    assert found == ["common.cuh"]
