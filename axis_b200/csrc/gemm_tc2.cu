@@ -255,7 +255,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
     if (warp == 1) { tmem_alloc2(smem_u32(tmem_slot), 512); tmem_relinquish2(); }
     tc_fence_before();
     __syncthreads();
-    cluster_sync();                                   // peer barriers are initialised before anyone signals them
+    cluster_sync();                                       // peer barriers are initialised before anyone signals them
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t full_leader = map_to_cta(bar_full, lead);  // cluster address of the leader's full[0]
@@ -427,7 +427,8 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
             // sums of the other parts in this CTA's operand ring: [part][lane quarter][chunk][4 columns][row], 512 bytes in a row per warp
             auto part_at = [&](int from, int c) { return ((from - (from > part)) * 4 + quad) * own * 4096 + c * 4096 + lane * 16; };
             if (CAN_SHARE && S > 1) {                           // one tile per cluster: every warp comes by here once
-                cluster_sync();                             // no ring has a reader or a writer left
+                ok = __all_sync(0xffffffffu, ok);               // lanes may have seen the wait or the flag differently: TMEM is read by whole warps
+                cluster_sync();                                 // no ring has a reader or a writer left
                 if (ok)
                     for (int q = 1; q < S; q++) {
                         const int to = (part + q) & (S - 1);
@@ -674,7 +675,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
     if (CAN_SHARE && S > 1 && warp < 2) { cluster_sync(); cluster_sync(); }      // the two of the epilogue
     tc_fence_before();
     __syncthreads();
-    cluster_sync();                                    // nobody frees TMEM while the peer may still use the pair
+    cluster_sync();                                        // nobody frees TMEM while the peer may still use the pair
     if (warp == 1) { __syncwarp(); tc_fence_after(); tmem_dealloc2(tmem_base, 512); }
     if (timing && threadIdx.x == 0) prof[7] = clock64();
 }
