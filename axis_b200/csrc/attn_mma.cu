@@ -445,6 +445,7 @@ static bool ma_served(const AttnShape& s) {
 int ax_attn_fwd_mma(const void* q, const void* k, const void* v, void* o, float* lse, const AttnShape& s, cudaStream_t st) {
     if (!ma_served(s) || !aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(o)) return -1;
     const dim3 grid(s.H * s.B, (s.T + MA_ROWS - 1) / MA_ROWS);
+    ax_variant = 0x82;
     auto go = [&](auto kern, int smem) {
         return ax_launch_chain(kern, grid, dim3(MA_TH), smem, st, (const bf16*)q, (const bf16*)k, (const bf16*)v, (bf16*)o, lse, s) == cudaSuccess ? 0 : 3;
     };
@@ -465,6 +466,7 @@ int ax_attn_bwd_mma(const void* q, const void* k, const void* v, const void* dO,
     const long long chain = (long long)(s.H / s.KV) * tiles, share = (long long)s.H * s.B * tiles * (tiles + 1) / 2 / (AX_SMS * (s.DH > 64 ? 1 : 2));
     int S = 1;
     while (S < (s.DH <= 32 ? 2 : 4) && S * 2 <= chain && chain > S * share) S *= 2;
+    ax_variant = 0x83 + 0x100 * S;
     auto go = [&](auto kq, auto kk, int smem) {
         if (ax_launch_chain(kq, gq, dim3(MA_TH), smem, st, (const bf16*)q, (const bf16*)k, (const bf16*)v, (const bf16*)dO, lse, Dv, (bf16*)dq, s, rope_cos, rope_sin) != cudaSuccess) return 3;
         cudaLaunchConfig_t cfg = {};

@@ -164,7 +164,8 @@ int eng_set_fallback(int mask);
 long long eng_bytes_allocated(void);
 /* Code of the kernel variant the last GEMM / cross-entropy op ran on (no counterpart in the reference; lets a
  * test assert that a shape was served by the kernel it means to check): 0x10 cross-entropy streaming rows,
- * 0x11 register-resident rows; 0x80 / 0x81 attention forward / backward with split probabilities on tcgen05; 0x20 general GEMM, 0x21 single-CTA tcgen05 GEMM, 0x22 paired-CTA tcgen05 GEMM, 0x23 a group of them, 0x26 small products,
+ * 0x11 register-resident rows; 0x80 / 0x81 attention forward / backward with split probabilities on tcgen05, 0x82 / 0x83 on mma.sync
+ * (the backward plus 0x100 times the CTAs that share a key tile); 0x20 general GEMM, 0x21 single-CTA tcgen05 GEMM, 0x22 paired-CTA tcgen05 GEMM, 0x23 a group of them, 0x26 small products,
  * the GEMM codes plus 0x100 times the split-K factor. */
 int eng_last_variant(void);
 /* Pairs of CTAs that shared the depth of a tile in the last paired-CTA tcgen05 launch: 1, 2 or 4. */

@@ -186,7 +186,7 @@ def test_attention_backward_with_the_inverse_rotary_inside(eng, dt, B, H, KV, T,
     (1, 2, 2, 128, 8), (2, 8, 4, 256, 32), (1, 3, 1, 130, 40),
     (1, 2, 1, 65, 72), (2, 2, 2, 200, 96), (1, 4, 2, 385, 128), (1, 2, 1, 1, 128)])
 def test_attention_on_ragged_tiles_and_narrow_heads(eng, B, H, KV, T, DH):
-    """Sequences that end inside a tile and heads narrower than the columns of a tile (`attn_mma.cu`), with guard rows behind every
+    """Sequences that end inside a tile and heads narrower than the columns of a tile (`attn_mma.cu`; T 1000 `attn_tcs.cu`), with guard rows behind every
     output (a store past the end of the sequence or the head would land there).  Tolerances: operands and results are bf16
     (half an ulp, 2^-8 at most) with fp32 sums over up to 1000 keys or queries, the largest element of a result is the scale: the limits of
     the whole-tile cases above are more than enough."""
@@ -238,20 +238,21 @@ def attention_f64(q, k, v, do, scale):
     return dict(o=o, dq=ds @ kk, dk=group(ds.transpose(0, 1, 3, 2) @ q), dv=group(p.transpose(0, 1, 3, 2) @ do))
 
 
-def run_bf16_attention(eng, q, k, v, do, scale, fallback, times=1):
-    """o, dq, dk, dv as bf16 bits in [B,T,heads,DH], one list per run"""
+def run_bf16_attention(eng, q, k, v, do, scale, fallback, times=1, rotary=()):
+    """o, dq, dk, dv as bf16 bits in [B,T,heads,DH], one list per run; rotary: cos and sin tables for dq and dk to be rotated back"""
     B, H, T, DH = q.shape
     KV = k.shape[1]
     t = lambda x: np.ascontiguousarray(x.transpose(0, 2, 1, 3))
     iq, ik, iv, ido = put(eng, t(q), 1), put(eng, t(k), 1), put(eng, t(v), 1), put(eng, t(do), 1)
     out = {n: (eng.alloc(a.size, 2), (B, T, a.shape[1], DH)) for n, a in (("o", q), ("dq", q), ("dk", k), ("dv", k))}
     ilse, iD = eng.alloc(B * H * T), eng.alloc(2 * B * H * (T + 128) + q.size)
+    tables = dict(zip(("beta", "gamma"), (float(put(eng, x, 0)) for x in rotary)))
     eng.set_fallback(fallback)
     runs = []
     for _ in range(times):
         eng.run([op(E.ATTN_FWD, a=iq, b=ik, d=iv, c=out["o"][0], sa=ilse, m=T, n=DH, k=KV, batch=B, tb=H, dt=1, alpha=scale),
                  op(E.ATTN_BWD, a=iq, b=ik, d=iv, c=ido, sa=ilse, sb=out["o"][0], tb=out["dq"][0], sc=out["dk"][0], oa=out["dv"][0],
-                    ob=H, oc=iD, m=T, n=DH, k=KV, batch=B, dt=1, alpha=scale)])
+                    ob=H, oc=iD, m=T, n=DH, k=KV, batch=B, dt=1, alpha=scale, **tables)])
         runs.append({n: eng.download_raw(i, sh, np.uint16) for n, (i, sh) in out.items()})
     eng.set_fallback(0)
     assert eng.device_status() == 0
@@ -260,10 +261,10 @@ def run_bf16_attention(eng, q, k, v, do, scale, fallback, times=1):
 
 @pytest.mark.parametrize("B,H,KV,T,DH", [(1, 4, 2, 1000, 64), (1, 6, 2, 321, 64), (2, 8, 4, 256, 32), (1, 3, 1, 130, 40),
                                          (2, 2, 2, 200, 96), (1, 4, 2, 385, 128),
-                                         (8, 24, 8, 320, 64), (16, 16, 16, 130, 64)])       # dK / dV over clusters of two, without one (others: four)
+                                         (8, 24, 8, 320, 64), (16, 16, 16, 130, 64)])       # on tcgen05; the backward without clusters
 def test_attention_of_other_shapes_keeps_fp32_probabilities(eng, B, H, KV, T, DH):
-    """Shapes that the tcgen05 kernels do not take had P and dS in fp32 on the general kernels (fallback 2) and the same bits on
-    every run; the tensor-core kernels for them may be no further from float64 than those and as reproducible.  P and dS enter
+    """Shapes that the whole-tile tcgen05 kernels do not take had P and dS in fp32 on the general kernels (fallback 2) and the same bits on
+    every run; the tensor-core kernels for them (attn_mma.cu, and attn_tcs.cu for (8, 24, 8, 320, 64) and T 1000) may be no further from float64 than those and as reproducible.  P and dS enter
     as two bf16 numbers, off by at most 2^-17 of an element; the results' own rounding to bf16 is up to 2^-8, so the 2-norm error
     grows by a part in 2^18, and the bound of one per cent leaves room for results that round the other way."""
     rng = np.random.default_rng(T + DH)
@@ -320,6 +321,51 @@ def test_attention_with_split_probabilities_on_tcgen05(eng, B, H, KV, T, DH, gai
     general = run_bf16_attention(eng, q, k, v, do, scale, 2)[0]
     for n, exact in attention_f64(q, k, v, do, scale).items():
         assert all(np.array_equal(runs[0][n], r[n]) for r in runs[1:]), n
+        err = lambda bits: float(np.linalg.norm(E.bf16_bits_to_f32(bits).transpose(0, 2, 1, 3) - exact) / np.linalg.norm(exact))
+        assert err(runs[0][n]) <= 1.01 * err(general[n]), (n, err(runs[0][n]), err(general[n]))
+
+
+@pytest.mark.parametrize("B,H,KV,T,DH,parts,launches", [
+    (4, 24, 8, 500, 64, 1, 3), (4, 12, 4, 129, 64, 2, 3), (2, 16, 2, 900, 64, 4, 3),       # rotated before they are rounded
+    (2, 16, 8, 500, 48, 2, 4), (4, 16, 16, 130, 40, 1, 4)])                                # the rotary as a launch of its own
+def test_split_probabilities_on_tcgen05_with_the_inverse_rotary_inside(eng, B, H, KV, T, DH, parts, launches):
+    """dq and dk of the tcgen05 backward leave ATTN_BWD rotated back, from one CTA to a key tile and from clusters: no further from float64 than the
+    general kernels, which round to bf16 in front of the rotation and behind it, and within that much (a wrong row, sign or pair of the
+    tables errs by as much as the result).  dv is not rotated."""
+    assert eng.lib.eng_attn_route(1, B, H, KV, T, DH) == parts
+    rng = np.random.default_rng(T + DH)
+    q, k, v, do = make(rng, B, H, KV, T, DH, 1)
+    scale = 1.0 / np.sqrt(DH)
+    cos, sin = O.rope_tables(T, DH)
+    eng.launch_count(reset=True)
+    runs = run_bf16_attention(eng, q, k, v, do, scale, 0, times=2, rotary=(cos, sin))
+    assert eng.last_variant() == 0x81 and eng.launch_count() == 2 * (1 + launches)
+    general = run_bf16_attention(eng, q, k, v, do, scale, 2, rotary=(cos, sin))[0]
+    ref = attention_f64(q, k, v, do, scale)
+    c, s = cos.astype(np.float64), sin.astype(np.float64)
+    for n in ("dq", "dk"):
+        g1, g2 = ref[n][..., :DH // 2], ref[n][..., DH // 2:]
+        ref[n] = np.concatenate([g1 * c + g2 * s, g2 * c - g1 * s], -1)
+    for n, exact in ref.items():
+        assert np.array_equal(runs[0][n], runs[1][n]), n
+        err = lambda bits: float(np.linalg.norm(E.bf16_bits_to_f32(bits).transpose(0, 2, 1, 3) - exact) / np.linalg.norm(exact))
+        assert err(runs[0][n]) <= 1.01 * err(general[n]) <= 1.01 * 2.0 ** -7, (n, err(runs[0][n]), err(general[n]))
+
+
+@pytest.mark.parametrize("B,H,KV,T,DH,parts", [
+    (8, 16, 16, 130, 96, 1), (8, 8, 4, 320, 128, 2), (1, 4, 2, 385, 72, 4), (16, 16, 16, 130, 32, 1), (8, 8, 4, 320, 24, 2),
+    (16, 16, 16, 130, 64, 1), (1, 8, 8, 100, 56, 2), (1, 8, 4, 500, 64, 4)])
+def test_attention_on_mma_sync_with_and_without_clusters(eng, B, H, KV, T, DH, parts):
+    """The head dims and the short or small shapes that stay on attn_mma.cu, by the number of CTAs that share a key tile in dK / dV: the bound of
+    the tests above against float64, and the same bits on every run."""
+    rng = np.random.default_rng(T + DH)
+    q, k, v, do = make(rng, B, H, KV, T, DH, 1)
+    scale = 1.0 / np.sqrt(DH)
+    runs = run_bf16_attention(eng, q, k, v, do, scale, 0, times=2)
+    assert eng.last_variant() == 0x83 + 0x100 * parts
+    general = run_bf16_attention(eng, q, k, v, do, scale, 2)[0]
+    for n, exact in attention_f64(q, k, v, do, scale).items():
+        assert np.array_equal(runs[0][n], runs[1][n]), n
         err = lambda bits: float(np.linalg.norm(E.bf16_bits_to_f32(bits).transpose(0, 2, 1, 3) - exact) / np.linalg.norm(exact))
         assert err(runs[0][n]) <= 1.01 * err(general[n]), (n, err(runs[0][n]), err(general[n]))
 
