@@ -867,6 +867,42 @@ def test_tile_depth_shared_over_a_cluster(eng, tb, dt, addend, m, n, k, parts):
     assert eng.device_status() == 0
 
 
+@pytest.mark.parametrize("tb", [0, 1, 2])
+@pytest.mark.parametrize("m,n,k,parts", [(1288, 776, 2064, 2), (1032, 1032, 1352, 2), (520, 776, 1352, 4), (520, 264, 2104, 4)])
+def test_tile_depth_shared_with_a_float_addend(eng, tb, m, n, k, parts):
+    """The same with fp32 output and addend: four or two 32-column pieces to a part, which take the staging buffers in turn."""
+    test_tile_depth_shared_over_a_cluster(eng, tb, 2, True, m, n, k, parts)
+
+
+@pytest.mark.parametrize("r", [0, 16])
+@pytest.mark.parametrize("m,T,k,ns,parts", [(1032, 258, 1352, (512, 256, 128), 2), (1032, 700, 1352, (512, 128, 264), 2), (520, 260, 1800, (256, 128, 64), 4)])
+def test_rotary_projections_of_tiles_shared_over_a_cluster(eng, m, T, k, ns, parts, r):
+    """Outputs of whole heads leave the launch rotated, from parts of 128 or 64 columns; the rotation meets the finished sum.
+    The sum's 2^-14 in `rounding` holds at this depth, too: errors of 2^-23 in random directions come to sqrt(k) 2^-23, 2^-17.5."""
+    rng = np.random.default_rng(m + T + r)
+    mk = lambda *sh: bf(rng.standard_normal(sh).astype(np.float32) * 0.4)
+    cos, sin = O.rope_tables(T, 64)
+    x, w, xa, xb = mk(m, k), [mk(k, n) for n in ns], [mk(m, 16) for _ in ns], [mk(16, n) for n in ns]
+    ix, ic, isn = put(eng, x, 1), put(eng, cos, 0), put(eng, sin, 0)
+    iw, ia, ib = ([put(eng, v, 1) for v in vs] for vs in (w, xa, xb))
+    out = [eng.alloc(m * n, 2) for n in ns]
+    pre = [op(E.GEMM_XSEG, a=ia[0], b=ia[1], d=ia[2], sa=ib[0], sb=ib[1], sc=ib[2], k=r, batch=3)] if r else []
+    eng.set_fallback(8)
+    eng.run(pre + [op(E.GEMM_GROUP, a=ix, b=iw[0], sa=iw[1], sb=iw[2], c=out[0], d=out[1], sc=out[2], m=m, k=k, n=ns[0], oa=ns[1], ob=ns[2],
+                      batch=3, oc=1, dt=1, beta=float(ic), gamma=float(isn))])
+    eng.set_fallback(0)
+    assert (eng.last_variant(), eng.last_gemm_parts()) == (0x23, parts)
+    f = lambda v: v.astype(np.float64)
+    c, s = (f(a)[np.arange(m) % T][:, None, :32] for a in (cos.reshape(T, -1), sin.reshape(T, -1)))
+    for g, n in enumerate(ns):
+        y = f(x) @ f(w[g]) + (f(xa[g]) @ f(xb[g]) if r else 0.0)
+        if g < 2:
+            h = y.reshape(m, n // 64, 64)
+            y = np.concatenate([h[..., :32] * c - h[..., 32:] * s, h[..., :32] * s + h[..., 32:] * c], -1).reshape(m, n)
+        rounding(eng.download_bf16(out[g], (m, n)), y)
+    assert eng.device_status() == 0
+
+
 @pytest.mark.parametrize("addend", [False, True])
 @pytest.mark.parametrize("n,variant,parts", [(776, 0x122, 4), (780, 0x222, 1)])
 def test_depth_is_not_shared_for_rows_that_tma_cannot_store(eng, addend, n, variant, parts):
