@@ -773,7 +773,6 @@ class CompiledTransformer:
                        tb=self.b_t, sc=self.b_wdflag, oa=self.b_sumsq, ob=nb, oc=self.b_gnorm,
                        alpha=float(self.max_grad_norm or 0.0), beta=self.wd, gamma=adam_eps)]
         self._plan_with_bucket_ops, self._bucket_norm, self._update_of_bucket_norms = plan_with_bucket_ops, bucket_norm, update_of_bucket_norms
-        self._n_buckets = nb
         self.bucket_norms = bool(cw == 1 and not zero and nb <= 64 and all(self._groups[0][b][1] > 0 for b in range(nb)))
         if self.bucket_norms:
             self.plan_step = plan_with_bucket_ops(bucket_norm) + update_of_bucket_norms()
@@ -899,7 +898,7 @@ class CompiledTransformer:
             inv = 1.0 / n
 
             def keep(*seg):
-                return self._acc_flat(SCALE, *seg, bufs=dict(a=self.a_grad, c=self.a_gacc), alpha=inv) if n > 1 else []
+                return self._acc_flat(SCALE, *seg, bufs=dict(a=self.a_grad, c=self.a_gacc), alpha=inv)
 
             def add_to(dst, *seg):
                 sc = self._acc_flat(SCALE, *seg, bufs=dict(a=self.a_grad, c=self.a_grad), alpha=inv, oa=1)
@@ -909,17 +908,14 @@ class CompiledTransformer:
                 # one GPU: a bucket's pass runs as soon as its gradients are complete, beside the backward where the weight gradients are, and
                 # the last one's is followed by the bucket's norm
                 seg = lambda b: self._groups[0][b]
-                tail = lambda b: add_to(self.a_grad, *seg(b)) if n > 1 else []
-                first = self._plan_with_bucket_ops(lambda b: keep(*seg(b)))
+                first = self._plan_with_bucket_ops(lambda b: keep(*seg(b)) if n > 1 else self._bucket_norm(b))
                 nxt = self._plan_with_bucket_ops(lambda b: add_to(self.a_gacc, *seg(b)))
-                last = self._plan_with_bucket_ops(lambda b: tail(b) + self._bucket_norm(b))
+                last = self._plan_with_bucket_ops(lambda b: add_to(self.a_grad, *seg(b)) + self._bucket_norm(b))
                 opt = self._update_of_bucket_norms()
             else:
-                first = self._gather_ops() + self.plan_fb + keep()
+                first = self._gather_ops() + self.plan_fb + (keep() if n > 1 else [])
                 nxt, last = self.plan_fb + add_to(self.a_gacc), self.plan_fb + add_to(self.a_grad)
                 opt = self.plan_ar + self._opt_ops(self.max_grad_norm)
-            if n == 1:
-                first = last if self.bucket_norms else first
             self._acc_plans[n] = (first, nxt, last, opt)
         first, nxt, last, opt = self._acc_plans[n]
         # the host queues the micro-batches without waiting for their losses, which come back through the read-back ring; the last
