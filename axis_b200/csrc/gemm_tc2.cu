@@ -129,7 +129,9 @@ __device__ __forceinline__ void tc_commit2_e(uint32_t bar, uint16_t mask) {
 //           epilogue fetches g (tmD) and u (tmC2) and writes dg (tmC) and du (tmC1).
 // Grouped launches write through TMA stores and do not split K; only mode 2 takes an addend.
 // A launch of so few tiles that pairs would be left without one takes a cluster of S pairs to a tile (S 2 or 4): each sums its part of
-// the depth, then gives the others, through distributed shared memory, their columns of its accumulator, and finishes its own.
+// the depth, then gives the others, through distributed shared memory, their columns of its accumulator, and finishes its own.  A kernel of
+// its own (SHARE): with S as a value in the one kernel, a launch that shares nothing took 0.6 us longer (0.4 with fp32 output), 7.3 us in place of
+// 6.6 for 904 x 1704 x 128.
 struct GemmGroup {
     int mode, count;
     int S;                   // pairs that share a tile's depth (1: a pair has tiles of its own)
@@ -149,7 +151,7 @@ void ax_gemm_group_rope(const float* cs, const float* sn, int T, int mask) {
     g_rope_req.rope_cos = cs; g_rope_req.rope_sin = sn; g_rope_req.rope_T = T; g_rope_req.rope_mask = mask;
 }
 
-template <int A_MN, int B_MN, typename TO, int EPI>
+template <int A_MN, int B_MN, typename TO, int EPI, bool SHARE>
 __global__ void __launch_bounds__(EpiCfg<EPI>::THREADS, 1)
 k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
            const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmD,
@@ -189,14 +191,14 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     const uint32_t smem_base = smem_u32(smem);
     constexpr int NH = EpiCfg<EPI>::NH, EW = EpiCfg<EPI>::EW;
-    constexpr bool swiglu = EPI == EPI_SWIGLU, swb = EPI == EPI_SWB, CAN_SHARE = !swiglu && !swb;
+    constexpr bool swiglu = EPI == EPI_SWIGLU, swb = EPI == EPI_SWB;
     const bool wide_stg = swiglu || swb || tma_out == 2;           // 64 KB of staging instead of 32, five stages
     const int nst = wide_stg ? STAGES2 - 1 : STAGES2;              // operand stages in use
     const uint32_t bar_d = smem_u32(bars + 20);                    // [EW warps][16 / EW buffers] arrival barriers of fetched pieces
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t crank = cluster_rank(), rank = crank & 1, lead = crank & ~1u;     // rank 0 of a pair leads it (issues the MMAs)
-    const int S = grp.S, part = crank >> 1;                // this pair's part of the depth
+    const int S = SHARE ? grp.S : 1, part = SHARE ? crank >> 1 : 0;      // this pair's part of the depth
     const int pair = blockIdx.x / (2 * S), npairs = gridDim.x / (2 * S);
     const uint16_t both = 3u << lead;                      // the pair's CTAs
     const int tiles_m = (m + 2 * BM2 - 1) / (2 * BM2);
@@ -236,7 +238,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
         return q;
     };
     const int kb_per = (kblocks_all + ksplit - 1) / ksplit;
-    const int kb_from = S > 1 ? kblocks_all * part / S : 0, kb_to = S > 1 ? kblocks_all * (part + 1) / S : kblocks_all;
+    const int kb_from = SHARE ? kblocks_all * part / S : 0, kb_to = SHARE ? kblocks_all * (part + 1) / S : kblocks_all;
     const int num_units = num_tiles * ksplit;
 
     if (threadIdx.x == 0) {
@@ -392,8 +394,8 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
             // pieces of this tile that this warp writes: half, half + NH, ...
             const int pw = swb ? 32 : cw;
             const int npt = (tma_out && !swiglu && row0 < m_g) ? (ncols + pw - 1) / pw : 0;
-            const int j0 = S > 1 ? part * (BN2 / cw / S) : 0;   // a shared tile: this part's 256 / S columns
-            const int npc = S > 1 ? max(0, min(npt - j0, BN2 / cw / S)) : (npt - half + NH - 1) / NH;
+            const int j0 = SHARE ? part * (BN2 / cw / S) : 0;   // a shared tile: this part's 256 / S columns
+            const int npc = SHARE ? max(0, min(npt - j0, BN2 / cw / S)) : (npt - half + NH - 1) / NH;
             const uint32_t pbase = pieces;
             const bool do_rope = EPI == EPI_ROPE && ((grp.rope_mask >> g) & 1);
             const int rope_t = do_rope ? (row < m_g ? row : 0) % grp.rope_T : 0;
@@ -426,7 +428,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
             const int own = 8 / S;                              // 32-column chunks of a part
             // sums of the other parts in this CTA's operand ring: [part][lane quarter][chunk][4 columns][row], 512 bytes in a row per warp
             auto part_at = [&](int from, int c) { return ((from - (from > part)) * 4 + quad) * own * 4096 + c * 4096 + lane * 16; };
-            if (CAN_SHARE && S > 1) {                           // one tile per cluster: every warp comes by here once
+            if (SHARE) {                                        // one tile per cluster: every warp comes by here once
                 ok = __all_sync(0xffffffffu, ok);               // lanes may have seen the wait or the flag differently: TMEM is read by whole warps
                 cluster_sync();                                 // no ring has a reader or a writer left
                 if (ok)
@@ -448,7 +450,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
             }
             if (!ok) break;
             auto part_add = [&](int c, uint32_t* r) {            // chunk c of this part, the parts in order behind the own sum
-                if (!CAN_SHARE || S == 1) return;
+                if (!SHARE) return;
                 for (int from = 0; from < S; from++) {
                     if (from == part) continue;
 #pragma unroll
@@ -672,7 +674,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
         if (tma_out && lane == 0) bulk_wait_read_all();       // staging stays valid until the last store has read it
         if (!ok && lane == 0) { *abort_flag = 1; atomicExch(status, STAT_GEMM2 | 3); }
     }
-    if (CAN_SHARE && S > 1 && warp < 2) { cluster_sync(); cluster_sync(); }      // the two of the epilogue
+    if (SHARE && warp < 2) { cluster_sync(); cluster_sync(); }      // the two of the epilogue
     tc_fence_before();
     __syncthreads();
     cluster_sync();                                        // nobody frees TMEM while the peer may still use the pair
@@ -694,7 +696,7 @@ template <int A_MN, int B_MN, typename TO, int EPI = EPI_PLAIN, int S = 1>
 static int clusters_for() {
     static int g_max = -1;
     if (g_max < 0) {
-        cudaFuncSetAttribute(k_gemm_tc2<A_MN, B_MN, TO, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM2);
+        cudaFuncSetAttribute(k_gemm_tc2<A_MN, B_MN, TO, EPI, (S > 1)>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM2);
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(AX_SMS / (2 * S) * 2 * S, 1, 1);
         cfg.blockDim = dim3(EpiCfg<EPI>::THREADS, 1, 1);
@@ -704,7 +706,7 @@ static int clusters_for() {
         at[0].val.clusterDim.x = 2 * S; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
         cfg.attrs = at; cfg.numAttrs = 1;
         int nc = 0;
-        if (cudaOccupancyMaxActiveClusters(&nc, k_gemm_tc2<A_MN, B_MN, TO, EPI>, &cfg) != cudaSuccess || nc < 1) { cudaGetLastError(); nc = 0; }
+        if (cudaOccupancyMaxActiveClusters(&nc, k_gemm_tc2<A_MN, B_MN, TO, EPI, (S > 1)>, &cfg) != cudaSuccess || nc < 1) { cudaGetLastError(); nc = 0; }
         g_max = nc;
     }
     return g_max;
@@ -769,6 +771,7 @@ template <int A_MN, int B_MN, typename TO, int EPI = EPI_PLAIN>
 static int gemm2_launch(int mode, int count, const void* const* A, const void* const* B, void* const* C, const void* D,
                         const int* mv, const int* nv, const int* kv, float alpha, float beta, int* status, int ksplit, cudaStream_t st,
                         const void* const* XA = nullptr, const void* const* XB = nullptr, int xk = 0, const SwbArgs* swb = nullptr) {
+    constexpr bool CAN_SHARE = EPI == EPI_PLAIN || EPI == EPI_ROPE;
     const int maxp = clusters_for<A_MN, B_MN, TO, EPI>();
     if (maxp < 1) return -1;
     const int m = mv[0], n = nv[0], k = kv[0];
@@ -834,7 +837,7 @@ static int gemm2_launch(int mode, int count, const void* const* A, const void* c
     if (mode == 2) { kb = 0; for (int g = 0; g < count; g++) kb += grp.kb[g]; }
     // (not beside the main chain, whose kernels fill the SMs and where a cluster waits for four or eight free ones in one place: a step of
     // 2 x 1536 tokens at D 1024 took 3522 us with the weight gradients shared, 3506 without)
-    grp.S = (EPI == EPI_PLAIN || EPI == EPI_ROPE) && ksplit == 1 && !ax_gemm_on_side() ? ax_gemm_tc2_share(units, kb, nullptr) : 1;
+    grp.S = CAN_SHARE && ksplit == 1 && !ax_gemm_on_side() ? ax_gemm_tc2_share(units, kb, nullptr) : 1;
     units *= ksplit;
     const int osz = ksplit > 1 ? 4 : (int)sizeof(TO);
     const bool has_d = D != nullptr && beta != 0.f && ksplit == 1;
@@ -897,8 +900,14 @@ static int gemm2_launch(int mode, int count, const void* const* A, const void* c
     static const bool want_prof = getenv("AXENG_GEMM_PROF") != nullptr;
     if (want_prof && (cudaMalloc(&prof, 64) != cudaSuccess || cudaMemset(prof, 0, 64) != cudaSuccess)) prof = nullptr;
 #endif
-    if (cudaLaunchKernelEx(&cfg, k_gemm_tc2<A_MN, B_MN, TO, EPI>, tmA[0], tmB[0], tmC[0], tmD, tmA[1], tmA[2], tmB[1], tmB[2], tmC[1], tmC[2],
-                           tmEA[0], tmEA[1], tmEA[2], tmEB[0], tmEB[1], tmEB[2], grp, tma_out, Cp, Dp, m, n, k, alpha, beta, status, ksplit, ws, prof) != cudaSuccess) return 3;
+    auto launch = [&](auto kern) {
+        return cudaLaunchKernelEx(&cfg, kern, tmA[0], tmB[0], tmC[0], tmD, tmA[1], tmA[2], tmB[1], tmB[2], tmC[1], tmC[2],
+                                  tmEA[0], tmEA[1], tmEA[2], tmEB[0], tmEB[1], tmEB[2], grp, tma_out, Cp, Dp, m, n, k, alpha, beta, status, ksplit, ws, prof);
+    };
+    cudaError_t err;
+    if constexpr (CAN_SHARE) err = grp.S > 1 ? launch(k_gemm_tc2<A_MN, B_MN, TO, EPI, true>) : launch(k_gemm_tc2<A_MN, B_MN, TO, EPI, false>);
+    else err = launch(k_gemm_tc2<A_MN, B_MN, TO, EPI, false>);
+    if (err != cudaSuccess) return 3;
 #ifdef AXENG_PROF
     if (prof) {
         long long h[8];
