@@ -440,14 +440,35 @@ static int attn_vec(int dt, const AttnShape& s, std::initializer_list<const void
     return ok;
 }
 
-// CTAs that share a block's walk of `chain` tiles: doubled up to four CTAs per SM and while each keeps half of `least` tiles.  fp32, forward / backward in us with 1 / 2 / 4 / (dK / dV) 8: B2 H8 KV4 T256 DH32 27, 21, 21 /
+// CTAs that fit the GPU, up to four per SM
+static long long attn_slots(size_t smem) {
+    const long long fit = (long long)(227 * 1024 / (smem + 1024));
+    return (fit < 1 ? 1 : fit < 4 ? fit : 4) * AX_SMS;
+}
+// CTAs that share a block's walk of `chain` tiles: doubled up to four per SM, while each keeps half of `least` tiles; with more than one per SM one and
+// a half, and with more than fit at once three (two fit: head dims above 64) or six (one fits: above 128).
+// Gain of a doubling (484 shapes, DH 8 to 256, T 7 to 900, forward / backward) by the CTAs that it leads to and the tiles that it leaves to each:
+// up to one per SM and one tile 1.16 / 1.11, two or three 1.31 / 1.18, four to seven 1.57 / 1.43; up to two per SM, where as many fit, one 1.07 / 0.90, two or
+// three 1.23 / 1.10; up to four, where two fit, one 0.72 / 0.81, two or three 0.97 / 0.96, four to seven 1.08 / 1.05; up to two, where one fits, two or
+// three 0.96 / 0.93, four to seven 1.12 / 0.99, eight to fifteen 1.34 / 1.20.
+// fp32, forward / backward in us with 1 / 2 / 4 / (dK / dV) 8: B2 H8 KV4 T256 DH32 27, 21, 21 /
 // 87, 79, 59, 47; B2 H4 KV2 T200 DH64 33, 24, 19 / 111, 73, 55, 44; B1 H8 KV8 T512 DH64 65, 45, 37 / 229, 130, 101, 107; B4 H8 KV4 T128 DH32
 // 17, 15, 16 / 51, 49, 43, 36; B1 H4 KV1 T300 DH64 43, 28, 22 / 225, 126, 77, 56.
-static int attn_share(long long ctas, int chain, int most, int least) {
+static int attn_share(long long ctas, int chain, int most, int least, size_t smem) {
+    const long long slots = attn_slots(smem);
     int S = 1;
-    while (S < most && ctas * S * 2 <= 4 * AX_SMS && chain >= least * S) S *= 2;
+    for (; S < most; S *= 2) {
+        const long long n = ctas * S * 2, half_tiles = n <= AX_SMS ? least : n <= slots ? 3 : 12 * AX_SMS / slots;
+        if (n > 4 * AX_SMS || chain < half_tiles * S) break;
+    }
     return S;
 }
+int ax_attn_simt_share(int which, const AttnShape& s) {
+    const int blocks = (s.T + ABLK - 1) / ABLK, rep = s.H / s.KV;
+    if (which == ATTN_DKV) return attn_share((long long)blocks * s.KV * s.B, blocks * rep, 8, 2, attn_smem(which, s.DH));
+    return attn_share((long long)blocks * s.H * s.B, blocks, 4, 3, attn_smem(which, s.DH));
+}
+
 template <typename K, typename... A>
 static int attn_launch(K kern, dim3 grid, size_t smem, int S, cudaStream_t st, A... args) {
     grid.x *= S;
@@ -467,7 +488,7 @@ static int attn_fwd_launch(const void* q, const void* k, const void* v, void* o,
     const size_t smem = attn_smem(ATTN_FWD, s.DH);
     if (!attn_smem_ok(smem, k_attn_fwd_simt<T, NJ>)) return 101;
     const dim3 grid((s.T + ABLK - 1) / ABLK, s.H, s.B);
-    return attn_launch(k_attn_fwd_simt<T, NJ>, grid, smem, attn_share((long long)grid.x * grid.y * grid.z, grid.x, 4, 3), st, (const T*)q, (const T*)k, (const T*)v, (T*)o, lse, s, vec);
+    return attn_launch(k_attn_fwd_simt<T, NJ>, grid, smem, ax_attn_simt_share(ATTN_FWD, s), st, (const T*)q, (const T*)k, (const T*)v, (T*)o, lse, s, vec);
 }
 template <typename T>
 static int attn_fwd_nj(const void* q, const void* k, const void* v, void* o, float* lse, const AttnShape& s, int vec, cudaStream_t st) {
@@ -490,9 +511,9 @@ static int attn_bwd_launch(const void* q, const void* k, const void* v, const vo
     const size_t smem_q = attn_smem(ATTN_DQ, s.DH), smem_kv = attn_smem(ATTN_DKV, s.DH);
     if (!attn_smem_ok(smem_q, k_attn_bwd_dq_simt<T, TO, NJ>) || !attn_smem_ok(smem_kv, k_attn_bwd_dkv_simt<T, TO, NJ>)) return 102;
     const dim3 g1((s.T + ABLK - 1) / ABLK, s.H, s.B), g2((s.T + ABLK - 1) / ABLK, s.KV, s.B);
-    const int rc = attn_launch(k_attn_bwd_dq_simt<T, TO, NJ>, g1, smem_q, attn_share((long long)g1.x * g1.y * g1.z, g1.x, 4, 3), st, (const T*)q, (const T*)k, (const T*)v,
+    const int rc = attn_launch(k_attn_bwd_dq_simt<T, TO, NJ>, g1, smem_q, ax_attn_simt_share(ATTN_DQ, s), st, (const T*)q, (const T*)k, (const T*)v,
                                (const T*)dO, lse, Dv, (TO*)dq, s, vec);
-    return rc ? rc : attn_launch(k_attn_bwd_dkv_simt<T, TO, NJ>, g2, smem_kv, attn_share((long long)g2.x * g2.y * g2.z, g2.x * (s.H / s.KV), 8, 2), st, (const T*)q, (const T*)k,
+    return rc ? rc : attn_launch(k_attn_bwd_dkv_simt<T, TO, NJ>, g2, smem_kv, ax_attn_simt_share(ATTN_DKV, s), st, (const T*)q, (const T*)k,
                                  (const T*)v, (const T*)dO, lse, Dv, (TO*)dk, (TO*)dv, s, vec);
 }
 template <typename T, typename TO>

@@ -115,6 +115,7 @@ int ax_attn_bwd_simt(int dt, int out_dt, const void* q, const void* k, const voi
                      const float* lse, const float* Dv, void* dq, void* dk, void* dv,
                      const AttnShape& s, cudaStream_t st);
 long long ax_attn_simt_smem(int which, int DH);      // see eng_attn_smem
+int ax_attn_simt_share(int which, const AttnShape& s);      // see eng_attn_share
 
 // gemm_tc2.cu — grouped launch of the paired-CTA GEMM (mode 1: shared A, per-problem B/C/n; mode 2: one C summed
 // over per-segment A/B/k; mode 3: independent problems A/B/C/m/n of one depth k).  -1 when not served.

@@ -120,6 +120,16 @@ def test_attention_route_of_invalid_shapes(lib):
         assert lib.eng_attn_route(0, *a) == lib.eng_attn_route(1, *a) == 0
 
 
+@pytest.mark.parametrize("B,H,KV,T,DH,parts", [
+    (2, 8, 4, 256, 32, (4, 4, 8)), (1, 4, 1, 300, 64, (4, 4, 8)), (1, 2, 1, 225, 8, (4, 4, 8)), (16, 8, 8, 65, 64, (1, 1, 1)), (1, 8, 8, 16, 64, (1, 1, 1)),
+    # one CTA of a wide head to an SM: none of two for each, unless a walk is long
+    (3, 12, 12, 128, 256, (1, 1, 1)), (4, 8, 4, 100, 256, (1, 1, 2)), (1, 4, 1, 200, 256, (4, 4, 8)), (1, 16, 4, 400, 256, (2, 2, 8)), (8, 8, 2, 64, 256, (1, 1, 4)),
+    # the third CTA of an SM is not worth a single tile
+    (8, 16, 16, 64, 64, (1, 1, 1)), (32, 8, 4, 64, 32, (1, 1, 2))])
+def test_ctas_to_a_walk_of_the_general_attention(lib, B, H, KV, T, DH, parts):
+    assert tuple(lib.eng_attn_share(w, B, H, KV, T, DH) for w in range(3)) == parts
+
+
 def test_cluster_barriers_are_met_by_converged_warps():
     """The aligned forms of the cluster barrier stand in one helper only, behind a __syncwarp(): lanes may come to them from a branch."""
     csrc = os.path.join(ROOT, "axis_b200", "csrc")
