@@ -99,6 +99,8 @@ __device__ __forceinline__ void attn_axpy(float (&acc)[AR][NJ], const float* w, 
 
 // Where rows are few, a cluster of S CTAs takes the tiles that a block of rows walks in turn, and the sums meet through distributed
 // shared memory: a unit is a warp's row of accumulators, [unit][i][thread], and each CTA finishes 1 / S of the units, in rank order.
+// Kernels of their own (SHARE): with S as a value, walks that nobody shares took up to 20 % longer (B1 H8 KV8 T900 DH256,
+// forward and backward: 1350 us so, 1650).
 __device__ __forceinline__ float attn_peer(const float* p, int rank) {
     float x;
     asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %1, %2;\n\tld.shared::cluster.f32 %0, [ra];\n\t}"
@@ -106,10 +108,10 @@ __device__ __forceinline__ float attn_peer(const float* p, int rank) {
     return x;
 }
 
-template <typename T, int NJ>
+template <typename T, int NJ, bool SHARE>
 __global__ void __launch_bounds__(ATH)
 k_attn_fwd_simt(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, T* __restrict__ o,
-                float* __restrict__ lse, AttnShape s, int vec, int S) {
+                float* __restrict__ lse, AttnShape s, int vec, int ctas) {
     extern __shared__ __align__(16) float smem[];
     const int DH = s.DH, LD = attn_ld(DH), q4 = (DH + 3) / 4, TILE = AKT * LD;
     float* Ks = smem;                    // two tiles each
@@ -118,13 +120,13 @@ k_attn_fwd_simt(const T* __restrict__ q, const T* __restrict__ k, const T* __res
     float* Ps = Qs + TILE;               // [warp][key][AR]
     const int b = blockIdx.z, h = blockIdx.y, g = h / (s.H / s.KV);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int part = blockIdx.x % S, r0 = (gridDim.x / S - 1 - blockIdx.x / S) * ABLK, t0 = r0 + warp * AR;      // the longest rows first
+    const int S = SHARE ? ctas : 1, part = SHARE ? blockIdx.x % S : 0, r0 = (gridDim.x / S - 1 - blockIdx.x / S) * ABLK, t0 = r0 + warp * AR;      // the longest rows first
     const T* kbase = k + b * s.kb + g * s.kh;
     const T* vbase = v + b * s.kb + g * s.kh;
     const int ntiles = min(r0 + ABLK - 1, s.T - 1) / AKT + 1;
     pdl_enter();
     attn_tile(Qs, q + b * s.qb + h * s.qh, s.qt, r0, s.T, DH, LD, vec);
-    if (part < ntiles) {
+    if (!SHARE || part < ntiles) {
         attn_tile(Ks, kbase, s.kt, part * AKT, s.T, DH, LD, vec);
         attn_tile(Vs, vbase, s.kt, part * AKT, s.T, DH, LD, vec);
     }
@@ -138,10 +140,10 @@ k_attn_fwd_simt(const T* __restrict__ q, const T* __restrict__ k, const T* __res
     }
     const float* myQ = Qs + warp * AR * LD;
     float* myP = Ps + warp * AKT * AR;
-    for (int kt = part, cur = 0; kt < ntiles; kt += S, cur ^= 1) {
+    for (int kt = part, it = 0; kt < ntiles; kt += S, it++) {
         attn_wait();
         __syncthreads();
-        const int nxt = cur ^ 1;
+        const int cur = it & 1, nxt = cur ^ 1;
         if (kt + S < ntiles) {
             attn_tile(Ks + nxt * TILE, kbase, s.kt, (kt + S) * AKT, s.T, DH, LD, vec);
             attn_tile(Vs + nxt * TILE, vbase, s.kt, (kt + S) * AKT, s.T, DH, LD, vec);
@@ -168,7 +170,7 @@ k_attn_fwd_simt(const T* __restrict__ q, const T* __restrict__ k, const T* __res
         attn_axpy<NJ>(acc, myP, Vs + cur * TILE, LD, DH, lane);
         __syncwarp();
     }
-    if (S > 1) {                         // merge: sums at the largest of the ranks' maxima
+    if (SHARE) {                         // merge: sums at the largest of the ranks' maxima
         attn_wait();
         __syncthreads();
         float* acc_x = smem + threadIdx.x;
@@ -221,11 +223,11 @@ k_attn_fwd_simt(const T* __restrict__ q, const T* __restrict__ k, const T* __res
 }
 
 // dQ: a warp owns AR query rows and walks the keys.
-template <typename T, typename TO, int NJ>
+template <typename T, typename TO, int NJ, bool SHARE>
 __global__ void __launch_bounds__(ATH)
 k_attn_bwd_dq_simt(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
                    const T* __restrict__ dO, const float* __restrict__ lse, const float* __restrict__ Dv,
-                   TO* __restrict__ dq, AttnShape s, int vec, int S) {
+                   TO* __restrict__ dq, AttnShape s, int vec, int ctas) {
     extern __shared__ __align__(16) float smem[];
     const int DH = s.DH, LD = attn_ld(DH), q4 = (DH + 3) / 4, TILE = AKT * LD;
     float* Ks = smem;
@@ -235,14 +237,14 @@ k_attn_bwd_dq_simt(const T* __restrict__ q, const T* __restrict__ k, const T* __
     float* Ps = Gs + TILE;
     const int b = blockIdx.z, h = blockIdx.y, g = h / (s.H / s.KV);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int part = blockIdx.x % S, r0 = (gridDim.x / S - 1 - blockIdx.x / S) * ABLK, t0 = r0 + warp * AR;
+    const int S = SHARE ? ctas : 1, part = SHARE ? blockIdx.x % S : 0, r0 = (gridDim.x / S - 1 - blockIdx.x / S) * ABLK, t0 = r0 + warp * AR;
     const T* kbase = k + b * s.kb + g * s.kh;
     const T* vbase = v + b * s.kb + g * s.kh;
     pdl_enter();
     attn_tile(Qs, q + b * s.qb + h * s.qh, s.qt, r0, s.T, DH, LD, vec);
     attn_tile(Gs, dO + b * s.qb + h * s.qh, s.qt, r0, s.T, DH, LD, vec);
     const int ntiles = min(r0 + ABLK - 1, s.T - 1) / AKT + 1;
-    if (part < ntiles) {
+    if (!SHARE || part < ntiles) {
         attn_tile(Ks, kbase, s.kt, part * AKT, s.T, DH, LD, vec);
         attn_tile(Vs, vbase, s.kt, part * AKT, s.T, DH, LD, vec);
     }
@@ -259,10 +261,10 @@ k_attn_bwd_dq_simt(const T* __restrict__ q, const T* __restrict__ k, const T* __
     const float* myQ = Qs + warp * AR * LD;
     const float* myG = Gs + warp * AR * LD;
     float* myP = Ps + warp * AKT * AR;
-    for (int kt = part, cur = 0; kt < ntiles; kt += S, cur ^= 1) {
+    for (int kt = part, it = 0; kt < ntiles; kt += S, it++) {
         attn_wait();
         __syncthreads();
-        const int nxt = cur ^ 1;
+        const int cur = it & 1, nxt = cur ^ 1;
         if (kt + S < ntiles) {
             attn_tile(Ks + nxt * TILE, kbase, s.kt, (kt + S) * AKT, s.T, DH, LD, vec);
             attn_tile(Vs + nxt * TILE, vbase, s.kt, (kt + S) * AKT, s.T, DH, LD, vec);
@@ -281,7 +283,7 @@ k_attn_bwd_dq_simt(const T* __restrict__ q, const T* __restrict__ k, const T* __
         attn_axpy<NJ>(acc, myP, Ks + cur * TILE, LD, DH, lane);
         __syncwarp();
     }
-    if (S > 1) {
+    if (SHARE) {
         attn_wait();
         __syncthreads();
         float* acc_x = smem + threadIdx.x;
@@ -319,11 +321,11 @@ k_attn_bwd_dq_simt(const T* __restrict__ q, const T* __restrict__ k, const T* __
 
 // dK, dV: a warp owns AR key rows of a kv head and walks the group's query heads and their causal query tiles — this is
 // where the GQA sum happens.
-template <typename T, typename TO, int NJ>
+template <typename T, typename TO, int NJ, bool SHARE>
 __global__ void __launch_bounds__(ATH)
 k_attn_bwd_dkv_simt(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
                     const T* __restrict__ dO, const float* __restrict__ lse, const float* __restrict__ Dv,
-                    TO* __restrict__ dk, TO* __restrict__ dv, AttnShape s, int vec, int S) {
+                    TO* __restrict__ dk, TO* __restrict__ dv, AttnShape s, int vec, int ctas) {
     extern __shared__ __align__(16) float smem[];
     const int DH = s.DH, LD = attn_ld(DH), q4 = (DH + 3) / 4, TILE = AKT * LD;
     float* Qs = smem;                    // two tiles each
@@ -333,7 +335,7 @@ k_attn_bwd_dkv_simt(const T* __restrict__ q, const T* __restrict__ k, const T* _
     float* Ps = Vr + TILE;               // [warp][query][AR]
     const int b = blockIdx.z, g = blockIdx.y, rep = s.H / s.KV;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int part = blockIdx.x % S, r0 = blockIdx.x / S * ABLK, j0 = r0 + warp * AR;       // the first key rows meet the most queries
+    const int S = SHARE ? ctas : 1, part = SHARE ? blockIdx.x % S : 0, r0 = blockIdx.x / S * ABLK, j0 = r0 + warp * AR;       // the first key rows meet the most queries
     const int qt0 = r0 / AKT, nq = (s.T + AKT - 1) / AKT - qt0, n_it = rep * nq;
     pdl_enter();
     attn_tile(Kr, k + b * s.kb + g * s.kh, s.kt, r0, s.T, DH, LD, vec);
@@ -344,7 +346,7 @@ k_attn_bwd_dkv_simt(const T* __restrict__ q, const T* __restrict__ k, const T* _
         attn_tile(Qs + cur * TILE, q + hb, s.qt, t, s.T, DH, LD, vec);
         attn_tile(Gs + cur * TILE, dO + hb, s.qt, t, s.T, DH, LD, vec);
     };
-    if (part < n_it) load(part, 0);
+    if (!SHARE || part < n_it) load(part, 0);
     attn_commit();
     float ak[AR][NJ], av[AR][NJ];
 #pragma unroll
@@ -354,7 +356,8 @@ k_attn_bwd_dkv_simt(const T* __restrict__ q, const T* __restrict__ k, const T* _
     const float* myK = Kr + warp * AR * LD;
     const float* myV = Vr + warp * AR * LD;
     float* myP = Ps + warp * AKT * AR;
-    for (int it = part, cur = 0; it < n_it; it += S, cur ^= 1) {
+    for (int it = part, step = 0; it < n_it; it += S, step++) {
+        const int cur = step & 1;
         const int h = g * rep + it / nq, t = (qt0 + it % nq) * AKT + lane;
         const bool live = t < s.T;
         const float L = live ? lse[((long long)b * s.H + h) * s.T + t] : 0.f;
@@ -382,7 +385,7 @@ k_attn_bwd_dkv_simt(const T* __restrict__ q, const T* __restrict__ k, const T* _
         attn_axpy<NJ>(ak, myP, Qt, LD, DH, lane);
         __syncwarp();
     }
-    if (S > 1) {                         // units: dK rows, then dV rows
+    if (SHARE) {                         // units: dK rows, then dV rows
         attn_wait();
         __syncthreads();
         float* acc_x = smem + threadIdx.x;
@@ -469,26 +472,29 @@ int ax_attn_simt_share(int which, const AttnShape& s) {
     return attn_share((long long)blocks * s.H * s.B, blocks, 4, 3, attn_smem(which, s.DH));
 }
 
+// the kernel of walks that CTAs share, or that of whole ones
 template <typename K, typename... A>
-static int attn_launch(K kern, dim3 grid, size_t smem, int S, cudaStream_t st, A... args) {
+static int attn_launch(K shared, K whole, dim3 grid, size_t smem, int S, cudaStream_t st, A... args) {
     grid.x *= S;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid; cfg.blockDim = dim3(ATH); cfg.dynamicSmemBytes = smem; cfg.stream = st;
     cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = S; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at; cfg.numAttrs = ax_gemm_pdl() ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, kern, args..., S) == cudaSuccess ? 0 : 3;
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = ax_gemm_pdl();
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = S; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
+    cfg.attrs = at; cfg.numAttrs = S > 1 ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, S > 1 ? shared : whole, args..., S) == cudaSuccess ? 0 : 3;
 }
 
 template <typename T, int NJ>
 static int attn_fwd_launch(const void* q, const void* k, const void* v, void* o, float* lse, const AttnShape& s, int vec, cudaStream_t st) {
     const size_t smem = attn_smem(ATTN_FWD, s.DH);
-    if (!attn_smem_ok(smem, k_attn_fwd_simt<T, NJ>)) return 101;
+    const auto shared = k_attn_fwd_simt<T, NJ, true>, whole = k_attn_fwd_simt<T, NJ, false>;
+    const int S = ax_attn_simt_share(ATTN_FWD, s);
+    if (!attn_smem_ok(smem, S > 1 ? shared : whole)) return 101;
     const dim3 grid((s.T + ABLK - 1) / ABLK, s.H, s.B);
-    return attn_launch(k_attn_fwd_simt<T, NJ>, grid, smem, ax_attn_simt_share(ATTN_FWD, s), st, (const T*)q, (const T*)k, (const T*)v, (T*)o, lse, s, vec);
+    return attn_launch(shared, whole, grid, smem, S, st, (const T*)q, (const T*)k, (const T*)v, (T*)o, lse, s, vec);
 }
 template <typename T>
 static int attn_fwd_nj(const void* q, const void* k, const void* v, void* o, float* lse, const AttnShape& s, int vec, cudaStream_t st) {
@@ -509,12 +515,13 @@ template <typename T, typename TO, int NJ>
 static int attn_bwd_launch(const void* q, const void* k, const void* v, const void* dO, const float* lse,
                            const float* Dv, void* dq, void* dk, void* dv, const AttnShape& s, int vec, cudaStream_t st) {
     const size_t smem_q = attn_smem(ATTN_DQ, s.DH), smem_kv = attn_smem(ATTN_DKV, s.DH);
-    if (!attn_smem_ok(smem_q, k_attn_bwd_dq_simt<T, TO, NJ>) || !attn_smem_ok(smem_kv, k_attn_bwd_dkv_simt<T, TO, NJ>)) return 102;
+    const auto q_shared = k_attn_bwd_dq_simt<T, TO, NJ, true>, q_whole = k_attn_bwd_dq_simt<T, TO, NJ, false>;
+    const auto kv_shared = k_attn_bwd_dkv_simt<T, TO, NJ, true>, kv_whole = k_attn_bwd_dkv_simt<T, TO, NJ, false>;
+    const int Sq = ax_attn_simt_share(ATTN_DQ, s), Skv = ax_attn_simt_share(ATTN_DKV, s);
+    if (!attn_smem_ok(smem_q, Sq > 1 ? q_shared : q_whole) || !attn_smem_ok(smem_kv, Skv > 1 ? kv_shared : kv_whole)) return 102;
     const dim3 g1((s.T + ABLK - 1) / ABLK, s.H, s.B), g2((s.T + ABLK - 1) / ABLK, s.KV, s.B);
-    const int rc = attn_launch(k_attn_bwd_dq_simt<T, TO, NJ>, g1, smem_q, ax_attn_simt_share(ATTN_DQ, s), st, (const T*)q, (const T*)k, (const T*)v,
-                               (const T*)dO, lse, Dv, (TO*)dq, s, vec);
-    return rc ? rc : attn_launch(k_attn_bwd_dkv_simt<T, TO, NJ>, g2, smem_kv, ax_attn_simt_share(ATTN_DKV, s), st, (const T*)q, (const T*)k,
-                                 (const T*)v, (const T*)dO, lse, Dv, (TO*)dk, (TO*)dv, s, vec);
+    const int rc = attn_launch(q_shared, q_whole, g1, smem_q, Sq, st, (const T*)q, (const T*)k, (const T*)v, (const T*)dO, lse, Dv, (TO*)dq, s, vec);
+    return rc ? rc : attn_launch(kv_shared, kv_whole, g2, smem_kv, Skv, st, (const T*)q, (const T*)k, (const T*)v, (const T*)dO, lse, Dv, (TO*)dk, (TO*)dv, s, vec);
 }
 template <typename T, typename TO>
 static int attn_bwd_nj(const void* q, const void* k, const void* v, const void* dO, const float* lse,
