@@ -472,15 +472,15 @@ int ax_attn_simt_share(int which, const AttnShape& s) {
     return attn_share((long long)blocks * s.H * s.B, blocks, 4, 3, attn_smem(which, s.DH));
 }
 
-// the kernel of walks that CTAs share, or that of whole ones
+// the kernel of walks that CTAs share, or that of whole ones; early: its CTAs may start before the grid in front of it in the stream has finished
 template <typename K, typename... A>
-static int attn_launch(K shared, K whole, dim3 grid, size_t smem, int S, cudaStream_t st, A... args) {
+static int attn_launch(K shared, K whole, dim3 grid, size_t smem, int S, bool early, cudaStream_t st, A... args) {
     grid.x *= S;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid; cfg.blockDim = dim3(ATH); cfg.dynamicSmemBytes = smem; cfg.stream = st;
     cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = ax_gemm_pdl();
+    at[0].val.programmaticStreamSerializationAllowed = early && ax_gemm_pdl();
     at[1].id = cudaLaunchAttributeClusterDimension;
     at[1].val.clusterDim.x = S; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
     cfg.attrs = at; cfg.numAttrs = S > 1 ? 2 : 1;
@@ -494,7 +494,7 @@ static int attn_fwd_launch(const void* q, const void* k, const void* v, void* o,
     const int S = ax_attn_simt_share(ATTN_FWD, s);
     if (!attn_smem_ok(smem, S > 1 ? shared : whole)) return 101;
     const dim3 grid((s.T + ABLK - 1) / ABLK, s.H, s.B);
-    return attn_launch(shared, whole, grid, smem, S, st, (const T*)q, (const T*)k, (const T*)v, (T*)o, lse, s, vec);
+    return attn_launch(shared, whole, grid, smem, S, true, st, (const T*)q, (const T*)k, (const T*)v, (T*)o, lse, s, vec);
 }
 template <typename T>
 static int attn_fwd_nj(const void* q, const void* k, const void* v, void* o, float* lse, const AttnShape& s, int vec, cudaStream_t st) {
@@ -520,8 +520,11 @@ static int attn_bwd_launch(const void* q, const void* k, const void* v, const vo
     const int Sq = ax_attn_simt_share(ATTN_DQ, s), Skv = ax_attn_simt_share(ATTN_DKV, s);
     if (!attn_smem_ok(smem_q, Sq > 1 ? q_shared : q_whole) || !attn_smem_ok(smem_kv, Skv > 1 ? kv_shared : kv_whole)) return 102;
     const dim3 g1((s.T + ABLK - 1) / ABLK, s.H, s.B), g2((s.T + ABLK - 1) / ABLK, s.KV, s.B);
-    const int rc = attn_launch(q_shared, q_whole, g1, smem_q, Sq, st, (const T*)q, (const T*)k, (const T*)v, (const T*)dO, lse, Dv, (TO*)dq, s, vec);
-    return rc ? rc : attn_launch(kv_shared, kv_whole, g2, smem_kv, Skv, st, (const T*)q, (const T*)k, (const T*)v, (const T*)dO, lse, Dv, (TO*)dk, (TO*)dv, s, vec);
+    const int rc = attn_launch(q_shared, q_whole, g1, smem_q, Sq, true, st, (const T*)q, (const T*)k, (const T*)v, (const T*)dO, lse, Dv, (TO*)dq, s, vec);
+    // dK / dV comes early only as a quarter of a full GPU: the CTAs of its longest walks, the first, would be stacked on the SMs that dQ leaves first
+    // (backward of B4 H8 KV4 T400 DH32 in us, in its turn / early: 130 / 159)
+    const bool early = (long long)g2.x * g2.y * g2.z * Skv * 4 <= attn_slots(smem_kv);
+    return rc ? rc : attn_launch(kv_shared, kv_whole, g2, smem_kv, Skv, early, st, (const T*)q, (const T*)k, (const T*)v, (const T*)dO, lse, Dv, (TO*)dk, (TO*)dv, s, vec);
 }
 template <typename T, typename TO>
 static int attn_bwd_nj(const void* q, const void* k, const void* v, const void* dO, const float* lse,
