@@ -361,7 +361,15 @@ int ax_gemm_tc(int out_bf16, int tb, const void* A, const void* B, void* C, cons
             if (cost < best2 - 1e-9) { best2 = cost; best2_s = sk; }
         }
         double shared;
-        if (!g_side && ax_gemm_tc2_by_tma(C, beta != 0.f ? D : nullptr, n, out_bf16 ? 2 : 4) && ax_gemm_tc2_share((int)tiles2, kblocks, &shared) > 1 && shared * 0.70 < best2) { best2 = shared * 0.70; best2_s = 1; }
+        const int S = !g_side && ax_gemm_tc2_by_tma(C, beta != 0.f ? D : nullptr, n, out_bf16 ? 2 : 4) ? ax_gemm_tc2_share((int)tiles2, kblocks, &shared) : 1;
+        if (S > 1) {
+            // Against a split through the workspace in us, fitted to 60 and 76 shapes (rms 1.0): set-up, k-blocks of a pair, and the sums, which stay in L2.
+            // Split / shared: 1472 x 744 x 7432 25.2 / 32.7, 1368 x 784 x 5264 22.8 / 25.5, 608 x 2304 x 6520 33.0 / 30.3, 760 x 848 x 4464 18.7 / 15.9.
+            const double split_us = 10.3 + 0.38 * ((tiles2 * best2_s + g_pairs_avail - 1) / g_pairs_avail) * ((kblocks + best2_s - 1) / best2_s) +
+                                    1.22e-7 * m * n * ((best2_s + 1) * 4.0 + (out_bf16 ? 2 : 4));
+            const double shared_us = 8.2 + 0.36 * ((kblocks + S - 1) / S) + 0.04 * S * tiles2;
+            if (best2_s == 1 || shared_us < split_us) { best2 = shared * 0.70 < best2 ? shared * 0.70 : best2; best2_s = 1; }
+        }
         if (g_pair_mode == 2 || best2 < best) {
             ax_variant = 0x22 + 0x100 * best2_s;
             const int rc = ax_gemm_tc2(out_bf16, tb, A, B, C, D, m, n, k, alpha, beta, status, best2_s, st);

@@ -915,6 +915,16 @@ def test_depth_is_not_shared_for_rows_that_tma_cannot_store(eng, addend, n, vari
     assert eng.device_status() == 0
 
 
+@pytest.mark.parametrize("m,n,k,tb,dt,variant,parts", [
+    (512, 2168, 6784, 1, 1, 0x422, 1), (1368, 784, 5264, 2, 1, 0x322, 1), (1472, 744, 7432, 1, 2, 0x422, 1),       # split: more pairs at work
+    (1224, 1464, 5240, 1, 1, 0x122, 2), (760, 848, 4464, 1, 1, 0x122, 4)])                                         # shared: no pass over the sums
+def test_deep_products_of_few_tiles_are_split_or_shared(eng, m, n, k, tb, dt, variant, parts):
+    got, ref = run_gemm(eng, np.random.default_rng(m + n), m, n, k, tb, dt, fallback=8)
+    assert (eng.last_variant(), eng.last_gemm_parts()) == (variant, parts)
+    check(got, ref, dt == 1, k)
+    assert eng.device_status() == 0
+
+
 @pytest.mark.parametrize("m,k,ns,r,parts", [(1032, 1352, (512, 264, 136), 16, 2), (520, 1800, (264, 136, 72), 8, 4)])
 def test_grouped_tiles_shared_over_a_cluster(eng, m, k, ns, r, parts):
     """The same for groups: one input and several outputs with a low-rank term each, and one output summed over K-segments."""
