@@ -1,6 +1,6 @@
 // Causal grouped-query attention in bf16 with the probabilities held to 32-bit accuracy, for the shapes that the tcgen05
 // kernels do not take (attn_tc.cu, attn_tc128.cu: whole 128-token tiles of head_dim 64 and 128; attn_tcs.cu: other lengths and head
-// dims from 40 to 64, once there is work for all SMs): [B,T,H,DH] layout, DH a multiple of 8 up to 128, any T.
+// dims from 40 to 64, where there is work for all SMs and the line in that file says so): [B,T,H,DH] layout, DH a multiple of 8 up to 128, any T.
 //
 // The products that take P and dS as an operand need them in bf16, and eight bits are not what fp32 arithmetic on CUDA cores
 // (attn_simt.cu) gives.  Here every P and dS enters as the sum of two bf16 numbers, hi = rn(x) and lo = rn(x - hi), in two MMAs
@@ -11,9 +11,9 @@
 //
 // A warp owns 16 rows (queries, or keys in the dK / dV kernel) and walks the other operand in steps of 32 rows; P and dS stay in
 // registers, where the accumulator layout of one mma.sync is the operand layout of the next.  On tcgen05
-// two 128-column accumulators leave no TMEM to double the scores of the dK / dV kernel (head_dim above 64), and a tile of 64 columns is
-// half empty for heads up to 32.  Bound by issue and by MMA latency: the MMA pipe (555 TFLOP/s by itself) is busy 44 / 56 / 50 % of the active cycles in
-// the forward, dQ and dK / dV kernels (B3 H24 KV8 T1000 DH64), and the schedulers issue in half of all cycles (exponentials, splits,
+// a tile of 64 columns is half empty for heads up to 32.  Heads above 64 have no such kernel yet: dV and dK of 128 columns and two S^T and dP^T of 64 each
+// would fill TMEM, with K and V read from shared memory by the score products.  Bound by issue and by MMA latency: the MMA pipe (555 TFLOP/s by itself) is busy 49 / 57 / 52 % of the active cycles in
+// the forward, dQ and dK / dV kernels (B2 H16 KV16 T1500 DH128: 119, 143 and 214 us), and the schedulers issue in 43 / 36 / 33 % of them (exponentials, splits,
 // operand reads).  Times in us, forward / backward with the row dots,
 // CUDA cores -> here (for comparison: tcgen05 with 8-bit P and dS; the first two and their like now run on attn_tcs.cu):
 //   B3 H24 KV8 T1000 DH64    628 / 2080 ->  70 / 203   (31 / 77)      B4 H24 KV8 T500 DH64   247 / 790 ->  33 / 102   (21 / 51)

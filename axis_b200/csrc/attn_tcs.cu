@@ -15,8 +15,8 @@
 //   dK / dV   CTA: 128 keys of a kv head, 64 queries a step; K and V in TMEM, S^T and dP^T doubled (448 columns), P^T and dS^T in
 //             place; issuing warps for the scores, dV and dK, sixteen softmax warps in two groups that take the steps in turn
 //
-// Bound by the softmax warps: the schedulers issue in 37 % (forward) and 46 % (dK / dV) of the cycles, the XU pipe (exponentials) is busy
-// 37 % and 23 %; what is left of a step is the round trip MMA -> TMEM load -> MMA, which two CTAs or two groups cover in part.
+// Bound by the softmax warps: the schedulers issue in 37 % (forward), 38 % (dQ) and 46 % (dK / dV) of the cycles, the XU pipe (exponentials) is busy
+// 37, 30 and 25 % (B3 H24 KV8 T1000 DH64: 34, 42 and 66 us); what is left of a step is the round trip MMA -> TMEM load -> MMA, which two CTAs or two groups cover in part.
 // Forward / backward with the row dots in us, mma.sync -> here (one cold launch each): B3 H24 KV8 T1000 DH64 70 / 203 -> 36 / 106,
 // B4 H24 KV8 T500 DH64 33 / 102 -> 22 / 60, B1 H12 KV4 T2500 DH64 88 / 225 -> 46 / 137, B8 H24 KV8 T320 DH64 29 / 85 -> 25 / 52.
 #include "common.cuh"
