@@ -691,7 +691,8 @@ static bool forward_here(const AttnShape& s) {
 // (kv heads as heads, up to 64 rows: 192 heads T20 12.4 / 18.6, 384 heads T64 18.5 / 27.7), two do while all of them are at work at
 // once (144 heads T65 24.1 / 16.5 and 296 heads T65 26.0 / 24.7, but 608 heads T65 45.2 / 51.1 and 384 heads T129 53.4 / 59.5).  And up to
 // two steps an SM the kernels there have SMs to spare as long as their 64-row tiles are few and the walks short: 8 heads KV 4 T500 28.8 / 30.9, 16
-// heads KV 8 T384 26.9 / 28.8, but 16 heads KV 2 T384 43.1 / 37.0, 8 heads KV 8 T640 36.9 / 32.9, 64 heads T129 24.7 / 18.6.
+// heads KV 8 T384 26.9 / 28.8, but 16 heads KV 2 T384 43.1 / 37.0, 8 heads KV 8 T640 36.9 / 32.9, 64 heads T129 24.7 / 18.6 (just
+// above the line 48 heads KV 16 T129 lose: 20.7 / 22.8).
 static long long steps(const AttnShape& s) {
     const long long tiles = (s.T + XT - 1) / XT, nq = (s.T + XQ - 1) / XQ;
     return s.B * s.H * (tiles * nq - tiles * (tiles - 1));

@@ -13,7 +13,8 @@
 //   0x26 small-product kernel (single or grouped), 0x23 grouped launch of the paired-CTA kernel,
 //   0x24 / 0x27 SwiGLU backward inside the product that makes dh on the small-product / the paired-CTA kernel,
 //   0x25 / 0x28 SwiGLU inside a projection pair with adapters on the same two,
-//   0x70 embedding scatter by scanning the ids, 0x71 by occurrence lists, 0x72 scale and add as one pass
+//   0x70 embedding scatter by scanning the ids, 0x71 by occurrence lists, 0x72 scale and add as one pass, 0x73 with the norm,
+//   0x80 / 0x81 attention forward / backward with split probabilities on tcgen05, 0x82 / 0x83 on mma.sync (0x83 + 0x100 * CTAs to a key tile)
 extern int ax_variant;
 extern int ax_gemm_parts;     // see eng_last_gemm_parts
 
