@@ -134,6 +134,7 @@ __device__ __forceinline__ void tc_commit2_e(uint32_t bar, uint16_t mask) {
 // 6.6 for 904 x 1704 x 128.
 struct GemmGroup {
     int mode, count;
+    int band;                // row tiles that are walked together, column by column (see band_of)
     int S;                   // pairs that share a tile's depth (1: a pair has tiles of its own)
     int n[3];
     int kb[6];
@@ -216,7 +217,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
         num_tiles = 0;
         for (int q = 0; q < grp.count; q++) num_tiles += ((grp.m[q] + 2 * BM2 - 1) / (2 * BM2)) * ((grp.n[q] + BN2 - 1) / BN2);
     }
-    // tile index -> problem g, row tile tm and column tile tl inside it (row tiles fastest)
+    // tile index -> problem g, row tile tm and column tile tl inside it (row tiles of a band fastest, bands slowest)
     auto locate = [&](int tile, int& tm, int& tl) -> int {
         int q = 0;
         if (grp.mode == 3) {
@@ -230,8 +231,11 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
             tm = tile % tmq; tl = tile / tmq;
             return q;
         }
-        tm = tile % tiles_m;
-        int tn = tile / tiles_m;
+        const int per = grp.band * tiles_n, b0 = tile / per * grp.band;
+        tile -= b0 * tiles_n;
+        const int rows = min(grp.band, tiles_m - b0);
+        tm = b0 + tile % rows;
+        int tn = tile / rows;
         if (grp.mode == 1)
             for (; q + 1 < grp.count; q++) { const int tq = (grp.n[q] + BN2 - 1) / BN2; if (tn < tq) break; tn -= tq; }
         tl = tn;
@@ -761,6 +765,17 @@ bool ax_gemm_tc2_by_tma(const void* C, const void* D, long long n, int osz) {
     return ax_gemm_tma_out() && ((uintptr_t)C & 15) == 0 && ((uintptr_t)D & 15) == 0 && n * osz % 16 == 0;
 }
 
+// Row tiles of a band.  74 pairs work on as many tiles at once.  While A stays in the L2 (126 MB, shared with B and the output), walking down
+// all row tiles of a column reads A and B from memory once; when it does not, every two or three columns read all of A again, and a block of
+// about 12 x 6 tiles reads the least.  us with one band / with bands of 12, by MB of A: 8192 x 4096 x 11008 (180) 575 / 545, 8192 x 32000 x 4096
+// (67) 1610 / 1470, 8192 x 2 * 11008 x 4096 (67) 1225 / 1145, 32000 x 4096 x 8192 (524) 1944 / 1730, 50000 x 1536 x 3000 (300) 480 / 410,
+// 8192 x 4096 x 3072 (50) 161 / 158; but 8192 x 32000 x 2048 (34) 770 / 805 and 6144 x 32000 x 3072 (38) 844 / 867, where bands read B again.
+// Bands of 8 and 16 differ from 12 by 1 % either way.
+static int band_of(int m, long long k) {
+    const int tiles_m = (m + 255) / 256;
+    return 2ll * m * k > 52000000ll && tiles_m > 12 ? 12 : tiles_m;
+}
+
 struct SwbArgs { const void* g; const void* u; void* du; };    // SwiGLU backward in the epilogue (C = dg)
 
 // One launch.  grp.mode 0: the plain GEMM (A, B, C, D are element 0 of the arrays).  Grouped modes: see GemmGroup;
@@ -880,6 +895,7 @@ static int gemm2_launch(int mode, int count, const void* const* A, const void* c
         if (mode != 4 && !swb && (!per_problem_c || g >= count || !tma_out)) tmC[g] = tmC[0];
     }
     const int pairs = units < maxp ? units : maxp;
+    grp.band = band_of(m, mode == 2 ? (long long)kb * BK2 : k);
     ax_gemm_parts = grp.S;
     size_t wsb = 0;
     float* ws = ax_splitk_ws(&wsb);

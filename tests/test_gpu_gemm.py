@@ -952,3 +952,12 @@ def test_grouped_tiles_shared_over_a_cluster(eng, m, k, ns, r, parts):
     assert eng.last_gemm_parts() == 4
     check(eng.download_bf16(c, (m, n)), sum(a @ b.T for a, b in zip(As, Bt)) + D, True, sum(ks))
     assert eng.device_status() == 0
+
+
+@pytest.mark.parametrize("m,n,k,tb,dt", [(3336, 776, 7816, 0, 1), (3128, 520, 8320, 1, 1), (6408, 264, 4104, 2, 2), (3072, 520, 8512, 2, 2)])
+def test_tall_products_walk_their_tiles_in_bands(eng, m, n, k, tb, dt):
+    """A above 52 MB: bands of twelve row tiles, the last one of two, one, two and twelve; every tile of the output is written once."""
+    assert 2 * m * k > 52000000
+    got, ref = run_gemm(eng, np.random.default_rng(m + n), m, n, k, tb, dt, fallback=8)
+    check(got, ref, dt == 1, k)
+    assert eng.device_status() == 0
