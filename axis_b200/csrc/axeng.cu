@@ -486,6 +486,20 @@ static int do_lora_proj(const EngOp* op) {
     return 0;
 }
 
+// whether the first xb bytes of buffer x and the first yb of y have none in common
+static bool apart(int x, long long xb, int y, long long yb) {
+    const char* p = (const char*)BUFP(x); const char* q = (const char*)BUFP(y);
+    return p + xb <= q || q + yb <= p;
+}
+// A group as one launch reads and writes in no order: its outputs lie apart from its inputs and from one another, or its members run one by one.
+static bool group_apart(const int* in, const long long* inb, int nin, const int* out, const long long* outb, int nout) {
+    for (int o = 0; o < nout; o++) {
+        for (int i = 0; i < nin; i++) if (!apart(out[o], outb[o], in[i], inb[i])) return false;
+        for (int q = 0; q < o; q++) if (!apart(out[o], outb[o], out[q], outb[q])) return false;
+    }
+    return true;
+}
+
 static int do_gemm_group(const EngOp* op) {
     const int count = op->batch, mode = op->oc;
     const auto xs = g_xseg;                   // consumed by this op whatever happens
@@ -506,6 +520,15 @@ static int do_gemm_group(const EngOp* op) {
             const int rc = ax_gemm_tc2_group(1, 0, 4, 2, A, B, C, &op->m, &op->n, &op->k, alpha, G.d_status, G.cur);
             if (rc == 0) { G.launches++; return 0; }
             if (rc > 0) { set_err("fused SwiGLU gemm failed rc=%d: %s", rc, cudaGetErrorString(cudaGetLastError())); return rc; }
+        }
+        if (dt4 == 0 && op->tb == 0 && !(G.fallback & 5)) {
+            const int in[3] = {op->a, op->b, op->sa}, out[3] = {op->c, op->d, op->sc};
+            const long long kn = (long long)op->k * op->n * 4, ib[3] = {(long long)op->m * op->k * 4, kn, kn}, ob[3] = {mn * 4, mn * 4, mn * 4};
+            const void* A[1] = {BUFP(op->a)}; const void* B[2] = {BUFP(op->b), BUFP(op->sa)};
+            void* C[3] = {BUFP(op->c), BUFP(op->d), BUFP(op->sc)};
+            const int rc = group_apart(in, ib, 3, out, ob, 3) ? ax_gemm_f32_group(0, 4, 2, A, B, C, &op->m, &op->n, &op->k, op->alpha == 0.f ? 1.f : op->alpha,
+                                                                                nullptr, 0.f, nullptr, nullptr, nullptr, G.cur) : -1;
+            if (rc >= 0) { G.launches++; ax_variant = 0x29; return rc; }
         }
         // unfused: two GEMMs and the activation kernel
         EngOp g1 = *op; g1.kind = ENG_GEMM_SB; g1.batch = 1; g1.sa = g1.sb = g1.sc = 0; g1.oa = g1.ob = g1.oc = 0; g1.d = -1; g1.beta = 0.f;
@@ -579,7 +602,36 @@ static int do_gemm_group(const EngOp* op) {
         if (rc == 0) { G.launches++; return 0; }
         if (rc > 0) { set_err("grouped tensor-core gemm failed rc=%d: %s", rc, cudaGetErrorString(cudaGetLastError())); return rc; }
     }
-    for (int g = 0; g < nsub; g++) {
+    bool grouped = false;
+    if (dt == 0 && (mode == 1 ? xs.n == 0 : mode == 2) && !(G.fallback & 5)) {
+        int in[13], out[6], mv[6], nv[6], kv[6];
+        long long ib[13], ob[6];
+        const void* A[6]; const void* B[6]; void* C[6];
+        bool bad = false;
+        const int nout = mode == 2 ? 1 : nsub;
+        int nin = 0;
+        for (int g = 0; g < nsub; g++) {
+            const EngOp* q = &sub[g];
+            NEED(q->a, (long long)q->m * q->k * 4); NEED(q->b, (long long)q->k * q->n * 4); NEED(q->c, (long long)q->m * q->n * 4);
+            in[nin] = q->a; ib[nin++] = (long long)q->m * q->k * 4;
+            in[nin] = q->b; ib[nin++] = (long long)q->k * q->n * 4;
+            out[g] = q->c; ob[g] = (long long)q->m * q->n * 4;
+            A[g] = BUFP(q->a); B[g] = BUFP(q->b); C[g] = BUFP(q->c); mv[g] = q->m; nv[g] = q->n; kv[g] = q->k;
+            bad = bad || q->m < 1 || q->n < 1 || q->k < 1;
+        }
+        const void* D = nullptr;
+        if (mode == 2 && xs.addend) {
+            NEED(xs.addend, ob[0]);
+            D = BUFP(xs.addend);
+            if (D != C[0]) { in[nin] = xs.addend; ib[nin++] = ob[0]; }       // (an addend that the sum replaces is read where it is written)
+        }
+        if (!bad && group_apart(in, ib, nin, out, ob, nout)) {
+            const int rc = ax_gemm_f32_group(op->tb, mode, nsub, A, B, C, mv, nv, kv, op->alpha == 0.f ? 1.f : op->alpha, D, xs.beta, nullptr, nullptr, nullptr, G.cur);
+            if (rc > 0) return rc;
+            if (rc == 0) { G.launches++; ax_variant = 0x29; grouped = true; }
+        }
+    }
+    for (int g = 0; g < nsub && !grouped; g++) {
         int rc = do_gemm(&sub[g], sub[g].kind == ENG_GEMM_EX);
         if (!rc && mode == 1 && g < xs.n) rc = do_gemm(&xsub[g], false);
         if (rc) return rc;
@@ -1083,48 +1135,45 @@ static int run_fused(const EngOp* ops, int n_ops, int i, int* last) {
         return ax_add_scaled((const float*)x, (const float*)g, (float*)BUFP(s->c), op->alpha, n, G.cur);
     }
     const bool group = op->kind == ENG_GEMM_GROUP;
-    if ((op->kind != ENG_GEMM_SB && !group) || op->dt != 1 || (G.fallback & 5) || G.cur != G.stream || i + 1 >= n_ops) return -1;
-    const long long mn = (long long)op->m * op->n;
-    if (op->m < 256 || op->n < 256) return -1;
+    if ((op->kind != ENG_GEMM_SB && !group) || op->dt > 1 || op->dt < 0 || (G.fallback & 5) || G.cur != G.stream || i + 1 >= n_ops) return -1;
+    const long long mn = (long long)op->m * op->n, es = esz(op->dt);
+    if (op->dt == 1 ? op->m < 256 || op->n < 256 : op->m < 1 || op->n < 1) return -1;
     const float alpha = op->alpha == 0.f ? 1.f : op->alpha;
-    auto apart = [](int x, long long xb, int y, long long yb) {
-        const char* p = (const char*)BUFP(x); const char* q = (const char*)BUFP(y);
-        return p + xb <= q || q + yb <= p;
-    };
     const auto xs = g_xseg;
     if (op->tb == 1 && (group ? op->oc == 2 : true)) {
         int j = i + 1;
         while (j < n_ops && ops[j].kind == ENG_EVENT && ops[j].tb == 2 && ops[j].sa == 0) j++;
         if (j >= n_ops) return -1;
         const EngOp* s = &ops[j];
-        if (s->kind != ENG_SILU_BWD || s->oa != 1 || s->dt != 1 || s->d != op->c || (long long)s->n != mn) return -1;
+        if (s->kind != ENG_SILU_BWD || s->oa != 1 || s->dt != op->dt || s->d != op->c || (long long)s->n != mn) return -1;
         if (group ? (op->batch < 1 || op->batch > 3 || xs.addend) : (op->batch > 1 || op->oa || op->ob || op->oc || op->beta != 0.f)) return -1;
         int a[6] = {op->a, op->sa, op->sb}, b[6] = {op->b, op->d, op->sc}, k[6] = {op->k, op->oa, op->ob};
         int ns = group ? op->batch : 1;
         if (group) for (int g = 0; g < xs.n; g++, ns++) { a[ns] = xs.a[g]; b[ns] = xs.b[g]; k[ns] = xs.k; }
         const void* A[6]; const void* B[6]; void* C[6]; int mv[6], nv[6];
         const int out[2] = {s->c, s->tb};
-        if (!have(out[0], mn * 2) || !have(out[1], mn * 2) || !have(s->a, mn * 2) || !have(s->b, mn * 2) || !apart(out[0], mn * 2, out[1], mn * 2)) return -1;
+        if (!have(out[0], mn * es) || !have(out[1], mn * es) || !have(s->a, mn * es) || !have(s->b, mn * es) || !apart(out[0], mn * es, out[1], mn * es)) return -1;
         for (int o = 0; o < 2; o++)
-            if (!apart(out[o], mn * 2, s->a, mn * 2) || !apart(out[o], mn * 2, s->b, mn * 2)) return -1;
+            if (!apart(out[o], mn * es, s->a, mn * es) || !apart(out[o], mn * es, s->b, mn * es)) return -1;
         for (int g = 0; g < ns; g++) {
-            if (k[g] < 1 || !have(a[g], (long long)op->m * k[g] * 2) || !have(b[g], (long long)op->n * k[g] * 2)) return -1;
+            if (k[g] < 1 || !have(a[g], (long long)op->m * k[g] * es) || !have(b[g], (long long)op->n * k[g] * es)) return -1;
             for (int o = 0; o < 2; o++)
-                if (!apart(out[o], mn * 2, a[g], (long long)op->m * k[g] * 2) || !apart(out[o], mn * 2, b[g], (long long)op->n * k[g] * 2)) return -1;
+                if (!apart(out[o], mn * es, a[g], (long long)op->m * k[g] * es) || !apart(out[o], mn * es, b[g], (long long)op->n * k[g] * es)) return -1;
             A[g] = BUFP(a[g]); B[g] = BUFP(b[g]); C[g] = BUFP(out[0]); mv[g] = op->m; nv[g] = op->n;
         }
         for (int e = i + 1; e < j; e++) { const int rc = exec_op(&ops[e]); if (rc) return rc; }
-        const int rc = ax_gemm_tc2_group(1, 1, 2, ns, A, B, C, mv, nv, k, alpha, G.d_status, G.cur, nullptr, nullptr, 0, nullptr, 0.f,
-                                         BUFP(s->a), BUFP(s->b), BUFP(out[1]));
+        const int rc = op->dt == 0 ? ax_gemm_f32_group(1, 2, ns, A, B, C, mv, nv, k, alpha, nullptr, 0.f, BUFP(s->a), BUFP(s->b), BUFP(out[1]), G.cur)
+                                   : ax_gemm_tc2_group(1, 1, 2, ns, A, B, C, mv, nv, k, alpha, G.d_status, G.cur, nullptr, nullptr, 0, nullptr, 0.f,
+                                                       BUFP(s->a), BUFP(s->b), BUFP(out[1]));
         if (rc < 0) return -1;
         if (rc > 0) { set_err("fused SwiGLU backward failed rc=%d: %s", rc, cudaGetErrorString(cudaGetLastError())); return rc; }
         if (group) g_xseg = {};                  // a plain product leaves pending segments to the group that follows
         G.launches++;
-        ax_variant = ax_variant == 0x26 ? 0x24 : 0x27;
+        ax_variant = op->dt == 0 ? 0x2a : ax_variant == 0x26 ? 0x24 : 0x27;
         *last = j;
         return 0;
     }
-    if (group && op->tb == 0 && op->oc == 1 && op->batch == 2 && op->oa == op->n && op->gamma <= 0.f && xs.n == 2 && !xs.addend) {
+    if (op->dt == 1 && group && op->tb == 0 && op->oc == 1 && op->batch == 2 && op->oa == op->n && op->gamma <= 0.f && xs.n == 2 && !xs.addend) {
         const EngOp* s = &ops[i + 1];
         if (s->kind != ENG_SILU_MUL || s->dt != 1 || s->a != op->c || s->b != op->d || (long long)s->n != mn) return -1;
         const int in[7] = {op->a, op->b, op->sa, xs.a[0], xs.a[1], xs.b[0], xs.b[1]}, out[3] = {op->c, op->d, s->c};

@@ -82,7 +82,7 @@ k_gemm_simt(const TI* __restrict__ A, const TI* __restrict__ B, TO* C, const TO*
 // product of 512 x 256 x 256 is 32 tiles of 64 x 64 for 148 SMs, and a tile that walks its depth one 16-deep step after
 // another pays a memory round trip per step.  So
 //   * the depth travels in steps of 64 through a ring of cp.async stages that is filled before the first FMA;
-//   * small tiles (32 x 32) cut every step among four groups of 64 threads;
+//   * small tiles (64 x 32, 32 x 32) cut every step among four groups of 64 threads;
 //   * where the tiles still leave SMs idle, a cluster of 2, 4 or 8 CTAs cuts the depth once more and adds its partial
 //     tiles through distributed shared memory.
 // 512 x 256 x 256, one cold launch: 46 us with 64 x 64 tiles, 16-deep steps and no prefetch, 7 us now; 512 x 512 x 256: 11 us.
@@ -119,28 +119,59 @@ struct F32Tile {
     static constexpr int EL = ST * (A_EL + B_EL) > RED ? ST * (A_EL + B_EL) : RED;
     static constexpr int SMEM = EL * 4;
 };
-template <int BM, int BN, int BK, int KG, int TM, int TN, int ST, bool A_MN, bool B_KM, bool VEC>
+// What one launch computes: up to three problems of one A-shape (their column tiles form one tile space), each the sum of its `nseg` segments
+// seg[g * nseg ...]; the plain product is one problem of one segment.  A group is latency like a product of its size, its members one
+// after the other are that many times as much.  With the tiles of `f32_gemm` the step of a 256-wide model of four layers, 512 tokens, takes 857 us
+// in place of 987 (58 products of it had launches of their own, four activations and their backward too).
+//   F32_SWIGLU: B and B2 are the gate and up weights; a tile holds BN / 2 columns of either; C = g, u, silu(g) * u
+//   F32_SWB: the product is dh of h = silu(g) * u and stays in registers; C = dg, du
+enum { F32_PLAIN, F32_SWIGLU, F32_SWB };
+struct F32Seg { const float* A; const float* B; const float* B2; int k; };
+struct F32Group {
+    F32Seg seg[6];
+    int nprob, nseg, n[3];
+    float* C[3];
+    const float* D;             // addend (one problem)
+    const float* G; const float* U;
+};
+template <int BM, int BN, int BK, int KG, int TM, int TN, int ST, bool A_MN, bool B_KM, bool VEC, int EPI>
 __global__ void __launch_bounds__(KG * (BM / TM) * (BN / TN))
-k_gemm_f32(const float* __restrict__ A, const float* __restrict__ B, float* C, const float* D, int m, int n, int k,
-           long long sa, long long sb, long long sc, int ksplit, float alpha, float beta) {
+k_gemm_f32(const __grid_constant__ F32Group a, int m, long long sa, long long sb, long long sc, int ksplit, float alpha, float beta) {
     using L = F32Tile<BM, BN, BK, KG, TM, TN, ST, A_MN, B_KM>;
-    constexpr int TH = L::THREADS, TX = BN / TN, TY = BM / TM, GT_ = TX * TY, KS = BK / KG;
+    constexpr int TH = L::THREADS, TX = BN / TN, TY = BM / TM, GT_ = TX * TY, KS = BK / KG, W = EPI == F32_SWIGLU ? BN / 2 : BN;
     extern __shared__ __align__(16) float sm[];
     pdl_enter();
-    const int bz = blockIdx.z;
-    A += (long long)bz * sa; B += (long long)bz * sb; C += (long long)bz * sc;
-    if (D) D += (long long)bz * sc;
-    const int split = blockIdx.x % ksplit, i0 = blockIdx.y * BM, j0 = (blockIdx.x / ksplit) * BN;
-    const int steps_all = (k + BK - 1) / BK, per = (steps_all + ksplit - 1) / ksplit;
+    const int split = blockIdx.x % ksplit, i0 = blockIdx.y * BM;
+    int tn = blockIdx.x / ksplit, g = 0;
+    for (; g + 1 < a.nprob; g++) {
+        const int t = (a.n[g] + W - 1) / W;
+        if (tn < t) break;
+        tn -= t;
+    }
+    const int n = a.n[g], j0 = tn * W;
+    const F32Seg* seg = a.seg + g * a.nseg;
+    const long long oa = blockIdx.z * sa, ob = blockIdx.z * sb, oc = blockIdx.z * sc;
+    float* C = a.C[g] + oc;
+    const float* D = a.D ? a.D + oc : nullptr;
+    int steps_all = 0;
+    for (int q = 0; q < a.nseg; q++) steps_all += (seg[q].k + BK - 1) / BK;
+    const int per = (steps_all + ksplit - 1) / ksplit;
     const int s0 = split * per, s1 = min(steps_all, s0 + per), steps = max(s1 - s0, 0);
     const int grp = threadIdx.x / GT_, tid = threadIdx.x % GT_, ty = tid / TX, tx = tid % TX;
-    auto load = [&](int st) {
-        float* as = sm + (st % ST) * (L::A_EL + L::B_EL);
+    int ls = 0, lk = s0;                                  // next step to load: segment and step inside it
+    auto load = [&](int slot) {
+        while (ls + 1 < a.nseg && lk >= (seg[ls].k + BK - 1) / BK) lk -= (seg[ls++].k + BK - 1) / BK;
+        float* as = sm + slot * (L::A_EL + L::B_EL);
         float* bs = as + L::A_EL;
-        const int k0 = (s0 + st) * BK;
+        const int k = seg[ls].k, k0 = lk++ * BK;
+        const float* A = seg[ls].A + oa; const float* B = seg[ls].B + ob;
         if (A_MN) tile_cp<BK, BM, L::AP, VEC, TH>(as, A, m, k0, i0, k, m);
         else tile_cp<BM, BK, L::AP, VEC, TH>(as, A, k, i0, k0, m, k);
-        if (B_KM) tile_cp<BN, BK, L::BP, VEC, TH>(bs, B, k, j0, k0, n, k);
+        if constexpr (EPI == F32_SWIGLU) {
+            tile_cp<BK, BN / 2, L::BP, VEC, TH>(bs, B, n, k0, j0, k, n);
+            tile_cp<BK, BN / 2, L::BP, VEC, TH>(bs + BN / 2, seg[ls].B2, n, k0, j0, k, n);
+        }
+        else if (B_KM) tile_cp<BN, BK, L::BP, VEC, TH>(bs, B, k, j0, k0, n, k);
         else tile_cp<BK, BN, L::BP, VEC, TH>(bs, B, n, k0, j0, k, n);
     };
     float acc[TM][TN];
@@ -159,7 +190,7 @@ k_gemm_f32(const float* __restrict__ A, const float* __restrict__ B, float* C, c
     for (int st = 0; st < steps; st++) {
         asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
         __syncthreads();                                  // stage st has landed and everyone has left stage st - 1
-        if (st + ST - 1 < steps) load(st + ST - 1);
+        if (st + ST - 1 < steps) load((st + ST - 1) % ST);
         asm volatile("cp.async.commit_group;" ::: "memory");
         const float* as = sm + (st % ST) * (L::A_EL + L::B_EL);
         const float* bs = as + L::A_EL;
@@ -206,7 +237,11 @@ k_gemm_f32(const float* __restrict__ A, const float* __restrict__ B, float* C, c
 #pragma unroll
     for (int p = 0; p < TM; p++)
 #pragma unroll
-        for (int q = 0; q < TN; q++) red[row_of(p) * RP + col_of(q)] = acc[p][q];
+        for (int q = 0; q < TN; q += B_KM ? 1 : 4) {
+            float* at = red + row_of(p) * RP + col_of(q);
+            if (B_KM) *at = acc[p][q];
+            else *reinterpret_cast<float4*>(at) = make_float4(acc[p][q], acc[p][q + (B_KM ? 0 : 1)], acc[p][q + (B_KM ? 0 : 2)], acc[p][q + (B_KM ? 0 : 3)]);
+        }
     __syncthreads();
     if (ksplit > 1) {
         if (KG > 1) {                                     // this CTA's groups first, so that peers read one tile
@@ -224,9 +259,7 @@ k_gemm_f32(const float* __restrict__ A, const float* __restrict__ B, float* C, c
     const int rows = ksplit > 1 ? BM / ksplit : BM, rb = ksplit > 1 ? split * rows : 0;
     const uint32_t smb = (uint32_t)__cvta_generic_to_shared(sm);
     const bool v4 = VEC && (n & 3) == 0;
-    for (int e = threadIdx.x; e < rows * (BN / 4); e += TH) {
-        const int r = rb + e / (BN / 4), c = e % (BN / 4) * 4;
-        const int gi = i0 + r, gj = j0 + c;
+    auto total = [&](int r, int c, float* f) {            // four columns of the tile's sum, times alpha
         float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
         if (ksplit > 1) {
             for (int q = 0; q < ksplit; q++) {            // in rank order
@@ -238,24 +271,55 @@ k_gemm_f32(const float* __restrict__ A, const float* __restrict__ B, float* C, c
             }
         } else {
 #pragma unroll
-            for (int g = 0; g < KG; g++) {
-                const float4 v = *reinterpret_cast<const float4*>(sm + g * BM * RP + r * RP + c);
+            for (int q = 0; q < KG; q++) {
+                const float4 v = *reinterpret_cast<const float4*>(sm + q * BM * RP + r * RP + c);
                 t.x += v.x; t.y += v.y; t.z += v.z; t.w += v.w;
             }
         }
-        if (gi >= m || gj >= n) continue;
-        const long long idx = (long long)gi * n + gj;
-        float f[4] = {alpha * t.x, alpha * t.y, alpha * t.z, alpha * t.w};
-        if (v4) {
-            if (beta != 0.f) {
-                const float4 d = *reinterpret_cast<const float4*>(D + idx);
-                f[0] += beta * d.x; f[1] += beta * d.y; f[2] += beta * d.z; f[3] += beta * d.w;
-            }
-            *reinterpret_cast<float4*>(C + idx) = make_float4(f[0], f[1], f[2], f[3]);
+        f[0] = alpha * t.x; f[1] = alpha * t.y; f[2] = alpha * t.z; f[3] = alpha * t.w;
+    };
+    auto put = [&](float* dst, long long idx, int gj, const float* f) {
+        if (v4) *reinterpret_cast<float4*>(dst + idx) = make_float4(f[0], f[1], f[2], f[3]);
+        else for (int q = 0; q < 4 && gj + q < n; q++) dst[idx + q] = f[q];
+    };
+    auto get = [&](const float* src, long long idx, int gj, float* f) {
+        if (v4) { const float4 v = *reinterpret_cast<const float4*>(src + idx); f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w; }
+        else for (int q = 0; q < 4; q++) f[q] = gj + q < n ? src[idx + q] : 0.f;
+    };
+    for (int e = threadIdx.x; e < rows * (W / 4); e += TH) {
+        const int r = rb + e / (W / 4), c = e % (W / 4) * 4;
+        const int gi = i0 + r, gj = j0 + c;
+        float f[4];
+        total(r, c, f);
+        if constexpr (EPI == F32_SWIGLU) {
+            float u[4], h[4];
+            total(r, c + W, u);
+            if (gi >= m || gj >= n) continue;
+            const long long idx = (long long)gi * n + gj;
+#pragma unroll
+            for (int q = 0; q < 4; q++) h[q] = f[q] / (1.f + expf(-f[q])) * u[q];
+            put(a.C[0], idx, gj, f); put(a.C[1], idx, gj, u); put(a.C[2], idx, gj, h);
         } else {
-            for (int q = 0; q < 4 && gj + q < n; q++) {
-                if (beta != 0.f) f[q] += beta * D[idx + q];
-                C[idx + q] = f[q];
+            if (gi >= m || gj >= n) continue;
+            const long long idx = (long long)gi * n + gj;
+            float d[4];
+            if constexpr (EPI == F32_SWB) {
+                float x[4], o[4];
+                get(a.G, idx, gj, x); get(a.U, idx, gj, d);
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const float sig = 1.f / (1.f + expf(-x[q]));
+                    o[q] = f[q] * d[q] * (sig * (1.f + x[q] * (1.f - sig)));
+                    f[q] *= x[q] * sig;
+                }
+                put(a.C[0], idx, gj, o); put(a.C[1], idx, gj, f);
+            } else {
+                if (beta != 0.f) {
+                    get(D, idx, gj, d);
+#pragma unroll
+                    for (int q = 0; q < 4; q++) f[q] += beta * d[q];
+                }
+                put(C, idx, gj, f);
             }
         }
     }
@@ -263,15 +327,17 @@ k_gemm_f32(const float* __restrict__ A, const float* __restrict__ B, float* C, c
         cluster_sync();
 }
 
-template <int BM, int BN, int BK, int KG, int TM, int TN, int ST, bool A_MN, bool B_KM, bool VEC>
-static int f32_launch(const float* A, const float* B, float* C, const float* D, int m, int n, int k, int batch,
-                      long long sa, long long sb, long long sc, int ksplit, float alpha, float beta, cudaStream_t st) {
+template <int BM, int BN, int BK, int KG, int TM, int TN, int ST, bool A_MN, bool B_KM, bool VEC, int EPI>
+static int f32_launch(const F32Group& a, int m, int batch, long long sa, long long sb, long long sc, int ksplit, float alpha, float beta, cudaStream_t st) {
     using L = F32Tile<BM, BN, BK, KG, TM, TN, ST, A_MN, B_KM>;
-    auto kern = k_gemm_f32<BM, BN, BK, KG, TM, TN, ST, A_MN, B_KM, VEC>;
+    constexpr int W = EPI == F32_SWIGLU ? BN / 2 : BN;
+    auto kern = k_gemm_f32<BM, BN, BK, KG, TM, TN, ST, A_MN, B_KM, VEC, EPI>;
     static const cudaError_t attr = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM);
     if (attr != cudaSuccess) return 125;
+    int cols = 0;
+    for (int g = 0; g < a.nprob; g++) cols += (a.n[g] + W - 1) / W;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((n + BN - 1) / BN * ksplit, (m + BM - 1) / BM, batch);
+    cfg.gridDim = dim3(cols * ksplit, (m + BM - 1) / BM, batch);
     if (cfg.gridDim.y > 65535 || cfg.gridDim.z > 65535) return 123;
     cfg.blockDim = dim3(L::THREADS); cfg.dynamicSmemBytes = L::SMEM; cfg.stream = st;
     cudaLaunchAttribute at[2];
@@ -287,27 +353,78 @@ static int f32_launch(const float* A, const float* B, float* C, const float* D, 
         na++;
     }
     cfg.attrs = at; cfg.numAttrs = na;
-    return cudaLaunchKernelEx(&cfg, kern, A, B, C, D, m, n, k, sa, sb, sc, ksplit, alpha, beta) == cudaSuccess ? 0 : 126;
+    return cudaLaunchKernelEx(&cfg, kern, a, m, sa, sb, sc, ksplit, alpha, beta) == cudaSuccess ? 0 : 126;
 }
-template <bool A_MN, bool B_KM>
-static int f32_gemm(const float* A, const float* B, float* C, const float* D, int m, int n, int k, int batch,
-                    long long sa, long long sb, long long sc, float alpha, float beta, cudaStream_t st) {
+template <bool A_MN, bool B_KM, int EPI = F32_PLAIN>
+static int f32_gemm(const F32Group& a, int m, int batch, long long sa, long long sb, long long sc, float alpha, float beta, cudaStream_t st) {
     // 16-byte copies need row pitches and starts on 16-byte boundaries
-    const bool vec = (A_MN ? m : k) % 4 == 0 && (B_KM ? k : n) % 4 == 0 && n % 4 == 0 && aligned16(A) && aligned16(B) && aligned16(C) &&
-                     (!D || aligned16(D)) && sa % 4 == 0 && sb % 4 == 0 && sc % 4 == 0;
-    auto tiles = [&](int bm, int bn) { return (long long)((m + bm - 1) / bm) * ((n + bn - 1) / bn) * batch; };
-#define F32L(BM, BN, BK, KG, TM, TN, ST, KSP)                                                                                        \
-    (vec ? f32_launch<BM, BN, BK, KG, TM, TN, ST, A_MN, B_KM, true>(A, B, C, D, m, n, k, batch, sa, sb, sc, KSP, alpha, beta, st)    \
-         : f32_launch<BM, BN, BK, KG, TM, TN, ST, A_MN, B_KM, false>(A, B, C, D, m, n, k, batch, sa, sb, sc, KSP, alpha, beta, st))
-    // the largest tile that still gives every SM one: a 128 x 128 tile has twice the FMAs per shared-memory read of a
-    // 64 x 64 one, but fewer than 148 of them leave SMs without work
+    bool vec = sa % 4 == 0 && sb % 4 == 0 && sc % 4 == 0 && (!A_MN || m % 4 == 0) && aligned16(a.D) && aligned16(a.G) && aligned16(a.U);
+    for (const float* c : a.C) vec = vec && aligned16(c);
+    for (int g = 0; g < a.nprob; g++) {
+        vec = vec && a.n[g] % 4 == 0;
+        for (const F32Seg* q = a.seg + g * a.nseg; q < a.seg + (g + 1) * a.nseg; q++)
+            vec = vec && ((A_MN && !B_KM) || q->k % 4 == 0) && aligned16(q->A) && aligned16(q->B) && aligned16(q->B2);
+    }
+    auto tiles = [&](int bm, int bn) {
+        long long cols = 0;
+        const int w = EPI == F32_SWIGLU ? bn / 2 : bn;
+        for (int g = 0; g < a.nprob; g++) cols += (a.n[g] + w - 1) / w;
+        return (long long)((m + bm - 1) / bm) * cols * batch;
+    };
+#define F32L(BM, BN, BK, KG, TM, TN, ST, KSP)                                                                                  \
+    (vec ? f32_launch<BM, BN, BK, KG, TM, TN, ST, A_MN, B_KM, true, EPI>(a, m, batch, sa, sb, sc, KSP, alpha, beta, st)        \
+         : f32_launch<BM, BN, BK, KG, TM, TN, ST, A_MN, B_KM, false, EPI>(a, m, batch, sa, sb, sc, KSP, alpha, beta, st))
+    // A 128 x 128 tile has the most FMAs per shared-memory read, but fewer than 148 of them leave SMs without work.
     if (tiles(128, 128) >= AX_SMS) return F32L(128, 128, 16, 1, 8, 8, 3, 1);
-    if (tiles(64, 64) >= AX_SMS) return F32L(64, 64, 32, 1, 4, 4, 3, 1);
-    // 32 x 32 tiles; a cluster splits the depth while CTAs are fewer than SMs and every CTA keeps two steps of 64
+    int steps = 0;
+    for (int q = 0; q < a.nseg; q++) steps += (a.seg[q].k + 63) / 64;
+    const long long small = tiles(32, 32), mid = tiles(64, 32);
+    if (tiles(64, 64) >= 2 * AX_SMS) return F32L(64, 64, 32, 2, 8, 8, 4, 1);
+    // Below, a launch is the latency of its steps: 64 x 32 tiles (8 x 4 sums to a thread, 43 % of the FMA pipe with two CTAs on an SM, which is what
+    // fits) with the depth cut over a cluster as far as two CTAs for each SM.  Where that leaves a third of the SMs idle or most with one CTA and some with two,
+    // or takes a second round, 32 x 32 tiles spread better; a product of two steps is over before a larger tile pays.  us, 64 x 32 with 1 / 2 / 4 CTAs to a tile |
+    // 32 x 32 alike | before: 512 x 256 x 256 8.6 / 7.9 / 6.2 | 8.8 / 7.6 / 10.1 | 7.6, 512 x 512 x 256 11.0 / 8.4 / 11.9 | 10.0 / 12.0 / 14.9 | 10.0,
+    // 512 x 256 x 688 21.1 / 16.4 / 10.8 | 20.2 / 14.8 / 15.3 | 14.8, 512 x 1024 x 256 12.2 / 17.1 / 24.3 | 14.4 / 19.2 / 26.5 | 14.4,
+    // 512 x 688 x 256 12.2 / 16.6 / 18.2 | 10.8 / 12.9 / 20.3 | 10.9, 512 x 1376 x 256 17.2 / 23.0 / 29.5 | 15.9 / 23.9 / 33.6 | 29.3 (64 x 64 tiles, 4 x 4 sums),
+    // 256 x 256 x 128 4.6 / 5.0 / 5.8 | 3.6 / 4.9 / 5.3 | 3.7, 300 x 128 x 344 10.0 / 7.4 / 7.6 | 6.9 / 6.6 / 7.3 | 6.7; 1024 x 1536 x 512 58 | 60 | 69 and with 64 x 64 tiles of 8 x 8 sums 50.
     int ks = 1;
-    while (ks < 8 && tiles(32, 32) * ks * 2 <= AX_SMS * 2 && (k + 63) / 64 >= 4 * ks) ks *= 2;
+    while (ks < 8 && mid * ks * 2 <= 2 * AX_SMS && steps >= 2 * ks) ks *= 2;
+    const long long ctas = mid * ks;
+    if (steps > 2 && 3 * ctas > 2 * AX_SMS && ctas <= 2 * AX_SMS && (ctas <= AX_SMS || 2 * ctas > 3 * AX_SMS)) return F32L(64, 32, 64, 4, 8, 4, 3, ks);
+    ks = 1;
+    while (ks < 8 && small * ks * 2 <= AX_SMS * 5 / 2 && steps >= 4 * ks) ks *= 2;
     return F32L(32, 32, 64, 4, 4, 4, 4, ks);
 #undef F32L
+}
+
+// Arguments as ax_gemm_tc2_group, fp32 operands and outputs (mode 0: one product).  -1: not for this kernel.
+int ax_gemm_f32_group(int tb, int mode, int count, const void* const* A, const void* const* B, void* const* C, const int* m, const int* n,
+                      const int* k, float alpha, const void* D, float beta, const void* swb_g, const void* swb_u, void* swb_du, cudaStream_t st) {
+    if (count < 1 || count > (mode == 2 ? 6 : 3) || m[0] < 1 || (mode != 1 && mode != 2 && mode != 4) || (D && mode != 2) || (swb_g && (mode != 2 || tb != 1 || D))) return -1;
+    F32Group a = {};
+    a.nprob = mode == 1 ? count : 1;
+    a.nseg = mode == 2 ? count : 1;
+    auto f = [](const void* p) { return (const float*)p; };
+    for (int g = 0; g < a.nprob; g++) { a.n[g] = n[g]; a.C[g] = (float*)C[g]; if (n[g] < 1) return -1; }
+    for (int g = 0; g < (mode == 4 ? 1 : count); g++) {
+        a.seg[g] = {f(A[mode == 2 ? g : 0]), f(B[g]), nullptr, k[mode == 2 ? g : 0]};
+        if (a.seg[g].k < 1) return -1;
+    }
+    a.D = beta != 0.f ? f(D) : nullptr;
+    if (!a.D) beta = 0.f;
+    if (mode == 4) {
+        if (tb != 0 || count != 2) return -1;
+        a.seg[0].B2 = f(B[1]);
+        a.C[1] = (float*)C[1]; a.C[2] = (float*)C[2];
+        return f32_gemm<false, false, F32_SWIGLU>(a, m[0], 1, 0, 0, 0, alpha, 0.f, st);
+    }
+    if (swb_g) {
+        a.G = f(swb_g); a.U = f(swb_u); a.C[1] = (float*)swb_du;
+        return f32_gemm<false, true, F32_SWB>(a, m[0], 1, 0, 0, 0, alpha, 0.f, st);
+    }
+    if (tb == 0) return f32_gemm<false, false>(a, m[0], 1, 0, 0, 0, alpha, beta, st);
+    if (tb == 1) return f32_gemm<false, true>(a, m[0], 1, 0, 0, 0, alpha, beta, st);
+    return f32_gemm<true, false>(a, m[0], 1, 0, 0, 0, alpha, beta, st);
 }
 
 int ax_gemm_simt(int in_bf16, int out_bf16, int tb, const void* A, const void* B, void* C, const void* D,
@@ -321,11 +438,12 @@ int ax_gemm_simt(int in_bf16, int out_bf16, int tb, const void* A, const void* B
     else { as_m = 1; as_k = m; bs_k = n; bs_n = 1; }
     if (beta != 0.f && !D) D = C;
     if (!in_bf16 && !out_bf16) {
-        const float* a = (const float*)A; const float* b = (const float*)B;
-        float* c = (float*)C; const float* d = beta != 0.f ? (const float*)D : nullptr;
-        if (tb == 0) return f32_gemm<false, false>(a, b, c, d, m, n, k, batch, sa, sb, sc, alpha, beta, st);
-        if (tb == 1) return f32_gemm<false, true>(a, b, c, d, m, n, k, batch, sa, sb, sc, alpha, beta, st);
-        return f32_gemm<true, false>(a, b, c, d, m, n, k, batch, sa, sb, sc, alpha, beta, st);
+        F32Group a = {};
+        a.seg[0] = {(const float*)A, (const float*)B, nullptr, k};
+        a.nprob = a.nseg = 1; a.n[0] = n; a.C[0] = (float*)C; a.D = beta != 0.f ? (const float*)D : nullptr;
+        if (tb == 0) return f32_gemm<false, false>(a, m, batch, sa, sb, sc, alpha, beta, st);
+        if (tb == 1) return f32_gemm<false, true>(a, m, batch, sa, sb, sc, alpha, beta, st);
+        return f32_gemm<true, false>(a, m, batch, sa, sb, sc, alpha, beta, st);
     }
     dim3 grid((n + GT - 1) / GT, (m + GT - 1) / GT, batch);
     if (grid.y > 65535 || grid.z > 65535) return 123;

@@ -12,6 +12,7 @@
 //   0x20 general GEMM, 0x21 single-CTA tcgen05 GEMM, 0x22 paired-CTA tcgen05 GEMM (+ 0x100 * split-K factor),
 //   0x26 small-product kernel (single or grouped), 0x23 grouped launch of the paired-CTA kernel,
 //   0x24 / 0x27 SwiGLU backward inside the product that makes dh on the small-product / the paired-CTA kernel,
+//   0x29 fp32 group as one launch, 0x2a SwiGLU backward inside the fp32 product that makes dh,
 //   0x25 / 0x28 SwiGLU inside a projection pair with adapters on the same two,
 //   0x70 embedding scatter by scanning the ids, 0x71 by occurrence lists, 0x72 scale and add as one pass, 0x73 with the norm,
 //   0x80 / 0x81 attention forward / backward with split probabilities on tcgen05, 0x82 / 0x83 on mma.sync (0x83 + 0x100 * CTAs to a key tile)
@@ -86,6 +87,9 @@ int ax_adamw_flat(float* p, const float* g, float* m, float* v, void* pbf, const
 int ax_gemm_simt(int in_bf16, int out_bf16, int tb, const void* A, const void* B, void* C, const void* D,
                  int m, int n, int k, int batch, long long sa, long long sb, long long sc,
                  float alpha, float beta, cudaStream_t st);
+// groups of fp32 products (and their SwiGLU epilogues) as one launch; -1 = not served
+int ax_gemm_f32_group(int tb, int mode, int count, const void* const* A, const void* const* B, void* const* C, const int* m, const int* n,
+                      const int* k, float alpha, const void* D, float beta, const void* swb_g, const void* swb_u, void* swb_du, cudaStream_t st);
 
 // gemm_tc.cu — tcgen05/TMEM/TMA bf16 GEMM. Returns -1 when the shape/alignment is not served.
 int ax_gemm_tc_init(void);

@@ -961,3 +961,85 @@ def test_tall_products_walk_their_tiles_in_bands(eng, m, n, k, tb, dt):
     got, ref = run_gemm(eng, np.random.default_rng(m + n), m, n, k, tb, dt, fallback=8)
     check(got, ref, dt == 1, k)
     assert eng.device_status() == 0
+
+
+F32_GROUPS = [(5, 7, (3, 9, 2)), (33, 66, (40, 8, 1)),              # rows that are no whole 16-byte pieces, less than a tile
+              (512, 256, (256, 128, 128)), (100, 1100, (36, 4, 200)),    # 32 x 32 tiles, the depth over a cluster of one, two and four
+              (700, 72, (520, 264, 132)), (1300, 36, (1032, 776, 516))]  # 64 x 64 and 128 x 128 tiles
+
+
+def f32_limit(k):
+    return 3e-6 * max(1.0, np.sqrt(k) / 4)             # as in `check`, of the largest element
+
+
+@pytest.mark.parametrize("tb", [0, 1, 2])
+@pytest.mark.parametrize("m,k,ns", F32_GROUPS)
+def test_fp32_products_of_one_input_as_one_launch(eng, tb, m, k, ns):
+    rng = np.random.default_rng(m + k + tb)
+    mk = lambda *sh: rng.standard_normal(sh).astype(np.float32)
+    x, w = mk(*((k, m) if tb == 2 else (m, k))), [mk(*((n, k) if tb == 1 else (k, n))) for n in ns]
+    ix, iw, ic = put(eng, x, 0), [put(eng, v, 0) for v in w], [put(eng, np.full((m, n), np.nan, np.float32), 0) for n in ns]
+    eng.launch_count(reset=True)
+    eng.run([op(E.GEMM_GROUP, a=ix, b=iw[0], sa=iw[1], sb=iw[2], c=ic[0], d=ic[1], sc=ic[2], m=m, k=k, n=ns[0], oa=ns[1], ob=ns[2], batch=3, oc=1, tb=tb, dt=0)])
+    assert (eng.launch_count(), eng.last_variant()) == (1, 0x29)
+    f = lambda v, t: (v.T if t else v).astype(np.float64)
+    for g, n in enumerate(ns):
+        check(eng.download(ic[g], (m, n)), f(x, tb == 2) @ f(w[g], tb == 1), False, k)
+    # an output that another member reads: the members run one by one, the last product meets the first one's result
+    if tb == 0 and ns[0] * m >= k * ns[2]:
+        eng.run([op(E.GEMM_GROUP, a=ix, b=iw[0], sa=iw[1], sb=ic[0], c=ic[0], d=ic[1], sc=ic[2], m=m, k=k, n=ns[0], oa=ns[1], ob=ns[2], batch=3, oc=1, dt=0)])
+        assert eng.last_variant() == 0x20
+        first = eng.download(ic[0], (m * ns[0],))[:k * ns[2]].reshape(k, ns[2])
+        check(eng.download(ic[2], (m, ns[2])), f(x, 0) @ f(first, 0), False, k)
+
+
+@pytest.mark.parametrize("addend", [0, 1, 2])                       # none, one of its own, the output itself
+@pytest.mark.parametrize("m,k,ns", F32_GROUPS)
+def test_fp32_sum_over_segments_as_one_launch(eng, m, k, ns, addend):
+    rng = np.random.default_rng(m + k + addend)
+    mk = lambda *sh: rng.standard_normal(sh).astype(np.float32)
+    n, r, ks = ns[0], 4, (k,) + ns[1:]
+    a, b, xa, xb, d = [mk(m, q) for q in ks], [mk(n, q) for q in ks], mk(m, r), mk(n, r), mk(m, n)
+    ia, ib, ixa, ixb, idd = [put(eng, v, 0) for v in a], [put(eng, v, 0) for v in b], put(eng, xa, 0), put(eng, xb, 0), put(eng, d, 0)
+    ic = idd if addend == 2 else put(eng, np.full((m, n), np.nan, np.float32), 0)
+    eng.launch_count(reset=True)
+    eng.run([op(E.GEMM_XSEG, a=ixa, sa=ixb, k=r, batch=1, c=idd if addend else 0, beta=-2.0),
+             op(E.GEMM_GROUP, c=ic, a=ia[0], sa=ia[1], sb=ia[2], b=ib[0], d=ib[1], sc=ib[2], m=m, n=n, k=ks[0], oa=ks[1], ob=ks[2], batch=3, oc=2, tb=1, dt=0,
+                alpha=0.5)])
+    assert (eng.launch_count(), eng.last_variant()) == (1, 0x29)
+    f = lambda v: v.astype(np.float64)
+    ref = 0.5 * (sum(f(x) @ f(w).T for x, w in zip(a, b)) + f(xa) @ f(xb).T) - (2.0 * f(d) if addend else 0.0)
+    check(eng.download(ic, (m, n)), ref, False, sum(ks) + r)
+
+
+@pytest.mark.parametrize("m,k,ns", F32_GROUPS)
+def test_fp32_swiglu_pair_and_its_backward_inside_their_products(eng, m, k, ns):
+    """g, u and h = silu(g) u from one launch; dg and du from the product that makes dh, which is not written.  Bounds: the error of a product, `f32_limit` of its
+    largest element, times what the outputs' derivatives make of it (silu' and sigmoid' g up to 1.1 and 0.5, sigmoid up to 1), and as much again for their own arithmetic."""
+    rng = np.random.default_rng(m + k)
+    mk = lambda *sh: rng.standard_normal(sh).astype(np.float32)
+    n = ns[0]
+    x, wg, wu = mk(m, k), mk(k, n), mk(k, n)
+    ix, ig, iu = put(eng, x, 0), put(eng, wg, 0), put(eng, wu, 0)
+    og, ou, oh = (put(eng, np.full((m, n), np.nan, np.float32), 0) for _ in range(3))
+    eng.launch_count(reset=True)
+    eng.run([op(E.GEMM_GROUP, a=ix, b=ig, sa=iu, c=og, d=ou, sc=oh, m=m, n=n, k=k, batch=2, oc=4, dt=0)])
+    assert (eng.launch_count(), eng.last_variant()) == (1, 0x29)
+    f = lambda v: v.astype(np.float64)
+    big = lambda v: np.abs(v).max()
+    g, u = f(x) @ f(wg), f(x) @ f(wu)
+    sig = lambda v: 1.0 / (1.0 + np.exp(-v))
+    check(eng.download(og, (m, n)), g, False, k)
+    check(eng.download(ou, (m, n)), u, False, k)
+    assert big(eng.download(oh, (m, n)) - g * sig(g) * u) <= 2 * f32_limit(k) * (1.1 * big(u) * big(g) + big(g) * big(u))
+    dy, wd = mk(m, k), mk(n, k)
+    idy, iwd, idh, idg, idu = put(eng, dy, 0), put(eng, wd, 0), put(eng, np.full((m, n), 7.0, np.float32), 0), eng.alloc(m * n), eng.alloc(m * n)
+    eng.launch_count(reset=True)
+    eng.run([op(E.GEMM_SB, a=idy, b=iwd, c=idh, m=m, n=n, k=k, batch=1, tb=1, dt=0), op(E.SILU_BWD, a=og, b=ou, d=idh, c=idg, tb=idu, n=m * n, dt=0, oa=1)])
+    assert (eng.launch_count(), eng.last_variant()) == (1, 0x2a) and np.all(eng.download(idh, (m, n)) == 7.0)
+    dh, s = f(dy) @ f(wd).T, sig(g)
+    assert big(eng.download(idg, (m, n)) - dh * u * s * (1 + g * (1 - s))) <= 2 * f32_limit(k) * big(dh) * big(u) * (1.1 + 0.5 * big(g) + 1.1)
+    assert big(eng.download(idu, (m, n)) - dh * g * s) <= 2 * f32_limit(k) * big(dh) * big(g) * (1 + 1.1)
+    # without the mark the gradient of h is kept: two launches
+    eng.run([op(E.GEMM_SB, a=idy, b=iwd, c=idh, m=m, n=n, k=k, batch=1, tb=1, dt=0), op(E.SILU_BWD, a=og, b=ou, d=idh, c=idg, tb=idu, n=m * n, dt=0)])
+    check(eng.download(idh, (m, n)), dh, False, k)
