@@ -40,6 +40,15 @@ template <int EPI> struct EpiCfg {
     static constexpr int THREADS = 64 + 32 * EW;                    // + TMA warp, MMA warp
 };
 
+// Bounded wait of a converged warp, with one answer for all of its lanes: a lane that left alone would be missed by the elect.sync of the others.
+// It also ends when another role has given up; that flag is looked at only while the phase is not complete.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, const volatile int* abort_flag) {
+    for (uint32_t i = 0; i < TC_SPIN_LIMIT; i++) {
+        if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
+        if (__any_sync(0xffffffffu, *abort_flag)) return false;
+    }
+    return false;
+}
 __device__ __forceinline__ uint32_t cluster_rank() {
     uint32_t r;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -71,11 +80,21 @@ __device__ __forceinline__ uint32_t pack2_bf16(float lo, float hi) {
     __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&h);
 }
-// tile load whose completion is counted on an mbarrier that may live in the peer CTA
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* m, uint32_t bar_cluster, int x, int y) {
+// tile loads by a converged warp (one elected lane issues), their completion counted on an mbarrier that may live in the peer CTA
+__device__ __forceinline__ void tma_load_2d_pair_e(uint32_t dst, const CUtensorMap* m, uint32_t bar_cluster, int x, int y) {
     asm volatile(
-        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+        "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+        "@q cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}"
         ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar_cluster), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_pair_e(uint32_t dst, const CUtensorMap* m, uint32_t bar_cluster, int x, int y, int z) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+        "@q cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n\t}"
+        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar_cluster), "r"(x), "r"(y), "r"(z) : "memory");
+}
+__device__ __forceinline__ void mbar_expect_tx_e(uint32_t bar, uint32_t bytes) {
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(bar), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void tmem_alloc2(uint32_t smem_dst, uint32_t ncols) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols) : "memory");
@@ -134,6 +153,7 @@ __device__ __forceinline__ void tc_commit2_e(uint32_t bar, uint16_t mask) {
 // 6.6 for 904 x 1704 x 128.
 struct GemmGroup {
     int mode, count;
+    int whole;               // M- and N-major operands have whole blocks of 64 along M and N: see map_mn
     int band;                // row tiles that are walked together, column by column (see band_of)
     int S;                   // pairs that share a tile's depth (1: a pair has tiles of its own)
     int n[3];
@@ -195,6 +215,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
     constexpr bool swiglu = EPI == EPI_SWIGLU, swb = EPI == EPI_SWB;
     const bool wide_stg = swiglu || swb || tma_out == 2;           // 64 KB of staging instead of 32, five stages
     const int nst = wide_stg ? STAGES2 - 1 : STAGES2;              // operand stages in use
+    const bool whole = grp.whole;
     const uint32_t bar_d = smem_u32(bars + 20);                    // [EW warps][16 / EW buffers] arrival barriers of fetched pieces
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -272,8 +293,13 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (timing && threadIdx.x == 0) prof[2] = clock64();
 
-    if (warp == 0 && lane == 0) {
-        // ── TMA producer (both CTAs): own 128 rows of A, own 128 columns of B ──
+    if (warp == 0) {
+        // ── TMA producer (both CTAs): own 128 rows of A, own 128 columns of B.  The whole warp runs the loop, one elected lane issues ──
+        // This loop was the bound: as one thread of a divergent warp that chose its maps anew for each k-block it took 418 cycles and 61 for each
+        // TMA instruction, 540 / 607 / 663 a k-block of 256 x 256 x 64 with both operands K-major / one / none (one pair alone, K 8192), where
+        // the MMAs need 512.  Converged, with the choice made once for a run of k-blocks and one instruction for each operand, all three take 512 (that
+        // is the tensor core's time).  8 launches in a row: 4096 x 1536 x 8192 (A^T B) 839 -> 746 us, 2000 x 1536 x 4096 (A B) 218 -> 201,
+        // 2000 x 4096 x 1536 (A B^T) 178 -> 176.
         uint32_t it = 0, ph = 0;
         int s = 0;
         bool ok = true;
@@ -283,51 +309,58 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
             int tm, tl;
             const int g = locate(tile, tm, tl);
             const int row0 = tm * 2 * BM2 + rank * BM2, col0 = swiglu ? tl * 128 : tl * BN2 + rank * 128;
-            // operand maps: modes 1 and 3 pick B by problem (mode 3 also A), mode 2 walks A and B through the K-segments,
-            // mode 4 gives CTA 0 the gate weights and CTA 1 the up weights (same 128 columns)
+            // A run: k-blocks whose operands lie one behind the other in the same two tensors.  Modes 1 and 3 pick B by problem (mode 3 also A), mode 4
+            // gives CTA 0 the gate weights and CTA 1 the up weights (same 128 columns).
             const CUtensorMap* pA = grp.mode == 3 ? (g == 0 ? &tmA : (g == 1 ? &tmA1 : &tmA2)) : &tmA;
             const CUtensorMap* pB = (grp.mode == 1 || grp.mode == 3) ? (g == 0 ? &tmB : (g == 1 ? &tmB1 : &tmB2))
                                     : (swiglu && rank == 1 ? &tmB1 : &tmB);
             int seg = 0, kl = kb0;                       // segment and k-block inside it
-            if (grp.mode == 2) while (seg + 1 < grp.count && kl >= grp.kb[seg]) { kl -= grp.kb[seg]; seg++; }
-            for (int kb = kb0; kb < kb1; kb++, kl++, it++, s = (s + 1 == nst ? 0 : s + 1), ph ^= (s == 0)) {
+            for (int kb = kb0; kb < kb1 && ok;) {
+                int run = kb1 - kb, yb = 0, ys = BK2;    // length; row of B when its rows run along K, and its step
                 if (grp.mode == 2) {
-                    while (seg + 1 < grp.count && kl >= grp.kb[seg]) { kl = 0; seg++; }
+                    while (seg + 1 < grp.count && kl >= grp.kb[seg]) kl -= grp.kb[seg++];
+                    run = min(run, grp.kb[seg] - kl);
                     pA = seg == 0 ? &tmA : seg == 1 ? &tmA1 : seg == 2 ? &tmA2 : seg == 3 ? &tmEA0 : seg == 4 ? &tmEA1 : &tmEA2;
                     pB = seg == 0 ? &tmB : seg == 1 ? &tmB1 : seg == 2 ? &tmB2 : seg == 3 ? &tmEB0 : seg == 4 ? &tmEB1 : &tmEB2;
-                } else if (grp.mode == 1 && kb >= kb_main) {         // the problem's own extra segment
+                } else if (kb < kb_main) {
+                    run = min(run, kb_main - kb);
+                } else if (grp.mode == 1) {              // the problem's own extra segment
                     kl = kb - kb_main;
                     pA = g == 0 ? &tmEA0 : (g == 1 ? &tmEA1 : &tmEA2);
                     pB = g == 0 ? &tmEB0 : (g == 1 ? &tmEB1 : &tmEB2);
-                }
-                int ybk = kl * BK2;                                  // row of B when its rows run along K
-                if (swiglu && kb >= kb_main) {                       // gate term, then up term; the other CTA reads zeros
+                } else if (swiglu) {                     // gate term, then up term; the other CTA reads zeros
                     const int e = kb - kb_main >= grp.xkb;
                     kl = kb - kb_main - e * grp.xkb;
+                    run = min(run, grp.xkb - kl);
                     pA = e ? &tmEA1 : &tmEA0;
                     pB = e ? &tmEB1 : &tmEB0;
-                    ybk = (int)rank == e ? kl * BK2 : grp.xk_pad;
+                    if ((int)rank != e) { yb = grp.xk_pad; ys = 0; }
                 }
-                if (it >= (uint32_t)nst && !mbar_wait(bar_empty + 8 * s, ph ^ 1)) { ok = false; break; }
-                if (*abort_flag) { ok = false; break; }
-                const uint32_t sa = smem_base + s * STAGE_BYTES2, sb = sa + A_BYTES2;
-                const uint32_t fb = full_leader + 8 * s;
-                if (rank == 0) mbar_expect_tx(bar_full + 8 * s, 2 * STAGE_BYTES2);   // both CTAs' bytes land on this barrier
-                if (A_MN) {
-#pragma unroll
-                    for (int b = 0; b < 2; b++) tma_load_2d_pair(sa + b * 8192, pA, fb, row0 + b * 64, kl * BK2);
-                } else {
-                    tma_load_2d_pair(sa, pA, fb, kl * BK2, row0);
-                }
-                if (B_MN) {
-#pragma unroll
-                    for (int b = 0; b < 2; b++) tma_load_2d_pair(sb + b * 8192, pB, fb, col0 + b * 64, ybk);
-                } else {
-                    tma_load_2d_pair(sb, pB, fb, kl * BK2, col0);
+                int x = kl * BK2;
+                if (ys) yb = x;
+                kb += run; kl += run;
+                for (; run > 0; run--, it++, s = (s + 1 == nst ? 0 : s + 1), ph ^= (s == 0), x += BK2, yb += ys) {
+                    if (it >= (uint32_t)nst && !mbar_wait_warp(bar_empty + 8 * s, ph ^ 1, abort_flag)) { ok = false; break; }
+                    const uint32_t sa = smem_base + s * STAGE_BYTES2, sb = sa + A_BYTES2;
+                    const uint32_t fb = full_leader + 8 * s;
+                    if (rank == 0) mbar_expect_tx_e(bar_full + 8 * s, 2 * STAGE_BYTES2);   // both CTAs' bytes land on this barrier
+                    if (A_MN) {
+                        if (whole) tma_load_3d_pair_e(sa, pA, fb, 0, x, row0 >> 6);
+                        else { tma_load_2d_pair_e(sa, pA, fb, row0, x); tma_load_2d_pair_e(sa + 8192, pA, fb, row0 + 64, x); }
+                    } else {
+                        tma_load_2d_pair_e(sa, pA, fb, x, row0);
+                    }
+                    if (B_MN) {
+                        if (whole) tma_load_3d_pair_e(sb, pB, fb, 0, yb, col0 >> 6);
+                        else { tma_load_2d_pair_e(sb, pB, fb, col0, yb); tma_load_2d_pair_e(sb + 8192, pB, fb, col0 + 64, yb); }
+                    } else {
+                        tma_load_2d_pair_e(sb, pB, fb, x, col0);
+                    }
                 }
             }
         }
-        if (!ok) { *abort_flag = 1; atomicExch(status, STAT_GEMM2 | 1); }
+        __syncwarp();
+        if (!ok && lane == 0) { *abort_flag = 1; atomicExch(status, STAT_GEMM2 | 1); }
     } else if (warp == 1 && rank == 0) {
         // ── MMA issuer (leader CTA only): the whole warp runs the loop converged, one elected lane issues ──
         constexpr uint32_t idesc = tc_idesc_bf16(256, BN2, A_MN, B_MN);
@@ -344,11 +377,11 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
             const int kb0 = kb_from + split * kb_per, kb1 = min(kb_to, kb0 + kb_per);
             const int acc = tcount & 1;
             const uint32_t aph = (tcount >> 1) & 1;
-            if (tcount >= 2 && !mbar_wait(bar_tempty + 8 * acc, aph ^ 1)) { ok = false; break; }
+            if (tcount >= 2 && !mbar_wait_warp(bar_tempty + 8 * acc, aph ^ 1, abort_flag)) { ok = false; break; }
             tc_fence_after();
             const uint32_t d_tmem = tmem_base + acc * BN2;
             for (int kb = kb0; kb < kb1; kb++, it++, s = (s + 1 == nst ? 0 : s + 1), ph ^= (s == 0)) {
-                if (!mbar_wait(bar_full + 8 * s, ph) || *abort_flag) { ok = false; break; }
+                if (!mbar_wait_warp(bar_full + 8 * s, ph, abort_flag)) { ok = false; break; }
                 tc_fence_after();
                 if (timing && it == 0 && lane == 0) prof[3] = clock64();
                 const uint32_t sa = smem_base + s * STAGE_BYTES2, sb = sa + A_BYTES2;
@@ -717,18 +750,18 @@ static int clusters_for() {
 }
 static int g_share_max[2] = {0, 0};      // the least of that over the kernels that share a tile, for 2 and 4 pairs
 
-// operand / output tensor maps of one problem
-template <int A_MN> static int map_a(CUtensorMap* t, const void* A, int m, int k) {
-    uint64_t dims[2], strides[1]; uint32_t box[2];
-    if (A_MN) { dims[0] = m; dims[1] = k; strides[0] = (uint64_t)m * 2; box[0] = 64; box[1] = BK2; }
-    else { dims[0] = k; dims[1] = m; strides[0] = (uint64_t)k * 2; box[0] = BK2; box[1] = BM2; }
-    return tc_make_tmap_bf16(t, A, 2, dims, strides, box, true);
+// operand / output tensor maps of one problem.  An M- or N-major operand [k, e] is loaded as two blocks of 64 elements by 64 rows, with one
+// instruction where its rows are whole blocks: as {64, k, e / 64}.  (A block that reached past the end of a row would read the next one.)
+static int map_mn(CUtensorMap* t, const void* p, int e, int k, bool whole) {
+    uint64_t dims[3] = {64, (uint64_t)k, (uint64_t)e / 64}, strides[2] = {(uint64_t)e * 2, 128};
+    uint32_t box[3] = {64, BK2, 2};
+    if (!whole) dims[0] = e;
+    return tc_make_tmap_bf16(t, p, whole ? 3 : 2, dims, strides, box, true);
 }
-template <int B_MN> static int map_b(CUtensorMap* t, const void* B, int n, int k) {
-    uint64_t dims[2], strides[1]; uint32_t box[2];
-    if (B_MN) { dims[0] = n; dims[1] = k; strides[0] = (uint64_t)n * 2; box[0] = 64; box[1] = BK2; }
-    else { dims[0] = k; dims[1] = n; strides[0] = (uint64_t)k * 2; box[0] = BK2; box[1] = 128; }
-    return tc_make_tmap_bf16(t, B, 2, dims, strides, box, true);
+static int map_km(CUtensorMap* t, const void* p, int e, int k) {
+    uint64_t dims[2] = {(uint64_t)k, (uint64_t)e}, strides[1] = {(uint64_t)k * 2};
+    uint32_t box[2] = {BK2, 128};
+    return tc_make_tmap_bf16(t, p, 2, dims, strides, box, true);
 }
 // {n, m, nz} tensor of osz-byte elements, pieces of 128 bytes (half_row: 64) x 32 rows
 static int map_c(CUtensorMap* t, void* base, int m, int n, int nz, int osz, bool half_row = false) {
@@ -800,19 +833,23 @@ static int gemm2_launch(int mode, int count, const void* const* A, const void* c
         for (int g = 0; g < count; g++) if (((grp.rope_mask >> g) & 1) && nv[g] % 64) return -1;
     }
     CUtensorMap tmA[3], tmB[3], tmC[3], tmD, tmEA[3], tmEB[3];
+    grp.whole = 1;
+    for (int g = 0; g < (mode == 1 || mode == 3 ? count : 1); g++) grp.whole = grp.whole && (!A_MN || mv[mode == 3 ? g : 0] % 64 == 0) && (!B_MN || nv[g] % 64 == 0);
+    auto map_a = [&](CUtensorMap* t, const void* p, int e, int depth) { return A_MN ? map_mn(t, p, e, depth, grp.whole) : map_km(t, p, e, depth); };
+    auto map_b = [&](CUtensorMap* t, const void* p, int e, int depth) { return B_MN ? map_mn(t, p, e, depth, grp.whole) : map_km(t, p, e, depth); };
     bool have_x = false;
     int tiles_n = 0;
     if (mode == 0) {
-        if (map_a<A_MN>(&tmA[0], A[0], m, k) || map_b<B_MN>(&tmB[0], B[0], n, k)) return 2;
+        if (map_a(&tmA[0], A[0], m, k) || map_b(&tmB[0], B[0], n, k)) return 2;
         tiles_n = (n + 255) / 256;
     } else if (mode == 1) {
-        if (map_a<A_MN>(&tmA[0], A[0], m, k)) return 2;
+        if (map_a(&tmA[0], A[0], m, k)) return 2;
         for (int g = 0; g < count; g++) {
-            if (map_b<B_MN>(&tmB[g], B[g], nv[g], k)) return 2;
+            if (map_b(&tmB[g], B[g], nv[g], k)) return 2;
             grp.n[g] = nv[g];
             tiles_n += (nv[g] + 255) / 256;
             if (XA && xk > 0) {
-                if (map_a<A_MN>(&tmEA[g], XA[g], m, xk) || map_b<B_MN>(&tmEB[g], XB[g], nv[g], xk)) return 2;
+                if (map_a(&tmEA[g], XA[g], m, xk) || map_b(&tmEB[g], XB[g], nv[g], xk)) return 2;
                 have_x = true;
             }
         }
@@ -822,22 +859,22 @@ static int gemm2_launch(int mode, int count, const void* const* A, const void* c
         for (int g = 0; g < count; g++) {
             CUtensorMap* ta = g < 3 ? &tmA[g] : &tmEA[g - 3];
             CUtensorMap* tb_ = g < 3 ? &tmB[g] : &tmEB[g - 3];
-            if (map_a<A_MN>(ta, A[g], m, kv[g]) || map_b<B_MN>(tb_, B[g], n, kv[g])) return 2;
+            if (map_a(ta, A[g], m, kv[g]) || map_b(tb_, B[g], n, kv[g])) return 2;
             grp.kb[g] = (kv[g] + BK2 - 1) / BK2;
         }
         have_x = count > 3;
         tiles_n = (n + 255) / 256;
     } else if (mode == 3) {
         for (int g = 0; g < count; g++) {
-            if (map_a<A_MN>(&tmA[g], A[g], mv[g], k) || map_b<B_MN>(&tmB[g], B[g], nv[g], k)) return 2;
+            if (map_a(&tmA[g], A[g], mv[g], k) || map_b(&tmB[g], B[g], nv[g], k)) return 2;
             grp.m[g] = mv[g]; grp.n[g] = nv[g];
         }
     } else {        // mode 4: gate and up weights of the same width n; outputs g, u, h
         if (sizeof(TO) != 2 || count != 2) return -1;
-        if (map_a<A_MN>(&tmA[0], A[0], m, k) || map_b<B_MN>(&tmB[0], B[0], n, k) || map_b<B_MN>(&tmB[1], B[1], n, k)) return 2;
+        if (map_a(&tmA[0], A[0], m, k) || map_b(&tmB[0], B[0], n, k) || map_b(&tmB[1], B[1], n, k)) return 2;
         if (XA && xk > 0) {                  // low-rank terms; the zeros come from rows of B behind the last
             for (int q = 0; q < 2; q++)
-                if (map_a<A_MN>(&tmEA[q], XA[q], m, xk) || map_b<B_MN>(&tmEB[q], XB[q], n, xk)) return 2;
+                if (map_a(&tmEA[q], XA[q], m, xk) || map_b(&tmEB[q], XB[q], n, xk)) return 2;
             have_x = true;
             grp.xkb = (xk + BK2 - 1) / BK2;
             grp.xk_pad = grp.xkb * BK2;

@@ -1043,3 +1043,13 @@ def test_fp32_swiglu_pair_and_its_backward_inside_their_products(eng, m, k, ns):
     # without the mark the gradient of h is kept: two launches
     eng.run([op(E.GEMM_SB, a=idy, b=iwd, c=idh, m=m, n=n, k=k, batch=1, tb=1, dt=0), op(E.SILU_BWD, a=og, b=ou, d=idh, c=idg, tb=idu, n=m * n, dt=0)])
     check(eng.download(idh, (m, n)), dh, False, k)
+
+
+@pytest.mark.parametrize("tb", [0, 2])
+@pytest.mark.parametrize("dt,m,n,k", [(1, 320, 448, 200), (2, 256, 256, 64), (1, 576, 1088, 72), (1, 320, 456, 200), (2, 328, 448, 200)])
+def test_operands_of_whole_64_blocks_and_others(eng, tb, dt, m, n, k):
+    """M- and N-major operands travel as two blocks of 64 columns in one instruction where their rows are whole blocks, ending in the first or the
+    second of a pair, else one by one."""
+    got, ref = run_gemm(eng, np.random.default_rng(m + n + k), m, n, k, tb, dt, fallback=8)
+    check(got, ref, dt == 1, k)
+    assert eng.device_status() == 0
