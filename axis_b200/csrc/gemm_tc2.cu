@@ -40,6 +40,9 @@ template <int EPI> struct EpiCfg {
     static constexpr int THREADS = 64 + 32 * EW;                    // + TMA warp, MMA warp
 };
 
+// The two halves of cluster_sync, for a converged warp
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // Bounded wait of a converged warp, with one answer for all of its lanes: a lane that left alone would be missed by the elect.sync of the others.
 // It also ends when another role has given up; that flag is looked at only while the phase is not complete.
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, const volatile int* abort_flag) {
@@ -193,7 +196,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
     // the sixth stage's memory doubles the staging area.
     // Epilogue warps: four (a warp per TMEM lane quarter), eight where the epilogue computes so much that four would
     // outlast the main loop of the next tile (SwiGLU backward); the two warps of a quarter then take the column pieces
-    // in turn.
+    // in turn.  Eight for plain products gain 1 % in chains of one round (2000 x 1536 x 1536) and lose as much where rounds follow one another.
     // prof (only in builds with -DAXENG_PROF, otherwise null and every stamp compiles out): clock64 stamps of
     // pair 0's leader CTA — [0] entry, [1] set-up done, [2] predecessor grid finished, [3] first operands landed,
     // [4] last MMA issued, [5] last accumulator complete, [6] last tile stored, [7] exit
@@ -219,9 +222,30 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
     const uint32_t bar_d = smem_u32(bars + 20);                    // [EW warps][16 / EW buffers] arrival barriers of fetched pieces
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // Set-up: barriers, tensor memory and tensor maps by three warps, one barrier of the cluster at its end, and what each warp has to know about its tiles
+    // while that barrier waits for the peer (2560 cycles from the entry before, when one thread did it and two barriers followed; 1850 now: steps of small tiles 0.3 to 2 % shorter).
+    static_assert(2 * STAGES2 + 4 == 16, "one barrier to a lane");
+    if (warp == 0) {
+        mbar_init(smem_u32(bars + (lane < 16 ? lane : lane + 4)), lane == 14 || lane == 15 ? 64 * EW : 1);
+        if (lane == 0) *abort_flag = 0;
+        mbar_fence_init();
+    } else if (warp == 1) {
+        tmem_alloc2(smem_u32(tmem_slot), 512);
+        tmem_relinquish2();
+    } else if (warp == 2 && lane == 0) {
+        tma_prefetch_desc(&tmA);
+        tma_prefetch_desc(&tmB);
+        if (grp.count > 1) { tma_prefetch_desc(grp.mode == 2 ? &tmA1 : &tmC1); tma_prefetch_desc(&tmB1); }
+        if (grp.count > 2) { tma_prefetch_desc(grp.mode == 2 ? &tmA2 : &tmC2); tma_prefetch_desc(&tmB2); }
+        if (tma_out) tma_prefetch_desc(&tmC);
+        if (tma_out == 2 || swb) tma_prefetch_desc(&tmD);
+    }
+    tc_fence_before();
+    __syncwarp();
+    cluster_arrive();
     const uint32_t crank = cluster_rank(), rank = crank & 1, lead = crank & ~1u;     // rank 0 of a pair leads it (issues the MMAs)
     const int S = SHARE ? grp.S : 1, part = SHARE ? crank >> 1 : 0;      // this pair's part of the depth
-    const int pair = blockIdx.x / (2 * S), npairs = gridDim.x / (2 * S);
+    const int pair = SHARE ? blockIdx.x / (2 * S) : blockIdx.x >> 1, npairs = SHARE ? gridDim.x / (2 * S) : gridDim.x >> 1;
     const uint16_t both = 3u << lead;                      // the pair's CTAs
     const int tiles_m = (m + 2 * BM2 - 1) / (2 * BM2);
     int tiles_n = (n + BN2 - 1) / BN2, kblocks_all = (k + BK2 - 1) / BK2;
@@ -252,37 +276,25 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
             tm = tile % tmq; tl = tile / tmq;
             return q;
         }
-        const int per = grp.band * tiles_n, b0 = tile / per * grp.band;
-        tile -= b0 * tiles_n;
-        const int rows = min(grp.band, tiles_m - b0);
-        tm = b0 + tile % rows;
+        int b0 = 0, rows = tiles_m;
+        if (grp.band < tiles_m) {
+            b0 = tile / (grp.band * tiles_n) * grp.band;
+            tile -= b0 * tiles_n;
+            rows = min(grp.band, tiles_m - b0);
+        }
         int tn = tile / rows;
+        tm = b0 + tile - tn * rows;
         if (grp.mode == 1)
             for (; q + 1 < grp.count; q++) { const int tq = (grp.n[q] + BN2 - 1) / BN2; if (tn < tq) break; tn -= tq; }
         tl = tn;
         return q;
     };
-    const int kb_per = (kblocks_all + ksplit - 1) / ksplit;
+    const int kb_per = ksplit == 1 ? kblocks_all : (kblocks_all + ksplit - 1) / ksplit;
     const int kb_from = SHARE ? kblocks_all * part / S : 0, kb_to = SHARE ? kblocks_all * (part + 1) / S : kblocks_all;
     const int num_units = num_tiles * ksplit;
 
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES2; s++) { mbar_init(bar_full + 8 * s, 1); mbar_init(bar_empty + 8 * s, 1); }
-        for (int a = 0; a < 2; a++) { mbar_init(bar_tfull + 8 * a, 1); mbar_init(bar_tempty + 8 * a, 64 * EW); }
-        for (int a = 0; a < 16; a++) mbar_init(bar_d + 8 * a, 1);
-        *abort_flag = 0;
-        mbar_fence_init();
-        tma_prefetch_desc(&tmA);
-        tma_prefetch_desc(&tmB);
-        if (grp.count > 1) { tma_prefetch_desc(grp.mode == 2 ? &tmA1 : &tmC1); tma_prefetch_desc(&tmB1); }
-        if (grp.count > 2) { tma_prefetch_desc(grp.mode == 2 ? &tmA2 : &tmC2); tma_prefetch_desc(&tmB2); }
-        if (tma_out) tma_prefetch_desc(&tmC);
-        if (tma_out == 2 || swb) tma_prefetch_desc(&tmD);
-    }
-    if (warp == 1) { tmem_alloc2(smem_u32(tmem_slot), 512); tmem_relinquish2(); }
-    tc_fence_before();
-    __syncthreads();
-    cluster_sync();                                       // peer barriers are initialised before anyone signals them
+    // the CTA's own warps and the peer's: barriers are initialised and tensor memory is there
+    cluster_wait();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t full_leader = map_to_cta(bar_full, lead);  // cluster address of the leader's full[0]
@@ -304,7 +316,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
         int s = 0;
         bool ok = true;
         for (int unit = pair; unit < num_units && ok; unit += npairs) {
-            const int tile = unit % num_tiles, split = unit / num_tiles;
+            const int split = ksplit == 1 ? 0 : unit / num_tiles, tile = unit - split * num_tiles;
             const int kb0 = kb_from + split * kb_per, kb1 = min(kb_to, kb0 + kb_per);
             int tm, tl;
             const int g = locate(tile, tm, tl);
@@ -373,7 +385,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
         int s = 0;
         bool ok = true;
         for (int unit = pair; unit < num_units && ok; unit += npairs, tcount++) {
-            const int split = unit / num_tiles;
+            const int split = ksplit == 1 ? 0 : unit / num_tiles;
             const int kb0 = kb_from + split * kb_per, kb1 = min(kb_to, kb0 + kb_per);
             const int acc = tcount & 1;
             const uint32_t aph = (tcount >> 1) & 1;
@@ -416,7 +428,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
         const uint32_t my_bar_d = bar_d + 8 * (16 / EW) * (EW == 4 ? quad : ew);
         uint32_t dpar = 0;                                      // phase parity of each arrival barrier
         for (int unit = pair; unit < num_units && ok; unit += npairs, tcount++) {
-            const int tile = unit % num_tiles, split = unit / num_tiles;
+            const int split = ksplit == 1 ? 0 : unit / num_tiles, tile = unit - split * num_tiles;
             int tm, tl;
             const int g = locate(tile, tm, tl);                  // grouped launch: which output, which tile of it
             const int tn = tl;
