@@ -583,7 +583,7 @@ static int map_bthd128(CUtensorMap* m, const void* base, int B, int T, int heads
     uint64_t dims[4] = {DH2, (uint64_t)heads, (uint64_t)T, (uint64_t)B};
     uint64_t strides[3] = {(uint64_t)DH2 * 2, (uint64_t)heads * DH2 * 2, (uint64_t)T * heads * DH2 * 2};
     uint32_t box[4] = {64, 1, (uint32_t)rows, 1};
-    return tc_make_tmap_bf16(m, base, 4, dims, strides, box, true);
+    return tc_make_tmap_bf16(m, base, 4, dims, strides, box, 128);
 }
 static int map_dq_f32_128(CUtensorMap* m, const void* base, int B, int T, int heads) {
     PFN_tmapEncodeTiled enc = tc_encode_fn();

@@ -672,7 +672,7 @@ static int map_rows(CUtensorMap* m, const void* base, const AttnShape& s, int he
     uint64_t dims[4] = {(uint64_t)s.DH, (uint64_t)heads, (uint64_t)s.T, (uint64_t)s.B};
     uint64_t strides[3] = {(uint64_t)s.DH * 2, (uint64_t)heads * s.DH * 2, (uint64_t)s.T * heads * s.DH * 2};
     uint32_t box[4] = {XD, 1, (uint32_t)rows, 1};
-    return tc_make_tmap_bf16(m, base, 4, dims, strides, box, true);
+    return tc_make_tmap_bf16(m, base, 4, dims, strides, box, 128);
 }
 // Where the line to attn_mma.cu lies.  Its 64-row tiles and lower set-up win where 128-row tiles are half empty or the SMs are not full.
 // Forward, us there / here (row after row of launches, heads = batch x heads): T64 384 heads 5.2 / 9.2, T20 960 heads 10.2 / 17.6, so up to 64

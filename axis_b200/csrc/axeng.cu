@@ -57,7 +57,7 @@ struct Engine {
 };
 static Engine G;
 int ax_variant = 0;
-int ax_gemm_parts = 0;
+int ax_gemm_parts = 0, ax_gemm_width = 0;
 
 static void set_err(const char* fmt, ...) {
     va_list ap; va_start(ap, fmt);
@@ -136,6 +136,7 @@ API int eng_set_fallback(int mask) {
 API long long eng_bytes_allocated(void) { return G.bytes; }
 API int eng_last_variant(void) { return ax_variant; }
 API int eng_last_gemm_parts(void) { return ax_gemm_parts; }
+API int eng_last_gemm_width(void) { return ax_gemm_width; }
 API long long eng_attn_smem(int which, int head_dim) { return which < 0 || which > 2 || head_dim < 1 || head_dim > 256 ? -1 : ax_attn_simt_smem(which, head_dim); }
 API int eng_sync(void) {
     int rc = (int)cudaStreamSynchronize(G.stream);
@@ -1202,7 +1203,7 @@ static int run_fused(const EngOp* ops, int n_ops, int i, int* last) {
 static int run_ops(const EngOp* ops, int n_ops) {
     G.fork_used = 0;
     G.cur = G.stream;
-    ax_gemm_side(0);
+    ax_gemm_plan_begin();
     for (int i = 0; i < n_ops; i++) {
         cudaEvent_t e0 = nullptr, e1 = nullptr;
         const bool prof = G.profile && ops[i].kind >= 0 && ops[i].kind < ENG_KIND_COUNT &&

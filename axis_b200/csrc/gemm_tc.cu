@@ -35,14 +35,14 @@ PFN_tmapEncodeTiled tc_encode_fn() {
     return g_encode;
 }
 int tc_make_tmap_bf16(CUtensorMap* out, const void* base, int rank, const uint64_t* dims, const uint64_t* strides_bytes,
-                      const uint32_t* box, bool swizzle128) {
+                      const uint32_t* box, int swizzle) {
     PFN_tmapEncodeTiled enc = tc_encode_fn();
     if (!enc) return 1;
     cuuint64_t gd[5]; cuuint64_t gs[4]; cuuint32_t bx[5]; cuuint32_t es[5];
     for (int i = 0; i < rank; i++) { gd[i] = dims[i]; bx[i] = box[i]; es[i] = 1; }
     for (int i = 0; i + 1 < rank; i++) gs[i] = strides_bytes[i];
     CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(base), gd, gs, bx, es,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : swizzle == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE,
                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? 0 : 2;
 }
@@ -236,7 +236,11 @@ static int g_pairs_avail = 0;      // co-resident CTA pairs of the paired kernel
 // launch (their predecessor in the stream is an event wait, not a kernel of the chain) and no split-K (the
 // split-K workspace is one buffer, owned by the main stream's launches)
 static int g_side = 0;
-void ax_gemm_side(int on) { g_side = on; }
+static bool g_beside = false;
+void ax_gemm_side(int on) { g_side = on; g_beside = g_beside || on; }
+// A plan that has queued products on the side stream has them running beside the main chain from then on (until the next plan starts)
+void ax_gemm_plan_begin(void) { g_side = 0; g_beside = false; }
+bool ax_gemm_beside(void) { return g_beside; }
 int ax_gemm_pdl(void) {
     static const int on = getenv("AXENG_NO_PDL") ? 0 : 1;
     return on && !g_side;
@@ -285,11 +289,11 @@ static int gemm_launch(const void* A, const void* B, void* C, const void* D, int
         uint64_t dims[2], strides[1]; uint32_t box[2];
         if (A_MN) { dims[0] = m; dims[1] = k; strides[0] = (uint64_t)m * 2; box[0] = 64; box[1] = BK; }
         else { dims[0] = k; dims[1] = m; strides[0] = (uint64_t)k * 2; box[0] = BK; box[1] = BM; }
-        if (tc_make_tmap_bf16(&tmA, A, 2, dims, strides, box, true)) return 2;
+        if (tc_make_tmap_bf16(&tmA, A, 2, dims, strides, box, 128)) return 2;
         // B: N-major [k,n] -> dims {n, k}, box {64, 64};  K-major [n,k] -> dims {k, n}, box {64, BN}
         if (B_MN) { dims[0] = n; dims[1] = k; strides[0] = (uint64_t)n * 2; box[0] = 64; box[1] = BK; }
         else { dims[0] = k; dims[1] = n; strides[0] = (uint64_t)k * 2; box[0] = BK; box[1] = BN; }
-        if (tc_make_tmap_bf16(&tmB, B, 2, dims, strides, box, true)) return 2;
+        if (tc_make_tmap_bf16(&tmB, B, 2, dims, strides, box, 128)) return 2;
     }
     const int units = ((m + BM - 1) / BM) * ((n + BN - 1) / BN) * ksplit;
     const int grid = units < AX_SMS ? units : AX_SMS;
@@ -360,19 +364,32 @@ int ax_gemm_tc(int out_bf16, int tb, const void* A, const void* B, void* C, cons
             if (sk > 1) cost += (2.0 * sk + 1.0) * m * n * 4.0 / 4.0e12 / 0.45e-6 + 4.0;
             if (cost < best2 - 1e-9) { best2 = cost; best2_s = sk; }
         }
+        const bool by_tma = ax_gemm_tc2_by_tma(C, beta != 0.f ? D : nullptr, n, out_bf16 ? 2 : 4);
+        // Against a split through the workspace in us, fitted to 60 and 76 shapes (rms 1.0): set-up, k-blocks of a pair, and the sums, which stay in L2.
+        // Split / shared: 1472 x 744 x 7432 25.2 / 32.7, 1368 x 784 x 5264 22.8 / 25.5, 608 x 2304 x 6520 33.0 / 30.3, 760 x 848 x 4464 18.7 / 15.9.
+        const double split_us = 10.3 + 0.38 * ((tiles2 * best2_s + g_pairs_avail - 1) / g_pairs_avail) * ((kblocks + best2_s - 1) / best2_s) +
+                                1.22e-7 * m * n * ((best2_s + 1) * 4.0 + (out_bf16 ? 2 : 4));
         double shared;
-        const int S = !g_side && ax_gemm_tc2_by_tma(C, beta != 0.f ? D : nullptr, n, out_bf16 ? 2 : 4) ? ax_gemm_tc2_share((int)tiles2, kblocks, &shared) : 1;
-        if (S > 1) {
-            // Against a split through the workspace in us, fitted to 60 and 76 shapes (rms 1.0): set-up, k-blocks of a pair, and the sums, which stay in L2.
-            // Split / shared: 1472 x 744 x 7432 25.2 / 32.7, 1368 x 784 x 5264 22.8 / 25.5, 608 x 2304 x 6520 33.0 / 30.3, 760 x 848 x 4464 18.7 / 15.9.
-            const double split_us = 10.3 + 0.38 * ((tiles2 * best2_s + g_pairs_avail - 1) / g_pairs_avail) * ((kblocks + best2_s - 1) / best2_s) +
-                                    1.22e-7 * m * n * ((best2_s + 1) * 4.0 + (out_bf16 ? 2 : 4));
+        const int S = !g_side && by_tma ? ax_gemm_tc2_share((int)tiles2, kblocks, &shared) : 1;
+        int width = 256;
+        if (g_pair_mode == 0 && !g_beside) {
+            const long long rows = (m + 255) / 256, tiles[3] = {tiles2, rows * ((n + 191) / 192), rows * ((n + 127) / 128)};
+            const TileTimes t = ax_gemm_tc2_width(tiles, kblocks, S > 1);
+            if (t.width != 256 && (best2_s == 1 || t.us < split_us)) {
+                width = t.width;
+                const double in_blocks = (t.us - 5.6) / 0.30 * 0.70;
+                best2 = in_blocks < best2 ? in_blocks : best2;
+                best2_s = 1;
+            }
+        }
+        if (width == 256 && S > 1) {
             const double shared_us = 8.2 + 0.36 * ((kblocks + S - 1) / S) + 0.04 * S * tiles2;
             if (best2_s == 1 || shared_us < split_us) { best2 = shared * 0.70 < best2 ? shared * 0.70 : best2; best2_s = 1; }
         }
         if (g_pair_mode == 2 || best2 < best) {
             ax_variant = 0x22 + 0x100 * best2_s;
-            const int rc = ax_gemm_tc2(out_bf16, tb, A, B, C, D, m, n, k, alpha, beta, status, best2_s, st);
+            ax_gemm_width = width;
+            const int rc = ax_gemm_tc2(out_bf16, tb, A, B, C, D, m, n, k, alpha, beta, status, best2_s, width, st);
             if (rc >= 0) return rc;
         }
     }

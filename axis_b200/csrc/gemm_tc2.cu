@@ -21,7 +21,6 @@
 #include "tc_common.cuh"
 
 #define BM2 128            // rows per CTA (256 per pair)
-#define BN2 256            // columns per pair (128 loaded by each CTA)
 #define BK2 64
 #define STAGES2 6
 #define STAT_GEMM2 0x400
@@ -40,9 +39,6 @@ template <int EPI> struct EpiCfg {
     static constexpr int THREADS = 64 + 32 * EW;                    // + TMA warp, MMA warp
 };
 
-// The two halves of cluster_sync, for a converged warp
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // Bounded wait of a converged warp, with one answer for all of its lanes: a lane that left alone would be missed by the elect.sync of the others.
 // It also ends when another role has given up; that flag is looked at only while the phase is not complete.
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, const volatile int* abort_flag) {
@@ -175,7 +171,10 @@ void ax_gemm_group_rope(const float* cs, const float* sn, int T, int mask) {
     g_rope_req.rope_cos = cs; g_rope_req.rope_sin = sn; g_rope_req.rope_T = T; g_rope_req.rope_mask = mask;
 }
 
-template <int A_MN, int B_MN, typename TO, int EPI, bool SHARE>
+// An N-major B comes in blocks of 64 columns by 64 rows (128-byte swizzle), of 32 (64-byte) where a CTA's columns are no multiple of 64
+__host__ __device__ constexpr int b_block(int bn) { return bn / 2 % 64 ? 32 : 64; }
+
+template <int A_MN, int B_MN, typename TO, int EPI, bool SHARE, int BN>
 __global__ void __launch_bounds__(EpiCfg<EPI>::THREADS, 1)
 k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
            const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmD,
@@ -216,14 +215,15 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
     const uint32_t smem_base = smem_u32(smem);
     constexpr int NH = EpiCfg<EPI>::NH, EW = EpiCfg<EPI>::EW;
     constexpr bool swiglu = EPI == EPI_SWIGLU, swb = EPI == EPI_SWB;
+    constexpr int B_BLK = b_block(BN);                             // columns of a block of an N-major B
     const bool wide_stg = swiglu || swb || tma_out == 2;           // 64 KB of staging instead of 32, five stages
     const int nst = wide_stg ? STAGES2 - 1 : STAGES2;              // operand stages in use
     const bool whole = grp.whole;
     const uint32_t bar_d = smem_u32(bars + 20);                    // [EW warps][16 / EW buffers] arrival barriers of fetched pieces
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // Set-up: barriers, tensor memory and tensor maps by three warps, one barrier of the cluster at its end, and what each warp has to know about its tiles
-    // while that barrier waits for the peer (2560 cycles from the entry before, when one thread did it and two barriers followed; 1850 now: steps of small tiles 0.3 to 2 % shorter).
+    // Set-up: barriers, tensor memory and tensor maps by three warps at the same time, what each warp has to know about its tiles, and one barrier of the
+    // cluster behind it (2560 cycles from the entry before, when one thread did it and two barriers followed; 1850 now: steps of small tiles 0.3 to 2 % shorter).
     static_assert(2 * STAGES2 + 4 == 16, "one barrier to a lane");
     if (warp == 0) {
         mbar_init(smem_u32(bars + (lane < 16 ? lane : lane + 4)), lane == 14 || lane == 15 ? 64 * EW : 1);
@@ -242,17 +242,16 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
     }
     tc_fence_before();
     __syncwarp();
-    cluster_arrive();
     const uint32_t crank = cluster_rank(), rank = crank & 1, lead = crank & ~1u;     // rank 0 of a pair leads it (issues the MMAs)
     const int S = SHARE ? grp.S : 1, part = SHARE ? crank >> 1 : 0;      // this pair's part of the depth
     const int pair = SHARE ? blockIdx.x / (2 * S) : blockIdx.x >> 1, npairs = SHARE ? gridDim.x / (2 * S) : gridDim.x >> 1;
     const uint16_t both = 3u << lead;                      // the pair's CTAs
     const int tiles_m = (m + 2 * BM2 - 1) / (2 * BM2);
-    int tiles_n = (n + BN2 - 1) / BN2, kblocks_all = (k + BK2 - 1) / BK2;
+    int tiles_n = (n + BN - 1) / BN, kblocks_all = (k + BK2 - 1) / BK2;
     const int kb_main = kblocks_all;                       // mode 1: k-blocks of the shared segment
     if (grp.mode == 1) {
         tiles_n = 0;
-        for (int q = 0; q < grp.count; q++) tiles_n += (grp.n[q] + BN2 - 1) / BN2;
+        for (int q = 0; q < grp.count; q++) tiles_n += (grp.n[q] + BN - 1) / BN;
         kblocks_all += grp.xkb;
     }
     if (grp.mode == 2) { kblocks_all = 0; for (int q = 0; q < grp.count; q++) kblocks_all += grp.kb[q]; }
@@ -260,7 +259,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
     int num_tiles = tiles_m * tiles_n;
     if (grp.mode == 3) {
         num_tiles = 0;
-        for (int q = 0; q < grp.count; q++) num_tiles += ((grp.m[q] + 2 * BM2 - 1) / (2 * BM2)) * ((grp.n[q] + BN2 - 1) / BN2);
+        for (int q = 0; q < grp.count; q++) num_tiles += ((grp.m[q] + 2 * BM2 - 1) / (2 * BM2)) * ((grp.n[q] + BN - 1) / BN);
     }
     // tile index -> problem g, row tile tm and column tile tl inside it (row tiles of a band fastest, bands slowest)
     auto locate = [&](int tile, int& tm, int& tl) -> int {
@@ -268,7 +267,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
         if (grp.mode == 3) {
             int tmq = (grp.m[0] + 2 * BM2 - 1) / (2 * BM2);
             for (; q + 1 < grp.count; q++) {
-                const int tq = tmq * ((grp.n[q] + BN2 - 1) / BN2);
+                const int tq = tmq * ((grp.n[q] + BN - 1) / BN);
                 if (tile < tq) break;
                 tile -= tq;
                 tmq = (grp.m[q + 1] + 2 * BM2 - 1) / (2 * BM2);
@@ -285,7 +284,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
         int tn = tile / rows;
         tm = b0 + tile - tn * rows;
         if (grp.mode == 1)
-            for (; q + 1 < grp.count; q++) { const int tq = (grp.n[q] + BN2 - 1) / BN2; if (tn < tq) break; tn -= tq; }
+            for (; q + 1 < grp.count; q++) { const int tq = (grp.n[q] + BN - 1) / BN; if (tn < tq) break; tn -= tq; }
         tl = tn;
         return q;
     };
@@ -294,7 +293,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
     const int num_units = num_tiles * ksplit;
 
     // the CTA's own warps and the peer's: barriers are initialised and tensor memory is there
-    cluster_wait();
+    cluster_sync();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t full_leader = map_to_cta(bar_full, lead);  // cluster address of the leader's full[0]
@@ -320,7 +319,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
             const int kb0 = kb_from + split * kb_per, kb1 = min(kb_to, kb0 + kb_per);
             int tm, tl;
             const int g = locate(tile, tm, tl);
-            const int row0 = tm * 2 * BM2 + rank * BM2, col0 = swiglu ? tl * 128 : tl * BN2 + rank * 128;
+            const int row0 = tm * 2 * BM2 + rank * BM2, col0 = swiglu ? tl * 128 : tl * BN + rank * (BN / 2);
             // A run: k-blocks whose operands lie one behind the other in the same two tensors.  Modes 1 and 3 pick B by problem (mode 3 also A), mode 4
             // gives CTA 0 the gate weights and CTA 1 the up weights (same 128 columns).
             const CUtensorMap* pA = grp.mode == 3 ? (g == 0 ? &tmA : (g == 1 ? &tmA1 : &tmA2)) : &tmA;
@@ -355,7 +354,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
                     if (it >= (uint32_t)nst && !mbar_wait_warp(bar_empty + 8 * s, ph ^ 1, abort_flag)) { ok = false; break; }
                     const uint32_t sa = smem_base + s * STAGE_BYTES2, sb = sa + A_BYTES2;
                     const uint32_t fb = full_leader + 8 * s;
-                    if (rank == 0) mbar_expect_tx_e(bar_full + 8 * s, 2 * STAGE_BYTES2);   // both CTAs' bytes land on this barrier
+                    if (rank == 0) mbar_expect_tx_e(bar_full + 8 * s, 2 * (A_BYTES2 + BN * BK2));   // both CTAs' bytes land on this barrier
                     if (A_MN) {
                         if (whole) tma_load_3d_pair_e(sa, pA, fb, 0, x, row0 >> 6);
                         else { tma_load_2d_pair_e(sa, pA, fb, row0, x); tma_load_2d_pair_e(sa + 8192, pA, fb, row0 + 64, x); }
@@ -363,8 +362,12 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
                         tma_load_2d_pair_e(sa, pA, fb, x, row0);
                     }
                     if (B_MN) {
-                        if (whole) tma_load_3d_pair_e(sb, pB, fb, 0, yb, col0 >> 6);
-                        else { tma_load_2d_pair_e(sb, pB, fb, col0, yb); tma_load_2d_pair_e(sb + 8192, pB, fb, col0 + 64, yb); }
+                        if (B_BLK == BN / 2) tma_load_2d_pair_e(sb, pB, fb, col0, yb);
+                        else if (whole) tma_load_3d_pair_e(sb, pB, fb, 0, yb, col0 / B_BLK);
+                        else {
+#pragma unroll
+                            for (int z = 0; z < BN / 2; z += B_BLK) tma_load_2d_pair_e(sb + z * BK2 * 2, pB, fb, col0 + z, yb);
+                        }
                     } else {
                         tma_load_2d_pair_e(sb, pB, fb, x, col0);
                     }
@@ -375,12 +378,13 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
         if (!ok && lane == 0) { *abort_flag = 1; atomicExch(status, STAT_GEMM2 | 1); }
     } else if (warp == 1 && rank == 0) {
         // ── MMA issuer (leader CTA only): the whole warp runs the loop converged, one elected lane issues ──
-        constexpr uint32_t idesc = tc_idesc_bf16(256, BN2, A_MN, B_MN);
-        // descriptor words: the upper one is a constant (SBO 1024, 128-byte swizzle), the lower one is
-        // (address >> 4) | (LBO >> 4) << 16; a k-step of 16 advances it by 2048 B (MN-major) or 32 B (K-major)
-        constexpr uint32_t dhi = (1024u >> 4) | (1u << 14) | (2u << 29);
-        constexpr uint32_t a_step = A_MN ? 128 : 2, b_step = B_MN ? 128 : 2;
-        constexpr uint32_t a_lbo = (A_MN ? 8192u : 16u) >> 4, b_lbo = (B_MN ? 8192u : 16u) >> 4;
+        constexpr uint32_t idesc = tc_idesc_bf16(256, BN, A_MN, B_MN);
+        // descriptor words: the upper one is a constant (SBO 1024, 128-byte swizzle; 512 and 64 for blocks of 32 columns), the lower one is
+        // (address >> 4) | (LBO >> 4) << 16; a k-step of 16 advances it by 2048 B (MN-major; 1024) or 32 B (K-major)
+        constexpr bool b64 = B_MN && B_BLK == 32;
+        constexpr uint32_t dhi = (1024u >> 4) | (1u << 14) | (2u << 29), dhi_b = b64 ? (512u >> 4) | (1u << 14) | (4u << 29) : dhi;
+        constexpr uint32_t a_step = A_MN ? 128 : 2, b_step = B_MN ? (b64 ? 64 : 128) : 2;
+        constexpr uint32_t a_lbo = (A_MN ? 8192u : 16u) >> 4, b_lbo = (B_MN ? B_BLK * BK2 * 2u : 16u) >> 4;
         uint32_t it = 0, tcount = 0, ph = 0;
         int s = 0;
         bool ok = true;
@@ -391,7 +395,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
             const uint32_t aph = (tcount >> 1) & 1;
             if (tcount >= 2 && !mbar_wait_warp(bar_tempty + 8 * acc, aph ^ 1, abort_flag)) { ok = false; break; }
             tc_fence_after();
-            const uint32_t d_tmem = tmem_base + acc * BN2;
+            const uint32_t d_tmem = tmem_base + acc * 256;
             for (int kb = kb0; kb < kb1; kb++, it++, s = (s + 1 == nst ? 0 : s + 1), ph ^= (s == 0)) {
                 if (!mbar_wait_warp(bar_full + 8 * s, ph, abort_flag)) { ok = false; break; }
                 tc_fence_after();
@@ -400,7 +404,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
                 const uint32_t a_lo = ((sa & 0x3FFFF) >> 4) | (a_lbo << 16), b_lo = ((sb & 0x3FFFF) >> 4) | (b_lbo << 16);
 #pragma unroll
                 for (int kk = 0; kk < BK2 / 16; kk++)
-                    tc_mma_ss2_e(d_tmem, ((uint64_t)dhi << 32) | (a_lo + kk * a_step), ((uint64_t)dhi << 32) | (b_lo + kk * b_step),
+                    tc_mma_ss2_e(d_tmem, ((uint64_t)dhi << 32) | (a_lo + kk * a_step), ((uint64_t)dhi_b << 32) | (b_lo + kk * b_step),
                                  idesc, (kb != kb0) || (kk != 0));
                 tc_commit2_e(bar_empty + 8 * s, both);       // frees the stage in both CTAs
             }
@@ -438,20 +442,20 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
             const int row = row0 + lane;
             const int cw = f32_out ? 32 : 64;                   // columns per 128-byte piece
             const CUtensorMap* pC = g == 0 ? &tmC : (g == 1 ? &tmC1 : &tmC2);
-            const int ncols = min(BN2, ((grp.mode == 1 || grp.mode == 3) ? grp.n[g] : n) - tl * BN2);
+            const int ncols = min(BN, ((grp.mode == 1 || grp.mode == 3) ? grp.n[g] : n) - tl * BN);
             const int m_g = grp.mode == 3 ? grp.m[g] : m;
             // pieces of this tile that this warp writes: half, half + NH, ...
             const int pw = swb ? 32 : cw;
             const int npt = (tma_out && !swiglu && row0 < m_g) ? (ncols + pw - 1) / pw : 0;
-            const int j0 = SHARE ? part * (BN2 / cw / S) : 0;   // a shared tile: this part's 256 / S columns
-            const int npc = SHARE ? max(0, min(npt - j0, BN2 / cw / S)) : (npt - half + NH - 1) / NH;
+            const int j0 = SHARE ? part * (BN / cw / S) : 0;   // a shared tile: this part's 256 / S columns
+            const int npc = SHARE ? max(0, min(npt - j0, BN / cw / S)) : (npt - half + NH - 1) / NH;
             const uint32_t pbase = pieces;
             const bool do_rope = EPI == EPI_ROPE && ((grp.rope_mask >> g) & 1);
             const int rope_t = do_rope ? (row < m_g ? row : 0) % grp.rope_T : 0;
             // lane 0: piece i of this warp of the addend, or of g and u, -> its buffer
             auto fetch_d = [&](int i) {
                 const uint32_t bi = (pbase + i) & (nbuf - 1);
-                const int x = tn * BN2 + (j0 + half + NH * i) * pw;
+                const int x = tn * BN + (j0 + half + NH * i) * pw;
                 mbar_expect_tx(my_bar_d + 8 * bi, 4096);
                 tma_load_3d(stg_u32 + bi * 4096, &tmD, my_bar_d + 8 * bi, x, row0, 0);
                 if (swb) tma_load_3d(stg_u32 + bi * 4096 + 2048, &tmC2, my_bar_d + 8 * bi, x, row0, 0);
@@ -473,7 +477,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
             if (!mbar_wait(bar_tfull + 8 * acc, aph) || *abort_flag) ok = false;
             tc_fence_after();
             if (timing && threadIdx.x == 64) prof[5] = clock64();
-            const uint32_t taddr = tmem_base + acc * BN2 + ((uint32_t)(quad * 32) << 16);
+            const uint32_t taddr = tmem_base + acc * 256 + ((uint32_t)(quad * 32) << 16);
             const int own = 8 / S;                              // 32-column chunks of a part
             // sums of the other parts in this CTA's operand ring: [part][lane quarter][chunk][4 columns][row], 512 bytes in a row per warp
             auto part_at = [&](int from, int c) { return ((from - (from > part)) * 4 + quad) * own * 4096 + c * 4096 + lane * 16; };
@@ -571,7 +575,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
                 for (int i = 0; i < npc; i++) {
                     const uint32_t bi = (pbase + i) & (nbuf - 1);
                     uint8_t* buf = stg + bi * 4096 + lane * 64;
-                    const int x = tn * BN2 + (half + NH * i) * 32;
+                    const int x = tn * BN + (half + NH * i) * 32;
                     uint32_t r[32];
                     tmem_ld32(taddr + (half + NH * i) * 32, r);
                     if (!mbar_wait(my_bar_d + 8 * bi, (dpar >> bi) & 1)) { ok = false; break; }
@@ -694,7 +698,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     __syncwarp();
                     if (lane == 0) {
-                        tma_store_3d(pC, stg_u32 + bi * 4096, tl * BN2 + c, row0, ksplit > 1 ? split : 0);
+                        tma_store_3d(pC, stg_u32 + bi * 4096, tl * BN + c, row0, ksplit > 1 ? split : 0);
                         bulk_commit2();
                     }
                     pieces++;
@@ -705,11 +709,11 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
                 const TO* drow = (D && beta != 0.f) ? D + (long long)row * n : nullptr;
                 float* wrow = ws + ((long long)split * m + row) * n;
 #pragma unroll 1
-                for (int c = half * (BN2 / NH); c < (half + 1) * (BN2 / NH); c += 32) {
+                for (int c = half * (BN / NH); c < (half + 1) * (BN / NH); c += 32) {
                     uint32_t r[32];
                     tmem_ld32(taddr + c, r);
                     tmem_ld_wait();
-                    const int col0 = tn * BN2 + c;
+                    const int col0 = tn * BN + c;
                     if (row < m && col0 < n) {
                         if (ksplit > 1) epi_store<float>(wrow, nullptr, r, col0, n - col0, 1.f, 0.f, (n & 3) == 0);
                         else epi_store<TO>(crow, drow, r, col0, n - col0, alpha, beta, vec_ok);
@@ -737,15 +741,16 @@ extern int ax_gemm_pdl(void);
 extern int ax_gemm_mode(void);
 extern int ax_gemm_tma_out(void);
 extern bool ax_gemm_on_side(void);
+extern bool ax_gemm_beside(void);
 template <typename TO>
 void ax_splitk_reduce_launch(const float* ws, int ksplit, TO* C, const TO* D, long long mn, float alpha, float beta, cudaStream_t st);
 
 // co-resident clusters of S pairs of this kernel (0: none)
-template <int A_MN, int B_MN, typename TO, int EPI = EPI_PLAIN, int S = 1>
+template <int A_MN, int B_MN, typename TO, int EPI = EPI_PLAIN, int S = 1, int BN = 256>
 static int clusters_for() {
     static int g_max = -1;
     if (g_max < 0) {
-        cudaFuncSetAttribute(k_gemm_tc2<A_MN, B_MN, TO, EPI, (S > 1)>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM2);
+        cudaFuncSetAttribute(k_gemm_tc2<A_MN, B_MN, TO, EPI, (S > 1), BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM2);
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(AX_SMS / (2 * S) * 2 * S, 1, 1);
         cfg.blockDim = dim3(EpiCfg<EPI>::THREADS, 1, 1);
@@ -755,25 +760,27 @@ static int clusters_for() {
         at[0].val.clusterDim.x = 2 * S; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
         cfg.attrs = at; cfg.numAttrs = 1;
         int nc = 0;
-        if (cudaOccupancyMaxActiveClusters(&nc, k_gemm_tc2<A_MN, B_MN, TO, EPI, (S > 1)>, &cfg) != cudaSuccess || nc < 1) { cudaGetLastError(); nc = 0; }
+        if (cudaOccupancyMaxActiveClusters(&nc, k_gemm_tc2<A_MN, B_MN, TO, EPI, (S > 1), BN>, &cfg) != cudaSuccess || nc < 1) { cudaGetLastError(); nc = 0; }
         g_max = nc;
     }
     return g_max;
 }
 static int g_share_max[2] = {0, 0};      // the least of that over the kernels that share a tile, for 2 and 4 pairs
 
-// operand / output tensor maps of one problem.  An M- or N-major operand [k, e] is loaded as two blocks of 64 elements by 64 rows, with one
-// instruction where its rows are whole blocks: as {64, k, e / 64}.  (A block that reached past the end of a row would read the next one.)
-static int map_mn(CUtensorMap* t, const void* p, int e, int k, bool whole) {
-    uint64_t dims[3] = {64, (uint64_t)k, (uint64_t)e / 64}, strides[2] = {(uint64_t)e * 2, 128};
-    uint32_t box[3] = {64, BK2, 2};
+// operand / output tensor maps of one problem.  An M- or N-major operand [k, e] is loaded as blocks of `blk` (64; 32: see b_block) elements by 64 rows, all of
+// a CTA's `ext` elements with one instruction where its rows are whole blocks: as {blk, k, e / blk}.  (A block that reached past the end of a row
+// would read the next one.)
+static int map_mn(CUtensorMap* t, const void* p, int e, int k, bool whole, int ext, int blk) {
+    uint64_t dims[3] = {(uint64_t)blk, (uint64_t)k, (uint64_t)e / blk}, strides[2] = {(uint64_t)e * 2, (uint64_t)blk * 2};
+    uint32_t box[3] = {(uint32_t)blk, BK2, (uint32_t)(ext / blk)};
+    whole = whole && ext > blk;
     if (!whole) dims[0] = e;
-    return tc_make_tmap_bf16(t, p, whole ? 3 : 2, dims, strides, box, true);
+    return tc_make_tmap_bf16(t, p, whole ? 3 : 2, dims, strides, box, blk == 64 ? 128 : 64);
 }
-static int map_km(CUtensorMap* t, const void* p, int e, int k) {
+static int map_km(CUtensorMap* t, const void* p, int e, int k, int ext) {
     uint64_t dims[2] = {(uint64_t)k, (uint64_t)e}, strides[1] = {(uint64_t)k * 2};
-    uint32_t box[2] = {BK2, 128};
-    return tc_make_tmap_bf16(t, p, 2, dims, strides, box, true);
+    uint32_t box[2] = {BK2, (uint32_t)ext};
+    return tc_make_tmap_bf16(t, p, 2, dims, strides, box, 128);
 }
 // {n, m, nz} tensor of osz-byte elements, pieces of 128 bytes (half_row: 64) x 32 rows
 static int map_c(CUtensorMap* t, void* base, int m, int n, int nz, int osz, bool half_row = false) {
@@ -821,18 +828,41 @@ static int band_of(int m, long long k) {
     return 2ll * m * k > 52000000ll && tiles_m > 12 ? 12 : tiles_m;
 }
 
+// Columns of a tile.  A launch is a set-up, a first load and the last tile's epilogue (f) and, for each round of tiles over the pairs, the
+// k-blocks (t), which for narrow tiles are bound by shared memory: 512 / 385 / 355 cycles by themselves.  us of 256 / 192 / 128 columns in chains of launches:
+// 2000 x 1536 x 1536 (48, 64, 96 tiles) 12.8 / 11.3 / 13.6, x 4096 24.8 / 21.8 / 28.1, 8192 x 768 x 2304 (96, 128, 192) 26.6 / 23.2 / 27.9, 1536 x 1024 x 1024
+// (24 shared by two pairs, 36, 48) 9.5 / 8.2 / 7.7, x 2816 15.3 / 14.8 / 13.0, x 5632 20.7 / 24.6 / 22.7, 2000 x 4096 x 1536 (128, 176, 256) 21.3 / 22.9 / 25.4.
+// Only while a plan has queued nothing beside the main chain (see ax_gemm_plan_begin): products on the side stream fill the pairs that wide tiles leave, and
+// the step of 8 x 1024 tokens at D 768 takes 5114 us with narrow ones throughout, 5037 without.  Steps with adapters are 1 to 2 % shorter, small ones up to 5.
+// With three rounds or more the rounds even out and the wide tile, which moves the least, is the best under the power limit: 8192 x 1536 x 2560 (192, 256, 384)
+// 48.6 / 49.5 / 58.4.
+static int g_pairs = 0;                  // pairs that run at once
+TileTimes ax_gemm_tc2_width(const long long* tiles /* of 256, 192, 128 columns */, int kb, bool may_share) {
+    static const int width[3] = {256, 192, 128};
+    static const double f[3] = {5.6, 4.95, 4.3}, t[3] = {0.30, 0.263, 0.185};
+    TileTimes best = {256, 0.0};
+    for (int i = 0; i < 3; i++) {
+        const long long rounds = g_pairs > 0 ? (tiles[i] + g_pairs - 1) / g_pairs : 1;
+        double us = f[i] + t[i] * rounds * kb, shared;
+        if (i == 0 && may_share && tiles[0] <= 33 && ax_gemm_tc2_share((int)tiles[0], kb, &shared) > 1) us = f[0] + t[0] * shared;
+        if (i == 0) best.us = us;
+        else if (tiles[0] <= 2 * g_pairs && us < best.us * 0.97) best = {width[i], us};
+    }
+    return best;
+}
+
 struct SwbArgs { const void* g; const void* u; void* du; };    // SwiGLU backward in the epilogue (C = dg)
 
 // One launch.  grp.mode 0: the plain GEMM (A, B, C, D are element 0 of the arrays).  Grouped modes: see GemmGroup;
 // n[] / k[] then hold the per-problem widths (mode 1) or per-segment depths (mode 2).
 // Extra K-segments of a grouped launch: mode 1 — problem g adds XA[g] XB[g] (depth xk) to its output; mode 2 — they are
 // appended to the launch's own segments (A, B, kv then hold count + xcount entries, at most 6).
-template <int A_MN, int B_MN, typename TO, int EPI = EPI_PLAIN>
+template <int A_MN, int B_MN, typename TO, int EPI = EPI_PLAIN, int BN = 256>
 static int gemm2_launch(int mode, int count, const void* const* A, const void* const* B, void* const* C, const void* D,
                         const int* mv, const int* nv, const int* kv, float alpha, float beta, int* status, int ksplit, cudaStream_t st,
                         const void* const* XA = nullptr, const void* const* XB = nullptr, int xk = 0, const SwbArgs* swb = nullptr) {
-    constexpr bool CAN_SHARE = EPI == EPI_PLAIN || EPI == EPI_ROPE;
-    const int maxp = clusters_for<A_MN, B_MN, TO, EPI>();
+    constexpr bool CAN_SHARE = BN == 256 && (EPI == EPI_PLAIN || EPI == EPI_ROPE);
+    const int maxp = clusters_for<A_MN, B_MN, TO, EPI, 1, BN>();
     if (maxp < 1) return -1;
     const int m = mv[0], n = nv[0], k = kv[0];
     GemmGroup grp = {};
@@ -846,20 +876,20 @@ static int gemm2_launch(int mode, int count, const void* const* A, const void* c
     }
     CUtensorMap tmA[3], tmB[3], tmC[3], tmD, tmEA[3], tmEB[3];
     grp.whole = 1;
-    for (int g = 0; g < (mode == 1 || mode == 3 ? count : 1); g++) grp.whole = grp.whole && (!A_MN || mv[mode == 3 ? g : 0] % 64 == 0) && (!B_MN || nv[g] % 64 == 0);
-    auto map_a = [&](CUtensorMap* t, const void* p, int e, int depth) { return A_MN ? map_mn(t, p, e, depth, grp.whole) : map_km(t, p, e, depth); };
-    auto map_b = [&](CUtensorMap* t, const void* p, int e, int depth) { return B_MN ? map_mn(t, p, e, depth, grp.whole) : map_km(t, p, e, depth); };
+    for (int g = 0; g < (mode == 1 || mode == 3 ? count : 1); g++) grp.whole = grp.whole && (!A_MN || mv[mode == 3 ? g : 0] % 64 == 0) && (!B_MN || nv[g] % b_block(BN) == 0);
+    auto map_a = [&](CUtensorMap* t, const void* p, int e, int depth) { return A_MN ? map_mn(t, p, e, depth, grp.whole, 128, 64) : map_km(t, p, e, depth, 128); };
+    auto map_b = [&](CUtensorMap* t, const void* p, int e, int depth) { return B_MN ? map_mn(t, p, e, depth, grp.whole, BN / 2, b_block(BN)) : map_km(t, p, e, depth, BN / 2); };
     bool have_x = false;
     int tiles_n = 0;
     if (mode == 0) {
         if (map_a(&tmA[0], A[0], m, k) || map_b(&tmB[0], B[0], n, k)) return 2;
-        tiles_n = (n + 255) / 256;
+        tiles_n = (n + BN - 1) / BN;
     } else if (mode == 1) {
         if (map_a(&tmA[0], A[0], m, k)) return 2;
         for (int g = 0; g < count; g++) {
             if (map_b(&tmB[g], B[g], nv[g], k)) return 2;
             grp.n[g] = nv[g];
-            tiles_n += (nv[g] + 255) / 256;
+            tiles_n += (nv[g] + BN - 1) / BN;
             if (XA && xk > 0) {
                 if (map_a(&tmEA[g], XA[g], m, xk) || map_b(&tmEB[g], XB[g], nv[g], xk)) return 2;
                 have_x = true;
@@ -875,7 +905,7 @@ static int gemm2_launch(int mode, int count, const void* const* A, const void* c
             grp.kb[g] = (kv[g] + BK2 - 1) / BK2;
         }
         have_x = count > 3;
-        tiles_n = (n + 255) / 256;
+        tiles_n = (n + BN - 1) / BN;
     } else if (mode == 3) {
         for (int g = 0; g < count; g++) {
             if (map_a(&tmA[g], A[g], mv[g], k) || map_b(&tmB[g], B[g], nv[g], k)) return 2;
@@ -895,7 +925,7 @@ static int gemm2_launch(int mode, int count, const void* const* A, const void* c
     const bool per_problem_c = mode == 1 || mode == 3;
     // output through TMA tile stores when the destination allows it: 1 = no addend to read, 2 = addend by TMA too
     int units = ((m + 255) / 256) * tiles_n;
-    if (mode == 3) { units = 0; for (int g = 0; g < count; g++) units += ((mv[g] + 255) / 256) * ((nv[g] + 255) / 256); }
+    if (mode == 3) { units = 0; for (int g = 0; g < count; g++) units += ((mv[g] + 255) / 256) * ((nv[g] + BN - 1) / BN); }
     if (mode == 4) units = ((m + 255) / 256) * ((n + 127) / 128);
     int kb = (k + BK2 - 1) / BK2 + grp.xkb;
     if (mode == 2) { kb = 0; for (int g = 0; g < count; g++) kb += grp.kb[g]; }
@@ -970,8 +1000,8 @@ static int gemm2_launch(int mode, int count, const void* const* A, const void* c
                                   tmEA[0], tmEA[1], tmEA[2], tmEB[0], tmEB[1], tmEB[2], grp, tma_out, Cp, Dp, m, n, k, alpha, beta, status, ksplit, ws, prof);
     };
     cudaError_t err;
-    if constexpr (CAN_SHARE) err = grp.S > 1 ? launch(k_gemm_tc2<A_MN, B_MN, TO, EPI, true>) : launch(k_gemm_tc2<A_MN, B_MN, TO, EPI, false>);
-    else err = launch(k_gemm_tc2<A_MN, B_MN, TO, EPI, false>);
+    if constexpr (CAN_SHARE) err = grp.S > 1 ? launch(k_gemm_tc2<A_MN, B_MN, TO, EPI, true, BN>) : launch(k_gemm_tc2<A_MN, B_MN, TO, EPI, false, BN>);
+    else err = launch(k_gemm_tc2<A_MN, B_MN, TO, EPI, false, BN>);
     if (err != cudaSuccess) return 3;
 #ifdef AXENG_PROF
     if (prof) {
@@ -996,26 +1026,34 @@ int ax_gemm_tc2_init(void) {
     const int v[9] = {ALL_KERNELS(1), clusters_for<0, 1, bf16, EPI_SWIGLU>(), clusters_for<0, 0, bf16, EPI_SWB>()};
     const int v2[7] = {ALL_KERNELS(2)}, v4[7] = {ALL_KERNELS(4)};
 #undef ALL_KERNELS
+#define NARROW(W) clusters_for<0, 1, bf16, EPI_PLAIN, 1, W>(), clusters_for<0, 1, float, EPI_PLAIN, 1, W>(), clusters_for<0, 0, bf16, EPI_PLAIN, 1, W>(),      \
+                  clusters_for<0, 0, float, EPI_PLAIN, 1, W>(), clusters_for<1, 1, bf16, EPI_PLAIN, 1, W>(), clusters_for<1, 1, float, EPI_PLAIN, 1, W>(), \
+                  clusters_for<0, 1, bf16, EPI_ROPE, 1, W>(), clusters_for<0, 0, bf16, EPI_SWB, 1, W>()
+    for (int x : {NARROW(192), NARROW(128)}) worst = x < worst ? x : worst;
+#undef NARROW
     g_share_max[0] = g_share_max[1] = AX_SMS;
     for (int i = 0; i < 7; i++) {
         g_share_max[0] = v2[i] < g_share_max[0] ? v2[i] : g_share_max[0];
         g_share_max[1] = v4[i] < g_share_max[1] ? v4[i] : g_share_max[1];
     }
     for (int i = 0; i < 9; i++) worst = v[i] < worst ? v[i] : worst;
+    g_pairs = worst;
     return worst;      // pairs that can run together (<= 0: the paired kernel is unavailable)
 }
 
 // Same argument meaning as ax_gemm_tc; returns -1 when the paired kernel cannot run here.
 int ax_gemm_tc2(int out_bf16, int tb, const void* A, const void* B, void* C, const void* D,
-                int m, int n, int k, float alpha, float beta, int* status, int ksplit, cudaStream_t st) {
+                int m, int n, int k, float alpha, float beta, int* status, int ksplit, int bn, cudaStream_t st) {
     const void* Av[1] = {A}; const void* Bv[1] = {B}; void* Cv[1] = {C};
-#define G2(AM, BMj)                                                                                                            \
-    (out_bf16 ? gemm2_launch<AM, BMj, bf16>(0, 1, Av, Bv, Cv, D, &m, &n, &k, alpha, beta, status, ksplit, st)                 \
-              : gemm2_launch<AM, BMj, float>(0, 1, Av, Bv, Cv, D, &m, &n, &k, alpha, beta, status, ksplit, st))
+#define G2W(AM, BMj, T, W) gemm2_launch<AM, BMj, T, EPI_PLAIN, W>(0, 1, Av, Bv, Cv, D, &m, &n, &k, alpha, beta, status, ksplit, st)
+#define G2T(AM, BMj, T) (bn == 256 ? G2W(AM, BMj, T, 256) : bn == 192 ? G2W(AM, BMj, T, 192) : G2W(AM, BMj, T, 128))
+#define G2(AM, BMj) (out_bf16 ? G2T(AM, BMj, bf16) : G2T(AM, BMj, float))
     if (tb == 0) return G2(0, 1);
     if (tb == 1) return G2(0, 0);
     return G2(1, 1);
 #undef G2
+#undef G2T
+#undef G2W
 }
 
 // Grouped launch (see GemmGroup).  mode 1: A[0] shared, B[g] / C[g] / n[g] per problem, m[0], k[0].  mode 2: A[s] / B[s] /
@@ -1053,14 +1091,27 @@ int ax_gemm_tc2_group(int out_bf16, int tb, int mode, int count, const void* con
         if (bad) { g_rope_req.rope_mask = 0; return -1; }
     }
     ax_variant = 0x23;
-#define G2X(AM, BMj, T, EPI) gemm2_launch<AM, BMj, T, EPI>(mode, count, A, B, C, D, m, n, k, alpha, D ? beta : 0.f, status, 1, st, XA, XB, xk, swb)
+    // (a caller who forces this kernel gets the wide tiles, and what they share, as they are)
+    int bn = 256;
+    if (ax_gemm_mode() == 0 && !ax_gemm_beside() && (mode == 1 || mode == 2)) {
+        long long tiles[3] = {0, 0, 0};
+        int kb = mode == 1 && XA ? (xk + BK2 - 1) / BK2 : 0;
+        for (int g = 0; g < (mode == 2 ? count : 1); g++) kb += (k[g] + BK2 - 1) / BK2;
+        for (int i = 0; i < 3; i++)
+            for (int g = 0; g < (mode == 1 ? count : 1); g++) tiles[i] += (long long)((m[0] + 255) / 256) * ((n[g] + 255 - 64 * i) / (256 - 64 * i));
+        bn = ax_gemm_tc2_width(tiles, kb, !swb).width;
+    }
+    ax_gemm_width = mode == 4 ? 256 : bn;
+#define G2W(AM, BMj, T, EPI, W) gemm2_launch<AM, BMj, T, EPI, W>(mode, count, A, B, C, D, m, n, k, alpha, D ? beta : 0.f, status, 1, st, XA, XB, xk, swb)
+#define G2X(AM, BMj, T, EPI) (bn == 256 ? G2W(AM, BMj, T, EPI, 256) : bn == 192 ? G2W(AM, BMj, T, EPI, 192) : G2W(AM, BMj, T, EPI, 128))
 #define G2(AM, BMj) (out_bf16 ? G2X(AM, BMj, bf16, EPI_PLAIN) : G2X(AM, BMj, float, EPI_PLAIN))
     if (swb) return G2X(0, 0, bf16, EPI_SWB);
-    if (mode == 4) return G2X(0, 1, bf16, EPI_SWIGLU);
+    if (mode == 4) return G2W(0, 1, bf16, EPI_SWIGLU, 256);
     if (rope_mask) return G2X(0, 1, bf16, EPI_ROPE);
     if (tb == 0) return G2(0, 1);
     if (tb == 1) return G2(0, 0);
     return G2(1, 1);
 #undef G2X
+#undef G2W
 #undef G2
 }

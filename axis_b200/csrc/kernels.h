@@ -18,6 +18,7 @@
 //   0x80 / 0x81 attention forward / backward with split probabilities on tcgen05, 0x82 / 0x83 on mma.sync (0x83 + 0x100 * CTAs to a key tile)
 extern int ax_variant;
 extern int ax_gemm_parts;     // see eng_last_gemm_parts
+extern int ax_gemm_width;     // see eng_last_gemm_width
 
 // elementwise.cu
 int ax_binary(int which, int dt, const void* a, const void* b, void* c, long long n, cudaStream_t st); // 0 add 1 mul 2 silu_mul
@@ -100,8 +101,10 @@ int ax_gemm_tc(int out_bf16, int tb, const void* A, const void* B, void* C, cons
 int ax_gemm_tc2_init(void);
 int ax_gemm_tc2_share(int tiles, int kb, double* cost);
 bool ax_gemm_tc2_by_tma(const void* C, const void* D, long long n, int osz);
+struct TileTimes { int width; double us; };
+TileTimes ax_gemm_tc2_width(const long long* tiles, int kb, bool may_share);      // tiles of 256, 192 and 128 columns
 int ax_gemm_tc2(int out_bf16, int tb, const void* A, const void* B, void* C, const void* D,
-                int m, int n, int k, float alpha, float beta, int* status, int ksplit, cudaStream_t st);
+                int m, int n, int k, float alpha, float beta, int* status, int ksplit, int width, cudaStream_t st);
 void ax_gemm_set_mode(int mode);      // 0 auto, 1 single-CTA only, 2 paired whenever possible
 
 // attn_simt.cu — exact-fp32 causal GQA attention on strided layouts.
@@ -125,6 +128,7 @@ int ax_attn_simt_share(int which, const AttnShape& s);      // see eng_attn_shar
 // gemm_tc2.cu — grouped launch of the paired-CTA GEMM (mode 1: shared A, per-problem B/C/n; mode 2: one C summed
 // over per-segment A/B/k; mode 3: independent problems A/B/C/m/n of one depth k).  -1 when not served.
 void ax_gemm_side(int on);
+void ax_gemm_plan_begin(void);
 // Rotary request for the NEXT ax_gemm_tc2_group call (mode 1, bf16 output, tb 0): outputs g with bit g of `mask` set are
 // [rows, heads * 64] projections and leave the launch rotated (tables fp32 [T, 32], row = batch * T + token).  The call
 // either honours the request or returns -1; it never ignores it.

@@ -139,4 +139,4 @@ typedef CUresult (*PFN_tmapEncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuin
 PFN_tmapEncodeTiled tc_encode_fn();
 // bf16 tensor of `rank` dims; dims[0] is the contiguous one; strides_bytes[i] is the stride of dims[i+1].
 int tc_make_tmap_bf16(CUtensorMap* out, const void* base, int rank, const uint64_t* dims, const uint64_t* strides_bytes,
-                      const uint32_t* box, bool swizzle128);
+                      const uint32_t* box, int swizzle);      // swizzle: bytes, 128 or 64 (0: none)

@@ -363,6 +363,10 @@ class Engine:
         """Pairs of CTAs that shared a tile's depth in the last paired-CTA launch (include/axeng.h)."""
         return int(self.lib.eng_last_gemm_parts())
 
+    def last_gemm_width(self) -> int:
+        """Columns of a tile in the last paired-CTA GEMM launch: 256, 192 or 128."""
+        return int(self.lib.eng_last_gemm_width())
+
     def bytes_allocated(self) -> int:
         return int(self.lib.eng_bytes_allocated())
 

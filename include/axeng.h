@@ -170,6 +170,8 @@ long long eng_bytes_allocated(void);
 int eng_last_variant(void);
 /* Pairs of CTAs that shared the depth of a tile in the last paired-CTA tcgen05 launch: 1, 2 or 4. */
 int eng_last_gemm_parts(void);
+/* Columns of a tile in the last launch of the paired-CTA GEMM: 256, 192 or 128. */
+int eng_last_gemm_width(void);
 /* Whether bf16 attention of this shape, in the layout of ENG_ATTN_FWD / ENG_ATTN_BWD and with aligned buffers, runs on the tcgen05
  * kernels with split probabilities once the whole-tile kernels have refused it (for the backward the number of CTAs that share a key tile,
  * 1, 2 or 4) or not (0): host arithmetic that needs no GPU. */

@@ -1053,3 +1053,69 @@ def test_operands_of_whole_64_blocks_and_others(eng, tb, dt, m, n, k):
     got, ref = run_gemm(eng, np.random.default_rng(m + n + k), m, n, k, tb, dt, fallback=8)
     check(got, ref, dt == 1, k)
     assert eng.device_status() == 0
+
+
+@pytest.mark.parametrize("tb", [0, 1, 2])
+@pytest.mark.parametrize("dt,addend", [(1, False), (1, True), (2, False), (2, True)])
+@pytest.mark.parametrize("m,n,k,width", [(2000, 1504, 640, 192), (2000, 1416, 712, 192), (1304, 776, 1000, 128), (1288, 640, 1000, 128)])
+def test_narrow_tiles_where_wide_ones_leave_pairs_idle(eng, tb, dt, addend, m, n, k, width):
+    """Tiles of 192 and 128 columns: last tiles of 160, 72, 8 and 128 columns, rows of B that are whole blocks of 32 or 64 and rows that are not.  A column's sum
+    does not depend on the tile: where the wide ones share no depth (40 or more of them) the bits are theirs."""
+    kw = dict(beta=-2.0, addend=True) if addend else dict(alpha=0.5)
+    got, ref = run_gemm(eng, np.random.default_rng(m + n), m, n, k, tb, dt, **kw)
+    assert (eng.last_variant(), eng.last_gemm_parts(), eng.last_gemm_width()) == (0x122, 1, width)
+    check(got, ref, dt == 1, k)
+    wide, _ = run_gemm(eng, np.random.default_rng(m + n), m, n, k, tb, dt, fallback=8, **kw)
+    assert eng.last_gemm_width() == 256 and (width != 192 or np.array_equal(got, wide))
+    assert eng.device_status() == 0
+
+
+@pytest.mark.parametrize("r", [0, 16])
+@pytest.mark.parametrize("m,k,ns,width", [(3000, 640, (768, 192, 192), 192), (2904, 264, (704, 192, 128), 192), (1800, 72, (576, 64, 72), 128)])
+def test_narrow_tiles_of_groups_have_the_bits_of_wide_ones(eng, m, k, ns, width, r):
+    """Projections of one input, two of them rotated, with and without low-rank terms; sums over segments with an addend; the SwiGLU backward.  Against the wide
+    tiles of the forced kernel (too many to share their depth, which has another order), whose tests compare them with float64."""
+    rng = np.random.default_rng(m + k + r)
+    mk = lambda *sh: put(eng, bf(rng.standard_normal(sh).astype(np.float32) * 0.3), 1)
+    cos, sin = O.rope_tables(m // 4, 64)
+    ix, iw, ia, ib = mk(m, k), [mk(k, n) for n in ns], [mk(m, 16) for _ in ns], [mk(16, n) for n in ns]
+    ic, isn = put(eng, cos, 0), put(eng, sin, 0)
+    n, gs, wt = ns[0], [mk(m, q) for q in ns], [mk(ns[0], q) for q in ns]
+    res, g, u = mk(m, n), mk(m, n), mk(m, n)
+    outs = [eng.alloc(m * q, 2) for q in ns] + [eng.alloc(m * n, 2) for _ in range(4)]
+    xseg = [op(E.GEMM_XSEG, a=ia[0], b=ia[1], d=ia[2], sa=ib[0], sb=ib[1], sc=ib[2], k=r, batch=3)] if r else []
+    addend = [op(E.GEMM_XSEG, a=0, b=0, d=0, sa=0, sb=0, sc=0, k=0, batch=0, c=res, beta=1.0)] if r else []
+    q, kk, v, y, dh, dg, du = outs
+    plans = [xseg + [op(E.GEMM_GROUP, a=ix, b=iw[0], sa=iw[1], sb=iw[2], c=q, d=kk, sc=v, m=m, k=k, n=ns[0], oa=ns[1], ob=ns[2], batch=3, oc=1, dt=1,
+                        beta=float(ic), gamma=float(isn))],
+             addend + [op(E.GEMM_GROUP, c=y, a=gs[0], sa=gs[1], sb=gs[2], b=wt[0], d=wt[1], sc=wt[2], m=m, n=n, k=ns[0], oa=ns[1], ob=ns[2], batch=3, oc=2, tb=1, dt=1)],
+             [op(E.GEMM_SB, a=gs[0], b=wt[0], c=dh, m=m, n=n, k=ns[0], batch=1, tb=1, dt=1), op(E.SILU_BWD, a=g, b=u, d=dh, c=dg, tb=du, n=m * n, dt=1, oa=1)]]
+    runs, widths = [], []
+    for mask in (0, 8):
+        eng.set_fallback(mask)
+        for p in plans:
+            eng.run(p)
+            widths.append(eng.last_gemm_width())
+        eng.set_fallback(0)
+        runs.append([eng.download_bf16(o, (m, w)) for o, w in zip(outs, list(ns) + [n, n, n, n]) if o != dh])
+    assert widths[0] == width and 256 not in widths[:3] and widths[3:] == [256] * 3
+    for a, b in zip(*runs):
+        assert np.array_equal(a, b)
+    assert eng.device_status() == 0
+
+
+def test_narrow_tiles_only_while_nothing_runs_beside_the_chain(eng):
+    """Products on the side stream take the pairs that wide tiles leave idle: behind the first of them in a plan the tiles are wide, and a new plan starts over."""
+    rng = np.random.default_rng(3)
+    mk = lambda *sh: put(eng, bf(rng.standard_normal(sh).astype(np.float32)), 1)
+    m, n, k = 2000, 1504, 640
+    a, b, c, d = mk(m, k), mk(k, n), eng.alloc(m * n, 2), eng.alloc(m * n, 2)
+    prod = lambda out: [op(E.GEMM_SB, a=a, b=b, c=out, m=m, n=n, k=k, batch=1, dt=1)]
+    eng.run(prod(c))
+    assert eng.last_gemm_width() == 192
+    eng.run([op(E.EVENT, tb=1, sa=0, oa=1), op(E.EVENT, tb=2, sa=2, oa=1), op(E.STREAM, tb=2)] + prod(d) + [op(E.EVENT, tb=1, sa=2, oa=2), op(E.STREAM, tb=0)] + prod(c) +
+            [op(E.EVENT, tb=2, sa=0, oa=2)])
+    assert eng.last_gemm_width() == 256
+    assert np.array_equal(eng.download_bf16(c, (m, n)), eng.download_bf16(d, (m, n)))
+    eng.run(prod(c))
+    assert eng.last_gemm_width() == 192
