@@ -87,3 +87,74 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* r) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
                  ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
+// two numbers each as the sum of two bf16 ones
+__device__ __forceinline__ void split_bf16(float x, float y, uint32_t& hi, uint32_t& lo) {
+    hi = pack_bf16(x, y);
+    lo = pack_bf16(x - __uint_as_float(hi << 16), y - __uint_as_float(hi & 0xffff0000u));
+}
+// columns c0 .. c0 + 7 (a) and as many HALF further on (b) of a gradient row, times f, rotated back where the tables are given (a pair's columns are
+// HALF apart): out1 = g1 c + g2 s, out2 = -g1 s + g2 c
+template <int HALF = 32>
+__device__ __forceinline__ void store_grad8(float* a, float* b, int c0, float f, const float* cr, const float* sr, bf16* row, int dh) {
+#pragma unroll
+    for (int z = 0; z < 8; z++) { a[z] *= f; b[z] *= f; }
+    if (cr) {
+#pragma unroll
+        for (int z = 0; z < 8; z += 4) {
+            const float4 c4 = *reinterpret_cast<const float4*>(cr + c0 + z), s4 = *reinterpret_cast<const float4*>(sr + c0 + z);
+            const float cc[4] = {c4.x, c4.y, c4.z, c4.w}, ss[4] = {s4.x, s4.y, s4.z, s4.w};
+#pragma unroll
+            for (int y = 0; y < 4; y++) {
+                const float g1 = a[z + y], g2 = b[z + y];
+                a[z + y] = g1 * cc[y] + g2 * ss[y];
+                b[z + y] = g2 * cc[y] - g1 * ss[y];
+            }
+        }
+    }
+    if (c0 < dh) *reinterpret_cast<uint4*>(row + c0) = make_uint4(pack_bf16(a[0], a[1]), pack_bf16(a[2], a[3]), pack_bf16(a[4], a[5]), pack_bf16(a[6], a[7]));
+    if (HALF + c0 < dh) *reinterpret_cast<uint4*>(row + HALF + c0) = make_uint4(pack_bf16(b[0], b[1]), pack_bf16(b[2], b[3]), pack_bf16(b[4], b[5]), pack_bf16(b[6], b[7]));
+}
+
+// Sixteen columns of a row of the sums that each CTA of a cluster has at `at` in its shared memory, added in rank order: eight, and eight HALF further on
+template <int HALF>
+__device__ __forceinline__ void cluster_sum16(uint32_t at, int S, float* a) {
+#pragma unroll
+    for (int z = 0; z < 16; z++) a[z] = 0.f;
+    for (int q = 0; q < S; q++)
+#pragma unroll
+        for (int z = 0; z < 16; z += 4) {
+            float4 x;
+            asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %4, %5;\n\tld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [ra];\n\t}"
+                         : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w) : "r"(at + ((z & 7) + (z >> 3) * HALF) * 4), "r"(q) : "memory");
+            a[z] += x.x; a[z + 1] += x.y; a[z + 2] += x.z; a[z + 3] += x.w;
+        }
+}
+// CTAs that share the walk of a key tile of 128 in the backward kernels of whole tiles (clusters, whose dK and dV meet through distributed shared memory).  One
+// CTA to a key tile and kv head is as long as its chain, the query tiles of all heads of the group; 74 clusters of two and 33 of four run at once.
+// Backward in us with 1 / 2 / 4 (CTAs at 1, chain), head_dim 64 | 128 where a tile of the chain costs twice as much:
+// B8 H24 KV8 T128 (64, 3) 20.6 / 22.1 / 37.1 | 31.6 / 26.8 / 48.7, B1 H8 KV2 T512 (8, 16) 39.9 / 27.5 / 23.2 | 72.3 / 44.6 / 34.1, B8 H16 KV4 T256 (64, 8)
+// 30.7 / 26.2 / 40.1 | 51.6 / 38.2 / 54.5, B2 H16 KV4 T1024 (64, 32) 73.2 / 47.5 / 53.0 | 142 / 83.4 / 77.2, B1 H16 KV4 T2048 (64, 64) 130 / 76 / 67 | 262 / 144 /
+// 107, B2 H16 KV8 T768 (96, 12) 38.1 / 36.7 / 58.5 | 65.6 / 48.8 / 76.4, B1 H8 KV8 T2048 (128, 16) 44.3 / 44.3 / 79 | 79.7 / 60.4 / 104, B1 H16 KV4 T4096
+// (128, 128) 252 / 137 / 185 | 514 / 275 / 329, B4 H24 KV8 T768 (192, 18) 54.0 / 72.6 / 126 | 104 / 117 / 181.
+static inline int attn_tile_parts(int head_dim, long long ctas, long long chain) {
+    const bool wide = head_dim > 64;
+    int S = 1;
+    if (ctas <= AX_SMS / 2 ? chain >= (wide ? 2 : 4) : ctas <= AX_SMS && chain >= (wide ? 2 : 12)) S = 2;
+    if (S == 2 && (ctas <= 33 ? chain >= 8 : ctas <= AX_SMS / 2 && chain >= (wide ? 32 : 48))) S = 4;
+    return S;
+}
+// Launch of a kernel whose CTAs form clusters of S (1: none).  Up to half a CTA for each SM start while the grid in front of them ends (the step of two layers of 512
+// tokens, D 256: 275 -> 259 us).  More would take SMs from what still runs, by side-stream products or by stacking the longest CTAs on the SMs that are free first:
+// all of them early cost the step of 8192 tokens with adapters 1.2 %, one of 22 x 80 tokens 5 %.
+template <typename... KA, typename... A>
+static inline cudaError_t attn_launch(void (*kern)(KA...), long long grid, int block, size_t smem, int S, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(grid * S)); cfg.blockDim = dim3(block); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = grid * S <= AX_SMS / 2 && ax_gemm_pdl();
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = S; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
+    cfg.attrs = at; cfg.numAttrs = S > 1 ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<KA>(args)...);
+}

@@ -81,6 +81,7 @@ k_attn_fwd_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     const uint32_t t_S = tmem, t_P = tmem + 128, t_O = tmem + 192;
+    pdl_enter();
 
     if (warp == 4) {
         // ── control warp (converged; one elected lane issues MMAs, lane 0 issues the TMA loads) ──
@@ -327,6 +328,8 @@ struct BwdSmem {
                          DQ = DS0 + 2 * 32768, STAT = DQ + 32768, BARS = STAT + 8192, TOTAL = BARS + 512 + 1024;
 };
 static_assert(BwdSmem::TOTAL <= 227 * 1024, "backward shared memory exceeds the per-CTA limit");
+#define BWD_PITCH 68           // floats of a row of sums of a cluster: rows of a warp fall in different banks
+static_assert(2 * AT * BWD_PITCH * 4 <= 2 * BWD_SLOTS * 8192, "the sums take the ring's place");
 static_assert(BwdSmem::DO0 % 1024 == 0 && BwdSmem::DS0 % 1024 == 0 && BwdSmem::DQ % 1024 == 0, "swizzled tiles need 1024-byte alignment");
 
 #ifdef AXENG_PROF
@@ -341,12 +344,13 @@ __device__ long long* g_bwd_prof = nullptr;
 #define PROF_FLUSH(lo, hi) do { } while (0)
 #endif
 
+template <bool SPLIT>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
 k_attn_bwd_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
               const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
               const __grid_constant__ CUtensorMap tmdQ, const float* __restrict__ lse, const float* __restrict__ Dv,
               bf16* __restrict__ dk, bf16* __restrict__ dv, int T, int H, int KV, float scale,
-              const float* __restrict__ rope_cos, const float* __restrict__ rope_sin, int* status) {
+              const float* __restrict__ rope_cos, const float* __restrict__ rope_sin, int ctas, int* status) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const uint32_t sb = smem_u32(smem);
@@ -371,11 +375,14 @@ k_attn_bwd_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     // 1-D grid ordered by decreasing work: key tile 0 (attended by every query tile) of all
     // (kv head, batch) pairs first
     const int rep = H / KV, nqt = T / AT;
-    const int ngb = gridDim.x / nqt;
-    const int j = blockIdx.x / ngb, gb = blockIdx.x % ngb;
+    const int S = SPLIT ? ctas : 1, part = SPLIT ? blockIdx.x % S : 0, blk = SPLIT ? blockIdx.x / S : blockIdx.x;
+    const int ngb = gridDim.x / (nqt * S);
+    const int j = blk / ngb, gb = blk % ngb;
     const int g = gb % KV, b = gb / KV;
     const int per_head = nqt - j;                                     // causal: query tiles j .. nqt-1
-    const int n_it = rep * per_head;                                  // 128-query tiles
+    const int n_it = (rep * per_head - part + S - 1) / S;             // 128-query tiles of this CTA: part, part + S, ... of the group's
+    // the tile S further on: its head of the group and its place among the head's causal tiles
+    auto step = [&](int& hh, int& ii, int by) { for (ii += by; ii >= per_head; ii -= per_head) hh++; };
     const int n_sub = 2 * n_it;                                       // 64-query sub-tiles
 
     if (threadIdx.x == 0) {
@@ -398,6 +405,7 @@ k_attn_bwd_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     // columns: S^T/P^T[2] 0..127, dP^T/dS^T[2] 128..255, dV 256..319, dK 320..383, dQ 384..447, K 448..479, V 480..511
     const uint32_t t_S = tmem, t_dP = tmem + 128, t_dV = tmem + 256, t_dK = tmem + 320, t_dQ = tmem + 384,
                    t_K = tmem + 448, t_V = tmem + 480;
+    pdl_enter();
 
     if (warp == CTRL_WARP || warp == CTRL_WARP + 1) {
         // ── issuers of S^T = K Q^T (warp CTRL_WARP, which also feeds the Q / dO ring) and dP^T = V dO^T
@@ -409,6 +417,7 @@ k_attn_bwd_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         const uint32_t tA = is_s ? t_K : t_V, tD = is_s ? t_S : t_dP;
         // ring producer state (S issuer only): next sub-tile to load, its head / causal tile, and the slot it goes to
         int lu = 0, lhh = 0, lii = 0;
+        if (SPLIT) step(lhh, lii, part);
         auto load_sub = [&](int slot) {
             if (lane == 0) {
                 const int i = j + lii, h = g * rep + lhh;
@@ -420,7 +429,7 @@ k_attn_bwd_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                 bulk_load_1d(sb + BwdSmem::STAT + 4096 + slot * 512, lse + sidx, 256, b_qf + 8 * slot);
                 bulk_load_1d(sb + BwdSmem::STAT + 4096 + slot * 512 + 256, Dv + sidx, 256, b_qf + 8 * slot);
             }
-            if ((lu & 1) && ++lii == per_head) { lii = 0; lhh++; }
+            if (lu & 1) step(lhh, lii, S);
             lu++;
         };
         if (is_s) {
@@ -518,6 +527,7 @@ k_attn_bwd_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
         bool ok = true;
         int hh = 0, ii = 0;
+        if (SPLIT) step(hh, ii, part);
         for (int t = 0; t < n_it && ok; t++) {
             const long long tm0 = PROF_T();
             if (!mbar_wait_park(b_dq + 8 * (t & 1), (t >> 1) & 1) || *abort_flag) { ok = false; break; }
@@ -549,7 +559,7 @@ k_attn_bwd_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                 tma_reduce_add_4d(&tmdQ, sb + BwdSmem::DQ + 16384, 32, h, i * AT, b);
                 bulk_commit();
             }
-            if (++ii == per_head) { ii = 0; hh++; }
+            step(hh, ii, S);
             PROF_ADD(13, PROF_T() - tm1);
         }
         if (dt_ == 0) bulk_wait0();
@@ -570,7 +580,7 @@ k_attn_bwd_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         float* my_stat = s_stat + warp * 64;                // [-lse*log2(e) 32 | -D 32]
         const float* ring_stat = s_stat + 1024;             // [slot][lse 64 | D 64]
         bool ok = true;
-        int sl_u = e, ph_u = 0, ii_c = 0;                    // ring slot (with fill parity) and causal tile index of the current sub-tile
+        int sl_u = e, ph_u = 0, ii_c = SPLIT ? part % per_head : 0;                    // ring slot (with fill parity) and causal tile index of the current sub-tile
         // K (group 0) / V (group 1) from the swizzled shared-memory tile into TMEM: a thread copies half of its row
         // (a row is 128 bytes = 32 packed columns; 16-byte chunk c sits at position c ^ (row & 7))
         if (!mbar_wait_park(b_kv, 0)) ok = false;
@@ -592,7 +602,7 @@ k_attn_bwd_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         for (int u = e; u < n_sub && ok; u += 2) {
             const int it = u >> 1;
             const bool diag = ii_c == 0;
-            if (++ii_c == per_head) ii_c = 0;
+            for (ii_c += S; ii_c >= per_head;) ii_c -= per_head;
             const float* L = my_stat;
             const float* Dr = L + 32;
             const long long ta0 = PROF_T();
@@ -669,8 +679,20 @@ k_attn_bwd_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         if (threadIdx.x == 0) PROF_FLUSH(0, 8);
         // dV (group 0) and dK (group 1): complete once the last sub-tile's dV and dK commits have fired.  Column half hc writes head
         // dimensions 16 hc .. 16 hc + 15 and their rotary partners 32 further on.
-        if (ok && !mbar_wait_park(b_qe + 8 * ((n_sub - 1) % BWD_SLOTS), ((n_sub - 1) / BWD_SLOTS) & 1)) ok = false;
-        if (ok) {
+        if (ok && (!SPLIT || n_sub) && !mbar_wait_park(b_qe + 8 * ((n_sub - 1) % BWD_SLOTS), ((n_sub - 1) / BWD_SLOTS) & 1)) ok = false;
+        if (SPLIT && ok) {
+            // [dV, dK][key][64] in the ring's place: its last reader has run
+            tc_fence_after();
+            float* row = reinterpret_cast<float*>(smem + BwdSmem::Q0) + (e * AT + r) * BWD_PITCH + hc * 32;
+            uint32_t v[32];
+            if (n_sub) {
+                tmem_ld32((e ? t_dK : t_dV) + lane_base + hc * 32, v);
+                tmem_ld_wait();
+            }
+#pragma unroll
+            for (int q = 0; q < 32; q += 4)
+                *reinterpret_cast<uint4*>(row + q) = n_sub ? make_uint4(v[q], v[q + 1], v[q + 2], v[q + 3]) : make_uint4(0, 0, 0, 0);
+        } else if (ok) {
             tc_fence_after();
             const int t = j * AT + r;
             const uint32_t ta = (e ? t_dK : t_dV) + lane_base + hc * 16;
@@ -724,10 +746,23 @@ k_attn_bwd_tc(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     tc_fence_before();
     __syncthreads();
     if (warp == CTRL_WARP) { __syncwarp(); tc_fence_after(); tmem_dealloc(tmem, 512); }
+    if (SPLIT) {
+        cluster_sync();
+        const int rows = AT / S;
+        for (int i = threadIdx.x; i < 2 * rows * 4; i += BWD_THREADS) {       // eight columns and their partners
+            const int m = i / (rows * 4), r = part * rows + (i >> 2) % rows, c0 = (i & 3) * 8, t = j * AT + r;
+            float a[16];
+            cluster_sum16<32>(sb + BwdSmem::Q0 + ((m * AT + r) * BWD_PITCH + c0) * 4, S, a);
+            store_grad8(a, a + 8, c0, m ? scale : 1.f, m && rope_cos ? rope_cos + (long long)t * 32 : nullptr, rope_sin + (long long)t * 32,
+                        (m ? dk : dv) + (((long long)b * T + t) * KV + g) * ADH, ADH);
+        }
+        cluster_sync();     // peers have read
+    }
 }
 
 // fp32 dq accumulator -> bf16 dq (same [B,T,H,DH] layout)
 __global__ void k_dq_convert(const float* __restrict__ src, bf16* __restrict__ dst, long long n8) {
+    pdl_enter();
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += stride) {
         float f[8];
@@ -740,6 +775,7 @@ __global__ void k_dq_convert(const float* __restrict__ src, bf16* __restrict__ d
 // 8 columns of the first half of a row and their partners; rows = B*T*H, t = (row / H) % T.
 __global__ void k_dq_convert_rope(const float* __restrict__ src, bf16* __restrict__ dst, const float* __restrict__ cs,
                                   const float* __restrict__ sn, long long rows, int T, int H) {
+    pdl_enter();
     const long long total = rows * 4;
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -762,7 +798,8 @@ __global__ void k_dq_convert_rope(const float* __restrict__ src, bf16* __restric
 int ax_attn_tc_init(void) {
     int rc = ax_attn_tc128_init();
     rc |= (int)cudaFuncSetAttribute(k_attn_fwd_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdSmem::TOTAL);
-    rc |= (int)cudaFuncSetAttribute(k_attn_bwd_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem::TOTAL);
+    rc |= (int)cudaFuncSetAttribute(k_attn_bwd_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem::TOTAL);
+    rc |= (int)cudaFuncSetAttribute(k_attn_bwd_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem::TOTAL);
     return rc;
 }
 
@@ -789,6 +826,11 @@ static int map_dq_f32(CUtensorMap* m, const void* base, int B, int T, int heads)
     return r == CUDA_SUCCESS ? 0 : 2;
 }
 
+int ax_attn_tc_parts(const AttnShape& s) {
+    if (s.DH != ADH && s.DH != 128) return 0;
+    if (s.T < AT || s.T % AT || s.KV < 1 || s.H % s.KV) return 0;
+    return attn_tile_parts(s.DH, (long long)(s.T / AT) * s.KV * s.B, (long long)s.H / s.KV * (s.T / AT));
+}
 int ax_attn_fwd_tc(const void* q, const void* k, const void* v, void* o, float* lse,
                    const AttnShape& s, int* status, cudaStream_t st) {
     if (s.DH == 128) return ax_attn_fwd_tc128(q, k, v, o, lse, s, status, st);
@@ -796,17 +838,13 @@ int ax_attn_fwd_tc(const void* q, const void* k, const void* v, void* o, float* 
     CUtensorMap tq, tk, tv;
     if (map_bthd(&tq, q, s.B, s.T, s.H) || map_bthd(&tk, k, s.B, s.T, s.KV) || map_bthd(&tv, v, s.B, s.T, s.KV)) return 2;
     dim3 grid((s.T / AT) * s.H * s.B);
-    k_attn_fwd_tc<<<grid, ATT_THREADS, FwdSmem::TOTAL, st>>>(tq, tk, tv, (bf16*)o, lse, s.T, s.H, s.KV, s.scale, status);
-    return 0;
+    return attn_launch(k_attn_fwd_tc, grid.x, ATT_THREADS, FwdSmem::TOTAL, 1, st, tq, tk, tv, (bf16*)o, lse, s.T, s.H, s.KV, s.scale, status) == cudaSuccess ? 0 : 3;
 }
 
 int ax_attn_bwd_tc(const void* q, const void* k, const void* v, const void* o, const void* dO,
                    const float* lse, float* Dscratch, float* g_dq_acc, void* dq, void* dk, void* dv,
                    const AttnShape& s, const float* rope_cos, const float* rope_sin, int* status, cudaStream_t st) {
-    if (s.DH == 128) {
-        if (rope_cos) return -1;                 // the inverse rotary is fused for head_dim 64 only
-        return ax_attn_bwd_tc128(q, k, v, o, dO, lse, Dscratch, g_dq_acc, dq, dk, dv, s, status, st);
-    }
+    if (s.DH == 128) return ax_attn_bwd_tc128(q, k, v, o, dO, lse, Dscratch, g_dq_acc, dq, dk, dv, s, rope_cos, rope_sin, status, st);
     if (!served(s) || !g_dq_acc || !aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(o) || !aligned16(dO) ||
         !aligned16(dq) || !aligned16(dk) || !aligned16(dv) || !aligned16(g_dq_acc)) return -1;
     if (rope_cos && (!rope_sin || !aligned16(rope_cos) || !aligned16(rope_sin))) return -1;
@@ -823,8 +861,9 @@ int ax_attn_bwd_tc(const void* q, const void* k, const void* v, const void* o, c
     if (want_prof && cudaMalloc(&prof, (size_t)nblk * 256) == cudaSuccess) cudaMemset(prof, 0, (size_t)nblk * 256); else prof = nullptr;
     cudaMemcpyToSymbol(g_bwd_prof, &prof, sizeof(prof));
 #endif
-    k_attn_bwd_tc<<<grid, BWD_THREADS, BwdSmem::TOTAL, st>>>(tq, tk, tv, tdo, tdq, lse, Dscratch, (bf16*)dk, (bf16*)dv,
-                                                              s.T, s.H, s.KV, s.scale, rope_cos, rope_sin, status);
+    const int S = attn_tile_parts(s.DH, grid.x, (long long)s.H / s.KV * (s.T / AT));
+    if (attn_launch(S > 1 ? k_attn_bwd_tc<true> : k_attn_bwd_tc<false>, grid.x, BWD_THREADS, BwdSmem::TOTAL, S, st, tq, tk, tv, tdo, tdq, lse, (const float*)Dscratch, (bf16*)dk, (bf16*)dv,
+                           s.T, s.H, s.KV, s.scale, rope_cos, rope_sin, S, status) != cudaSuccess) return 3;
 #ifdef AXENG_PROF
     if (prof) {
         std::vector<long long> h((size_t)nblk * 32);
@@ -841,10 +880,10 @@ int ax_attn_bwd_tc(const void* q, const void* k, const void* v, const void* o, c
     }
 #endif
     if (rope_cos) {
-        k_dq_convert_rope<<<ew_grid(rows * 4, 256), 256, 0, st>>>(g_dq_acc, (bf16*)dq, rope_cos, rope_sin, rows, s.T, s.H);
+        if (attn_launch(k_dq_convert_rope, ew_grid(rows * 4, 256), 256, 0, 1, st, (const float*)g_dq_acc, (bf16*)dq, rope_cos, rope_sin, rows, s.T, s.H) != cudaSuccess) return 3;
     } else {
         const long long n8 = rows * ADH / 8;
-        k_dq_convert<<<ew_grid(n8, 256), 256, 0, st>>>(g_dq_acc, (bf16*)dq, n8);
+        if (attn_launch(k_dq_convert, ew_grid(n8, 256), 256, 0, 1, st, (const float*)g_dq_acc, (bf16*)dq, n8) != cudaSuccess) return 3;
     }
     return 0;
 }

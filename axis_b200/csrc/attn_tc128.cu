@@ -80,6 +80,7 @@ k_attn_fwd_tc128(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     const uint32_t t_S = tmem, t_O = tmem + 128;
+    pdl_enter();
 
     if (warp == 4) {
         {   // the whole warp runs the loop converged; lane 0 issues the TMA loads, one elected lane the MMAs
@@ -287,6 +288,8 @@ struct Bwd128Smem {
     static constexpr int K = 0, V = 32768, Q0 = 65536, DO0 = Q0 + QST * 16384, DS = DO0 + QST * 16384, DQ = DS + 2 * 16384,
                          STAT = DQ + 32768, BARS = STAT + QST * 512, TOTAL = BARS + 256 + 1024;
 };
+#define BWD128_PITCH 132       // floats of a row of sums of a cluster: rows of a warp fall in different banks
+static_assert(2 * AT * BWD128_PITCH * 4 <= Bwd128Smem::DS, "the sums take the place of K, V and the ring");
 static_assert(Bwd128Smem::TOTAL <= 227 * 1024, "head_dim-128 backward shared memory exceeds the per-CTA limit");
 
 // One CTA per (128 keys, head) walks the query sub-tiles (64 queries) of the causal range.  Per sub-tile:
@@ -299,11 +302,13 @@ static_assert(Bwd128Smem::TOTAL <= 227 * 1024, "head_dim-128 backward shared mem
 // always has the independent half of the work queued.  TMEM (512 columns): S^T 64, dP^T 64, dV 128, dK 128, dQ^T 64,
 // P^T 32, dS^T 32.  dQ^T is single: the softmax warps move it out (transposing staging + TMA reduce-add) right after
 // they have handed over P^T / dS^T of the following sub-tile.
+template <bool SPLIT>
 __global__ void __launch_bounds__(BWD128_THREADS, 1)
 k_attn_bwd_tc128(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
                  const __grid_constant__ CUtensorMap tmdQ, const float* __restrict__ lse, const float* __restrict__ Dv,
-                 bf16* __restrict__ dk, bf16* __restrict__ dv, int T, int H, int KV, float scale, int* status) {
+                 bf16* __restrict__ dk, bf16* __restrict__ dv, int T, int H, int KV, float scale,
+                 const float* __restrict__ rope_cos, const float* __restrict__ rope_sin, int ctas, int* status) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const uint32_t sb = smem_u32(smem);
@@ -318,11 +323,12 @@ k_attn_bwd_tc128(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // 1-D grid ordered by decreasing work: key tile 0 of all (kv head, batch) pairs first
     const int rep = H / KV, nkt = T / AT;
-    const int ngb = gridDim.x / nkt;
-    const int j = blockIdx.x / ngb, gb = blockIdx.x % ngb;
+    const int S = SPLIT ? ctas : 1, part = SPLIT ? blockIdx.x % S : 0, blk = SPLIT ? blockIdx.x / S : blockIdx.x;
+    const int ngb = gridDim.x / (nkt * S);
+    const int j = blk / ngb, gb = blk % ngb;
     const int g = gb % KV, b = gb / KV;
     const int per_head = 2 * (nkt - j);                               // causal: query sub-tiles 2j .. 2 nkt - 1
-    const int n_it = rep * per_head;
+    const int n_it = (rep * per_head - part + S - 1) / S;             // this CTA: sub-tiles part, part + S, ... of the group's
 
     if (threadIdx.x == 0) {
         mbar_init(b_kv, 1);
@@ -339,6 +345,7 @@ k_attn_bwd_tc128(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     // columns: S^T 0..63, dP^T 64..127, dV 128..255, dK 256..383, dQ^T 384..447, P^T 448..479, dS^T 480..511 (packed bf16)
     const uint32_t t_S = tmem, t_dP = tmem + 64, t_dV = tmem + 128, t_dK = tmem + 256, t_dQ = tmem + 384, t_P = tmem + 448,
                    t_dS = tmem + 480;
+    pdl_enter();
 
     if (warp == 8) {
         {   // the whole warp runs the loop converged; lane 0 issues the TMA loads, one elected lane the MMAs
@@ -360,7 +367,7 @@ k_attn_bwd_tc128(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             }
             auto load_q = [&](int it) {
                 if (lane != 0) return;
-                const int s = it % QST, hh = it / per_head, u = 2 * j + it % per_head, h = g * rep + hh;
+                const int s = it % QST, i = part + it * S, hh = i / per_head, u = 2 * j + i % per_head, h = g * rep + hh;
                 mbar_expect_tx(b_qf + 8 * s, 32768 + 512);
                 // the sub-tile's row statistics ride on the same barrier (a softmax warp that loaded them from global
                 // memory itself would expose that latency at its next scoreboard wait)
@@ -372,7 +379,7 @@ k_attn_bwd_tc128(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 tma_load_4d(sb + Bwd128Smem::DO0 + s * 16384, &tmdO, b_qf + 8 * s, 0, h, u * QS, b);
                 tma_load_4d(sb + Bwd128Smem::DO0 + s * 16384 + 8192, &tmdO, b_qf + 8 * s, 64, h, u * QS, b);
             };
-            load_q(0);
+            if (!SPLIT || n_it) load_q(0);
             __syncwarp();
             if (!mbar_wait(b_kv, 0)) ok = false;
             // iteration it: S^T / dP^T of sub-tile it, then dV, dK and dQ^T of sub-tile it - 1 (one more round at the end)
@@ -451,7 +458,7 @@ k_attn_bwd_tc128(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             fence_async_smem();
             named_bar_sync(1, 256);
             if (threadIdx.x == 0) {
-                const int hh = t / per_head, u = 2 * j + t % per_head, h = g * rep + hh;
+                const int i = part + t * S, hh = i / per_head, u = 2 * j + i % per_head, h = g * rep + hh;
 #pragma unroll
                 for (int blk = 0; blk < 4; blk++)
                     tma_reduce_add_4d(&tmdQ, sb + Bwd128Smem::DQ + blk * 8192, blk * 32, h, u * QS, b);
@@ -461,7 +468,7 @@ k_attn_bwd_tc128(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         };
         const float c_l = -LOG2E;
         for (int it = 0; it < n_it && ok; it++) {
-            const int u = 2 * j + it % per_head;              // query sub-tile
+            const int u = 2 * j + (part + it * S) % per_head; // query sub-tile
             if (!mbar_wait(b_sdp, it & 1) || *abort_flag) { ok = false; break; }
             // the stage's barrier completed before S^T was issued; observing it makes the bulk-copied statistics visible
             if (!mbar_wait(b_qf + 8 * (it % QST), (it / QST) & 1)) { ok = false; break; }
@@ -519,29 +526,40 @@ k_attn_bwd_tc128(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             // dQ^T of the previous sub-tile: its MMA was issued right after that sub-tile's P^T / dS^T were handed over
             if (it >= 1 && !drain(it - 1)) { ok = false; break; }
         }
-        if (ok && !drain(n_it - 1)) ok = false;
+        if (SPLIT && n_it == 0) {
+            if (!mbar_wait(b_kv, 0)) ok = false;             // zeros replace K and V: not before these have landed
+        } else if (ok && !drain(n_it - 1)) ok = false;
         if (threadIdx.x == 0) bulk_wait0();
         if (ok) {
             // dV (half 0 threads) and dK (half 1 threads): complete once the last commit has fired — waited in drain
             const int t = j * AT + r;
-            const uint32_t ta = hf ? t_dK : t_dV;
-            const float f = hf ? scale : 1.f;
-            bf16* dst = (hf ? dk : dv) + (((long long)b * T + t) * KV + g) * DH2;
+            const uint32_t ta = (hf ? t_dK : t_dV) + lane_base;
+            if (SPLIT) {                                     // [dV, dK][key][128] in the place of K, V and the ring, whose last readers have run
+                float* row = reinterpret_cast<float*>(smem) + (hf * AT + r) * BWD128_PITCH;
 #pragma unroll 1
-            for (int ch = 0; ch < DH2 / 32; ch++) {
-                uint32_t v[32];
-                tmem_ld32(ta + lane_base + ch * 32, v);
-                tmem_ld_wait();
-                if (t < T) {
-#pragma unroll
-                    for (int q = 0; q < 32; q += 8) {
-                        uint4 pk;
-                        pk.x = pack_bf16(__uint_as_float(v[q]) * f, __uint_as_float(v[q + 1]) * f);
-                        pk.y = pack_bf16(__uint_as_float(v[q + 2]) * f, __uint_as_float(v[q + 3]) * f);
-                        pk.z = pack_bf16(__uint_as_float(v[q + 4]) * f, __uint_as_float(v[q + 5]) * f);
-                        pk.w = pack_bf16(__uint_as_float(v[q + 6]) * f, __uint_as_float(v[q + 7]) * f);
-                        *reinterpret_cast<uint4*>(dst + ch * 32 + q) = pk;
+                for (int ch = 0; ch < DH2 / 32; ch++) {
+                    uint32_t v[32];
+                    if (n_it) {
+                        tmem_ld32(ta + ch * 32, v);
+                        tmem_ld_wait();
                     }
+#pragma unroll
+                    for (int q = 0; q < 32; q += 4)
+                        *reinterpret_cast<uint4*>(row + ch * 32 + q) = n_it ? make_uint4(v[q], v[q + 1], v[q + 2], v[q + 3]) : make_uint4(0, 0, 0, 0);
+                }
+            } else {
+                bf16* dst = (hf ? dk : dv) + (((long long)b * T + t) * KV + g) * DH2;
+                const float* cr = hf && rope_cos ? rope_cos + (long long)t * (DH2 / 2) : nullptr;
+                const float* sr = rope_sin + (long long)t * (DH2 / 2);
+#pragma unroll 1
+                for (int ch = 0; ch < DH2 / 32; ch++) {      // sixteen columns and their rotary partners
+                    uint32_t v1[16], v2[16];
+                    tmem_ld16(ta + ch * 16, v1);
+                    tmem_ld16(ta + DH2 / 2 + ch * 16, v2);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int q = 0; q < 16; q += 8)
+                        store_grad8<DH2 / 2>(reinterpret_cast<float*>(v1 + q), reinterpret_cast<float*>(v2 + q), ch * 16 + q, hf ? scale : 1.f, cr, sr, dst, DH2);
                 }
             }
         } else if (lane == 0) {
@@ -552,10 +570,37 @@ k_attn_bwd_tc128(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     tc_fence_before();
     __syncthreads();
     if (warp == 8) { __syncwarp(); tc_fence_after(); tmem_dealloc(tmem, 512); }
+    if (SPLIT) {
+        cluster_sync();
+        const int rows = AT / S;
+        for (int i = threadIdx.x; i < 2 * rows * 8; i += BWD128_THREADS) {       // eight columns and their partners
+            const int m = i / (rows * 8), r = part * rows + (i >> 3) % rows, c0 = (i & 7) * 8, t = j * AT + r;
+            float a[16];
+            cluster_sum16<DH2 / 2>(sb + ((m * AT + r) * BWD128_PITCH + c0) * 4, S, a);
+            store_grad8<DH2 / 2>(a, a + 8, c0, m ? scale : 1.f, m && rope_cos ? rope_cos + (long long)t * (DH2 / 2) : nullptr, rope_sin + (long long)t * (DH2 / 2),
+                                 (m ? dk : dv) + (((long long)b * T + t) * KV + g) * DH2, DH2);
+        }
+        cluster_sync();     // peers have read
+    }
 }
 
-// fp32 dq accumulator -> bf16 dq (same [B,T,H,DH] layout)
+// fp32 dq accumulator -> bf16 dq (same [B,T,H,DH] layout), with the inverse rotary on the way where the tables are given: a thread takes 8 columns of
+// the first half of a row and their partners; rows = B*T*H, t = (row / H) % T
+__global__ void k_dq_convert128_rope(const float* __restrict__ src, bf16* __restrict__ dst, const float* __restrict__ cs, const float* __restrict__ sn,
+                                     long long rows, int T, int H) {
+    pdl_enter();
+    const long long total = rows * 8, stride = (long long)gridDim.x * blockDim.x;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
+        const long long row = i >> 3;
+        const int c0 = (int)(i & 7) * 8, t = (int)((row / H) % T);
+        float a[8], b[8];
+        Vec<float>::ld(src + row * DH2 + c0, a); Vec<float>::ld(src + row * DH2 + c0 + 4, a + 4);
+        Vec<float>::ld(src + row * DH2 + DH2 / 2 + c0, b); Vec<float>::ld(src + row * DH2 + DH2 / 2 + c0 + 4, b + 4);
+        store_grad8<DH2 / 2>(a, b, c0, 1.f, cs + (long long)t * (DH2 / 2), sn + (long long)t * (DH2 / 2), dst + row * DH2, DH2);
+    }
+}
 __global__ void k_dq_convert128(const float* __restrict__ src, bf16* __restrict__ dst, long long n8) {
+    pdl_enter();
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += stride) {
         float f[8];
@@ -569,7 +614,8 @@ __global__ void k_dq_convert128(const float* __restrict__ src, bf16* __restrict_
 int ax_attn_tc128_init(void) {
     int rc = 0;
     rc |= (int)cudaFuncSetAttribute(k_attn_fwd_tc128, cudaFuncAttributeMaxDynamicSharedMemorySize, Fwd128Smem::TOTAL);
-    rc |= (int)cudaFuncSetAttribute(k_attn_bwd_tc128, cudaFuncAttributeMaxDynamicSharedMemorySize, Bwd128Smem::TOTAL);
+    rc |= (int)cudaFuncSetAttribute(k_attn_bwd_tc128<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Bwd128Smem::TOTAL);
+    rc |= (int)cudaFuncSetAttribute(k_attn_bwd_tc128<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Bwd128Smem::TOTAL);
     return rc;
 }
 
@@ -603,13 +649,13 @@ int ax_attn_fwd_tc128(const void* q, const void* k, const void* v, void* o, floa
     CUtensorMap tq, tk, tv;
     if (map_bthd128(&tq, q, s.B, s.T, s.H, AT) || map_bthd128(&tk, k, s.B, s.T, s.KV, AT) || map_bthd128(&tv, v, s.B, s.T, s.KV, AT)) return 2;
     dim3 grid((s.T / AT) * s.H * s.B);
-    k_attn_fwd_tc128<<<grid, ATT_THREADS, Fwd128Smem::TOTAL, st>>>(tq, tk, tv, (bf16*)o, lse, s.T, s.H, s.KV, s.scale, status);
-    return 0;
+    return attn_launch(k_attn_fwd_tc128, grid.x, ATT_THREADS, Fwd128Smem::TOTAL, 1, st, tq, tk, tv, (bf16*)o, lse, s.T, s.H, s.KV, s.scale, status) == cudaSuccess ? 0 : 3;
 }
 
 int ax_attn_bwd_tc128(const void* q, const void* k, const void* v, const void* o, const void* dO,
                       const float* lse, float* Dscratch, float* g_dq_acc, void* dq, void* dk, void* dv,
-                      const AttnShape& s, int* status, cudaStream_t st) {
+                      const AttnShape& s, const float* rope_cos, const float* rope_sin, int* status, cudaStream_t st) {
+    if (rope_cos && (!rope_sin || !aligned16(rope_cos) || !aligned16(rope_sin))) return -1;
     if (!served128(s) || !g_dq_acc || !aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(o) || !aligned16(dO) ||
         !aligned16(dq) || !aligned16(dk) || !aligned16(dv) || !aligned16(g_dq_acc)) return -1;
     CUtensorMap tq, tk, tv, tdo, tdq;
@@ -618,9 +664,14 @@ int ax_attn_bwd_tc128(const void* q, const void* k, const void* v, const void* o
     const long long rows = (long long)s.B * s.T * s.H;
     if (ax_launch_chain(k_attn_bwd_prep128, dim3(ew_grid(rows * 16, 256)), dim3(256), 0, st, (const bf16*)o, (const bf16*)dO, Dscratch, g_dq_acc, s.B, s.T, s.H) != cudaSuccess) return 3;
     dim3 grid((s.T / AT) * s.KV * s.B);
-    k_attn_bwd_tc128<<<grid, BWD128_THREADS, Bwd128Smem::TOTAL, st>>>(tq, tk, tv, tdo, tdq, lse, Dscratch, (bf16*)dk, (bf16*)dv,
-                                                                       s.T, s.H, s.KV, s.scale, status);
-    const long long n8 = rows * DH2 / 8;
-    k_dq_convert128<<<ew_grid(n8, 256), 256, 0, st>>>(g_dq_acc, (bf16*)dq, n8);
+    const int S = attn_tile_parts(s.DH, grid.x, (long long)s.H / s.KV * (s.T / AT));
+    if (attn_launch(S > 1 ? k_attn_bwd_tc128<true> : k_attn_bwd_tc128<false>, grid.x, BWD128_THREADS, Bwd128Smem::TOTAL, S, st, tq, tk, tv, tdo, tdq, lse, (const float*)Dscratch, (bf16*)dk, (bf16*)dv,
+                           s.T, s.H, s.KV, s.scale, rope_cos, rope_sin, S, status) != cudaSuccess) return 3;
+    if (rope_cos) {
+        if (attn_launch(k_dq_convert128_rope, ew_grid(rows * 8, 256), 256, 0, 1, st, (const float*)g_dq_acc, (bf16*)dq, rope_cos, rope_sin, rows, s.T, s.H) != cudaSuccess) return 3;
+    } else {
+        const long long n8 = rows * DH2 / 8;
+        if (attn_launch(k_dq_convert128, ew_grid(n8, 256), 256, 0, 1, st, (const float*)g_dq_acc, (bf16*)dq, n8) != cudaSuccess) return 3;
+    }
     return 0;
 }

@@ -31,32 +31,6 @@
 #define STAT_XDQ 0xa00
 #define STAT_XDKV 0xb00
 
-// two numbers each as the sum of two bf16 ones
-__device__ __forceinline__ void split_bf16(float x, float y, uint32_t& hi, uint32_t& lo) {
-    hi = pack_bf16(x, y);
-    lo = pack_bf16(x - __uint_as_float(hi << 16), y - __uint_as_float(hi & 0xffff0000u));
-}
-// columns c0 .. c0 + 7 (a) and c0 + 32 .. c0 + 39 (b) of a gradient row, times f, rotated back where the tables are given (pairs 32
-// columns apart: out1 = g1 c + g2 s, out2 = -g1 s + g2 c), to bf16
-__device__ __forceinline__ void store_grad8(float* a, float* b, int c0, float f, const float* cr, const float* sr, bf16* row, int dh) {
-#pragma unroll
-    for (int z = 0; z < 8; z++) { a[z] *= f; b[z] *= f; }
-    if (cr) {
-#pragma unroll
-        for (int z = 0; z < 8; z += 4) {
-            const float4 c4 = *reinterpret_cast<const float4*>(cr + c0 + z), s4 = *reinterpret_cast<const float4*>(sr + c0 + z);
-            const float cc[4] = {c4.x, c4.y, c4.z, c4.w}, ss[4] = {s4.x, s4.y, s4.z, s4.w};
-#pragma unroll
-            for (int y = 0; y < 4; y++) {
-                const float g1 = a[z + y], g2 = b[z + y];
-                a[z + y] = g1 * cc[y] + g2 * ss[y];
-                b[z + y] = g2 * cc[y] - g1 * ss[y];
-            }
-        }
-    }
-    if (c0 < dh) *reinterpret_cast<uint4*>(row + c0) = make_uint4(pack_bf16(a[0], a[1]), pack_bf16(a[2], a[3]), pack_bf16(a[4], a[5]), pack_bf16(a[6], a[7]));
-    if (32 + c0 < dh) *reinterpret_cast<uint4*>(row + 32 + c0) = make_uint4(pack_bf16(b[0], b[1]), pack_bf16(b[2], b[3]), pack_bf16(b[4], b[5]), pack_bf16(b[6], b[7]));
-}
 // the same for a thread's columns c0 .. c0 + 15 and c0 + 32 .. c0 + 47 of an accumulator in TMEM
 __device__ __forceinline__ void store_grad_row(uint32_t taddr, int c0, float f, const float* cr, const float* sr, bf16* row, int dh, bool live) {
     uint32_t v1[16], v2[16];
@@ -641,15 +615,8 @@ k_attn_dkv_tcs(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             const int m = i / (rows * 4), r = part * rows + (i >> 2) % rows, c0 = (i & 3) * 8, t = j * XT + r;
             if (t >= T) continue;
             const uint32_t at = sb + XdKVSmem::Q0 + ((m * XT + r) * XK_PITCH + c0) * 4;
-            float a[16] = {};
-            for (int q = 0; q < S; q++)
-#pragma unroll
-                for (int z = 0; z < 16; z += 4) {
-                    float4 x;
-                    asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %4, %5;\n\tld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [ra];\n\t}"
-                                 : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w) : "r"(at + ((z & 7) + (z >> 3) * 32) * 4), "r"(q) : "memory");
-                    a[z] += x.x; a[z + 1] += x.y; a[z + 2] += x.z; a[z + 3] += x.w;
-                }
+            float a[16];
+            cluster_sum16<32>(at, S, a);
             store_grad8(a, a + 8, c0, m ? s.scale : 1.f, m && rope_cos ? rope_cos + (long long)t * 32 : nullptr, rope_sin + (long long)t * 32,
                         (m ? dk : dv) + (((long long)b * T + t) * KV + g) * s.DH, s.DH);
         }

@@ -413,3 +413,32 @@ def test_inverse_rotary_of_other_shapes_is_rounded_once(eng, B, H, KV, T, DH):
         base = err(E.bf16_bits_to_f32(plain[n]).transpose(0, 2, 1, 3), ref[n])
         assert err(eng.download_bf16(i, (B, T, heads, DH)).transpose(0, 2, 1, 3), want) <= (1.05 if fused else 1.6) * base
     assert eng.device_status() == 0
+
+
+@pytest.mark.parametrize("rotary", [False, True])
+@pytest.mark.parametrize("DH", [64, 128])
+@pytest.mark.parametrize("B,H,KV,T,parts", [
+    (1, 2, 2, 1024, 4), (2, 2, 1, 512, 4), (3, 12, 4, 512, 2), (3, 8, 4, 256, 2), (1, 10, 10, 512, 2), (3, 30, 10, 768, 1)])       # the first: CTAs with nothing to walk
+def test_whole_tile_backward_with_key_tiles_shared_over_a_cluster(eng, B, H, KV, T, DH, parts, rotary):
+    """dq, dk and dv against float64, from one CTA to a key tile and from clusters of two and four, plain and rotated back inside.  Bound: bf16 P or dS, result and (in
+    the row dots) o, three roundings of at most 2^-9 and 2^-9 / sqrt(3) on average, in quadrature 2.0e-3 in the 2-norm; twice that.  A tile or a pair in the wrong
+    place errs by as much as the result."""
+    assert eng.lib.eng_attn_tile_parts(B, H, KV, T, DH) == parts
+    rng = np.random.default_rng(T + DH + H)
+    q, k, v, do = make(rng, B, H, KV, T, DH, 1)
+    scale = 1.0 / np.sqrt(DH)
+    cos, sin = O.rope_tables(T, DH)
+    eng.launch_count(reset=True)
+    runs = run_bf16_attention(eng, q, k, v, do, scale, 0, times=2, rotary=(cos, sin) if rotary else ())
+    assert eng.launch_count() == 8
+    ref = attention_f64(q, k, v, do, scale)
+    if rotary:
+        c, s = cos.astype(np.float64), sin.astype(np.float64)
+        for n in ("dq", "dk"):
+            g1, g2 = ref[n][..., :DH // 2], ref[n][..., DH // 2:]
+            ref[n] = np.concatenate([g1 * c + g2 * s, g2 * c - g1 * s], -1)
+    for n, exact in ref.items():
+        got = E.bf16_bits_to_f32(runs[0][n]).transpose(0, 2, 1, 3)
+        assert np.linalg.norm(got - exact) <= 4e-3 * np.linalg.norm(exact), n
+        assert n == "dq" or np.array_equal(runs[0][n], runs[1][n]), n            # dq is added in the order of arrival
+    assert eng.device_status() == 0
