@@ -1,6 +1,6 @@
 // Causal grouped-query attention on CUDA cores with exact fp32 arithmetic —
-// the parity-mode path (fp32 storage, any head_dim <= 256, any T) and the
-// general path for shapes the tensor-core kernels do not take.  Layout is
+// the general path (any head_dim <= 256, any T, any strides) for shapes that neither the
+// tensor-core kernels nor attn_f32.cu (fp32 storage, head dims 12 to 64) take.  Layout is
 // given by element strides, so [B,H,T,DH] and [B,T,H,DH] are both served.
 // No atomics: dK/dV are accumulated per key row over the whole query group.
 //
@@ -507,6 +507,10 @@ int ax_attn_fwd_simt(int dt, const void* q, const void* k, const void* v, void* 
                      const AttnShape& s, cudaStream_t st) {
     if (s.DH > 256 || s.DH < 1 || s.KV < 1 || s.H % s.KV) return 101;
     if (s.B <= 0 || s.T <= 0) return 0;
+    if (dt == 0) {
+        const int rc = ax_attn_fwd_f32((const float*)q, (const float*)k, (const float*)v, (float*)o, lse, s, st);
+        if (rc >= 0) return rc;
+    }
     const int vec = attn_vec(dt, s, {q, k, v});
     return dt == 1 ? attn_fwd_nj<bf16>(q, k, v, o, lse, s, vec, st) : attn_fwd_nj<float>(q, k, v, o, lse, s, vec, st);
 }
@@ -539,6 +543,10 @@ int ax_attn_bwd_simt(int dt, int out_dt, const void* q, const void* k, const voi
                      const AttnShape& s, cudaStream_t st) {
     if (s.DH > 256 || s.DH < 1 || s.KV < 1 || s.H % s.KV) return 102;
     if (s.B <= 0 || s.T <= 0) return 0;
+    if (dt == 0 && out_dt == 0) {
+        const int rc = ax_attn_bwd_f32((const float*)q, (const float*)k, (const float*)v, (const float*)dO, lse, Dv, (float*)dq, (float*)dk, (float*)dv, s, st);
+        if (rc >= 0) return rc;
+    }
     const int vec = attn_vec(dt, s, {q, k, v, dO});
     if (dt == 1 && out_dt == 1) return attn_bwd_nj<bf16, bf16>(q, k, v, dO, lse, Dv, dq, dk, dv, s, vec, st);
     if (dt == 1) return attn_bwd_nj<bf16, float>(q, k, v, dO, lse, Dv, dq, dk, dv, s, vec, st);

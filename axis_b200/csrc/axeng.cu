@@ -114,7 +114,7 @@ API int eng_init(void) {
     if (cudaMalloc(&G.d_status, 64)) { set_err("status alloc failed"); return 3; }
     cudaMemset(G.d_status, 0, 64);
     if (ax_gemm_tc_init()) { set_err("tensor-core GEMM init failed: %s", cudaGetErrorString(cudaGetLastError())); return 4; }
-    if (ax_attn_mma_init() || ax_attn_tc_init() || ax_attn_tcs_init()) { set_err("tensor-core attention init failed: %s", cudaGetErrorString(cudaGetLastError())); return 4; }
+    if (ax_attn_f32_init() || ax_attn_mma_init() || ax_attn_tc_init() || ax_attn_tcs_init()) { set_err("tensor-core attention init failed: %s", cudaGetErrorString(cudaGetLastError())); return 4; }
     memset(G.prof_ms, 0, sizeof(G.prof_ms));
     memset(G.prof_calls, 0, sizeof(G.prof_calls));
     G.inited = true; G.rank = 0; G.world = 1; G.fallback = 0;

@@ -179,10 +179,10 @@ int eng_attn_route(int backward, int B, int H, int KV, int T, int head_dim);
 /* Dynamic shared memory in bytes of the general attention kernels, 0 forward, 1 dQ, 2 dK / dV, for a head dim of 1 to 256
  * (else -1): host arithmetic that needs no GPU. */
 long long eng_attn_smem(int which, int head_dim);
-/* CTAs that share a key tile of the whole-tile tcgen05 attention backward (head_dim 64 or 128, T a multiple of 128): 1, 2 or 4; 0 = not such a shape. */
-int eng_attn_tile_parts(int B, int H, int KV, int T, int head_dim);
 /* CTAs that share a block's walk in those kernels (1: none do; 0: not a shape): host arithmetic, too. */
 int eng_attn_share(int which, int B, int H, int KV, int T, int head_dim);
+/* CTAs that share a key tile of the whole-tile tcgen05 attention backward (head_dim 64 or 128, T a multiple of 128): 1, 2 or 4; 0 = not such a shape. */
+int eng_attn_tile_parts(int B, int H, int KV, int T, int head_dim);
 
 /* Fused RMSNorm backward that allocates nothing (no counterpart in the
  * reference).  dx = (res ? res : 0) + d(rmsnorm)/dx, dw = sum over rows of

@@ -442,3 +442,37 @@ def test_whole_tile_backward_with_key_tiles_shared_over_a_cluster(eng, B, H, KV,
         assert np.linalg.norm(got - exact) <= 4e-3 * np.linalg.norm(exact), n
         assert n == "dq" or np.array_equal(runs[0][n], runs[1][n]), n            # dq is added in the order of arrival
     assert eng.device_status() == 0
+
+
+@pytest.mark.parametrize("B,H,KV,T,DH", [
+    (1, 2, 1, 3, 64), (2, 2, 2, 17, 12), (1, 4, 2, 31, 32), (3, 6, 2, 64, 20), (1, 2, 1, 65, 36), (2, 8, 8, 130, 64), (2, 8, 4, 256, 32), (40, 8, 2, 100, 48), (1, 3, 3, 449, 16),
+    (2, 16, 16, 333, 64)])
+def test_fp32_attention_of_head_dims_up_to_64(eng, B, H, KV, T, DH):
+    """Rows that end inside a lane's four, a warp's sixteen and a block's 64, heads narrower than the columns of a tile, one CTA to a block and clusters of up to eight (some with
+    no tile): o, lse, dq, dk and dv against float64 within the bound of the fp32 tests above, nothing behind the last row, the same bits on every run.  (With one
+    token dq and dk are zero, the difference of two equal sums, and a bound by the largest element says nothing.)"""
+    rng = np.random.default_rng(T + DH)
+    q, k, v, do = make(rng, B, H, KV, T, DH, 0)
+    scale = 1.0 / np.sqrt(DH)
+    t = lambda x: np.ascontiguousarray(x.transpose(0, 2, 1, 3))
+    iq, ik, iv, ido = put(eng, t(q), 0), put(eng, t(k), 0), put(eng, t(v), 0), put(eng, t(do), 0)
+    guard = 256
+    out = {n: (eng.alloc(a.size + guard), a.shape[1], a.size) for n, a in (("o", q), ("dq", q), ("dk", k), ("dv", k))}
+    for i, _, n in out.values():
+        eng.upload(i, np.full(n + guard, 7.0, np.float32))
+    ilse, iD = eng.alloc(B * H * T), eng.alloc(B * H * T)
+    runs = []
+    for _ in range(2):
+        eng.run([op(E.ATTN_FWD, a=iq, b=ik, d=iv, c=out["o"][0], sa=ilse, m=T, n=DH, k=KV, batch=B, tb=H, dt=0, alpha=scale)])
+        assert eng.last_variant() == 0x84
+        eng.run([op(E.ATTN_BWD, a=iq, b=ik, d=iv, c=ido, sa=ilse, sb=out["o"][0], tb=out["dq"][0], sc=out["dk"][0], oa=out["dv"][0], ob=H, oc=iD, m=T, n=DH, k=KV,
+                    batch=B, dt=0, alpha=scale)])
+        assert eng.last_variant() == 0x85
+        runs.append({n: eng.download(i, (sz + guard,)) for n, (i, _, sz) in out.items()})
+    for n, ref in attention_f64(q, k, v, do, scale).items():
+        heads, sz = out[n][1:]
+        got = runs[0][n][:sz].reshape(B, T, heads, DH).transpose(0, 2, 1, 3)
+        assert np.abs(got - ref).max() <= 2e-5 * np.abs(ref).max() + 1e-30, n
+        assert np.array_equal(runs[0][n], runs[1][n]) and np.all(runs[0][n][sz:] == 7.0), n
+    assert np.abs(eng.download(ilse, (B, H, T)) - O.attention_fwd(q, k, v, scale)[1]).max() <= 2e-5
+    assert eng.device_status() == 0
