@@ -207,11 +207,15 @@ int ax_lora_grad(int count, const void* const* X, const void* const* S, float* c
 
 // ── the skinny products of an adapter: out[N, R] = alpha * X W (W [F, R]) or alpha * X W^T (W [R, F]) ──────────────────
 // u = x A in the forward and t = g B^T in the backward: again a stream over the wide operand with 16 flops per byte.
-// A CTA takes 32 tokens and walks F in pieces of 256 columns (three cp.async stages); its eight warps are two row tiles
-// times four quarters of a piece's depth, and the four partial accumulators of a row tile meet in shared memory.
-#define LP_TOK 32
-#define LP_COLS 256
-#define LP_STAGES 3
+// A CTA takes TOK tokens and walks F in pieces of COLS columns; its eight warps are the row tiles times equal shares of a
+// piece's depth, and the partial accumulators of a row tile meet in shared memory.  What bounds it is what an SM takes in:
+// besides its X a CTA reads all of W, from L2, so that 32 tokens a CTA moved as much W as X (rank 16: 32 bytes of W against
+// 64 of X a column).  Hence 64 tokens, and products of one X (the adapters of q, k and v, of gate and up) as M members
+// of one CTA, where X is staged once for all of them; one barrier a piece, all stages in flight from the start, and
+// neighbouring token blocks begin at different pieces, or all SMs ask for the same lines of W at the same time.
+// Rank 16, three products of one X, 8192 x 1536: 25.4 us with 32 tokens and a CTA per product, 17.0 with 64 and members,
+// 15.5 with the pieces turned, 15.1 with all stages in flight; one product of 8192 x 4096 24.0 -> 16.4; two of their own
+// 8192 x 4096 39.6 -> 25.0 (5.4 TB/s).
 
 struct LoraProjProb {
     const bf16* X;
@@ -233,162 +237,174 @@ __device__ __forceinline__ void ldsm_x2(uint32_t addr, uint32_t* r) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0, %1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(addr));
 }
 
-// TB = 0: W is [F, R] (row pitch of its stage R*2+16 bytes); TB = 1: W is [R, F] (row pitch LG_XS).  grid = (token blocks, products)
-template <int NT, int TB>
-__global__ void __launch_bounds__(256) k_lora_proj(const LoraProjArgs a) {
-    constexpr int R = NT * 8;
-    constexpr int WS = TB ? LG_XS : R * 2 + 16;
-    constexpr int WROWS = TB ? R : LP_COLS;
-    constexpr int XBYTES = LP_TOK * LG_XS;
-    constexpr int STAGE = XBYTES + WROWS * WS;
+// TB = 0: W is [F, R]; TB = 1: W is [R, F].
+// grid = (token blocks * S, products); M > 1: one row of blocks for M products of the same X and F.
+// TOK 64 with pieces of 128 columns (64 where the members' W would leave one CTA to an SM), or 32 with pieces of 256.
+template <int NT, int TB, int M, int TOK> struct LoraProj {
+    static constexpr int R = NT * 8, COLS = TOK == 32 ? 256 : (R * M > 64 ? 64 : 128);
+    static constexpr int XS = COLS * 2 + 16, WS = TB ? XS : (R == 8 ? 16 : R * 2 + 16), WROWS = TB ? R : COLS;    // padded pitches: conflict-free ldmatrix
+    static constexpr int XBYTES = TOK * XS, WBYTES = WROWS * WS, STAGE = XBYTES + M * WBYTES;
+    static constexpr int ROOM = 113 * 1024;                // two CTAs to an SM
+    static constexpr int STAGES = STAGE * 4 <= ROOM ? 4 : 3;
+    static constexpr int RT = TOK / 16, KQ = 8 / RT;       // row tiles, shares of a piece's depth: one warp each
+    static constexpr int RP = M * R % 16 ? M * R : M * R + 8;              // row pitch of the sums in floats: rows of a fragment in banks of their own
+    static constexpr int RED = (KQ + 1) * TOK * RP * 4; // the shares and their sum
+    static constexpr int SMEM = STAGES * STAGE > RED ? STAGES * STAGE : RED;
+    static_assert(SMEM <= ROOM, "two CTAs to an SM");
+};
+template <int NT, int TB, int M, int TOK>
+__global__ void __launch_bounds__(256) k_lora_proj(const __grid_constant__ LoraProjArgs a) {
+    using L = LoraProj<NT, TB, M, TOK>;
+    constexpr int R = L::R, COLS = L::COLS, XS = L::XS, WS = L::WS, XBYTES = L::XBYTES, WBYTES = L::WBYTES, STAGE = L::STAGE, STAGES = L::STAGES, RM = R * M, RP = L::RP;
     extern __shared__ __align__(128) uint8_t lg_smem[];
     const uint32_t sbase = lg_smem_u32(lg_smem);
-    const LoraProjProb P = a.p[blockIdx.y];
-    const int part = blockIdx.x % a.S, t0 = blockIdx.x / a.S * LP_TOK;     // a.S CTAs along x are one cluster
+    const int g0 = blockIdx.y;                             // 0 where M > 1
+    const bf16* const X = a.p[g0].X;
+    const int F = a.p[g0].F;
+    const int part = blockIdx.x % a.S, t0 = blockIdx.x / a.S * TOK;     // a.S CTAs along x are one cluster
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int pieces = (P.F + LP_COLS - 1) / LP_COLS;
+    const int pieces = (F + COLS - 1) / COLS;
     const int st0 = (int)((long long)pieces * part / a.S), nstage = (int)((long long)pieces * (part + 1) / a.S) - st0;
+    int at = nstage > 0 ? st0 + (int)(blockIdx.x / a.S) % nstage : 0;       // the piece to load next: neighbours start apart
     pdl_enter();
 
     auto load_stage = [&](int st) {
-        const int f0 = (st0 + st) * LP_COLS;
-        const uint32_t xs = sbase + (st % LP_STAGES) * STAGE, ws_ = xs + XBYTES;
+        const int f0 = at * COLS;
+        at = at + 1 == st0 + nstage ? st0 : at + 1;
+        const uint32_t xs = sbase + (st % STAGES) * STAGE;
 #pragma unroll
-        for (int q = 0; q < (LP_TOK * LP_COLS / 8) / 256; q++) {        // X: 32 rows x 32 chunks
+        for (int q = 0; q < TOK * (COLS / 8) / 256; q++) {           // X: 64 rows of COLS / 8 chunks
             const int idx = q * 256 + tid;
-            const int r = idx >> 5, c8 = idx & 31;
+            const int r = idx / (COLS / 8), c8 = idx % (COLS / 8);
             const int t = t0 + r, f = f0 + c8 * 8;
-            const bool ok = t < a.N && f < P.F;
-            cp_async16(xs + r * LG_XS + c8 * 16, ok ? (const void*)(P.X + (long long)t * P.F + f) : (const void*)P.X, ok ? 16 : 0);
+            const bool ok = t < a.N && f < F;
+            cp_async16(xs + r * XS + c8 * 16, ok ? (const void*)(X + (long long)t * F + f) : (const void*)X, ok ? 16 : 0);
         }
-        if (TB) {                                                       // W [R, F]: R rows x 32 chunks
 #pragma unroll
-            for (int q = 0; q < (R * 32 + 255) / 256; q++) {
-                const int idx = q * 256 + tid;
-                const int r = idx >> 5, c8 = idx & 31;
-                const int f = f0 + c8 * 8;
-                if (r < R) {
-                    const bool ok = f < P.F;
-                    cp_async16(ws_ + r * WS + c8 * 16, ok ? (const void*)(P.W + (long long)r * P.F + f) : (const void*)P.W, ok ? 16 : 0);
-                }
-            }
-        } else {                                                        // W [F, R]: 256 rows x NT chunks
+        for (int m = 0; m < M; m++) {
+            const bf16* const W = a.p[M > 1 ? m : g0].W;
+            const uint32_t ws_ = xs + XBYTES + m * WBYTES;
 #pragma unroll
-            for (int q = 0; q < NT; q++) {
+            for (int q = 0; q < (R * COLS / 8 + 255) / 256; q++) {      // W: R * COLS / 8 chunks either way
                 const int idx = q * 256 + tid;
-                const int r = idx / NT, c8 = idx % NT;
-                const int f = f0 + r;
-                const bool ok = f < P.F;
-                cp_async16(ws_ + r * WS + c8 * 16, ok ? (const void*)(P.W + (long long)f * R + c8 * 8) : (const void*)P.W, ok ? 16 : 0);
+                if (R * COLS / 8 % 256 && idx >= R * COLS / 8) break;
+                const int r = TB ? idx / (COLS / 8) : idx / NT, c8 = TB ? idx % (COLS / 8) : idx % NT;
+                const int f = TB ? f0 + c8 * 8 : f0 + r;
+                const bool ok = f < F;
+                cp_async16(ws_ + r * WS + c8 * 16, ok ? (const void*)(W + (TB ? (long long)r * F + f : (long long)f * R + c8 * 8)) : (const void*)W, ok ? 16 : 0);
             }
         }
-        cp_async_commit();
     };
 
-    float acc[NT][4];
+    float acc[M * NT][4];
 #pragma unroll
-    for (int j = 0; j < NT; j++)
+    for (int j = 0; j < M * NT; j++)
 #pragma unroll
         for (int e = 0; e < 4; e++) acc[j][e] = 0.f;
-    const int mt = warp & 1, kq = warp >> 1;               // row tile, quarter of the piece's depth
+    const int mt = warp % L::RT, kq = warp / L::RT;        // row tile, share of the piece's depth
     const int mi = lane >> 3, ri = lane & 7;
 
-    for (int st = 0; st < LP_STAGES - 1 && st < nstage; st++) load_stage(st);
+#pragma unroll
+    for (int st = 0; st < STAGES; st++) { if (st < nstage) load_stage(st); cp_async_commit(); }
     for (int st = 0; st < nstage; st++) {
-        if (st + LP_STAGES - 1 < nstage) { load_stage(st + LP_STAGES - 1); cp_async_wait<LP_STAGES - 1>(); }
-        else if (st + 2 == nstage) cp_async_wait<1>();
-        else if (st + 1 == nstage) cp_async_wait<0>();
-        else cp_async_wait<LP_STAGES - 2>();
-        __syncthreads();
-        const uint32_t xs = sbase + (st % LP_STAGES) * STAGE, ws_ = xs + XBYTES;
+        if (st == 0) cp_async_wait<STAGES - 1>(); else cp_async_wait<STAGES - 2>();
+        __syncthreads();                                    // piece st is there, and everyone has left piece st - 1
+        if (st) { if (st - 1 + STAGES < nstage) load_stage(st - 1 + STAGES); cp_async_commit(); }
+        const uint32_t xs = sbase + (st % STAGES) * STAGE;
 #pragma unroll
-        for (int ks = 0; ks < 4; ks++) {
-            const int k0 = kq * 64 + ks * 16;
+        for (int ks = 0; ks < COLS / L::KQ / 16; ks++) {
+            const int k0 = kq * (COLS / L::KQ) + ks * 16;
             uint32_t afr[4];                                 // X fragments: (rows 0-7, k 0-7) (rows 8-15, k 0-7) (rows 0-7, k 8-15) (rows 8-15, k 8-15)
-            ldsm_x4(xs + (mt * 16 + (mi & 1) * 8 + ri) * LG_XS + (k0 + (mi >> 1) * 8) * 2, afr);
+            ldsm_x4(xs + (mt * 16 + (mi & 1) * 8 + ri) * XS + (k0 + (mi >> 1) * 8) * 2, afr);
 #pragma unroll
-            for (int nt = 0; nt < NT; nt++) {
-                uint32_t bfr[2];
-                if (TB) ldsm_x2(ws_ + (nt * 8 + ri) * WS + (k0 + (mi & 1) * 8) * 2, bfr);           // W^T stored [n][k]
-                else ldsm_x2_t(ws_ + (k0 + (mi & 1) * 8 + ri) * WS + nt * 16, bfr);                  // W stored [k][n]
-                mma_bf16_16816(acc[nt], afr, bfr);
+            for (int m = 0; m < M; m++) {
+                const uint32_t ws_ = xs + XBYTES + m * WBYTES;
+#pragma unroll
+                for (int nt = 0; nt < NT; nt += 2) {         // W^T stored [n][k], or W stored [k][n]; two column tiles a load
+                    uint32_t bfr[4];
+                    const int n8 = nt + (NT > 1 ? mi >> 1 : 0);
+                    const uint32_t at = TB ? ws_ + (n8 * 8 + ri) * WS + (k0 + (mi & 1) * 8) * 2 : ws_ + (k0 + (mi & 1) * 8 + ri) * WS + n8 * 16;
+                    if (NT == 1) { if (TB) ldsm_x2(at, bfr); else ldsm_x2_t(at, bfr); }
+                    else { if (TB) ldsm_x4(at, bfr); else ldsm_x4_t(at, bfr); }
+                    mma_bf16_16816(acc[m * NT + nt], afr, bfr);
+                    if (NT > 1) mma_bf16_16816(acc[m * NT + (nt + 1) % NT], afr, bfr + 2);
+                }
             }
         }
-        __syncthreads();
     }
-    // the four depth quarters of a row tile meet in shared memory (the operand stages are free now)
-    float* red = reinterpret_cast<float*>(lg_smem);         // [kq][32 rows][R]
+    cp_async_wait<0>();
+    __syncthreads();
+    // the depth shares of a row tile meet in shared memory (the operand stages are free now)
+    float* red = reinterpret_cast<float*>(lg_smem);         // [kq][TOK rows][M * R]
     const int gq = lane >> 2, q2 = (lane & 3) * 2;
 #pragma unroll
     for (int h = 0; h < 2; h++)
 #pragma unroll
-        for (int nt = 0; nt < NT; nt++)
-            *reinterpret_cast<float2*>(red + ((kq * LP_TOK) + mt * 16 + h * 8 + gq) * R + nt * 8 + q2) = make_float2(acc[nt][h * 2], acc[nt][h * 2 + 1]);
+        for (int nt = 0; nt < M * NT; nt++)
+            *reinterpret_cast<float2*>(red + (kq * TOK + mt * 16 + h * 8 + gq) * RP + nt * 8 + q2) = make_float2(acc[nt][h * 2], acc[nt][h * 2 + 1]);
     __syncthreads();
-    auto quarters = [&](int r, int c) {
-        float2 s = make_float2(0.f, 0.f);
+    auto shares = [&](int j) {
+        const int i = j / RM * RP + j % RM;
+        float2 u = *reinterpret_cast<const float2*>(red + i);
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const float2 v = *reinterpret_cast<const float2*>(red + (q * LP_TOK + r) * R + c);
-            s.x += v.x; s.y += v.y;
+        for (int q = 1; q < L::KQ; q++) {
+            const float2 v = *reinterpret_cast<const float2*>(red + q * TOK * RP + i);
+            u.x += v.x; u.y += v.y;
         }
-        return s;
+        return u;
+    };
+    auto store = [&](int i, float2 s) {
+        const int r = i / RM, m = i % RM / R, c = i % R;
+        if (t0 + r < a.N) *reinterpret_cast<__nv_bfloat162*>(a.p[M > 1 ? m : g0].out + (long long)(t0 + r) * R + c) = __floats2bfloat162_rn(a.alpha * s.x, a.alpha * s.y);
     };
     if (a.S == 1) {
-        for (int i = tid; i < LP_TOK * R / 2; i += 256) {
-            const int r = (i * 2) / R, c = (i * 2) % R;
-            const float2 s = quarters(r, c);
-            if (t0 + r < a.N) *reinterpret_cast<__nv_bfloat162*>(P.out + (long long)(t0 + r) * R + c) = __floats2bfloat162_rn(a.alpha * s.x, a.alpha * s.y);
-        }
+        for (int i = tid * 2; i < TOK * RM; i += 512) store(i, shares(i));
         return;
     }
     // the cluster's parts: every CTA leaves its sum, then finishes 1 / S of the rows from all CTAs' sums, in part order
-    float* mine = red + 4 * LP_TOK * R;
-    for (int i = tid; i < LP_TOK * R / 2; i += 256) *reinterpret_cast<float2*>(mine + i * 2) = quarters((i * 2) / R, (i * 2) % R);
+    float* mine = red + L::KQ * TOK * RP;
+    for (int i = tid * 2; i < TOK * RM; i += 512) *reinterpret_cast<float2*>(mine + i) = shares(i);
     cluster_sync();
-    const int rows = LP_TOK / a.S;
-    for (int i = tid; i < rows * R / 2; i += 256) {
-        const int r = part * rows + (i * 2) / R, c = (i * 2) % R;
+    const int share = TOK / a.S * RM;
+    for (int i = part * share + tid * 2; i < (part + 1) * share; i += 512) {
         float2 s = make_float2(0.f, 0.f);
-        const uint32_t at = lg_smem_u32(mine + r * R + c);
+        const uint32_t at = lg_smem_u32(mine + i);
         for (int p = 0; p < a.S; p++) {
             float2 v;
             asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %2, %3;\n\tld.shared::cluster.v2.f32 {%0, %1}, [ra];\n\t}"
                          : "=f"(v.x), "=f"(v.y) : "r"(at), "r"(p) : "memory");
             s.x += v.x; s.y += v.y;
         }
-        if (t0 + r < a.N) *reinterpret_cast<__nv_bfloat162*>(P.out + (long long)(t0 + r) * R + c) = __floats2bfloat162_rn(a.alpha * s.x, a.alpha * s.y);
+        store(i, s);
     }
     cluster_sync();   // peers have read
 }
 
-template <int NT, int TB> static size_t lora_proj_smem() {
-    constexpr int R = NT * 8;
-    return (size_t)LP_STAGES * (LP_TOK * LG_XS + (TB ? R * LG_XS : LP_COLS * (R * 2 + 16)));
-}
-template <int NT, int TB> static int lora_proj_launch(const LoraProjArgs& a, cudaStream_t st) {
-    static bool attr = false;
-    const size_t smem = lora_proj_smem<NT, TB>();
-    if (!attr) { cudaFuncSetAttribute(k_lora_proj<NT, TB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); attr = true; }
-    // Depth split: 32 tokens a CTA leave SMs idle below 296 CTAs (two fit an SM), and a CTA that walks all of F alone is a chain of
-    // round trips: x A of 2048 x 4096 at rank 16 17 us on 64 CTAs, 8.6 us on 256.  Never beyond one resident wave: 8192 x 1536
-    // 11.0 us on 256 CTAs, 13.9 us on 512.
-    const int blocks = (a.N + LP_TOK - 1) / LP_TOK;
+template <int NT, int TB, int M, int TOK> static int lora_proj_launch(const LoraProjArgs& a, cudaStream_t st) {
+    using L = LoraProj<NT, TB, M, TOK>;
+    static const cudaError_t attr = cudaFuncSetAttribute(k_lora_proj<NT, TB, M, TOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM);
+    if (attr != cudaSuccess) return 3;
+    const int blocks = (a.N + TOK - 1) / TOK, rows = M > 1 ? 1 : a.count;
     int least = 1 << 30;
     for (int g = 0; g < a.count; g++) least = a.p[g].F < least ? a.p[g].F : least;
-    const int pieces = (least + LP_COLS - 1) / LP_COLS;
+    const int pieces = (least + L::COLS - 1) / L::COLS;
+    // Depth split: a CTA that walks all of F alone is a chain of round trips, and few token blocks leave SMs idle.  Never beyond
+    // one resident wave (two CTAs an SM): x A of 8192 x 1536 in blocks of 32 tokens 11.0 us on 256 CTAs, 13.9 us on 512.
     LoraProjArgs b = a;
     b.S = 1;
-    while (b.S < 8 && blocks * a.count * 2 * b.S <= 2 * AX_SMS && pieces >= 3 * b.S) b.S *= 2;
+    while (b.S < 8 && blocks * rows * 2 * b.S <= 2 * AX_SMS && pieces >= 2 * b.S) b.S *= 2;
+    // Where even the split leaves SMs without a CTA the walk's length counts, not W's traffic: 32 tokens and wide pieces.
+    // Rank 16, one product: 70 x 4096 4.4 us in blocks of 64, 3.5 of 32; 1024 x 4096 6.3 and 5.2; above, 2048 x 4096 7.3 and 8.1.
+    if (M == 1 && TOK == 64 && blocks * rows * b.S <= AX_SMS) return lora_proj_launch<NT, TB, 1, 32>(a, st);
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(blocks * b.S, a.count); cfg.blockDim = dim3(256); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    cfg.gridDim = dim3(blocks * b.S, rows); cfg.blockDim = dim3(256); cfg.dynamicSmemBytes = L::SMEM; cfg.stream = st;
     cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = b.S; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
     at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at; cfg.numAttrs = ax_gemm_pdl() ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, k_lora_proj<NT, TB>, b) == cudaSuccess ? 0 : 3;
+    return cudaLaunchKernelEx(&cfg, k_lora_proj<NT, TB, M, TOK>, b) == cudaSuccess ? 0 : 3;
 }
 
 // out[g] [N, R] bf16 = alpha * X[g] [N, F[g]] W[g]; tb 0: W [F, R], tb 1: W [R, F].  -1 when not served.
@@ -401,7 +417,16 @@ int ax_lora_proj(int count, int tb, const void* const* X, const void* const* W, 
         if (F[g] < 8 || F[g] % 8 || !aligned16(X[g]) || !aligned16(W[g]) || !out[g] || ((uintptr_t)out[g] & 3)) return -1;
         a.p[g].X = (const bf16*)X[g]; a.p[g].W = (const bf16*)W[g]; a.p[g].out = (bf16*)out[g]; a.p[g].F = F[g];
     }
-#define LP(NT_) (tb ? lora_proj_launch<NT_, 1>(a, st) : lora_proj_launch<NT_, 0>(a, st))
+    // Members of one X pay where a CTA per product would go beyond a resident wave (three products of rank 32, 8192 x 1536:
+    // 18.6 us as members, 24.3 each), or where token blocks alone occupy the SMs with a short member loop (rank 16, three of
+    // 2048 x 4096 10.5 and 15.0 us, two of 3000 x 2048 7.9 and 9.1; rank 32, three of 3000 x 1536 11.3 and 9.4; two of 256 x 1024 3.8 and 3.4).
+    bool one_x = true;
+    for (int g = 1; g < count; g++) one_x = one_x && X[g] == X[0] && F[g] == F[0];
+    const int blocks = (N + 63) / 64;                      // token blocks
+    const int members = one_x && ((blocks >= 32 && R * count <= 64) || blocks * count > 2 * AX_SMS) ? count : 1;
+#define LPM(NT_, TB_) (members == 3 ? lora_proj_launch<NT_, TB_, 3, 64>(a, st) : (members == 2 ? lora_proj_launch<NT_, TB_, 2, 64>(a, st) : lora_proj_launch<NT_, TB_, 1, 64>(a, st)))
+#define LP(NT_) (tb ? LPM(NT_, 1) : LPM(NT_, 0))
     return R == 8 ? LP(1) : (R == 16 ? LP(2) : LP(4));
 #undef LP
+#undef LPM
 }

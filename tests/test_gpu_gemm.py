@@ -670,6 +670,34 @@ def test_adapter_skinny_products_with_the_depth_split_over_a_cluster(eng, tb, N,
         assert np.all(runs[0][g][N * R:] == 3.0)
 
 
+@pytest.mark.parametrize("tb", [0, 1])
+@pytest.mark.parametrize("N,F,R,count,one", [(2031, 1544, 16, 3, 1), (2048, 264, 32, 2, 1), (6401, 136, 32, 3, 1), (1985, 8, 8, 3, 1),
+                                             (1984, 1032, 16, 3, 1), (2500, 520, 16, 3, 0), (1200, 4096, 16, 1, 1)])
+def test_adapter_skinny_products_of_one_input_as_members(eng, tb, N, F, R, count, one):
+    """Products of one X share its stage (from 32 token blocks on, rank * count <= 64, or beyond one wave of CTAs), on both
+    sides of that line.  Widths end inside a piece, token counts inside a block; nothing is written past an output."""
+    rng = np.random.default_rng(N + F + R + tb)
+    Xs = [bf(rng.standard_normal((N, F)).astype(np.float32)) for _ in range(1 if one else count)]
+    Xs = Xs * count if one else Xs
+    Ws = [bf(rng.standard_normal((R, F) if tb else (F, R)).astype(np.float32) * 0.1) for _ in range(count)]
+    ix = [put(eng, X, 1) for X in (Xs[:1] if one else Xs)]
+    ix = (ix * count if one else ix) + [0, 0]
+    iw = [put(eng, w, 1) for w in Ws] + [0, 0]
+    io = [eng.alloc(N * R + 64, 2) for _ in range(count)] + [0, 0]
+    for o_ in io[:count]:
+        eng.upload_bf16(o_, np.full(N * R + 64, 3.0, np.float32))
+    eng.launch_count(reset=True)
+    eng.run([op(E.LORA_PROJ, a=ix[0], sa=ix[1], sb=ix[2], b=iw[0], d=iw[1], sc=iw[2], c=io[0], oa=io[1], ob=io[2], n=F, k=F, oc=F,
+                m=N, batch=count, tb=tb, gamma=float(R), alpha=0.5, dt=1)])
+    assert eng.last_variant() == 0x62 and eng.launch_count() == 1
+    for g in range(count):
+        got = eng.download_bf16(io[g], (N * R + 64,))
+        ref = 0.5 * (Xs[g].astype(np.float64) @ (Ws[g].T if tb else Ws[g]).astype(np.float64))
+        assert np.abs(got[:N * R].reshape(N, R) - ref).max() <= 1.02 * 2.0 ** -8 * np.abs(ref).max()      # one rounding to bf16
+        assert np.all(got[N * R:] == 3.0)
+    assert eng.device_status() == 0
+
+
 @pytest.mark.parametrize("fused", [0, 1])
 def test_a_fused_product_leaves_pending_segments_to_their_group(eng, fused):
     """GEMM_XSEG announces operands for the next GEMM_GROUP; a plain product with its SwiGLU backward may stand between the two,
