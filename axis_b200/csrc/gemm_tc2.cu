@@ -1,11 +1,12 @@
 // bf16 GEMM with paired CTAs (tcgen05 cta_group::2): a cluster of two CTAs on
-// neighbouring SMs computes one 256 x 256 output tile.  Each CTA loads its own
-// 128 rows of A and its own 128 columns of B (plain TMA tile loads — nothing is
+// neighbouring SMs computes one output tile of 256 x 256 (or, by a rule at
+// ax_gemm_width, 192 or 128 columns).  Each CTA loads its own 128 rows of A and
+// its own half of the columns of B (plain TMA tile loads — nothing is
 // multicast; the pair shares B through the MMA unit, which reads both CTAs'
 // shared memory), so a k-block costs 32 KB of L2->smem traffic per SM instead of
 // the 48 KB of the single-CTA 128 x 256 tile, and half the smem operand reads
 // per flop.  CTA 0 of the pair issues the MMAs (M = 256); accumulators live in
-// both CTAs' TMEM (128 lanes x 256 columns each, double-buffered); completion is
+// both CTAs' TMEM (128 lanes x the tile's columns, double-buffered); completion is
 // signalled to both CTAs with multicast commits; every CTA writes its own 128
 // rows of C.
 //

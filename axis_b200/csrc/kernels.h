@@ -186,7 +186,7 @@ int ax_attn_fwd_tc(const void* q, const void* k, const void* v, void* o, float* 
                    const AttnShape& s, int* status, cudaStream_t st);
 // dq_acc: fp32 accumulator of B*T*H*DH elements for the dQ reduce-add (null -> not served).
 // rope_cos / rope_sin (fp32 [T, DH/2], may be null): when given, the inverse rotary is applied to dq and dk
-// before they are rounded to bf16 (head_dim 64 only; -1 otherwise, the caller then runs the rotary op itself).
+// before they are rounded to bf16 (-1: not a shape of these kernels; other kernels leave the rotary to an op of its own).
 int ax_attn_tc_parts(const AttnShape& s);      // CTAs to a key tile in the backward of whole tiles (0: not such a shape)
 int ax_attn_bwd_tc(const void* q, const void* k, const void* v, const void* o, const void* dO,
                    const float* lse, float* Dscratch, float* dq_acc, void* dq, void* dk, void* dv,

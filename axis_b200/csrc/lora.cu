@@ -209,8 +209,7 @@ int ax_lora_grad(int count, const void* const* X, const void* const* S, float* c
 // u = x A in the forward and t = g B^T in the backward: again a stream over the wide operand with 16 flops per byte.
 // A CTA takes TOK tokens and walks F in pieces of COLS columns; its eight warps are the row tiles times equal shares of a
 // piece's depth, and the partial accumulators of a row tile meet in shared memory.  What bounds it is what an SM takes in:
-// besides its X a CTA reads all of W, from L2, so that 32 tokens a CTA moved as much W as X (rank 16: 32 bytes of W against
-// 64 of X a column).  Hence 64 tokens, and products of one X (the adapters of q, k and v, of gate and up) as M members
+// besides its X a CTA reads all of W, from L2: at 32 tokens a CTA half as many bytes as X at rank 16, as many at rank 32.  Hence 64 tokens, and products of one X (the adapters of q, k and v, of gate and up) as M members
 // of one CTA, where X is staged once for all of them; one barrier a piece, all stages in flight from the start, and
 // neighbouring token blocks begin at different pieces, or all SMs ask for the same lines of W at the same time.
 // Rank 16, three products of one X, 8192 x 1536: 25.4 us with 32 tokens and a CTA per product, 17.0 with 64 and members,

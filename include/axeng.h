@@ -165,8 +165,10 @@ long long eng_bytes_allocated(void);
 /* Code of the kernel variant the last GEMM / cross-entropy op ran on (no counterpart in the reference; lets a
  * test assert that a shape was served by the kernel it means to check): 0x10 cross-entropy streaming rows,
  * 0x11 register-resident rows; 0x80 / 0x81 attention forward / backward with split probabilities on tcgen05, 0x82 / 0x83 on mma.sync
- * (the backward plus 0x100 times the CTAs that share a key tile); 0x20 general GEMM, 0x21 single-CTA tcgen05 GEMM, 0x22 paired-CTA tcgen05 GEMM, 0x23 a group of them, 0x26 small products,
- * the GEMM codes plus 0x100 times the split-K factor. */
+ * (the backward plus 0x100 times the CTAs that share a key tile), 0x84 / 0x85 in fp32 at head dims 12 to 64; 0x20 general GEMM, 0x21 single-CTA
+ * tcgen05 GEMM, 0x22 paired-CTA tcgen05 GEMM, 0x23 a group of them, 0x26 small products, 0x24 / 0x27 / 0x2a the SwiGLU backward
+ * inside a small / paired-CTA / fp32 product, 0x25 / 0x28 the SwiGLU inside a pair with adapters on the first two, 0x29 a group
+ * of fp32 products as one launch, the GEMM codes plus 0x100 times the split-K factor; 0x60 / 0x62 the adapters' gradients / skinny products. */
 int eng_last_variant(void);
 /* Pairs of CTAs that shared the depth of a tile in the last paired-CTA tcgen05 launch: 1, 2 or 4. */
 int eng_last_gemm_parts(void);
@@ -176,7 +178,8 @@ int eng_last_gemm_width(void);
  * kernels with split probabilities once the whole-tile kernels have refused it (for the backward the number of CTAs that share a key tile,
  * 1, 2 or 4) or not (0): host arithmetic that needs no GPU. */
 int eng_attn_route(int backward, int B, int H, int KV, int T, int head_dim);
-/* Dynamic shared memory in bytes of the general attention kernels, 0 forward, 1 dQ, 2 dK / dV, for a head dim of 1 to 256
+/* Dynamic shared memory in bytes of the general attention kernels (those of the general head dims; the fp32 kernels of head dims 12 to 64
+ * are others), 0 forward, 1 dQ, 2 dK / dV, for a head dim of 1 to 256
  * (else -1): host arithmetic that needs no GPU. */
 long long eng_attn_smem(int which, int head_dim);
 /* CTAs that share a block's walk in those kernels (1: none do; 0: not a shape): host arithmetic, too. */
