@@ -132,15 +132,29 @@ __device__ __forceinline__ void cluster_sum16(uint32_t at, int S, float* a) {
 // CTAs that share the walk of a key tile of 128 in the backward kernels of whole tiles (clusters, whose dK and dV meet through distributed shared memory).  One
 // CTA to a key tile and kv head is as long as its chain, the query tiles of all heads of the group; 74 clusters of two and 33 of four run at once.
 // Backward in us with 1 / 2 / 4 (CTAs at 1, chain), head_dim 64 | 128 where a tile of the chain costs twice as much:
-// B8 H24 KV8 T128 (64, 3) 20.6 / 22.1 / 37.1 | 31.6 / 26.8 / 48.7, B1 H8 KV2 T512 (8, 16) 39.9 / 27.5 / 23.2 | 72.3 / 44.6 / 34.1, B8 H16 KV4 T256 (64, 8)
-// 30.7 / 26.2 / 40.1 | 51.6 / 38.2 / 54.5, B2 H16 KV4 T1024 (64, 32) 73.2 / 47.5 / 53.0 | 142 / 83.4 / 77.2, B1 H16 KV4 T2048 (64, 64) 130 / 76 / 67 | 262 / 144 /
-// 107, B2 H16 KV8 T768 (96, 12) 38.1 / 36.7 / 58.5 | 65.6 / 48.8 / 76.4, B1 H8 KV8 T2048 (128, 16) 44.3 / 44.3 / 79 | 79.7 / 60.4 / 104, B1 H16 KV4 T4096
-// (128, 128) 252 / 137 / 185 | 514 / 275 / 329, B4 H24 KV8 T768 (192, 18) 54.0 / 72.6 / 126 | 104 / 117 / 181.
-static inline int attn_tile_parts(int head_dim, long long ctas, long long chain) {
+// B1 H8 KV2 T512 (8, 16) 39.9 / 27.5 / 23.2 | 72.3 / 44.6 / 34.1, B8 H16 KV4 T256 (64, 8) 30.7 / 26.2 / 40.1 | 51.6 / 38.2 / 54.5, B2 H16 KV4 T1024 (64, 32) 73.2 /
+// 47.5 / 53.0 | 142 / 83.4 / 77.2, B1 H16 KV4 T2048 (64, 64) 130 / 76 / 67 | 262 / 144 / 107.  Short chains: B3 H8 KV4 T256 (24, 4) 17.6 / 17.2, B24 H2 KV1 T256
+// (48, 4) 18.1 / 19.1, B8 H6 KV3 T384 (72, 6) 23.0 / 21.9 | B11 H4 KV2 T128 (22, 2) 19.1 / 18.8, B31 H2 KV2 T256 (62, 2) 19.6 / 20.6, B27 H6 KV2 T128 (54, 3) 26.4 / 25.6.
+// A cluster that starts late is another set-up, first load and merge, 9 tiles of the chain at head_dim 64 and 4.5 at 128, behind the shortest walks of the first
+// round: it pays where the walks of a head's key tiles differ enough.  Two CTAs, beyond 74 key tiles (CTAs, key tiles to a head, heads of a group): T128 (80, 1, 2)
+// 17 / 30 | 23.9 / 38.3, (96, 1, 4) | 38.0 / 53.8, T256 (96, 2, 2) | 31.9 / 40.0, (88, 2, 4) | 51.2 / 53.1, T512 (96, 4, 3) 36.5 / 38.6, (84, 4, 2) | 46.1 / 39.7, T768
+// (96, 6, 2) 38.1 / 36.7, T640 (100, 5, 3) | 75.2 / 58.7, T1536 (84, 12, 3) 78.3 / 50.4, (144, 12, 3) | 157 / 114, T4096 (128, 32, 3) 186 / 108; B4 H24 KV8 T768 (192, 6, 3)
+// 54.0 / 72.6 | 104 / 117.  Four CTAs beyond 33 key tiles, 2 / 4: T2048 (64, 16, 16) 256 / 167, T1024 (64, 8, 8) 78.9 / 71.8, T256 (40, 2, 32) | 179 / 141; T128
+// (36, 1, 48) 85 / 104 | (40, 1, 32) 121 / 141.
+static inline int attn_tile_parts(int head_dim, long long ctas, int key_tiles /* of a head */, int rep) {
     const bool wide = head_dim > 64;
+    const long long chain = (long long)rep * key_tiles;
+    // Clusters of S, `fit` of which run at once, the longest first: twice S times what they take less than one CTA for each does, in tiles of the chain.  The last to
+    // start in the second round waits for walk number 2 fit - ctas of the first.
+    auto gain = [&](int S, int fit) {
+        const long long late = ctas - fit, heads = ctas / key_tiles;
+        if (late > fit) return -1ll;
+        const long long first = (fit - late) / heads;
+        return S * chain - rep * (key_tiles - first + 1);
+    };
     int S = 1;
-    if (ctas <= AX_SMS / 2 ? chain >= (wide ? 2 : 4) : ctas <= AX_SMS && chain >= (wide ? 2 : 12)) S = 2;
-    if (S == 2 && (ctas <= 33 ? chain >= 8 : ctas <= AX_SMS / 2 && chain >= (wide ? 32 : 48))) S = 4;
+    if (ctas <= AX_SMS / 2 ? chain >= (wide ? 2 : 4) + (ctas <= 40 ? 0 : wide ? 1 : 2) : ctas <= AX_SMS && gain(2, AX_SMS / 2) > (wide ? 9 : 15)) S = 2;
+    if (S == 2 && (ctas <= 33 ? chain >= 8 : ctas <= AX_SMS / 2 && key_tiles > 1 && chain >= (wide ? 32 : 48))) S = 4;
     return S;
 }
 // Launch of a kernel whose CTAs form clusters of S (1: none).  Up to half a CTA for each SM start while the grid in front of them ends (the step of two layers of 512

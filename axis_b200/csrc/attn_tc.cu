@@ -829,7 +829,7 @@ static int map_dq_f32(CUtensorMap* m, const void* base, int B, int T, int heads)
 int ax_attn_tc_parts(const AttnShape& s) {
     if (s.DH != ADH && s.DH != 128) return 0;
     if (s.T < AT || s.T % AT || s.KV < 1 || s.H % s.KV) return 0;
-    return attn_tile_parts(s.DH, (long long)(s.T / AT) * s.KV * s.B, (long long)s.H / s.KV * (s.T / AT));
+    return attn_tile_parts(s.DH, (long long)(s.T / AT) * s.KV * s.B, s.T / AT, s.H / s.KV);
 }
 int ax_attn_fwd_tc(const void* q, const void* k, const void* v, void* o, float* lse,
                    const AttnShape& s, int* status, cudaStream_t st) {
@@ -861,7 +861,7 @@ int ax_attn_bwd_tc(const void* q, const void* k, const void* v, const void* o, c
     if (want_prof && cudaMalloc(&prof, (size_t)nblk * 256) == cudaSuccess) cudaMemset(prof, 0, (size_t)nblk * 256); else prof = nullptr;
     cudaMemcpyToSymbol(g_bwd_prof, &prof, sizeof(prof));
 #endif
-    const int S = attn_tile_parts(s.DH, grid.x, (long long)s.H / s.KV * (s.T / AT));
+    const int S = attn_tile_parts(s.DH, grid.x, s.T / AT, s.H / s.KV);
     if (attn_launch(S > 1 ? k_attn_bwd_tc<true> : k_attn_bwd_tc<false>, grid.x, BWD_THREADS, BwdSmem::TOTAL, S, st, tq, tk, tv, tdo, tdq, lse, (const float*)Dscratch, (bf16*)dk, (bf16*)dv,
                            s.T, s.H, s.KV, s.scale, rope_cos, rope_sin, S, status) != cudaSuccess) return 3;
 #ifdef AXENG_PROF

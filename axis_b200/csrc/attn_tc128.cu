@@ -664,7 +664,7 @@ int ax_attn_bwd_tc128(const void* q, const void* k, const void* v, const void* o
     const long long rows = (long long)s.B * s.T * s.H;
     if (ax_launch_chain(k_attn_bwd_prep128, dim3(ew_grid(rows * 16, 256)), dim3(256), 0, st, (const bf16*)o, (const bf16*)dO, Dscratch, g_dq_acc, s.B, s.T, s.H) != cudaSuccess) return 3;
     dim3 grid((s.T / AT) * s.KV * s.B);
-    const int S = attn_tile_parts(s.DH, grid.x, (long long)s.H / s.KV * (s.T / AT));
+    const int S = attn_tile_parts(s.DH, grid.x, s.T / AT, s.H / s.KV);
     if (attn_launch(S > 1 ? k_attn_bwd_tc128<true> : k_attn_bwd_tc128<false>, grid.x, BWD128_THREADS, Bwd128Smem::TOTAL, S, st, tq, tk, tv, tdo, tdq, lse, (const float*)Dscratch, (bf16*)dk, (bf16*)dv,
                            s.T, s.H, s.KV, s.scale, rope_cos, rope_sin, S, status) != cudaSuccess) return 3;
     if (rope_cos) {

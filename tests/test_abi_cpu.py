@@ -115,6 +115,19 @@ def test_ctas_to_a_key_tile_of_the_attention_backward(lib, B, H, KV, T, parts):
     assert lib.eng_attn_route(1, B, H, KV, T, 64 if T % 128 else 56) == parts
 
 
+@pytest.mark.parametrize("B,H,KV,T,parts64,parts128", [
+    # short chains: the second CTA's set-up and the merge cost more than half a chain
+    (22, 1, 1, 128, 1, 1), (4, 24, 12, 128, 1, 1), (2, 24, 12, 256, 1, 2), (13, 16, 4, 128, 1, 2), (1, 10, 10, 512, 2, 2), (2, 16, 4, 1024, 2, 4), (1, 16, 4, 1024, 4, 4),
+    # one key tile to a head: no shorter walk for a cluster to wait for, beyond what runs at once not even for the longest chain
+    (10, 16, 8, 128, 1, 1), (6, 64, 16, 128, 1, 1), (23, 12, 4, 128, 1, 1), (16, 128, 8, 128, 1, 1), (40, 32, 1, 128, 2, 2), (24, 32, 1, 128, 4, 4),
+    # clusters that start late: only where the walks of the first round differ enough
+    (16, 12, 4, 256, 1, 1), (12, 8, 4, 256, 1, 1), (22, 8, 2, 256, 1, 1), (13, 2, 2, 384, 1, 1), (6, 12, 4, 512, 1, 2), (25, 3, 1, 512, 1, 2), (11, 9, 3, 512, 1, 1), (3, 8, 8, 512, 1, 1),
+    (7, 6, 3, 512, 1, 2), (20, 3, 1, 640, 2, 2), (2, 16, 8, 768, 2, 2), (6, 16, 4, 768, 2, 2), (7, 3, 1, 1536, 2, 2), (9, 2, 1, 2048, 2, 2), (2, 6, 2, 4096, 2, 2), (4, 24, 8, 768, 1, 1)])
+def test_ctas_to_a_key_tile_of_whole_tiles(lib, B, H, KV, T, parts64, parts128):
+    assert [lib.eng_attn_tile_parts(B, H, KV, T, dh) for dh in (64, 128)] == [parts64, parts128]
+    assert lib.eng_attn_tile_parts(B, H, KV, T + 8, 64) == lib.eng_attn_tile_parts(B, H, KV, T, 96) == 0
+
+
 def test_attention_route_of_invalid_shapes(lib):
     for a in ((0, 8, 4, 500, 64), (1, 0, 4, 500, 64), (1, 8, 0, 500, 64), (1, 8, 3, 500, 64), (1, 8, 4, 0, 64), (1, 8, 4, 500, 0)):
         assert lib.eng_attn_route(0, *a) == lib.eng_attn_route(1, *a) == 0
