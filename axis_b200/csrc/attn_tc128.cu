@@ -534,32 +534,37 @@ k_attn_bwd_tc128(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             // dV (half 0 threads) and dK (half 1 threads): complete once the last commit has fired — waited in drain
             const int t = j * AT + r;
             const uint32_t ta = (hf ? t_dK : t_dV) + lane_base;
-            if (SPLIT) {                                     // [dV, dK][key][128] in the place of K, V and the ring, whose last readers have run
+            // Sums that meet others, or that are rotated back, go through [dV, dK][key][128] in the place of K, V and the ring, whose last readers have run.
+            if (SPLIT || (hf && rope_cos)) {
                 float* row = reinterpret_cast<float*>(smem) + (hf * AT + r) * BWD128_PITCH;
 #pragma unroll 1
                 for (int ch = 0; ch < DH2 / 32; ch++) {
                     uint32_t v[32];
-                    if (n_it) {
+                    if (!SPLIT || n_it) {
                         tmem_ld32(ta + ch * 32, v);
                         tmem_ld_wait();
                     }
 #pragma unroll
                     for (int q = 0; q < 32; q += 4)
-                        *reinterpret_cast<uint4*>(row + ch * 32 + q) = n_it ? make_uint4(v[q], v[q + 1], v[q + 2], v[q + 3]) : make_uint4(0, 0, 0, 0);
+                        *reinterpret_cast<uint4*>(row + ch * 32 + q) = !SPLIT || n_it ? make_uint4(v[q], v[q + 1], v[q + 2], v[q + 3]) : make_uint4(0, 0, 0, 0);
                 }
             } else {
                 bf16* dst = (hf ? dk : dv) + (((long long)b * T + t) * KV + g) * DH2;
-                const float* cr = hf && rope_cos ? rope_cos + (long long)t * (DH2 / 2) : nullptr;
-                const float* sr = rope_sin + (long long)t * (DH2 / 2);
+                const float f = hf ? scale : 1.f;
 #pragma unroll 1
-                for (int ch = 0; ch < DH2 / 32; ch++) {      // sixteen columns and their rotary partners
-                    uint32_t v1[16], v2[16];
-                    tmem_ld16(ta + ch * 16, v1);
-                    tmem_ld16(ta + DH2 / 2 + ch * 16, v2);
+                for (int ch = 0; ch < DH2 / 32; ch++) {      // 64 bytes of a row
+                    uint32_t v[32];
+                    tmem_ld32(ta + ch * 32, v);
                     tmem_ld_wait();
 #pragma unroll
-                    for (int q = 0; q < 16; q += 8)
-                        store_grad8<DH2 / 2>(reinterpret_cast<float*>(v1 + q), reinterpret_cast<float*>(v2 + q), ch * 16 + q, hf ? scale : 1.f, cr, sr, dst, DH2);
+                    for (int q = 0; q < 32; q += 8) {
+                        uint4 pk;
+                        pk.x = pack_bf16(__uint_as_float(v[q]) * f, __uint_as_float(v[q + 1]) * f);
+                        pk.y = pack_bf16(__uint_as_float(v[q + 2]) * f, __uint_as_float(v[q + 3]) * f);
+                        pk.z = pack_bf16(__uint_as_float(v[q + 4]) * f, __uint_as_float(v[q + 5]) * f);
+                        pk.w = pack_bf16(__uint_as_float(v[q + 6]) * f, __uint_as_float(v[q + 7]) * f);
+                        *reinterpret_cast<uint4*>(dst + ch * 32 + q) = pk;
+                    }
                 }
             }
         } else if (lane == 0) {
@@ -581,6 +586,16 @@ k_attn_bwd_tc128(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                                  (m ? dk : dv) + (((long long)b * T + t) * KV + g) * DH2, DH2);
         }
         cluster_sync();     // peers have read
+    } else if (rope_cos) {
+        // dK: eight threads to a row, whose tables they read and whose result they write side by side.  (From a thread to a row 2 us more for a CTA.)
+        for (int i = threadIdx.x; i < AT * 8; i += BWD128_THREADS) {
+            const int r = i >> 3, c0 = (i & 7) * 8, t = j * AT + r;
+            const float* row = reinterpret_cast<const float*>(smem) + (AT + r) * BWD128_PITCH + c0;
+            float a[16];
+#pragma unroll
+            for (int z = 0; z < 16; z += 4) *reinterpret_cast<float4*>(a + z) = *reinterpret_cast<const float4*>(row + (z & 7) + (z >> 3) * (DH2 / 2));
+            store_grad8<DH2 / 2>(a, a + 8, c0, scale, rope_cos + (long long)t * (DH2 / 2), rope_sin + (long long)t * (DH2 / 2), dk + (((long long)b * T + t) * KV + g) * DH2, DH2);
+        }
     }
 }
 
@@ -592,7 +607,7 @@ __global__ void k_dq_convert128_rope(const float* __restrict__ src, bf16* __rest
     const long long total = rows * 8, stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
         const long long row = i >> 3;
-        const int c0 = (int)(i & 7) * 8, t = (int)((row / H) % T);
+        const int c0 = (int)(i & 7) * 8, t = (int)((unsigned)row / H % T);       // (rows of 512 bytes: fewer than 2^32)
         float a[8], b[8];
         Vec<float>::ld(src + row * DH2 + c0, a); Vec<float>::ld(src + row * DH2 + c0 + 4, a + 4);
         Vec<float>::ld(src + row * DH2 + DH2 / 2 + c0, b); Vec<float>::ld(src + row * DH2 + DH2 / 2 + c0 + 4, b + 4);

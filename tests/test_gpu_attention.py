@@ -444,6 +444,30 @@ def test_whole_tile_backward_with_key_tiles_shared_over_a_cluster(eng, B, H, KV,
     assert eng.device_status() == 0
 
 
+@pytest.mark.parametrize("B,H,KV,T", [(20, 8, 8, 128), (10, 8, 8, 512)])
+def test_rotary_inside_the_head_dim_128_backward_takes_no_longer_than_a_launch_of_its_own(eng, B, H, KV, T):
+    """Many short walks of one CTA each, where the end of a CTA counts (us inside / as a launch of its own on one B200: 30.4 / 33.8 and 62.6 / 66.0; 36 and 70 when each thread rotated a row)."""
+    DH = 128
+    rng = np.random.default_rng(T)
+    q, k, v, do = make(rng, B, H, KV, T, DH, 1)
+    t = lambda x: np.ascontiguousarray(x.transpose(0, 2, 1, 3))
+    iq, ik, iv, ido = (put(eng, t(x), 1) for x in (q, k, v, do))
+    io, ilse, iD = eng.alloc(q.size, 2), eng.alloc(B * H * T), eng.alloc(B * H * T + q.size)
+    idq, idk, idv = eng.alloc(q.size, 2), eng.alloc(k.size, 2), eng.alloc(k.size, 2)
+    cos, sin = O.rope_tables(T, DH)
+    ic, isn = put(eng, cos, 0), put(eng, sin, 0)
+    eng.run([op(E.ATTN_FWD, a=iq, b=ik, d=iv, c=io, sa=ilse, m=T, n=DH, k=KV, batch=B, tb=H, dt=1, alpha=DH ** -0.5)])
+    bwd = lambda **kw: op(E.ATTN_BWD, a=iq, b=ik, d=iv, c=ido, sa=ilse, sb=io, tb=idq, sc=idk, oa=idv, ob=H, oc=iD, m=T, n=DH, k=KV, batch=B, dt=1, alpha=DH ** -0.5, **kw)
+    inside = [bwd(beta=float(ic), gamma=float(isn))] * 40
+    apart = [bwd(), op(E.ROPE_BTHD, a=idq, b=ic, d=isn, c=idq, batch=B, m=T, k=H, n=DH, tb=1, sa=idk, sb=idk, sc=KV, dt=1)] * 40
+    times = {n: [] for n in ("inside", "apart")}
+    for _ in range(6):
+        for n, plan in (("inside", inside), ("apart", apart)):
+            times[n].append(eng.time_plan(plan, reps=1, flush_l2=False))
+    assert min(times["inside"]) <= min(times["apart"]), times
+    assert eng.device_status() == 0
+
+
 @pytest.mark.parametrize("B,H,KV,T,DH", [
     (1, 2, 1, 3, 64), (2, 2, 2, 17, 12), (1, 4, 2, 31, 32), (3, 6, 2, 64, 20), (1, 2, 1, 65, 36), (2, 8, 8, 130, 64), (2, 8, 4, 256, 32), (40, 8, 2, 100, 48), (1, 3, 3, 449, 16),
     (2, 16, 16, 333, 64)])
