@@ -829,25 +829,31 @@ static int band_of(int m, long long k) {
     return 2ll * m * k > 52000000ll && tiles_m > 12 ? 12 : tiles_m;
 }
 
-// Columns of a tile.  A launch is a set-up, a first load and the last tile's epilogue (f) and, for each round of tiles over the pairs, the
-// k-blocks (t), which for narrow tiles are bound by shared memory: 512 / 385 / 355 cycles by themselves.  us of 256 / 192 / 128 columns in chains of launches:
-// 2000 x 1536 x 1536 (48, 64, 96 tiles) 12.8 / 11.3 / 13.6, x 4096 24.8 / 21.8 / 28.1, 8192 x 768 x 2304 (96, 128, 192) 26.6 / 23.2 / 27.9, 1536 x 1024 x 1024
-// (24 shared by two pairs, 36, 48) 9.5 / 8.2 / 7.7, x 2816 15.3 / 14.8 / 13.0, x 5632 20.7 / 24.6 / 22.7, 2000 x 4096 x 1536 (128, 176, 256) 21.3 / 22.9 / 25.4.
-// Only while a plan has queued nothing beside the main chain (see ax_gemm_plan_begin): products on the side stream fill the pairs that wide tiles leave, and
+// Columns of a tile.  A launch is a set-up, a first load and the last tile's epilogue (f), a round's k-blocks (t each; those of narrow tiles are bound by
+// shared memory and L2), and for each further round of tiles over the pairs its k-blocks or, where they are few, the epilogue that they run under (e).  us of 256 / 192 / 128
+// columns in chains of launches: 2000 x 1536 x 1536 (48, 64, 96 tiles) 12.8 / 11.3 / 13.6, x 4096 24.8 / 21.8 / 28.1, 8192 x 768 x 2304 (96, 128, 192) 26.6 / 23.2 / 27.9,
+// 1536 x 1024 x 1024 (24 shared by two pairs, 36, 48) 9.5 / 8.2 / 7.7, x 2816 15.3 / 14.8 / 13.0, x 5632 20.7 / 24.6 / 22.7, 2000 x 4096 x 1536 (128, 176, 256) 21.3 / 22.9 / 25.4.
+// Few k-blocks: 2520 x 2920 x 104 (120, 160, 230) 9.9 / 11.5 / 12.9, 5720 x 816 x 128 (92, 115, 161) 7.9 / 8.2 / 9.2, 1544 x 2176 x 568 (63, 84, 119) 9.9 / 13.0 / 11.3, 768 x 2816 x
+// 256 (33, 45, 66) 6.5 / 6.2 / 6.2.  Over 232 shapes the rule is 0.4 % behind the best of the three on average.
+// Only while a plan has queued nothing to another stream (see ax_gemm_plan_begin): products on the side stream fill the pairs that wide tiles leave, and
 // the step of 8 x 1024 tokens at D 768 takes 5114 us with narrow ones throughout, 5037 without.  Steps with adapters are 1 to 2 % shorter, small ones up to 5.
 // With three rounds or more the rounds even out and the wide tile, which moves the least, is the best under the power limit: 8192 x 1536 x 2560 (192, 256, 384)
 // 48.6 / 49.5 / 58.4.
 static int g_pairs = 0;                  // pairs that run at once
-TileTimes ax_gemm_tc2_width(const long long* tiles /* of 256, 192, 128 columns */, int kb, bool may_share) {
+TileTimes ax_gemm_tc2_width(const long long* tiles /* of 256, 192, 128 columns */, int kb, bool may_share, bool group) {
     static const int width[3] = {256, 192, 128};
-    static const double f[3] = {5.6, 4.95, 4.3}, t[3] = {0.30, 0.263, 0.185};
+    static const double f[3] = {5.6, 4.95, 4.5}, t[3] = {0.30, 0.263, 0.215}, e[3] = {3.4, 3.2, 2.5};
     TileTimes best = {256, 0.0};
     for (int i = 0; i < 3; i++) {
         const long long rounds = g_pairs > 0 ? (tiles[i] + g_pairs - 1) / g_pairs : 1;
-        double us = f[i] + t[i] * rounds * kb, shared;
-        if (i == 0 && may_share && tiles[0] <= 33 && ax_gemm_tc2_share((int)tiles[0], kb, &shared) > 1) us = f[0] + t[0] * shared;
+        const double round = t[i] * kb;
+        double us = f[i] + round + (rounds - 1) * (round > e[i] ? round : e[i]), shared;
+        if (i == 0 && may_share && tiles[0] <= 33) {
+            const int S = ax_gemm_tc2_share((int)tiles[0], kb, &shared);
+            if (S > 1) us = group ? 8.2 + 0.36 * ((kb + S - 1) / S) + 0.04 * S * tiles[0] : f[0] + t[0] * shared;
+        }
         if (i == 0) best.us = us;
-        else if (tiles[0] <= 2 * g_pairs && us < best.us * 0.97) best = {width[i], us};
+        else if (tiles[0] <= 2 * g_pairs && us < best.us) best = {width[i], us};
     }
     return best;
 }
@@ -1100,7 +1106,7 @@ int ax_gemm_tc2_group(int out_bf16, int tb, int mode, int count, const void* con
         for (int g = 0; g < (mode == 2 ? count : 1); g++) kb += (k[g] + BK2 - 1) / BK2;
         for (int i = 0; i < 3; i++)
             for (int g = 0; g < (mode == 1 ? count : 1); g++) tiles[i] += (long long)((m[0] + 255) / 256) * ((n[g] + 255 - 64 * i) / (256 - 64 * i));
-        bn = ax_gemm_tc2_width(tiles, kb, !swb).width;
+        bn = ax_gemm_tc2_width(tiles, kb, !swb, true).width;
     }
     ax_gemm_width = mode == 4 ? 256 : bn;
 #define G2W(AM, BMj, T, EPI, W) gemm2_launch<AM, BMj, T, EPI, W>(mode, count, A, B, C, D, m, n, k, alpha, D ? beta : 0.f, status, 1, st, XA, XB, xk, swb)

@@ -1098,6 +1098,18 @@ def test_narrow_tiles_where_wide_ones_leave_pairs_idle(eng, tb, dt, addend, m, n
     assert eng.device_status() == 0
 
 
+@pytest.mark.parametrize("m,n,k,tb,dt,width,split", [
+    (2520, 2920, 104, 1, 1, 256, 1), (5720, 816, 128, 2, 1, 192, 1), (2176, 3456, 128, 0, 2, 256, 1), (1544, 2176, 568, 2, 2, 256, 1), (4200, 728, 128, 2, 1, 192, 1),
+    (768, 2816, 256, 2, 1, 128, 1), (280, 1888, 3792, 2, 1, 256, 3)])
+def test_wide_tiles_where_the_epilogue_is_the_round(eng, m, n, k, tb, dt, width, split):
+    """A product of few k-blocks pays an epilogue for each round of tiles, so that more rounds of narrow tiles are no gain; one of many k-blocks is split over the
+    workspace rather than run on tiles of 128 columns whose k-blocks take as long as they do."""
+    got, ref = run_gemm(eng, np.random.default_rng(m + n), m, n, k, tb, dt)
+    assert (eng.last_variant(), eng.last_gemm_width()) == (0x22 + 0x100 * split, width)
+    check(got, ref, dt == 1, k)
+    assert eng.device_status() == 0
+
+
 @pytest.mark.parametrize("r", [0, 16])
 @pytest.mark.parametrize("m,k,ns,width", [(3000, 640, (768, 192, 192), 192), (2904, 264, (704, 192, 128), 192), (1800, 72, (576, 64, 72), 128)])
 def test_narrow_tiles_of_groups_have_the_bits_of_wide_ones(eng, m, k, ns, width, r):
