@@ -2,6 +2,8 @@
 // token-mean cross-entropy with ignored targets (target < 0).
 #include <cuda_fp16.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "kernels.h"
 #include "attn_common.cuh"
@@ -136,12 +138,12 @@ __global__ void k_embed_link(const int* __restrict__ ids, unsigned* __restrict__
 // Bound by the chain of loads that depend on one another: the id, then its first and last row, then everything that a token with one row needs, its
 // gradient row and the table's, at once; only tokens with more walk a list.  (With the list walked first and two slices of 128 threads for a row:
 // N 8192 D 1536 V 32000 92 us, N 8192 D 768 V 32000 44 us; 56 and 15 now; the memory that it has to move takes 19 and 10.)
-template <typename T>
+template <typename T, int PER>
 __global__ void __launch_bounds__(EB_THREADS)
 k_embed_bwd_list(const T* __restrict__ g, const int* __restrict__ ids, const unsigned* __restrict__ first, const int* __restrict__ last,
                  const int* __restrict__ link, float* __restrict__ dT, int N, int D, int rows) {
     constexpr int VN = Vec<T>::N;
-    __shared__ int s_list[EB_THREADS], s_wcnt[EB_THREADS / 32];
+    __shared__ int s_list[EB_THREADS], s_wcnt[2][EB_THREADS / 32];
     const int r = blockIdx.x, tok = ids[r];
     if (tok < 0 || tok >= rows) return;
     const unsigned head = first[tok];
@@ -191,19 +193,49 @@ k_embed_bwd_list(const T* __restrict__ g, const int* __restrict__ ids, const uns
             __syncthreads();
             add_rows(s_list, cnt);
         } else {
-            for (int base = r; base < N; base += blockDim.x) {
-                const int idx = base + (int)threadIdx.x;
-                const bool hit = idx < N && ids[idx] == tok;
-                const unsigned bal = __ballot_sync(0xffffffffu, hit);
-                const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-                if (!lane) s_wcnt[wp] = __popc(bal);
-                __syncthreads();
+            const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+            if (PER == 1) {
+                for (int base = r; base < N; base += blockDim.x) {
+                    const int idx = base + (int)threadIdx.x;
+                    const bool hit = idx < N && ids[idx] == tok;
+                    const unsigned bal = __ballot_sync(0xffffffffu, hit);
+                    if (!lane) s_wcnt[0][wp] = __popc(bal);
+                    __syncthreads();
+                    int off = 0, n = 0;
+                    for (int q = 0; q < warps; q++) { if (q < wp) off += s_wcnt[0][q]; n += s_wcnt[0][q]; }
+                    if (hit) s_list[off + __popc(bal & ((1u << lane) - 1))] = idx;
+                    __syncthreads();
+                    add_rows(s_list, n);
+                    __syncthreads();
+                }
+            }
+            // Blocks of few warps, those of narrow rows: turns of some 256 ids all the same.  With an id to a thread the scan of one warp took three times as long as that
+            // of the four warps that such rows had before (N 8000 D 128 V 1000 fp32, tokens of up to 31 rows: 30 us with four warps, 88 with one, 35 so).  Each warp has ids
+            // of its own behind one another and does nothing where it finds none, which is most of the time.
+            for (int base = r, turn = 0; PER > 1 && base < N; base += blockDim.x * PER, turn ^= 1) {
+                const int mine = base + wp * 32 * PER + lane;
+                unsigned hits = 0;
+#pragma unroll
+                for (int q = 0; q < PER; q++)
+                    if (mine + q * 32 < N && ids[mine + q * 32] == tok) hits |= 1u << q;
+                int cnt = 0;
+                if (__any_sync(0xffffffffu, hits))
+#pragma unroll
+                    for (int q = 0; q < PER; q++) cnt += __popc(__ballot_sync(0xffffffffu, hits >> q & 1));
+                if (!lane) s_wcnt[turn][wp] = cnt;
+                __syncthreads();                           // (also: everyone has left the list of the turn before)
                 int off = 0, n = 0;
-                for (int q = 0; q < (int)blockDim.x / 32; q++) { if (q < wp) off += s_wcnt[q]; n += s_wcnt[q]; }
-                if (hit) s_list[off + __popc(bal & ((1u << lane) - 1))] = idx;
+                for (int w = 0; w < warps; w++) { if (w == wp) off = n; n += s_wcnt[turn][w]; }
+                if (!n) continue;
+                if (cnt)
+#pragma unroll
+                    for (int q = 0; q < PER; q++) {
+                        const unsigned bal = __ballot_sync(0xffffffffu, hits >> q & 1);
+                        if (hits >> q & 1) s_list[off + __popc(bal & ((1u << lane) - 1))] = mine + q * 32;
+                        off += __popc(bal);
+                    }
                 __syncthreads();
                 add_rows(s_list, n);
-                __syncthreads();
             }
         }
     }
@@ -227,8 +259,15 @@ int ax_embed_bwd_det(int g_dt, const void* g, const int* ids, float* dT, int N, 
         k_embed_link<<<(N + 255) / 256, 256, 0, st>>>(ids, first, last, link, N, rows, status);
         const int warps = (D / vn + 31) / 32, slices = (warps * 32 + EB_THREADS - 1) / EB_THREADS, threads = (warps + slices - 1) / slices * 32;
         const dim3 grid(N, slices);
-        if (g_dt >= 1) k_embed_bwd_list<bf16><<<grid, threads, 0, st>>>((const bf16*)g, ids, first, last, link, dT, N, D, rows);
-        else k_embed_bwd_list<float><<<grid, threads, 0, st>>>((const float*)g, ids, first, last, link, dT, N, D, rows);
+        auto launch = [&](auto per) {                      // ids of a thread in a turn of the scan: some 256 a block
+            constexpr int PER = decltype(per)::value;
+            if (g_dt >= 1) k_embed_bwd_list<bf16, PER><<<grid, threads, 0, st>>>((const bf16*)g, ids, first, last, link, dT, N, D, rows);
+            else k_embed_bwd_list<float, PER><<<grid, threads, 0, st>>>((const float*)g, ids, first, last, link, dT, N, D, rows);
+        };
+        if (threads <= 32) launch(std::integral_constant<int, 8>());
+        else if (threads <= 64) launch(std::integral_constant<int, 4>());
+        else if (threads < 128) launch(std::integral_constant<int, 2>());
+        else launch(std::integral_constant<int, 1>());
         ax_variant = 0x71;
         return 0;
     }

@@ -449,6 +449,21 @@ def test_embedding_scatter_by_occurrence_lists(eng, dt, N, V, D, kind):
     assert eng.device_status() == 0
 
 
+def test_embedding_scatter_of_narrow_rows_takes_no_longer_than_of_wide_ones(eng):
+    """Tokens of more rows than a list holds are gathered by a scan of the ids, whose length must not depend on the few threads that a narrow row needs."""
+    rng = np.random.default_rng(5)
+    N, V = 8000, 1000
+    ids = rng.integers(0, V, N)
+    assert np.bincount(ids).max() > 16
+    iid, times = eng.alloc(N), {}
+    eng.upload_raw(iid, ids.astype(np.int32))
+    for D in (128, 512):
+        ig, idT = put(eng, rnd(rng, (N, D), 0), 0), eng.alloc(V * D)
+        plan = [op(E.EMBED_BWD_DET, a=ig, b=iid, c=idT, m=N, n=D, dt=0)] * 20
+        times[D] = min(eng.time_plan(plan, reps=1, flush_l2=False) for _ in range(5))
+    assert times[128] <= times[512], times
+
+
 @pytest.mark.parametrize("n", [1, 3, 4, 1023, 70001])
 @pytest.mark.parametrize("into", ["a", "b", "other"])
 def test_scale_then_add_as_one_pass(eng, n, into):
