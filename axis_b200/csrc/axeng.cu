@@ -667,6 +667,9 @@ API int eng_attn_route(int backward, int B, int H, int KV, int T, int head_dim) 
     if (B < 1 || H < 1 || KV < 1 || T < 1 || head_dim < 1) return 0;
     return ax_attn_tcs_route(backward, shape_bthd(B, H, KV, T, head_dim, 1.f));
 }
+API int eng_lora_proj_cut(int count, int one_x, int N, int F, int R) {
+    return count < 1 || count > 3 || N < 1 || F < 1 || R < 1 ? 0 : ax_lora_proj_cut(count, one_x, N, F, R);
+}
 API int eng_attn_tile_parts(int B, int H, int KV, int T, int head_dim) {
     if (B < 1 || H < 1 || KV < 1 || T < 1) return 0;
     return ax_attn_tc_parts(shape_bthd(B, H, KV, T, head_dim, 1.f));

@@ -162,6 +162,7 @@ float* ax_splitk_ws(size_t* bytes);
 // out[g] [N, R] bf16 = alpha * X[g] [N, F[g]] W[g] with W [F, R] (tb 0) or [R, F] (tb 1): the skinny products of an adapter.
 int ax_lora_proj(int count, int tb, const void* const* X, const void* const* W, void* const* out, const int* F, int N, int R,
                  float alpha, cudaStream_t st);
+int ax_lora_proj_cut(int count, int one_x, int N, int F, int R);      // see eng_lora_proj_cut
 int ax_lora_grad(int count, const void* const* X, const void* const* S, float* const* out, const int* F, const int* layout,
                  int N, int R, float alpha, float* ws, size_t ws_bytes, cudaStream_t st);
 

@@ -379,27 +379,47 @@ __global__ void __launch_bounds__(256) k_lora_proj(const __grid_constant__ LoraP
     cluster_sync();   // peers have read
 }
 
-template <int NT, int TB, int M, int TOK> static int lora_proj_launch(const LoraProjArgs& a, cudaStream_t st) {
+// How a launch of `count` products of N tokens, F columns (the narrowest) and rank R is cut: products as members of one CTA, tokens of a CTA, CTAs that share a CTA's walk.
+struct LoraProjCut { int members, tokens, S; };
+static LoraProjCut lora_proj_cut(int count, bool one_x, int N, int F, int R) {
+    // Members of one X pay where a CTA per product would go beyond a resident wave (three products of rank 32, 8192 x 1536: 18.6 us as members, 24.3 each),
+    // or where token blocks alone occupy the SMs, the walk is long and the member loop short (rank 16, three of 2048 x 4096 10.5 and 15.0 us, two of 3000 x 2048 7.9 and 9.1;
+    // rank 32, three of 3000 x 1536 11.3 and 9.4; two of 256 x 1024 3.8 and 3.4; rank 16, three of 4999 x 776 8.5 and 6.7, of 2006 x 864 7.9 and 5.6).
+    const int blocks = (N + 63) / 64;
+    LoraProjCut c = {one_x && ((blocks >= 32 && R * count <= 64 && F >= 1536) || blocks * count > 2 * AX_SMS) ? count : 1, 64, 1};
+    const int rows = c.members > 1 ? 1 : count;
+    // Depth split: a CTA that walks all of F alone is a chain of round trips, and few token blocks leave SMs idle.  Never beyond one resident wave, two CTAs an SM, which is 148
+    // clusters of two, 72 of four or 32 of eight: x A of 8192 x 1536 in blocks of 32 tokens 11.0 us on 256 CTAs, 13.9 us on 512; 74 clusters of four, 4707 x 6376 rank 32,
+    // 35.8 us, 24.9 in two; 34 of eight, 538 x 2320 rank 8, 6.8, 4.4 in four.  The barriers and the sum take 1 us, what some 500 columns do, one CTA / two: rank 8, 6510 x 232
+    // 2.1 / 3.4, 9458 x 160 2.4 / 3.8; rank 16, 5241 x 320 3.1 / 4.4, 3196 x 712 4.1 / 4.6; 1936 columns 10.7 / 8.9.
+    auto fits = [](long long n, int S) { return n <= (S == 2 ? AX_SMS : S == 4 ? 72 : 32); };
+    while (c.S < 8 && fits((long long)blocks * rows, 2 * c.S) && F >= 1024 && F * c.members >= 1024 * c.S) c.S *= 2;
+    // Where even the split leaves SMs without a CTA the walk's length counts, not W's traffic: 32 tokens and pieces of 256 columns.
+    // Rank 16, one product: 70 x 4096 4.4 us in blocks of 64, 3.5 of 32; 1024 x 4096 6.3 and 5.2, 4160 x 416 3.8 and 3.1; above, 2048 x 4096 7.3 and 8.1.
+    if (c.members == 1 && blocks * rows * c.S <= AX_SMS) {
+        const int small = (N + 31) / 32;
+        c.tokens = 32;
+        c.S = 1;
+        while (c.S < 8 && fits((long long)small * rows, 2 * c.S) && F >= (c.S == 1 ? 768 : 512 * c.S)) c.S *= 2;
+    }
+    return c;
+}
+int ax_lora_proj_cut(int count, int one_x, int N, int F, int R) {
+    const LoraProjCut c = lora_proj_cut(count, one_x != 0, N, F, R);
+    return c.members << 16 | c.tokens << 8 | c.S;
+}
+
+template <int NT, int TB, int M, int TOK> static int lora_proj_launch(const LoraProjArgs& a, int S, cudaStream_t st) {
     using L = LoraProj<NT, TB, M, TOK>;
     static const cudaError_t attr = cudaFuncSetAttribute(k_lora_proj<NT, TB, M, TOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM);
     if (attr != cudaSuccess) return 3;
-    const int blocks = (a.N + TOK - 1) / TOK, rows = M > 1 ? 1 : a.count;
-    int least = 1 << 30;
-    for (int g = 0; g < a.count; g++) least = a.p[g].F < least ? a.p[g].F : least;
-    const int pieces = (least + L::COLS - 1) / L::COLS;
-    // Depth split: a CTA that walks all of F alone is a chain of round trips, and few token blocks leave SMs idle.  Never beyond
-    // one resident wave (two CTAs an SM): x A of 8192 x 1536 in blocks of 32 tokens 11.0 us on 256 CTAs, 13.9 us on 512.
     LoraProjArgs b = a;
-    b.S = 1;
-    while (b.S < 8 && blocks * rows * 2 * b.S <= 2 * AX_SMS && pieces >= 2 * b.S) b.S *= 2;
-    // Where even the split leaves SMs without a CTA the walk's length counts, not W's traffic: 32 tokens and wide pieces.
-    // Rank 16, one product: 70 x 4096 4.4 us in blocks of 64, 3.5 of 32; 1024 x 4096 6.3 and 5.2; above, 2048 x 4096 7.3 and 8.1.
-    if (M == 1 && TOK == 64 && blocks * rows * b.S <= AX_SMS) return lora_proj_launch<NT, TB, 1, 32>(a, st);
+    b.S = S;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(blocks * b.S, rows); cfg.blockDim = dim3(256); cfg.dynamicSmemBytes = L::SMEM; cfg.stream = st;
+    cfg.gridDim = dim3((a.N + TOK - 1) / TOK * S, M > 1 ? 1 : a.count); cfg.blockDim = dim3(256); cfg.dynamicSmemBytes = L::SMEM; cfg.stream = st;
     cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = b.S; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    at[0].val.clusterDim.x = S; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
     at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at; cfg.numAttrs = ax_gemm_pdl() ? 2 : 1;
@@ -416,14 +436,12 @@ int ax_lora_proj(int count, int tb, const void* const* X, const void* const* W, 
         if (F[g] < 8 || F[g] % 8 || !aligned16(X[g]) || !aligned16(W[g]) || !out[g] || ((uintptr_t)out[g] & 3)) return -1;
         a.p[g].X = (const bf16*)X[g]; a.p[g].W = (const bf16*)W[g]; a.p[g].out = (bf16*)out[g]; a.p[g].F = F[g];
     }
-    // Members of one X pay where a CTA per product would go beyond a resident wave (three products of rank 32, 8192 x 1536:
-    // 18.6 us as members, 24.3 each), or where token blocks alone occupy the SMs with a short member loop (rank 16, three of
-    // 2048 x 4096 10.5 and 15.0 us, two of 3000 x 2048 7.9 and 9.1; rank 32, three of 3000 x 1536 11.3 and 9.4; two of 256 x 1024 3.8 and 3.4).
     bool one_x = true;
-    for (int g = 1; g < count; g++) one_x = one_x && X[g] == X[0] && F[g] == F[0];
-    const int blocks = (N + 63) / 64;                      // token blocks
-    const int members = one_x && ((blocks >= 32 && R * count <= 64) || blocks * count > 2 * AX_SMS) ? count : 1;
-#define LPM(NT_, TB_) (members == 3 ? lora_proj_launch<NT_, TB_, 3, 64>(a, st) : (members == 2 ? lora_proj_launch<NT_, TB_, 2, 64>(a, st) : lora_proj_launch<NT_, TB_, 1, 64>(a, st)))
+    int least = F[0];
+    for (int g = 1; g < count; g++) { one_x = one_x && X[g] == X[0] && F[g] == F[0]; least = F[g] < least ? F[g] : least; }
+    const LoraProjCut c = lora_proj_cut(count, one_x, N, least, R);
+#define LPM(NT_, TB_) (c.members == 3 ? lora_proj_launch<NT_, TB_, 3, 64>(a, c.S, st) : c.members == 2 ? lora_proj_launch<NT_, TB_, 2, 64>(a, c.S, st) \
+                       : c.tokens == 64 ? lora_proj_launch<NT_, TB_, 1, 64>(a, c.S, st) : lora_proj_launch<NT_, TB_, 1, 32>(a, c.S, st))
 #define LP(NT_) (tb ? LPM(NT_, 1) : LPM(NT_, 0))
     return R == 8 ? LP(1) : (R == 16 ? LP(2) : LP(4));
 #undef LP

@@ -186,6 +186,9 @@ long long eng_attn_smem(int which, int head_dim);
 int eng_attn_share(int which, int B, int H, int KV, int T, int head_dim);
 /* CTAs that share a key tile of the whole-tile tcgen05 attention backward (head_dim 64 or 128, T a multiple of 128): 1, 2 or 4; 0 = not such a shape. */
 int eng_attn_tile_parts(int B, int H, int KV, int T, int head_dim);
+/* How a launch of the adapters' skinny products is cut (`count` of N tokens and rank R, the narrowest with F columns, one_x: all of one input): products in a CTA * 65536 +
+ * tokens of a CTA * 256 + CTAs that share its columns; 0 = not a shape.  Host arithmetic that needs no GPU. */
+int eng_lora_proj_cut(int count, int one_x, int N, int F, int R);
 
 /* Fused RMSNorm backward that allocates nothing (no counterpart in the
  * reference).  dx = (res ? res : 0) + d(rmsnorm)/dx, dw = sum over rows of

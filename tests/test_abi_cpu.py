@@ -128,6 +128,19 @@ def test_ctas_to_a_key_tile_of_whole_tiles(lib, B, H, KV, T, parts64, parts128):
     assert lib.eng_attn_tile_parts(B, H, KV, T + 8, 64) == lib.eng_attn_tile_parts(B, H, KV, T, 96) == 0
 
 
+@pytest.mark.parametrize("count,one_x,N,F,R,members,tokens,ctas", [
+    # narrow inputs: a barrier and a sum across CTAs take as long as 500 columns
+    (1, 1, 6510, 232, 8, 1, 32, 1), (1, 1, 9480, 160, 8, 1, 64, 1), (1, 0, 5241, 320, 16, 1, 32, 1), (3, 1, 615, 456, 8, 1, 32, 1), (2, 0, 4088, 288, 32, 1, 32, 1),
+    (1, 0, 3196, 712, 16, 1, 32, 1), (1, 1, 45, 488, 8, 1, 32, 1), (3, 1, 302, 552, 16, 1, 32, 1),
+    # members of a CTA: a long walk, or more products than a wave
+    (3, 1, 2048, 4096, 16, 3, 64, 8), (2, 1, 3000, 2048, 16, 2, 64, 4), (3, 1, 4999, 776, 16, 1, 64, 1), (3, 1, 8572, 376, 8, 3, 64, 1), (3, 0, 8572, 376, 8, 1, 64, 1), (3, 1, 8192, 1536, 32, 3, 64, 2),
+    # few blocks and long walks: 32 tokens, the columns over a cluster
+    (1, 1, 70, 4096, 16, 1, 32, 8), (1, 1, 1024, 4096, 16, 1, 32, 8), (1, 1, 2048, 4096, 16, 1, 64, 8), (2, 1, 192, 1472, 32, 1, 32, 4), (1, 0, 4741, 1936, 16, 1, 64, 2), (1, 1, 8192, 4096, 16, 1, 64, 2)])
+def test_cut_of_the_adapters_products(lib, count, one_x, N, F, R, members, tokens, ctas):
+    cut = lib.eng_lora_proj_cut(count, one_x, N, F, R)
+    assert (cut >> 16, cut >> 8 & 255, cut & 255) == (members, tokens, ctas)
+
+
 def test_attention_route_of_invalid_shapes(lib):
     for a in ((0, 8, 4, 500, 64), (1, 0, 4, 500, 64), (1, 8, 0, 500, 64), (1, 8, 3, 500, 64), (1, 8, 4, 0, 64), (1, 8, 4, 500, 0)):
         assert lib.eng_attn_route(0, *a) == lib.eng_attn_route(1, *a) == 0
