@@ -134,33 +134,33 @@ struct F32Group {
     const float* D;             // addend (one problem)
     const float* G; const float* U;
 };
-template <int BM, int BN, int BK, int KG, int TM, int TN, int ST, bool A_MN, bool B_KM, bool VEC, int EPI>
+template <int BM, int BN, int BK, int KG, int TM, int TN, int ST, bool A_MN, bool B_KM, bool VEC, int EPI, bool ONE>
 __global__ void __launch_bounds__(KG * (BM / TM) * (BN / TN))
 k_gemm_f32(const __grid_constant__ F32Group a, int m, long long sa, long long sb, long long sc, int ksplit, float alpha, float beta) {
     using L = F32Tile<BM, BN, BK, KG, TM, TN, ST, A_MN, B_KM>;
     constexpr int TH = L::THREADS, TX = BN / TN, TY = BM / TM, GT_ = TX * TY, KS = BK / KG, W = EPI == F32_SWIGLU ? BN / 2 : BN;
+    const int nprob = ONE ? 1 : a.nprob, nseg = ONE ? 1 : a.nseg;
     extern __shared__ __align__(16) float sm[];
-    pdl_enter();
     const int split = blockIdx.x % ksplit, i0 = blockIdx.y * BM;
     int tn = blockIdx.x / ksplit, g = 0;
-    for (; g + 1 < a.nprob; g++) {
+    for (; g + 1 < nprob; g++) {
         const int t = (a.n[g] + W - 1) / W;
         if (tn < t) break;
         tn -= t;
     }
     const int n = a.n[g], j0 = tn * W;
-    const F32Seg* seg = a.seg + g * a.nseg;
+    const F32Seg* seg = a.seg + g * nseg;
     const long long oa = blockIdx.z * sa, ob = blockIdx.z * sb, oc = blockIdx.z * sc;
     float* C = a.C[g] + oc;
     const float* D = a.D ? a.D + oc : nullptr;
     int steps_all = 0;
-    for (int q = 0; q < a.nseg; q++) steps_all += (seg[q].k + BK - 1) / BK;
+    for (int q = 0; q < nseg; q++) steps_all += (seg[q].k + BK - 1) / BK;
     const int per = (steps_all + ksplit - 1) / ksplit;
     const int s0 = split * per, s1 = min(steps_all, s0 + per), steps = max(s1 - s0, 0);
     const int grp = threadIdx.x / GT_, tid = threadIdx.x % GT_, ty = tid / TX, tx = tid % TX;
     int ls = 0, lk = s0;                                  // next step to load: segment and step inside it
     auto load = [&](int slot) {
-        while (ls + 1 < a.nseg && lk >= (seg[ls].k + BK - 1) / BK) lk -= (seg[ls++].k + BK - 1) / BK;
+        while (ls + 1 < nseg && lk >= (seg[ls].k + BK - 1) / BK) lk -= (seg[ls++].k + BK - 1) / BK;
         float* as = sm + slot * (L::A_EL + L::B_EL);
         float* bs = as + L::A_EL;
         const int k = seg[ls].k, k0 = lk++ * BK;
@@ -179,6 +179,7 @@ k_gemm_f32(const __grid_constant__ F32Group a, int m, long long sa, long long sb
     for (int p = 0; p < TM; p++)
 #pragma unroll
         for (int q = 0; q < TN; q++) acc[p][q] = 0.f;
+    pdl_enter();                                          // which tile this is comes from the arguments alone
 #pragma unroll
     for (int st = 0; st < ST - 1; st++) {
         if (st < steps) load(st);
@@ -327,11 +328,11 @@ k_gemm_f32(const __grid_constant__ F32Group a, int m, long long sa, long long sb
         cluster_sync();
 }
 
-template <int BM, int BN, int BK, int KG, int TM, int TN, int ST, bool A_MN, bool B_KM, bool VEC, int EPI>
+template <int BM, int BN, int BK, int KG, int TM, int TN, int ST, bool A_MN, bool B_KM, bool VEC, int EPI, bool ONE>
 static int f32_launch(const F32Group& a, int m, int batch, long long sa, long long sb, long long sc, int ksplit, float alpha, float beta, cudaStream_t st) {
     using L = F32Tile<BM, BN, BK, KG, TM, TN, ST, A_MN, B_KM>;
     constexpr int W = EPI == F32_SWIGLU ? BN / 2 : BN;
-    auto kern = k_gemm_f32<BM, BN, BK, KG, TM, TN, ST, A_MN, B_KM, VEC, EPI>;
+    auto kern = k_gemm_f32<BM, BN, BK, KG, TM, TN, ST, A_MN, B_KM, VEC, EPI, ONE>;
     static const cudaError_t attr = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM);
     if (attr != cudaSuccess) return 125;
     int cols = 0;
@@ -355,7 +356,7 @@ static int f32_launch(const F32Group& a, int m, int batch, long long sa, long lo
     cfg.attrs = at; cfg.numAttrs = na;
     return cudaLaunchKernelEx(&cfg, kern, a, m, sa, sb, sc, ksplit, alpha, beta) == cudaSuccess ? 0 : 126;
 }
-template <bool A_MN, bool B_KM, int EPI = F32_PLAIN>
+template <bool A_MN, bool B_KM, int EPI = F32_PLAIN, bool ONE = false>
 static int f32_gemm(const F32Group& a, int m, int batch, long long sa, long long sb, long long sc, float alpha, float beta, cudaStream_t st) {
     // 16-byte copies need row pitches and starts on 16-byte boundaries
     bool vec = sa % 4 == 0 && sb % 4 == 0 && sc % 4 == 0 && (!A_MN || m % 4 == 0) && aligned16(a.D) && aligned16(a.G) && aligned16(a.U);
@@ -372,8 +373,8 @@ static int f32_gemm(const F32Group& a, int m, int batch, long long sa, long long
         return (long long)((m + bm - 1) / bm) * cols * batch;
     };
 #define F32L(BM, BN, BK, KG, TM, TN, ST, KSP)                                                                                  \
-    (vec ? f32_launch<BM, BN, BK, KG, TM, TN, ST, A_MN, B_KM, true, EPI>(a, m, batch, sa, sb, sc, KSP, alpha, beta, st)        \
-         : f32_launch<BM, BN, BK, KG, TM, TN, ST, A_MN, B_KM, false, EPI>(a, m, batch, sa, sb, sc, KSP, alpha, beta, st))
+    (vec ? f32_launch<BM, BN, BK, KG, TM, TN, ST, A_MN, B_KM, true, EPI, ONE>(a, m, batch, sa, sb, sc, KSP, alpha, beta, st)        \
+         : f32_launch<BM, BN, BK, KG, TM, TN, ST, A_MN, B_KM, false, EPI, ONE>(a, m, batch, sa, sb, sc, KSP, alpha, beta, st))
     // A 128 x 128 tile has the most FMAs per shared-memory read, but fewer than 148 of them leave SMs without work.
     if (tiles(128, 128) >= AX_SMS) return F32L(128, 128, 16, 1, 8, 8, 3, 1);
     int steps = 0;
@@ -441,9 +442,9 @@ int ax_gemm_simt(int in_bf16, int out_bf16, int tb, const void* A, const void* B
         F32Group a = {};
         a.seg[0] = {(const float*)A, (const float*)B, nullptr, k};
         a.nprob = a.nseg = 1; a.n[0] = n; a.C[0] = (float*)C; a.D = beta != 0.f ? (const float*)D : nullptr;
-        if (tb == 0) return f32_gemm<false, false>(a, m, batch, sa, sb, sc, alpha, beta, st);
-        if (tb == 1) return f32_gemm<false, true>(a, m, batch, sa, sb, sc, alpha, beta, st);
-        return f32_gemm<true, false>(a, m, batch, sa, sb, sc, alpha, beta, st);
+        if (tb == 0) return f32_gemm<false, false, F32_PLAIN, true>(a, m, batch, sa, sb, sc, alpha, beta, st);
+        if (tb == 1) return f32_gemm<false, true, F32_PLAIN, true>(a, m, batch, sa, sb, sc, alpha, beta, st);
+        return f32_gemm<true, false, F32_PLAIN, true>(a, m, batch, sa, sb, sc, alpha, beta, st);
     }
     dim3 grid((n + GT - 1) / GT, (m + GT - 1) / GT, batch);
     if (grid.y > 65535 || grid.z > 65535) return 123;
