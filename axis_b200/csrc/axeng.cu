@@ -137,6 +137,10 @@ API long long eng_bytes_allocated(void) { return G.bytes; }
 API int eng_last_variant(void) { return ax_variant; }
 API int eng_last_gemm_parts(void) { return ax_gemm_parts; }
 API int eng_last_gemm_width(void) { return ax_gemm_width; }
+API int eng_last_f32_cut(void) { return ax_f32_cut; }
+API int eng_gemm_f32_cut(int tb, int m, int n, int k, int batch, int aligned) {
+    return tb < 0 || tb > 2 || m < 1 || n < 1 || k < 1 || batch < 1 ? 0 : ax_gemm_f32_cut(tb, m, n, k, batch, aligned);
+}
 API long long eng_attn_smem(int which, int head_dim) { return which < 0 || which > 2 || head_dim < 1 || head_dim > 256 ? -1 : ax_attn_simt_smem(which, head_dim); }
 API int eng_sync(void) {
     int rc = (int)cudaStreamSynchronize(G.stream);

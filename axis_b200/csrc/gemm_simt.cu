@@ -85,7 +85,7 @@ k_gemm_simt(const TI* __restrict__ A, const TI* __restrict__ B, TO* C, const TO*
 //   * small tiles (64 x 32, 32 x 32) cut every step among four groups of 64 threads;
 //   * where the tiles still leave SMs idle, a cluster of 2, 4 or 8 CTAs cuts the depth once more and adds its partial
 //     tiles through distributed shared memory.
-// 512 x 256 x 256, one cold launch: 46 us with 64 x 64 tiles, 16-deep steps and no prefetch, 7 us now; 512 x 512 x 256: 11 us.
+// 512 x 256 x 256 took 46 us with 64 x 64 tiles, 16-deep steps and no prefetch; what each tile takes now stands at f32_cut.
 // All partial sums meet in a fixed order: run-to-run identical.  Operands keep their layout in shared memory: a
 // K-major operand is read as 16-byte pieces along K (row pitch BK + 4: the rows of a warp fall in different banks), an
 // M/N-major one as 16-byte pieces along M/N.
@@ -356,6 +356,45 @@ static int f32_launch(const F32Group& a, int m, int batch, long long sa, long lo
     cfg.attrs = at; cfg.numAttrs = na;
     return cudaLaunchKernelEx(&cfg, kern, a, m, sa, sb, sc, ksplit, alpha, beta) == cudaSuccess ? 0 : 126;
 }
+// How a launch is cut: tile, sums of a thread (rows), CTAs that share a tile's depth.  By the tiles that it would have, the 64-deep steps of its sums and whether rows are whole
+// 16-byte pieces.
+struct F32Cut { int rows, cols, sums, ctas; };
+static F32Cut f32_cut(int tb, bool plain, long long t128, long long t64, long long t64x32, long long t32, int steps, long long depth, bool vec) {
+    // A 128 x 128 tile has the most FMAs per shared-memory read, but fewer than 148 of them leave SMs without work, and so does a last round that is mostly empty (one CTA
+    // to an SM; us there / with 64 x 64 tiles: 171 tiles, 1072 x 2360 x 944 238 / 160, 189 tiles, 2688 x 1152 x 376 85 / 71; 210 tiles, 1760 x 1848 x 112 28.2 / 28.7).
+    if (t128 >= AX_SMS && 10 * t128 >= 7 * AX_SMS * ((t128 + AX_SMS - 1) / AX_SMS)) return {128, 128, 8, 1};
+    // Shallow products of many tiles are set-up, one load and the stores: 64 x 64 tiles of 4 x 4 sums with 32-deep steps, which leave an SM room for more CTAs.  us there / with 64 x 64
+    // tiles of 8 x 8 sums or 32 x 32: 2232 x 368 x 24 4.8 / 6.9, 680 x 2792 x 32 7.9 / 10.0, 1184 x 960 x 24 5.8 / 9.2, 1968 x 912 x 16 8.2 / 10.7; A B^T 1992 x 1072 x 136 25.8 / 31.5,
+    // 1552 x 1176 x 104 21.2 / 25.5; but 1008 x 656 x 40 7.2 / 6.3.
+    if (plain && t64 >= AX_SMS && (depth <= 32 || (tb == 1 && steps <= 3 && t64 >= 2 * AX_SMS))) return {64, 64, 4, 1};
+    if (t64 >= 2 * AX_SMS) return {64, 64, 8, 1};
+    // Below, a launch is the latency of its steps: 64 x 32 tiles (8 x 4 sums to a thread, 43 % of the FMA pipe with two CTAs on an SM, which is what
+    // fits) with the depth cut over a cluster as far as two CTAs for each SM.  Where that leaves a third of the SMs idle or most with one CTA and some with two,
+    // or takes a second round, 32 x 32 tiles spread better; a product of two steps is over before a larger tile pays.  us, 64 x 32 with 1 / 2 / 4 CTAs to a tile |
+    // 32 x 32 alike: 512 x 256 x 256 8.6 / 7.9 / 6.2 | 8.8 / 7.6 / 10.1, 512 x 512 x 256 11.0 / 8.4 / 11.9 | 10.0 / 12.0 / 14.9, 512 x 256 x 688 21.1 / 16.4 / 10.8 | 20.2 / 14.8 /
+    // 15.3, 512 x 1024 x 256 12.2 / 17.1 / 24.3 | 14.4 / 19.2 / 26.5, 512 x 688 x 256 12.2 / 16.6 / 18.2 | 10.8 / 12.9 / 20.3, 256 x 256 x 128 4.6 / 5.0 / 5.8 | 3.6 / 4.9 / 5.3,
+    // 300 x 128 x 344 10.0 / 7.4 / 7.6 | 6.9 / 6.6 / 7.3; 1024 x 1536 x 512 58 | 60 and with 64 x 64 tiles of 8 x 8 sums 50.
+    // Not where 64-row tiles are much larger than their rows (32 x 1656 x 144 5.8 / 7.1 | 4.4, 16 x 2208 x 320 7.9 / 9.2 / 7.9 | 5.8 / 6.0), where the steps do not go evenly into the
+    // CTAs (704 x 192 x 176, 2 + 1 steps, 7.5 | 5.1; 856 x 142 x 348, 2 + 2 + 2 + 0, 11.7 | 14.0 / 10.6), nor for shared tiles of A B by 4-byte copies (215 x 569 x 2021 - / - / 47.9 | - / 37.3).
+    int ks = 1, ks32 = 1;
+    while (ks < 8 && t64x32 * ks * 2 <= 2 * AX_SMS && steps >= 2 * ks) ks *= 2;
+    while (ks32 < 8 && t32 * ks32 * 2 <= AX_SMS * 5 / 2 && steps >= 4 * ks32) ks32 *= 2;
+    const long long ctas = t64x32 * ks;
+    if (steps > 2 && 3 * ctas > 2 * AX_SMS && ctas <= 2 * AX_SMS && (ctas <= AX_SMS || 2 * ctas > 3 * AX_SMS) && 40 * t64x32 <= (ks > ks32 ? 28 : 23) * t32 &&
+        (steps + ks - 1) / ks * ks * 100 <= steps * 127 && (vec || ks == 1 || tb)) return {64, 32, 8, ks};
+    // 4-byte copies count for each CTA that reads a tile of an operand: 64 x 64 tiles from one for each SM on (1964 x 456 x 3179 296 | 385 us, 2196 x 412 x 402 41 | 58, 270 x 2271 x 220 25.0 | 28.2).
+    if (plain && !vec && tb != 2 && depth > 64 && t64 >= AX_SMS) return {64, 64, 4, 1};
+    return {32, 32, 4, ks32};
+}
+static int cut_code(const F32Cut& c) { return c.rows << 20 | c.cols << 8 | c.sums << 4 | c.ctas; }
+int ax_f32_cut = 0;
+// of one product of `batch`
+int ax_gemm_f32_cut(int tb, int m, int n, int k, int batch, int aligned) {
+    auto tiles = [&](int bm, int bn) { return (long long)((m + bm - 1) / bm) * ((n + bn - 1) / bn) * batch; };
+    const bool vec = aligned && (tb != 2 || m % 4 == 0) && n % 4 == 0 && (tb == 2 || k % 4 == 0);
+    return cut_code(f32_cut(tb, true, tiles(128, 128), tiles(64, 64), tiles(64, 32), tiles(32, 32), (k + 63) / 64, k, vec));
+}
+
 template <bool A_MN, bool B_KM, int EPI = F32_PLAIN, bool ONE = false>
 static int f32_gemm(const F32Group& a, int m, int batch, long long sa, long long sb, long long sc, float alpha, float beta, cudaStream_t st) {
     // 16-byte copies need row pitches and starts on 16-byte boundaries
@@ -375,26 +414,17 @@ static int f32_gemm(const F32Group& a, int m, int batch, long long sa, long long
 #define F32L(BM, BN, BK, KG, TM, TN, ST, KSP)                                                                                  \
     (vec ? f32_launch<BM, BN, BK, KG, TM, TN, ST, A_MN, B_KM, true, EPI, ONE>(a, m, batch, sa, sb, sc, KSP, alpha, beta, st)        \
          : f32_launch<BM, BN, BK, KG, TM, TN, ST, A_MN, B_KM, false, EPI, ONE>(a, m, batch, sa, sb, sc, KSP, alpha, beta, st))
-    // A 128 x 128 tile has the most FMAs per shared-memory read, but fewer than 148 of them leave SMs without work.
-    if (tiles(128, 128) >= AX_SMS) return F32L(128, 128, 16, 1, 8, 8, 3, 1);
     int steps = 0;
-    for (int q = 0; q < a.nseg; q++) steps += (a.seg[q].k + 63) / 64;
-    const long long small = tiles(32, 32), mid = tiles(64, 32);
-    if (tiles(64, 64) >= 2 * AX_SMS) return F32L(64, 64, 32, 2, 8, 8, 4, 1);
-    // Below, a launch is the latency of its steps: 64 x 32 tiles (8 x 4 sums to a thread, 43 % of the FMA pipe with two CTAs on an SM, which is what
-    // fits) with the depth cut over a cluster as far as two CTAs for each SM.  Where that leaves a third of the SMs idle or most with one CTA and some with two,
-    // or takes a second round, 32 x 32 tiles spread better; a product of two steps is over before a larger tile pays.  us, 64 x 32 with 1 / 2 / 4 CTAs to a tile |
-    // 32 x 32 alike | before: 512 x 256 x 256 8.6 / 7.9 / 6.2 | 8.8 / 7.6 / 10.1 | 7.6, 512 x 512 x 256 11.0 / 8.4 / 11.9 | 10.0 / 12.0 / 14.9 | 10.0,
-    // 512 x 256 x 688 21.1 / 16.4 / 10.8 | 20.2 / 14.8 / 15.3 | 14.8, 512 x 1024 x 256 12.2 / 17.1 / 24.3 | 14.4 / 19.2 / 26.5 | 14.4,
-    // 512 x 688 x 256 12.2 / 16.6 / 18.2 | 10.8 / 12.9 / 20.3 | 10.9, 512 x 1376 x 256 17.2 / 23.0 / 29.5 | 15.9 / 23.9 / 33.6 | 29.3 (64 x 64 tiles, 4 x 4 sums),
-    // 256 x 256 x 128 4.6 / 5.0 / 5.8 | 3.6 / 4.9 / 5.3 | 3.7, 300 x 128 x 344 10.0 / 7.4 / 7.6 | 6.9 / 6.6 / 7.3 | 6.7; 1024 x 1536 x 512 58 | 60 | 69 and with 64 x 64 tiles of 8 x 8 sums 50.
-    int ks = 1;
-    while (ks < 8 && mid * ks * 2 <= 2 * AX_SMS && steps >= 2 * ks) ks *= 2;
-    const long long ctas = mid * ks;
-    if (steps > 2 && 3 * ctas > 2 * AX_SMS && ctas <= 2 * AX_SMS && (ctas <= AX_SMS || 2 * ctas > 3 * AX_SMS)) return F32L(64, 32, 64, 4, 8, 4, 3, ks);
-    ks = 1;
-    while (ks < 8 && small * ks * 2 <= AX_SMS * 5 / 2 && steps >= 4 * ks) ks *= 2;
-    return F32L(32, 32, 64, 4, 4, 4, 4, ks);
+    long long depth = 0;
+    for (int q = 0; q < a.nseg; q++) { steps += (a.seg[q].k + 63) / 64; depth += a.seg[q].k; }
+    const F32Cut c = f32_cut(A_MN ? 2 : B_KM, EPI == F32_PLAIN, tiles(128, 128), tiles(64, 64), tiles(64, 32), tiles(32, 32), steps, depth, vec);
+    ax_f32_cut = cut_code(c);
+    if (c.rows == 128) return F32L(128, 128, 16, 1, 8, 8, 3, 1);
+    if constexpr (EPI == F32_PLAIN)
+        if (c.cols == 64 && c.sums == 4) return F32L(64, 64, 32, 1, 4, 4, 3, 1);
+    if (c.cols == 64) return F32L(64, 64, 32, 2, 8, 8, 4, 1);
+    if (c.rows == 64) return F32L(64, 32, 64, 4, 8, 4, 3, c.ctas);
+    return F32L(32, 32, 64, 4, 4, 4, 4, c.ctas);
 #undef F32L
 }
 

@@ -89,6 +89,8 @@ int ax_adamw_flat(float* p, const float* g, float* m, float* v, void* pbf, const
 int ax_gemm_simt(int in_bf16, int out_bf16, int tb, const void* A, const void* B, void* C, const void* D,
                  int m, int n, int k, int batch, long long sa, long long sb, long long sc,
                  float alpha, float beta, cudaStream_t st);
+extern int ax_f32_cut;        // see eng_last_f32_cut
+int ax_gemm_f32_cut(int tb, int m, int n, int k, int batch, int aligned);
 // groups of fp32 products (and their SwiGLU epilogues) as one launch; -1 = not served
 int ax_gemm_f32_group(int tb, int mode, int count, const void* const* A, const void* const* B, void* const* C, const int* m, const int* n,
                       const int* k, float alpha, const void* D, float beta, const void* swb_g, const void* swb_u, void* swb_du, cudaStream_t st);

@@ -367,6 +367,11 @@ class Engine:
         """Columns of a tile in the last paired-CTA GEMM launch: 256, 192 or 128."""
         return int(self.lib.eng_last_gemm_width())
 
+    def last_f32_cut(self) -> Tuple[int, int, int, int]:
+        """Rows and columns of a tile, rows of a thread's sums and CTAs that share a tile's depth in the last fp32 product."""
+        c = int(self.lib.eng_last_f32_cut())
+        return c >> 20, c >> 8 & 0xfff, c >> 4 & 0xf, c & 0xf
+
     def bytes_allocated(self) -> int:
         return int(self.lib.eng_bytes_allocated())
 

@@ -174,6 +174,10 @@ int eng_last_variant(void);
 int eng_last_gemm_parts(void);
 /* Columns of a tile in the last launch of the paired-CTA GEMM: 256, 192 or 128. */
 int eng_last_gemm_width(void);
+/* Cut of the last launch of an fp32 product or group: rows of a tile << 20 | columns << 8 | rows of a thread's sums << 4 | CTAs that share a tile's depth.  And of a product of
+ * `batch` of these sizes (aligned: its operands start on 16-byte boundaries; 0 = not a shape): host arithmetic that needs no GPU. */
+int eng_last_f32_cut(void);
+int eng_gemm_f32_cut(int tb, int m, int n, int k, int batch, int aligned);
 /* Whether bf16 attention of this shape, in the layout of ENG_ATTN_FWD / ENG_ATTN_BWD and with aligned buffers, runs on the tcgen05
  * kernels with split probabilities once the whole-tile kernels have refused it (for the backward the number of CTAs that share a key tile,
  * 1, 2 or 4) or not (0): host arithmetic that needs no GPU. */

@@ -141,6 +141,24 @@ def test_cut_of_the_adapters_products(lib, count, one_x, N, F, R, members, token
     assert (cut >> 16, cut >> 8 & 255, cut & 255) == (members, tokens, ctas)
 
 
+@pytest.mark.parametrize("tb,m,n,k,batch,aligned,cut", [
+    # few steps for 64-row tiles, or half of their rows empty, or steps that do not go evenly into the CTAs
+    (0, 512, 256, 256, 1, 1, (64, 32, 8, 4)), (2, 512, 512, 256, 1, 1, (64, 32, 8, 2)), (1, 512, 256, 688, 1, 1, (64, 32, 8, 4)), (0, 512, 688, 256, 1, 1, (32, 32, 4, 1)),
+    (0, 19, 1648, 176, 1, 1, (32, 32, 4, 1)), (1, 32, 1656, 144, 1, 1, (32, 32, 4, 1)), (0, 16, 2208, 320, 1, 1, (32, 32, 4, 2)), (2, 32, 528, 888, 1, 1, (32, 32, 4, 4)),
+    (1, 704, 192, 176, 1, 1, (32, 32, 4, 1)), (1, 144, 2488, 184, 1, 1, (32, 32, 4, 1)), (0, 1104, 40, 384, 1, 1, (32, 32, 4, 2)), (0, 64, 984, 1168, 1, 1, (64, 32, 8, 8)),
+    # shallow products of many tiles
+    (0, 1184, 960, 24, 1, 1, (64, 64, 4, 1)), (1, 1968, 912, 16, 1, 1, (64, 64, 4, 1)), (0, 680, 2792, 32, 1, 1, (64, 64, 4, 1)), (1, 1552, 1176, 104, 1, 1, (64, 64, 4, 1)),
+    (0, 1552, 1176, 104, 1, 1, (64, 64, 8, 1)), (2, 1008, 656, 40, 1, 1, (32, 32, 4, 1)),
+    # rows that are no whole 16-byte pieces
+    (0, 1964, 456, 3179, 1, 1, (64, 64, 4, 1)), (1, 270, 2271, 220, 1, 1, (64, 64, 4, 1)), (2, 270, 2271, 220, 1, 1, (32, 32, 4, 1)), (0, 2422, 201, 324, 1, 1, (64, 32, 8, 1)),
+    (0, 215, 569, 2021, 1, 1, (32, 32, 4, 2)), (1, 202, 504, 677, 1, 1, (64, 32, 8, 4)), (0, 512, 256, 256, 1, 0, (32, 32, 4, 2)), (0, 1100, 1100, 100, 1, 1, (64, 64, 8, 1)),
+    (0, 200, 200, 72, 19, 1, (64, 64, 8, 1)), (0, 1664, 1540, 96, 1, 1, (64, 64, 8, 1)), (0, 2000, 1700, 96, 1, 1, (128, 128, 8, 1)), (2, 2001, 1701, 40, 1, 1, (128, 128, 8, 1))])
+def test_tiles_of_the_fp32_products(lib, tb, m, n, k, batch, aligned, cut):
+    c = lib.eng_gemm_f32_cut(tb, m, n, k, batch, aligned)
+    assert (c >> 20, c >> 8 & 0xfff, c >> 4 & 0xf, c & 0xf) == cut
+    assert lib.eng_gemm_f32_cut(3, m, n, k, batch, aligned) == lib.eng_gemm_f32_cut(tb, 0, n, k, batch, aligned) == 0
+
+
 def test_attention_route_of_invalid_shapes(lib):
     for a in ((0, 8, 4, 500, 64), (1, 0, 4, 500, 64), (1, 8, 0, 500, 64), (1, 8, 3, 500, 64), (1, 8, 4, 0, 64), (1, 8, 4, 500, 0)):
         assert lib.eng_attn_route(0, *a) == lib.eng_attn_route(1, *a) == 0

@@ -468,13 +468,13 @@ def test_adapter_gradients_noted_and_run_as_one_launch(eng):
 
 
 @pytest.mark.parametrize("m,n,k,batch", [
-    (1, 1, 1, 1), (31, 33, 65, 1), (512, 256, 256, 1), (256, 256, 1024, 1), (64, 48, 2048, 1), (32, 32, 250, 3),   # 32 x 32 tiles, split 1 to 8
-    (700, 820, 100, 1), (830, 770, 33, 1), (200, 200, 72, 12),                                                     # 64 x 64 tiles
-    (1664, 1540, 96, 1), (1601, 1603, 17, 1)])                                                                     # 128 x 128 tiles
+    (1, 1, 1, 1), (31, 33, 65, 1), (512, 256, 256, 1), (256, 256, 1024, 1), (64, 48, 2048, 1), (32, 32, 250, 3),   # 32 x 32 and 64 x 32 tiles, split 1 to 8
+    (700, 820, 100, 1), (830, 770, 33, 1), (200, 200, 72, 12),                                                     # 32 x 32 tiles, more than run at once
+    (1664, 1540, 96, 1), (1601, 1603, 17, 1)])                                                                     # 64 x 64 tiles
 @pytest.mark.parametrize("tb", [0, 1, 2])
 def test_fp32_gemm_tiles_and_splits(eng, m, n, k, batch, tb):
-    """Every tile of the fp32 GEMM, with remainders in each dimension, pitches that do and do not allow 16-byte copies, and
-    the depth split over a cluster.  Limit: k products of N(0,1) pairs summed in fp32 in any order err by about
+    """fp32 GEMM over its sizes, with remainders in each dimension, pitches that do and do not allow 16-byte copies, and
+    the depth split over a cluster (each tile by name: `test_fp32_products_on_the_tiles_they_are_cut_into`).  Limit: k products of N(0,1) pairs summed in fp32 in any order err by about
     2^-24 sqrt(k) of the result's rms sqrt(k) per element; ten times that covers the largest of 2.6 million elements."""
     rng = np.random.default_rng(m * 7 + n * 3 + k + tb)
     a = rng.standard_normal((batch, k, m) if tb == 2 else (batch, m, k)).astype(np.float32)
@@ -492,6 +492,69 @@ def test_fp32_gemm_tiles_and_splits(eng, m, n, k, batch, tb):
     assert np.abs(out[:d.size].reshape(ref.shape) - ref).max() <= 10 * 2.0 ** -24 * (k + 4)
     eng.run(plan)
     assert np.array_equal(out, eng.download(ic, d.size + 64))       # run-to-run identical
+
+
+@pytest.mark.parametrize("m,n,k,batch,cuts", [           # cuts of A B, A B^T, A^T B
+    (1100, 1100, 200, 1, [(64, 64, 8, 1)] * 3), (1093, 1101, 267, 1, [(64, 64, 8, 1)] * 3), (200, 200, 72, 19, [(64, 64, 8, 1), (64, 64, 4, 1), (64, 64, 8, 1)]),
+    (1100, 900, 24, 1, [(64, 64, 4, 1)] * 3), (1085, 907, 31, 1, [(64, 64, 4, 1)] * 3), (700, 1050, 451, 1, [(64, 64, 4, 1)] * 2 + [(32, 32, 4, 1)]),
+    (512, 256, 256, 1, [(64, 32, 8, 4)] * 3), (517, 250, 251, 1, [(32, 32, 4, 2)] + [(64, 32, 8, 4)] * 2), (523, 781, 300, 1, [(64, 32, 8, 1)] * 3), (120, 424, 1960, 1, [(64, 32, 8, 8)] * 3),
+    (31, 33, 65, 1, [(32, 32, 4, 1)] * 3), (90, 70, 1021, 1, [(32, 32, 4, 8)] * 3), (2000, 1700, 96, 1, [(128, 128, 8, 1)] * 3), (2001, 1701, 40, 1, [(128, 128, 8, 1)] * 3)])
+@pytest.mark.parametrize("tb", [0, 1, 2])
+def test_fp32_products_on_the_tiles_they_are_cut_into(eng, m, n, k, batch, cuts, tb):
+    """Every tile with and without whole 16-byte pieces and remainders, by what the launch says it was cut into; limit as in `test_fp32_gemm_tiles_and_splits`."""
+    rng = np.random.default_rng(m + n + k + tb)
+    a = rng.standard_normal((batch, k, m) if tb == 2 else (batch, m, k)).astype(np.float32)
+    b = rng.standard_normal((batch, n, k) if tb == 1 else (batch, k, n)).astype(np.float32)
+    d = rng.standard_normal((batch, m, n)).astype(np.float32)
+    ia, ib, ic, idd = eng.new_tensor(a), eng.new_tensor(b), eng.alloc(d.size + 64), eng.new_tensor(d)
+    eng.upload(ic, np.full(d.size + 64, 7.0, np.float32))
+    eng.run([op(E.GEMM_EX, a=ia, b=ib, c=ic, d=idd, m=m, n=n, k=k, batch=batch, tb=tb, sa=m * k, sb=k * n, sc=m * n, alpha=0.5, beta=-2.0)])
+    assert eng.last_f32_cut() == cuts[tb] and eng.last_variant() == 0x20
+    out = eng.download(ic, d.size + 64)
+    assert np.all(out[d.size:] == 7.0)
+    a64, b64 = a.astype(np.float64), b.astype(np.float64)
+    ref = 0.5 * ((a64.transpose(0, 2, 1) if tb == 2 else a64) @ (b64.transpose(0, 2, 1) if tb == 1 else b64)) - 2.0 * d
+    assert np.abs(out[:d.size].reshape(ref.shape) - ref).max() <= 10 * 2.0 ** -24 * (k + 4)
+
+
+def test_fp32_groups_on_64_by_64_tiles(eng):
+    """Products of one input, a sum over segments, a SwiGLU pair and its backward, each of 296 tiles of 64 x 64 or more and fewer than 148 of 128 x 128, with remainders; bounds as in the
+    tests of those groups."""
+    rng = np.random.default_rng(64)
+    mk = lambda *sh: rng.standard_normal(sh).astype(np.float32)
+    f = lambda v: v.astype(np.float64)
+    big = lambda v: np.abs(v).max()
+    m, k, ns = 1000, 204, (520, 776, 132)
+    x, w = mk(m, k), [mk(k, n) for n in ns]
+    ix, iw, ic = put(eng, x, 0), [put(eng, v, 0) for v in w], [eng.alloc(m * n) for n in ns]
+    eng.run([op(E.GEMM_GROUP, a=ix, b=iw[0], sa=iw[1], sb=iw[2], c=ic[0], d=ic[1], sc=ic[2], m=m, k=k, n=ns[0], oa=ns[1], ob=ns[2], batch=3, oc=1, tb=0, dt=0)])
+    assert eng.last_variant() == 0x29 and eng.last_f32_cut() == (64, 64, 8, 1)
+    for g, n in enumerate(ns):
+        check(eng.download(ic[g], (m, n)), f(x) @ f(w[g]), False, k)
+    n, ks = 1220, (100, 40, 72)
+    a, b = [mk(m, q) for q in ks], [mk(n, q) for q in ks]
+    ia, ib, io = [put(eng, v, 0) for v in a], [put(eng, v, 0) for v in b], eng.alloc(m * n)
+    eng.run([op(E.GEMM_GROUP, c=io, a=ia[0], sa=ia[1], sb=ia[2], b=ib[0], d=ib[1], sc=ib[2], m=m, n=n, k=ks[0], oa=ks[1], ob=ks[2], batch=3, oc=2, tb=1, dt=0)])
+    assert eng.last_variant() == 0x29 and eng.last_f32_cut() == (64, 64, 8, 1)
+    check(eng.download(io, (m, n)), sum(f(p) @ f(q).T for p, q in zip(a, b)), False, sum(ks))
+    for n in (640, 1220):                                # the pair's tiles hold 32 columns of either
+        wg, wu = mk(k, n), mk(k, n)
+        ig, iu, og, ou, oh = put(eng, wg, 0), put(eng, wu, 0), eng.alloc(m * n), eng.alloc(m * n), eng.alloc(m * n)
+        eng.run([op(E.GEMM_GROUP, a=ix, b=ig, sa=iu, c=og, d=ou, sc=oh, m=m, n=n, k=k, batch=2, oc=4, dt=0)])
+        assert eng.last_variant() == 0x29 and (n > 640 or eng.last_f32_cut() == (64, 64, 8, 1))
+        g, u = f(x) @ f(wg), f(x) @ f(wu)
+        s = 1.0 / (1.0 + np.exp(-g))
+        check(eng.download(og, (m, n)), g, False, k)
+        check(eng.download(ou, (m, n)), u, False, k)
+        assert big(eng.download(oh, (m, n)) - g * s * u) <= 4.1 * f32_limit(k) * big(g) * big(u)
+    wd, dy = mk(n, k), mk(m, k)
+    iwd, idy, idh, idg, idu = put(eng, wd, 0), put(eng, dy, 0), eng.alloc(m * n), eng.alloc(m * n), eng.alloc(m * n)
+    eng.run([op(E.GEMM_SB, a=idy, b=iwd, c=idh, m=m, n=n, k=k, batch=1, tb=1, dt=0), op(E.SILU_BWD, a=og, b=ou, d=idh, c=idg, tb=idu, n=m * n, dt=0, oa=1)])
+    assert eng.last_variant() == 0x2a and eng.last_f32_cut() == (64, 64, 8, 1)
+    dh = f(dy) @ f(wd).T
+    assert big(eng.download(idg, (m, n)) - dh * u * s * (1 + g * (1 - s))) <= 2 * f32_limit(k) * big(dh) * big(u) * (2.2 + 0.5 * big(g))
+    assert big(eng.download(idu, (m, n)) - dh * g * s) <= 2 * f32_limit(k) * big(dh) * big(g) * 2.1
+    assert eng.device_status() == 0
 
 
 @pytest.mark.parametrize("extra", [0, 1])
@@ -992,8 +1055,8 @@ def test_tall_products_walk_their_tiles_in_bands(eng, m, n, k, tb, dt):
 
 
 F32_GROUPS = [(5, 7, (3, 9, 2)), (33, 66, (40, 8, 1)),              # rows that are no whole 16-byte pieces, less than a tile
-              (512, 256, (256, 128, 128)), (100, 1100, (36, 4, 200)),    # 32 x 32 tiles, the depth over a cluster of one, two and four
-              (700, 72, (520, 264, 132)), (1300, 36, (1032, 776, 516))]  # 64 x 64 and 128 x 128 tiles
+              (512, 256, (256, 128, 128)), (100, 1100, (36, 4, 200)),    # 64 x 32 and 32 x 32 tiles, the depth over a cluster
+              (700, 72, (520, 264, 132)), (1300, 36, (1032, 776, 516))]  # 32 x 32, 64 x 64 and 128 x 128 tiles
 
 
 def f32_limit(k):
