@@ -9,6 +9,7 @@
 // fixed order.  B2 H8 KV4 T256 DH32, us in attn_simt.cu / here, forward and backward with the row
 // dots: 14.8 and 42.4 / 12.4 and 30.6; B2 H12 KV4 T900 DH64 214 and 639 / 130 and 455.  2-norm errors against float64 (T 128 to 900) are 0.79 to 1.01 times those there.
 #include <initializer_list>
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -21,7 +22,7 @@
 template <int DHP> struct F32Att {
     static constexpr int LD = DHP + 4, NC = DHP / 8, TILE = FT * LD, OWN = FB * LD, P = FT * 16;     // floats; LD: rows kg, kg + 1, ... in different banks
 };
-// ROWS rows of `stride` floats from r0 of a [T, DH] window; rows past T and columns past DH are zeros
+// ROWS rows of `stride` floats from r0 of a [T, DH] window; rows past T are zeros, columns past DH stay what they were (their sums are never stored)
 template <int DHP, int ROWS>
 __device__ __forceinline__ void fa_load(float* dst, const float* src, long long stride, int r0, int T, int DH) {
     constexpr int Q = DHP / 4;
@@ -29,22 +30,22 @@ __device__ __forceinline__ void fa_load(float* dst, const float* src, long long 
 #pragma unroll
     for (int i = 0; i < ROWS * Q / FTH; i++) {
         const int e = threadIdx.x + i * FTH, r = e / Q, d = e % Q * 4;
-        const bool in = r0 + r < T && d < DH;
+        const bool in = r0 + r < T;
         const float* p = in ? src + (long long)(r0 + r) * stride + d : src;
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(base + (r * F32Att<DHP>::LD + d) * 4), "l"(p), "r"(in ? 16 : 0) : "memory");
+        if (d < DH) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(base + (r * F32Att<DHP>::LD + d) * 4), "l"(p), "r"(in ? 16 : 0) : "memory");
     }
 }
 __device__ __forceinline__ void fa_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void fa_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 // out[i][j] = <row i of this lane, column j of this lane>; a and b point at the first of either
-template <int DHP> __device__ __forceinline__ void fa_dot(const float* a, const float* b, float (&out)[4][4]) {
+template <int DHP> __device__ __forceinline__ void fa_dot(const float* a, const float* b, int DH, float (&out)[4][4]) {
     constexpr int LD = F32Att<DHP>::LD;
 #pragma unroll
     for (int i = 0; i < 4; i++)
 #pragma unroll
         for (int j = 0; j < 4; j++) out[i][j] = 0.f;
 #pragma unroll 4
-    for (int d = 0; d < DHP; d += 4) {
+    for (int d = 0; d < DH; d += 4) {
         float4 x[4], y[4];
 #pragma unroll
         for (int i = 0; i < 4; i++) { x[i] = *reinterpret_cast<const float4*>(a + i * 4 * LD + d); y[i] = *reinterpret_cast<const float4*>(b + i * 8 * LD + d); }
@@ -91,11 +92,42 @@ template <int NC> __device__ __forceinline__ void fa_store(float* row, const flo
     for (int c = 0; c < NC; c += 4)
         if (c * 8 + kg * 4 < DH) *reinterpret_cast<float4*>(row + c * 8 + kg * 4) = make_float4(a[c] * f, a[c + 1] * f, a[c + 2] * f, a[c + 3] * f);
 }
-__device__ __forceinline__ float fa_peer(const float* p, int rank) {
-    float x;
-    asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %1, %2;\n\tld.shared::cluster.f32 %0, [ra];\n\t}"
-                 : "=f"(x) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank) : "memory");
+// What a cluster merges lies in shared memory as [piece][thread] of float4.  The pieces at `at` of all S ranks, added in rank order (SUM of a stored one: times w[rank]).  All S
+// reads are under way before the first is used: where each waited for the one before it, a merge took 6 us (dK / dV of B5 H12 KV12 T13 DH16 over two CTAs: 12.0 us,
+// 6.2 with one CTA and no merge).
+__device__ __forceinline__ float4 fa_peer4(const float4* p, int rank) {
+    float4 x;
+    asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %4, %5;\n\tld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [ra];\n\t}"
+                 : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank) : "memory");
     return x;
+}
+template <int S, int N> __device__ __forceinline__ void fa_gather(const float4* at, const float* w, float* a) {
+#pragma unroll
+    for (int c = 0; c < N; c += 4) {
+        float4 x[S];
+#pragma unroll
+        for (int z = 0; z < S; z++) x[z] = fa_peer4(at + c / 4 * FTH, z);
+        float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int z = 0; z < S; z++) {
+            const float f = w ? w[z] : 1.f;
+            t.x = fmaf(x[z].x, f, t.x); t.y = fmaf(x[z].y, f, t.y); t.z = fmaf(x[z].z, f, t.z); t.w = fmaf(x[z].w, f, t.w);
+        }
+        a[c] = t.x; a[c + 1] = t.y; a[c + 2] = t.z; a[c + 3] = t.w;
+    }
+}
+// rows of this lane's four (N columns each, from piece 0 of a) -> pieces
+template <int N> __device__ __forceinline__ void fa_leave(float4* x, const float (&a)[4][N]) {
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int c = 0; c < N; c += 4) x[(i * N + c) / 4 * FTH] = make_float4(a[i][c], a[i][c + 1], a[i][c + 2], a[i][c + 3]);
+}
+// f(integral constant S) for the sizes of a cluster
+template <typename F> __device__ __forceinline__ void fa_of_size(int S, F f) {
+    if (S == 2) f(std::integral_constant<int, 2>());
+    else if (S == 4) f(std::integral_constant<int, 4>());
+    else f(std::integral_constant<int, 8>());
 }
 // over the eight lanes of a row
 __device__ __forceinline__ float fa_max8(float x) {
@@ -145,7 +177,7 @@ k_attn_fwd_f32(const float* __restrict__ q, const float* __restrict__ k, const f
         fa_commit();
         if (kt * FT > t0 + 15) continue;
         float sc[4][4];
-        fa_dot<DHP>(Qs + (warp * 16 + rg) * F::LD, Ks + cur * F::TILE + kg * F::LD, sc);
+        fa_dot<DHP>(Qs + (warp * 16 + rg) * F::LD, Ks + cur * F::TILE + kg * F::LD, s.DH, sc);
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             const int last = t0 + rg + 4 * i - kt * FT - kg;                  // 8 j of the row's own key
@@ -174,33 +206,31 @@ k_attn_fwd_f32(const float* __restrict__ q, const float* __restrict__ k, const f
     if (SHARE) {                         // merge: sums at the largest of the ranks' maxima
         fa_wait();
         __syncthreads();
-        float* x = smem + threadIdx.x;
+        float4* x = reinterpret_cast<float4*>(smem) + threadIdx.x;       // [row: maximum and sum; columns]
+        float4* y = x + 4 * FTH;
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            x[(i * (F::NC + 2)) * FTH] = m[i];
-            x[(i * (F::NC + 2) + 1) * FTH] = l[i];
-#pragma unroll
-            for (int c = 0; c < F::NC; c++) x[(i * (F::NC + 2) + 2 + c) * FTH] = acc[i][c];
-        }
+        for (int i = 0; i < 4; i++) x[i * FTH] = make_float4(m[i], l[i], 0.f, 0.f);
+        fa_leave<F::NC>(y, acc);
         cluster_sync();
-        for (int i = part * 4 / S; i < (part + 1) * 4 / S; i++) {
-            const float* y = x + i * (F::NC + 2) * FTH;
-            float mx = -3.0e38f, ls = 0.f, a[F::NC];
-            for (int z = 0; z < S; z++) mx = fmaxf(mx, fa_peer(y, z));
+        fa_of_size(S, [&](auto size) {
+            constexpr int SS = decltype(size)::value;
+            for (int i = part * 4 / SS; i < (part + 1) * 4 / SS; i++) {
+                float4 ml[SS];
+                float mx = -3.0e38f, ls = 0.f, w[SS], a[F::NC];
 #pragma unroll
-            for (int c = 0; c < F::NC; c++) a[c] = 0.f;
-            for (int z = 0; z < S; z++) {
-                const float f = expf(fa_peer(y, z) - mx);
-                ls += fa_peer(y + FTH, z) * f;
+                for (int z = 0; z < SS; z++) ml[z] = fa_peer4(x + i * FTH, z);
 #pragma unroll
-                for (int c = 0; c < F::NC; c++) a[c] += fa_peer(y + (2 + c) * FTH, z) * f;
+                for (int z = 0; z < SS; z++) mx = fmaxf(mx, ml[z].x);
+#pragma unroll
+                for (int z = 0; z < SS; z++) { w[z] = expf(ml[z].x - mx); ls += ml[z].y * w[z]; }
+                fa_gather<SS, F::NC>(y + i * (F::NC / 4) * FTH, w, a);
+                ls = fa_sum8(ls);
+                const int t = t0 + rg + 4 * i;
+                if (t >= s.T) continue;
+                fa_store<F::NC>(o + b * s.qb + h * s.qh + (long long)t * s.qt, a, 1.f / ls, kg, s.DH);
+                if (lse && kg == 0) lse[((long long)b * s.H + h) * s.T + t] = mx + logf(ls);
             }
-            ls = fa_sum8(ls);
-            const int t = t0 + rg + 4 * i;
-            if (t >= s.T) continue;
-            fa_store<F::NC>(o + b * s.qb + h * s.qh + (long long)t * s.qt, a, 1.f / ls, kg, s.DH);
-            if (lse && kg == 0) lse[((long long)b * s.H + h) * s.T + t] = mx + logf(ls);
-        }
+        });
         cluster_sync();                  // peers have read
         return;
     }
@@ -258,8 +288,8 @@ k_attn_dq_f32(const float* __restrict__ q, const float* __restrict__ k, const fl
         fa_commit();
         if (kt * FT > t0 + 15) continue;
         float sc[4][4], dp[4][4];
-        fa_dot<DHP>(Qs + (warp * 16 + rg) * F::LD, Ks + cur * F::TILE + kg * F::LD, sc);
-        fa_dot<DHP>(Gs + (warp * 16 + rg) * F::LD, Vs + cur * F::TILE + kg * F::LD, dp);
+        fa_dot<DHP>(Qs + (warp * 16 + rg) * F::LD, Ks + cur * F::TILE + kg * F::LD, s.DH, sc);
+        fa_dot<DHP>(Gs + (warp * 16 + rg) * F::LD, Vs + cur * F::TILE + kg * F::LD, s.DH, dp);
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             const int t = t0 + rg + 4 * i, last = t - kt * FT - kg;
@@ -275,22 +305,18 @@ k_attn_dq_f32(const float* __restrict__ q, const float* __restrict__ k, const fl
     if (SHARE) {
         fa_wait();
         __syncthreads();
-        float* x = smem + threadIdx.x;
-#pragma unroll
-        for (int i = 0; i < 4; i++)
-#pragma unroll
-            for (int c = 0; c < F::NC; c++) x[(i * F::NC + c) * FTH] = acc[i][c];
+        float4* x = reinterpret_cast<float4*>(smem) + threadIdx.x;
+        fa_leave<F::NC>(x, acc);
         cluster_sync();
-        for (int i = part * 4 / S; i < (part + 1) * 4 / S; i++) {
-            float a[F::NC];
-#pragma unroll
-            for (int c = 0; c < F::NC; c++) {
-                a[c] = 0.f;
-                for (int z = 0; z < S; z++) a[c] += fa_peer(x + (i * F::NC + c) * FTH, z);
+        fa_of_size(S, [&](auto size) {
+            constexpr int SS = decltype(size)::value;
+            for (int i = part * 4 / SS; i < (part + 1) * 4 / SS; i++) {
+                float a[F::NC];
+                fa_gather<SS, F::NC>(x + i * (F::NC / 4) * FTH, nullptr, a);
+                const int t = t0 + rg + 4 * i;
+                if (t < s.T) fa_store<F::NC>(out + (long long)t * s.qt, a, 1.f, kg, s.DH);
             }
-            const int t = t0 + rg + 4 * i;
-            if (t < s.T) fa_store<F::NC>(out + (long long)t * s.qt, a, 1.f, kg, s.DH);
-        }
+        });
         cluster_sync();                  // peers have read
         return;
     }
@@ -346,8 +372,8 @@ k_attn_dkv_f32(const float* __restrict__ q, const float* __restrict__ k, const f
         const float* Qt = Qs + cur * F::TILE;
         const float* Gt = Gs + cur * F::TILE;
         float sc[4][4], dp[4][4];
-        fa_dot<DHP>(Kr + (warp * 16 + rg) * F::LD, Qt + kg * F::LD, sc);
-        fa_dot<DHP>(Vr + (warp * 16 + rg) * F::LD, Gt + kg * F::LD, dp);
+        fa_dot<DHP>(Kr + (warp * 16 + rg) * F::LD, Qt + kg * F::LD, s.DH, sc);
+        fa_dot<DHP>(Vr + (warp * 16 + rg) * F::LD, Gt + kg * F::LD, s.DH, dp);
 #pragma unroll
         for (int i = 0; i < 4; i++)
 #pragma unroll
@@ -370,22 +396,19 @@ k_attn_dkv_f32(const float* __restrict__ q, const float* __restrict__ k, const f
     if (SHARE) {                         // units: dK rows, then dV rows
         fa_wait();
         __syncthreads();
-        float* x = smem + threadIdx.x;
-#pragma unroll
-        for (int i = 0; i < 4; i++)
-#pragma unroll
-            for (int c = 0; c < F::NC; c++) { x[(i * F::NC + c) * FTH] = ak[i][c]; x[((4 + i) * F::NC + c) * FTH] = av[i][c]; }
+        float4* x = reinterpret_cast<float4*>(smem) + threadIdx.x;
+        fa_leave<F::NC>(x, ak);
+        fa_leave<F::NC>(x + F::NC * FTH, av);
         cluster_sync();
-        for (int u = part * 8 / S; u < (part + 1) * 8 / S; u++) {
-            float a[F::NC];
-#pragma unroll
-            for (int c = 0; c < F::NC; c++) {
-                a[c] = 0.f;
-                for (int z = 0; z < S; z++) a[c] += fa_peer(x + (u * F::NC + c) * FTH, z);
+        fa_of_size(S, [&](auto size) {
+            constexpr int SS = decltype(size)::value;
+            for (int u = part * 8 / SS; u < (part + 1) * 8 / SS; u++) {
+                float a[F::NC];
+                fa_gather<SS, F::NC>(x + u * (F::NC / 4) * FTH, nullptr, a);
+                const int t = j0 + rg + 4 * (u & 3);
+                if (t < s.T) fa_store<F::NC>((u < 4 ? ok : ov) + (long long)t * s.kt, a, 1.f, kg, s.DH);
             }
-            const int t = j0 + rg + 4 * (u & 3);
-            if (t < s.T) fa_store<F::NC>((u < 4 ? ok : ov) + (long long)t * s.kt, a, 1.f, kg, s.DH);
-        }
+        });
         cluster_sync();                  // peers have read
         return;
     }
@@ -404,7 +427,7 @@ template <int DHP> static constexpr int fa_smem(int which) {      // (the merge 
     return ((which == FA_FWD ? 1 : 2) * F32Att<DHP>::OWN + 4 * F32Att<DHP>::TILE + FW * F32Att<DHP>::P) * 4;
 }
 template <int DHP> static constexpr int fa_merge(int which) {
-    return (which == FA_FWD ? 4 * (F32Att<DHP>::NC + 2) : which == FA_DQ ? 4 * F32Att<DHP>::NC : 8 * F32Att<DHP>::NC) * FTH * 4;
+    return (which == FA_FWD ? 4 * (F32Att<DHP>::NC + 4) : which == FA_DQ ? 4 * F32Att<DHP>::NC : 8 * F32Att<DHP>::NC) * FTH * 4;
 }
 static_assert(fa_merge<32>(FA_FWD) <= fa_smem<32>(FA_FWD) && fa_merge<64>(FA_FWD) <= fa_smem<64>(FA_FWD) && fa_merge<32>(FA_DKV) <= fa_smem<32>(FA_DKV) &&
               fa_merge<64>(FA_DKV) <= fa_smem<64>(FA_DKV), "what a cluster merges takes the tiles' place");
