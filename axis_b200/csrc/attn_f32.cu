@@ -1,5 +1,5 @@
 // Causal grouped-query attention in exact fp32 for head dims from 12 to 64 (rows in whole 16-byte pieces): the parity mode at its usual sizes.
-// attn_simt.cu serves everything else.
+// attn_simt.cu serves everything else, and what is faster there (see ax_attn_f32_ctas).
 //
 // Bound by shared-memory reads and latency there: a lane of attn_simt.cu owns one row of the walked tile, and 16 FMAs take one read of its own row and four
 // broadcasts, eight cycles of the shared-memory pipe for four of the FMA pipes.  Here a warp owns 16 rows and a lane 4 x 4 of its 16 x 32 scores (rows rg + 4 i, columns
@@ -7,7 +7,9 @@
 // four rows and DH / 8 columns to a lane, with the probabilities going through shared memory as [column][16 rows].  A block is four warps, 64 rows; tiles of
 // 32 rows of the walked operands are double-buffered by cp.async, and where blocks are few a cluster takes the tiles in turn (see attn_simt.cu).  No atomics, sums in a
 // fixed order.  B2 H8 KV4 T256 DH32, us in attn_simt.cu / here, forward and backward with the row
-// dots: 14.8 and 42.4 / 12.4 and 30.6; B2 H12 KV4 T900 DH64 214 and 639 / 130 and 455.  2-norm errors against float64 (T 128 to 900) are 0.79 to 1.01 times those there.
+// dots: 14.9 and 42.2 / 12.3 and 30.4; B2 H12 KV4 T900 DH64 215 and 633 / 127 and 431.  2-norm errors against float64 (T 128 to 900) are 0.79 to 1.01 times those there.
+#include <math.h>
+
 #include <initializer_list>
 #include <type_traits>
 
@@ -447,23 +449,43 @@ static bool fa_served(const AttnShape& s, std::initializer_list<const void*> ptr
     for (const void* p : ptrs) ok = ok && aligned16(p);
     return ok;
 }
-// CTAs that share a block's walk of `chain` tiles: doubled up to four (dK / dV eight), the more CTAs there are then, the more tiles have to be left to each.  us with
-// 1 / 2 / 4 CTAs (blocks, chain): forward B2 H8 T256 DH32 (64, 8) 22.7 / 15.7 / 12.4, B4 H8 T128 DH32 (64, 4) 12.5 / 9.6 / 8.6, B2 H8 T300 DH16 (80, 10) 27.7 / 20.6 / 16.6,
-// B8 H8 T128 DH64 (128, 4) 19.7 / 18.0 / 20.2, B2 H8 T512 DH32 (128, 16) 49 / 35 / 23, B2 H12 T900 DH64 (360, 29) 191 / 137 / 129, B4 H16 T500 DH48 (512, 16) 116 / 104 / 108;
-// backward with four CTAs for dQ and 4 / 8 for dK / dV: B2 H8 KV4 T256 DH32 (32, 16) 34.5 / 30.6, B2 H8 KV4 T512 DH32 (64, 32) 83 / 73, B2 H8 KV8 T300 DH16 (80, 10) 39 / 43.
-static int fa_share(long long ctas, int chain, int most) {
-    int S = 1;
-    for (int n = 2; n <= most; n *= 2) {
-        const long long c = ctas * n;
-        if (!(c <= AX_SMS ? chain >= n / 2 : c <= 2 * AX_SMS ? chain >= n : c <= 3 * AX_SMS ? chain >= 2 * n : c <= 10 * AX_SMS && chain >= 4 * n)) break;
-        S = n;
-    }
-    return S;
+// CTAs that share a block's walk (powers of two, up to four, dK / dV eight), or 0: attn_simt.cu is faster, whose blocks are half as long and whose steps are shorter.
+//
+// The number is that of the least estimate: launch, steps of a CTA, the chip's work (steps and set-ups for each SM), which add up nearly, and a merge.  Constants are fitted to 680
+// seeded shapes (T 8 to 1500, H 1 to 48; rms 10 to 12 %).  us with 1 / 2 / 4 / 8 CTAs and there (blocks, tiles of the longest walk): forward B2 H8 T256 DH32 (64, 8) 22.9 / 14.7 / 12.2
+// and 14.8, B2 H16 T333 DH64 (192, 11) 65 / 41 / 40 and 63; with row dots dQ of the former 27.3 / 16.7 / 14.0 and 20.9; dK / dV of B2 H8 KV4 T256 DH32 (32, 16) 63.5 / 35.5 / 20.5 / 17.8
+// and 22.8, B40 H8 KV2 T100 DH48 (160, 16) 129 / 97 / 77 / 86 and 140.  Over the 680: 0.80, 0.85 and 0.88 of the time there.
+//
+// There, dQ | dK / dV with row dots, here / there: sequences of one tile, which fill half a block: B240 H16 KV4 T10 DH48 104 / 73 | 124 / 86, B7 H8 KV8 T22 DH32 - | 6.5 / 6.5, B12 H24 KV12
+// T14 DH16 - | 9.6 / 8.2, forward B33 H12 T17 DH32 8.9 / 7.2; few blocks with long walks, which are the latency of their steps: B1 H3 T976 DH16 32 / 24 | 51 / 41, B1 H8 KV2 T928 DH64 - | 144 / 125,
+// B6 H2 KV1 T192 DH12 - | 15.1 / 11.9.
+static double fa_us(int which, int DH, double walk, double work, double ctas, int S) {
+    static const struct { double launch, chip, step, step_dh, step_cols, cta_col, merge, merge_col; } k[3] = {
+        {1.39, 0.678, 1.33, 0.0220, 0.0141, 0.0149, 1.16, 0.0082}, {2.47, 0.767, 0.81, 0.0364, 0.0237, 0.0165, 1.45, 0.0070}, {1.83, 0.730, 1.49, 0.0342, 0.0341, 0.0450, 1.84, 0.0089}};
+    const auto& c = k[which];
+    const int cols = DH <= 32 ? 32 : 64;
+    const double step = c.step + c.step_dh * DH + c.step_cols * cols;
+    return c.launch + pow(pow(step * walk, 1.35) + pow(c.chip * step * work + c.cta_col * cols * ctas, 1.35), 1 / 1.35) + (S > 1 ? c.merge + c.merge_col * cols : 0);
 }
-static int fa_share(int which, const AttnShape& s) {
-    const long long blocks = (s.T + FB - 1) / FB;
-    const int tiles = (s.T + FT - 1) / FT;
-    return which == FA_DKV ? fa_share(blocks * s.KV * s.B, s.H / s.KV * tiles, 8) : fa_share(blocks * s.H * s.B, tiles, 4);
+int ax_attn_f32_ctas(int which, const AttnShape& s) {
+    if (s.DH <= 8 || s.DH > 64 || s.DH % 4 || s.B < 1 || s.T < 1 || s.KV < 1 || s.H < 1 || s.H % s.KV) return 0;
+    const long long nb = (s.T + FB - 1) / FB, tiles = (s.T + FT - 1) / FT, rep = s.H / s.KV, heads = (long long)(which == FA_DKV ? s.KV : s.H) * s.B;
+    const long long blocks = nb * heads, chain = which == FA_DKV ? rep * tiles : tiles;
+    long long work = 0;                  // tiles that all blocks of a head walk
+    for (long long i = 0; i < nb; i++) work += which == FA_DKV ? rep * (tiles - i * (FB / FT)) : tiles < (i + 1) * (FB / FT) ? tiles : (i + 1) * (FB / FT);
+    const bool half = s.T <= FT;         // of a block's rows
+    if (which == FA_FWD && half && blocks >= 2 * AX_SMS && (s.DH > 32 || blocks < 4 * AX_SMS)) return 0;
+    if (which == FA_DQ && ((half && s.DH > 32) || (blocks <= AX_SMS / 2 && chain > 8 && s.DH <= 16) || (blocks <= AX_SMS / 4 && chain > 20 && s.DH <= 32))) return 0;
+    if (which == FA_DKV && ((half && (s.DH > 32 ? chain == 1 || blocks > AX_SMS : s.DH < 32 && blocks <= AX_SMS)) || (s.T > 96 && blocks < 12) ||
+                            (blocks <= AX_SMS / 4 && chain > 60 && s.DH != 32) || (blocks <= 20 && chain > 8 && s.DH < 32))) return 0;
+    int best = 1;
+    double least = 0;
+    for (int S = 1; S <= (which == FA_DKV ? 8 : 4) && S < 2 * chain; S *= 2) {
+        if (S > chain && blocks * S > AX_SMS) break;     // CTAs without a tile only on SMs that have nothing else
+        const double us = fa_us(which, s.DH, (double)((chain + S - 1) / S), (double)work * heads / AX_SMS, (double)blocks * S / AX_SMS, S);
+        if (S == 1 || us < least) { least = us; best = S; }
+    }
+    return best;
 }
 template <typename K, typename... A>
 static int fa_launch(K shared, K whole, const AttnShape& s, int heads, int smem, int S, bool early, cudaStream_t st, A... args) {
@@ -478,26 +500,34 @@ static int fa_launch(K shared, K whole, const AttnShape& s, int heads, int smem,
     return cudaLaunchKernelEx(&cfg, S > 1 ? shared : whole, args..., S) == cudaSuccess ? 0 : 3;
 }
 template <int DHP>
-static int fa_fwd(const float* q, const float* k, const float* v, float* o, float* lse, const AttnShape& s, cudaStream_t st) {
-    return fa_launch(k_attn_fwd_f32<DHP, true>, k_attn_fwd_f32<DHP, false>, s, s.H, fa_smem<DHP>(FA_FWD), fa_share(FA_FWD, s), true, st, q, k, v, o, lse, s);
+static int fa_fwd(const float* q, const float* k, const float* v, float* o, float* lse, const AttnShape& s, int S, cudaStream_t st) {
+    return fa_launch(k_attn_fwd_f32<DHP, true>, k_attn_fwd_f32<DHP, false>, s, s.H, fa_smem<DHP>(FA_FWD), S, true, st, q, k, v, o, lse, s);
 }
 template <int DHP>
-static int fa_bwd(const float* q, const float* k, const float* v, const float* dO, const float* lse, const float* Dv, float* dq, float* dk, float* dv, const AttnShape& s, cudaStream_t st) {
-    const int rc = fa_launch(k_attn_dq_f32<DHP, true>, k_attn_dq_f32<DHP, false>, s, s.H, fa_smem<DHP>(FA_DQ), fa_share(FA_DQ, s), true, st, q, k, v, dO, lse, Dv, dq, s);
-    return rc ? rc : fa_launch(k_attn_dkv_f32<DHP, true>, k_attn_dkv_f32<DHP, false>, s, s.KV, fa_smem<DHP>(FA_DKV), fa_share(FA_DKV, s), false, st, q, k, v, dO, lse, Dv, dk, dv, s);
+static int fa_dq(const float* q, const float* k, const float* v, const float* dO, const float* lse, const float* Dv, float* dq, const AttnShape& s, int S, cudaStream_t st) {
+    return fa_launch(k_attn_dq_f32<DHP, true>, k_attn_dq_f32<DHP, false>, s, s.H, fa_smem<DHP>(FA_DQ), S, true, st, q, k, v, dO, lse, Dv, dq, s);
 }
-// -1: not for these kernels
+template <int DHP>
+static int fa_dkv(const float* q, const float* k, const float* v, const float* dO, const float* lse, const float* Dv, float* dk, float* dv, const AttnShape& s, int S, cudaStream_t st) {
+    // Its CTAs come while dQ ends where they are few: 8 % of the backward with 74 and narrow heads, 3 % with wide ones; behind the larger blocks of the general dQ kernel only with 37, as
+    // 74 to 111 took up to 1.4 times as long there.
+    const bool early = (long long)((s.T + FB - 1) / FB) * s.KV * s.B * S <= (ax_attn_f32_ctas(FA_DQ, s) ? AX_SMS / 2 : AX_SMS / 4);
+    return fa_launch(k_attn_dkv_f32<DHP, true>, k_attn_dkv_f32<DHP, false>, s, s.KV, fa_smem<DHP>(FA_DKV), S, early, st, q, k, v, dO, lse, Dv, dk, dv, s);
+}
+// -1: not for these kernels.  dQ and dK / dV are chosen each by itself.
 int ax_attn_fwd_f32(const float* q, const float* k, const float* v, float* o, float* lse, const AttnShape& s, cudaStream_t st) {
-    if (!fa_served(s, {q, k, v, o})) return -1;
+    const int S = ax_attn_f32_ctas(FA_FWD, s);
+    if (!S || !fa_served(s, {q, k, v, o})) return -1;
     ax_variant = 0x84;
-    return s.DH <= 32 ? fa_fwd<32>(q, k, v, o, lse, s, st) : fa_fwd<64>(q, k, v, o, lse, s, st);
+    return s.DH <= 32 ? fa_fwd<32>(q, k, v, o, lse, s, S, st) : fa_fwd<64>(q, k, v, o, lse, s, S, st);
 }
-int ax_attn_bwd_f32(const float* q, const float* k, const float* v, const float* dO, const float* lse, const float* Dv, float* dq, float* dk, float* dv,
-                    const AttnShape& s, cudaStream_t st) {
-    if (!fa_served(s, {q, k, v, dO, dq, dk, dv}) || !lse) return -1;
-    // long walks of a few key blocks: the blocks of 32 rows there are twice as many (B1 H4 KV1 T300 DH64 49 / 55 us)
-    const long long kv = (long long)((s.T + FB - 1) / FB) * s.KV * s.B;
-    if (kv * 8 <= AX_SMS / 2 && (long long)s.H / s.KV * ((s.T + FT - 1) / FT) >= 32) return -1;
-    ax_variant = 0x85;
-    return s.DH <= 32 ? fa_bwd<32>(q, k, v, dO, lse, Dv, dq, dk, dv, s, st) : fa_bwd<64>(q, k, v, dO, lse, Dv, dq, dk, dv, s, st);
+int ax_attn_dq_f32(const float* q, const float* k, const float* v, const float* dO, const float* lse, const float* Dv, float* dq, const AttnShape& s, cudaStream_t st) {
+    const int S = ax_attn_f32_ctas(FA_DQ, s);
+    if (!S || !lse || !fa_served(s, {q, k, v, dO, dq})) return -1;
+    return s.DH <= 32 ? fa_dq<32>(q, k, v, dO, lse, Dv, dq, s, S, st) : fa_dq<64>(q, k, v, dO, lse, Dv, dq, s, S, st);
+}
+int ax_attn_dkv_f32(const float* q, const float* k, const float* v, const float* dO, const float* lse, const float* Dv, float* dk, float* dv, const AttnShape& s, cudaStream_t st) {
+    const int S = ax_attn_f32_ctas(FA_DKV, s);
+    if (!S || !lse || !fa_served(s, {q, k, v, dO, dk, dv})) return -1;
+    return s.DH <= 32 ? fa_dkv<32>(q, k, v, dO, lse, Dv, dk, dv, s, S, st) : fa_dkv<64>(q, k, v, dO, lse, Dv, dk, dv, s, S, st);
 }

@@ -511,12 +511,13 @@ int ax_attn_fwd_simt(int dt, const void* q, const void* k, const void* v, void* 
         const int rc = ax_attn_fwd_f32((const float*)q, (const float*)k, (const float*)v, (float*)o, lse, s, st);
         if (rc >= 0) return rc;
     }
+    ax_variant = 0x86;
     const int vec = attn_vec(dt, s, {q, k, v});
     return dt == 1 ? attn_fwd_nj<bf16>(q, k, v, o, lse, s, vec, st) : attn_fwd_nj<float>(q, k, v, o, lse, s, vec, st);
 }
 
 template <typename T, typename TO, int NJ>
-static int attn_bwd_launch(const void* q, const void* k, const void* v, const void* dO, const float* lse,
+static int attn_bwd_launch(int part, const void* q, const void* k, const void* v, const void* dO, const float* lse,
                            const float* Dv, void* dq, void* dk, void* dv, const AttnShape& s, int vec, cudaStream_t st) {
     const size_t smem_q = attn_smem(ATTN_DQ, s.DH), smem_kv = attn_smem(ATTN_DKV, s.DH);
     const auto q_shared = k_attn_bwd_dq_simt<T, TO, NJ, true>, q_whole = k_attn_bwd_dq_simt<T, TO, NJ, false>;
@@ -524,32 +525,38 @@ static int attn_bwd_launch(const void* q, const void* k, const void* v, const vo
     const int Sq = ax_attn_simt_share(ATTN_DQ, s), Skv = ax_attn_simt_share(ATTN_DKV, s);
     if (!attn_smem_ok(smem_q, Sq > 1 ? q_shared : q_whole) || !attn_smem_ok(smem_kv, Skv > 1 ? kv_shared : kv_whole)) return 102;
     const dim3 g1((s.T + ABLK - 1) / ABLK, s.H, s.B), g2((s.T + ABLK - 1) / ABLK, s.KV, s.B);
-    const int rc = attn_launch(q_shared, q_whole, g1, smem_q, Sq, true, st, (const T*)q, (const T*)k, (const T*)v, (const T*)dO, lse, Dv, (TO*)dq, s, vec);
+    if (part == 0) return attn_launch(q_shared, q_whole, g1, smem_q, Sq, true, st, (const T*)q, (const T*)k, (const T*)v, (const T*)dO, lse, Dv, (TO*)dq, s, vec);
     // dK / dV comes early only as a quarter of a full GPU: the CTAs of its longest walks, the first, would be stacked on the SMs that dQ leaves first
     // (backward of B4 H8 KV4 T400 DH32 in us, in its turn / early: 130 / 159)
     const bool early = (long long)g2.x * g2.y * g2.z * Skv * 4 <= attn_slots(smem_kv);
-    return rc ? rc : attn_launch(kv_shared, kv_whole, g2, smem_kv, Skv, early, st, (const T*)q, (const T*)k, (const T*)v, (const T*)dO, lse, Dv, (TO*)dk, (TO*)dv, s, vec);
+    return attn_launch(kv_shared, kv_whole, g2, smem_kv, Skv, early, st, (const T*)q, (const T*)k, (const T*)v, (const T*)dO, lse, Dv, (TO*)dk, (TO*)dv, s, vec);
 }
 template <typename T, typename TO>
-static int attn_bwd_nj(const void* q, const void* k, const void* v, const void* dO, const float* lse,
+static int attn_bwd_nj(int part, const void* q, const void* k, const void* v, const void* dO, const float* lse,
                        const float* Dv, void* dq, void* dk, void* dv, const AttnShape& s, int vec, cudaStream_t st) {
-    if (s.DH <= 32) return attn_bwd_launch<T, TO, 1>(q, k, v, dO, lse, Dv, dq, dk, dv, s, vec, st);
-    if (s.DH <= 64) return attn_bwd_launch<T, TO, 2>(q, k, v, dO, lse, Dv, dq, dk, dv, s, vec, st);
-    if (s.DH <= 128) return attn_bwd_launch<T, TO, 4>(q, k, v, dO, lse, Dv, dq, dk, dv, s, vec, st);
-    return attn_bwd_launch<T, TO, 8>(q, k, v, dO, lse, Dv, dq, dk, dv, s, vec, st);
+    if (s.DH <= 32) return attn_bwd_launch<T, TO, 1>(part, q, k, v, dO, lse, Dv, dq, dk, dv, s, vec, st);
+    if (s.DH <= 64) return attn_bwd_launch<T, TO, 2>(part, q, k, v, dO, lse, Dv, dq, dk, dv, s, vec, st);
+    if (s.DH <= 128) return attn_bwd_launch<T, TO, 4>(part, q, k, v, dO, lse, Dv, dq, dk, dv, s, vec, st);
+    return attn_bwd_launch<T, TO, 8>(part, q, k, v, dO, lse, Dv, dq, dk, dv, s, vec, st);
 }
 int ax_attn_bwd_simt(int dt, int out_dt, const void* q, const void* k, const void* v, const void* dO,
                      const float* lse, const float* Dv, void* dq, void* dk, void* dv,
                      const AttnShape& s, cudaStream_t st) {
     if (s.DH > 256 || s.DH < 1 || s.KV < 1 || s.H % s.KV) return 102;
     if (s.B <= 0 || s.T <= 0) return 0;
-    if (dt == 0 && out_dt == 0) {
-        const int rc = ax_attn_bwd_f32((const float*)q, (const float*)k, (const float*)v, (const float*)dO, lse, Dv, (float*)dq, (float*)dk, (float*)dv, s, st);
-        if (rc >= 0) return rc;
-    }
+    if (dt == 0 && out_dt != 0) return 102;
     const int vec = attn_vec(dt, s, {q, k, v, dO});
-    if (dt == 1 && out_dt == 1) return attn_bwd_nj<bf16, bf16>(q, k, v, dO, lse, Dv, dq, dk, dv, s, vec, st);
-    if (dt == 1) return attn_bwd_nj<bf16, float>(q, k, v, dO, lse, Dv, dq, dk, dv, s, vec, st);
-    if (out_dt == 0) return attn_bwd_nj<float, float>(q, k, v, dO, lse, Dv, dq, dk, dv, s, vec, st);
-    return 102;
+    const bool f32 = dt == 0;
+    bool there = false;
+    for (int part = 0; part < 2; part++) {               // dQ, then dK / dV
+        int rc = !f32 ? -1 : part == 0 ? ax_attn_dq_f32((const float*)q, (const float*)k, (const float*)v, (const float*)dO, lse, Dv, (float*)dq, s, st)
+                                       : ax_attn_dkv_f32((const float*)q, (const float*)k, (const float*)v, (const float*)dO, lse, Dv, (float*)dk, (float*)dv, s, st);
+        there = there || rc >= 0;
+        if (rc < 0)
+            rc = f32 ? attn_bwd_nj<float, float>(part, q, k, v, dO, lse, Dv, dq, dk, dv, s, vec, st) : out_dt == 1 ? attn_bwd_nj<bf16, bf16>(part, q, k, v, dO, lse, Dv, dq, dk, dv, s, vec, st)
+                                                                                                          : attn_bwd_nj<bf16, float>(part, q, k, v, dO, lse, Dv, dq, dk, dv, s, vec, st);
+        if (rc) return rc;
+    }
+    ax_variant = there ? 0x85 : 0x87;
+    return 0;
 }

@@ -678,6 +678,9 @@ API int eng_attn_tile_parts(int B, int H, int KV, int T, int head_dim) {
     if (B < 1 || H < 1 || KV < 1 || T < 1) return 0;
     return ax_attn_tc_parts(shape_bthd(B, H, KV, T, head_dim, 1.f));
 }
+API int eng_attn_f32_ctas(int which, int B, int H, int KV, int T, int head_dim) {
+    return which < 0 || which > 2 || B < 1 || H < 1 || KV < 1 || T < 1 || head_dim < 1 ? 0 : ax_attn_f32_ctas(which, shape_bthd(B, H, KV, T, head_dim, 1.f));
+}
 API int eng_attn_share(int which, int B, int H, int KV, int T, int head_dim) {
     if (which < 0 || which > 2 || B < 1 || H < 1 || KV < 1 || H % KV || T < 1 || head_dim < 1 || head_dim > 256) return 0;
     return ax_attn_simt_share(which, shape_bthd(B, H, KV, T, head_dim, 1.f));

@@ -16,7 +16,7 @@
 //   0x25 / 0x28 SwiGLU inside a projection pair with adapters on the same two,
 //   0x70 embedding scatter by scanning the ids, 0x71 by occurrence lists, 0x72 scale and add as one pass, 0x73 with the norm,
 //   0x80 / 0x81 attention forward / backward with split probabilities on tcgen05, 0x82 / 0x83 on mma.sync (0x83 + 0x100 * CTAs to a key tile),
-//   0x84 / 0x85 attention forward / backward in fp32 with head dims 12 to 64 (attn_f32.cu)
+//   0x84 / 0x85 attention forward / backward (dQ, dK / dV or both) in fp32 with head dims 12 to 64 (attn_f32.cu), 0x86 / 0x87 on the general kernels (attn_simt.cu)
 extern int ax_variant;
 extern int ax_gemm_parts;     // see eng_last_gemm_parts
 extern int ax_gemm_width;     // see eng_last_gemm_width
@@ -121,9 +121,10 @@ struct AttnShape {
 };
 // attn_f32.cu — exact fp32 attention of head dims 12 to 64; -1 = not served
 int ax_attn_f32_init(void);
+int ax_attn_f32_ctas(int which, const AttnShape& s);      // see eng_attn_f32_ctas
 int ax_attn_fwd_f32(const float* q, const float* k, const float* v, float* o, float* lse, const AttnShape& s, cudaStream_t st);
-int ax_attn_bwd_f32(const float* q, const float* k, const float* v, const float* dO, const float* lse, const float* Dv, float* dq, float* dk, float* dv,
-                    const AttnShape& s, cudaStream_t st);
+int ax_attn_dq_f32(const float* q, const float* k, const float* v, const float* dO, const float* lse, const float* Dv, float* dq, const AttnShape& s, cudaStream_t st);
+int ax_attn_dkv_f32(const float* q, const float* k, const float* v, const float* dO, const float* lse, const float* Dv, float* dk, float* dv, const AttnShape& s, cudaStream_t st);
 int ax_attn_fwd_simt(int dt, const void* q, const void* k, const void* v, void* o, float* lse,
                      const AttnShape& s, cudaStream_t st);
 // out_dt: storage type of dq/dk/dv (0 fp32, 1 bf16)

@@ -165,7 +165,7 @@ long long eng_bytes_allocated(void);
 /* Code of the kernel variant the last GEMM / cross-entropy op ran on (no counterpart in the reference; lets a
  * test assert that a shape was served by the kernel it means to check): 0x10 cross-entropy streaming rows,
  * 0x11 register-resident rows; 0x80 / 0x81 attention forward / backward with split probabilities on tcgen05, 0x82 / 0x83 on mma.sync
- * (the backward plus 0x100 times the CTAs that share a key tile), 0x84 / 0x85 in fp32 at head dims 12 to 64; 0x20 general GEMM, 0x21 single-CTA
+ * (the backward plus 0x100 times the CTAs that share a key tile), 0x84 / 0x85 on the fp32 kernels of head dims 12 to 64 (0x85: dQ, dK / dV or both), 0x86 / 0x87 on the general ones; 0x20 general GEMM, 0x21 single-CTA
  * tcgen05 GEMM, 0x22 paired-CTA tcgen05 GEMM, 0x23 a group of them, 0x26 small products, 0x24 / 0x27 / 0x2a the SwiGLU backward
  * inside a small / paired-CTA / fp32 product, 0x25 / 0x28 the SwiGLU inside a pair with adapters on the first two, 0x29 a group
  * of fp32 products as one launch, the GEMM codes plus 0x100 times the split-K factor; 0x60 / 0x62 the adapters' gradients / skinny products. */
@@ -182,12 +182,14 @@ int eng_gemm_f32_cut(int tb, int m, int n, int k, int batch, int aligned);
  * kernels with split probabilities once the whole-tile kernels have refused it (for the backward the number of CTAs that share a key tile,
  * 1, 2 or 4) or not (0): host arithmetic that needs no GPU. */
 int eng_attn_route(int backward, int B, int H, int KV, int T, int head_dim);
-/* Dynamic shared memory in bytes of the general attention kernels (those of the general head dims; the fp32 kernels of head dims 12 to 64
- * are others), 0 forward, 1 dQ, 2 dK / dV, for a head dim of 1 to 256
+/* Dynamic shared memory in bytes of the general attention kernels, which fp32 shapes with eng_attn_f32_ctas above 0 reach only from unaligned buffers, 0 forward, 1 dQ, 2 dK / dV, for a head dim of 1 to 256
  * (else -1): host arithmetic that needs no GPU. */
 long long eng_attn_smem(int which, int head_dim);
 /* CTAs that share a block's walk in those kernels (1: none do; 0: not a shape): host arithmetic, too. */
 int eng_attn_share(int which, int B, int H, int KV, int T, int head_dim);
+/* CTAs that share a block's walk in the fp32 kernels of head dims 12 to 64 (attn_f32.cu; which: 0 forward, 1 dQ, 2 dK / dV), or 0: the general kernels serve the shape.  They also serve
+ * what these can't, rows that are no whole 16-byte pieces.  Host arithmetic, too. */
+int eng_attn_f32_ctas(int which, int B, int H, int KV, int T, int head_dim);
 /* CTAs that share a key tile of the whole-tile tcgen05 attention backward (head_dim 64 or 128, T a multiple of 128): 1, 2 or 4; 0 = not such a shape. */
 int eng_attn_tile_parts(int B, int H, int KV, int T, int head_dim);
 /* How a launch of the adapters' skinny products is cut (`count` of N tokens and rank R, the narrowest with F columns, one_x: all of one input): products in a CTA * 65536 +

@@ -174,6 +174,19 @@ def test_ctas_to_a_walk_of_the_general_attention(lib, B, H, KV, T, DH, parts):
     assert tuple(lib.eng_attn_share(w, B, H, KV, T, DH) for w in range(3)) == parts
 
 
+@pytest.mark.parametrize("B,H,KV,T,DH,ctas", [
+    (2, 8, 4, 256, 32, (4, 4, 8)), (2, 16, 16, 333, 64, (4, 4, 4)), (40, 8, 2, 100, 48, (1, 1, 4)), (2, 8, 8, 130, 64, (4, 4, 4)),
+    # one tile: nothing to share, and half of a block's rows empty
+    (11, 1, 1, 13, 12, (1, 1, 0)), (3, 8, 8, 26, 12, (1, 1, 0)), (4, 1, 1, 27, 64, (1, 0, 0)), (240, 16, 4, 10, 48, (0, 0, 0)), (33, 12, 12, 17, 32, (0, 1, 1)), (1, 2, 1, 3, 64, (1, 0, 2)),
+    # few blocks with long walks
+    (1, 3, 1, 976, 16, (4, 0, 0)), (1, 8, 2, 928, 64, (4, 4, 0)), (6, 2, 1, 192, 12, (4, 4, 0)), (5, 1, 1, 73, 32, (4, 4, 4)),
+    # not for these kernels
+    (2, 8, 4, 256, 8, (0, 0, 0)), (2, 8, 4, 256, 34, (0, 0, 0)), (2, 8, 4, 256, 68, (0, 0, 0)), (2, 8, 3, 256, 64, (0, 0, 0)), (0, 8, 4, 256, 64, (0, 0, 0))])
+def test_fp32_attention_goes_where_it_is_faster(lib, B, H, KV, T, DH, ctas):
+    assert tuple(lib.eng_attn_f32_ctas(w, B, H, KV, T, DH) for w in range(3)) == ctas
+    assert lib.eng_attn_f32_ctas(3, B, H, KV, T, DH) == 0
+
+
 def test_cluster_barriers_are_met_by_converged_warps():
     """The aligned forms of the cluster barrier stand in one helper only, behind a __syncwarp(): lanes may come to them from a branch."""
     csrc = os.path.join(ROOT, "axis_b200", "csrc")

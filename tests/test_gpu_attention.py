@@ -2,6 +2,8 @@
 reference layout ops (FLASH / ROWDOT / FLASH_BWD on [B,H,T,DH], fp32 outputs)
 and the fused ops on [B,T,H,DH]; fp32 and bf16; head_dim 16..128; ragged T;
 MHA / GQA / MQA; determinism."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -282,8 +284,8 @@ def test_attention_of_other_shapes_keeps_fp32_probabilities(eng, B, H, KV, T, DH
 @pytest.mark.parametrize("B,H,KV,T,DH", [(2, 8, 4, 256, 32), (1, 2, 1, 225, 8), (1, 4, 2, 97, 40), (1, 3, 3, 130, 128), (1, 2, 1, 64, 256), (16, 8, 8, 65, 64),
                                              (1, 4, 1, 33, 1), (2, 2, 2, 40, 2), (1, 8, 4, 150, 4), (1, 8, 1, 96, 256)])
 def test_fp32_attention_over_clusters(eng, B, H, KV, T, DH):
-    """Few rows: clusters of two to eight CTAs share a block's tiles, some of them without one (the last case has none: it fills the
-    SMs).  Sums of T products of N(0,1) numbers in fp32 in any order err by less than 2^-24 sqrt(T) a term: 2e-5 of the largest
+    """Few rows: clusters of two to eight CTAs share a block's tiles, some of them without one ((16, 8, 8, 65, 64) fills the SMs).  Head dims of 32, 40 and 64 run on attn_f32.cu
+    here, on the general kernels in the test below.  Sums of T products of N(0,1) numbers in fp32 in any order err by less than 2^-24 sqrt(T) a term: 2e-5 of the largest
     result, as for one CTA; a second run gives the same bits."""
     rng = np.random.default_rng(T + DH)
     q, k, v, do = make(rng, B, H, KV, T, DH, 0)
@@ -304,6 +306,63 @@ def test_fp32_attention_over_clusters(eng, B, H, KV, T, DH):
         assert np.abs(runs[0][n] - ref).max() <= 2e-5 * np.abs(ref).max(), n
     assert np.abs(lse - O.attention_fwd(q, k, v, scale)[1]).max() <= 2e-5
     assert eng.device_status() == 0
+
+
+@pytest.mark.parametrize("B,H,KV,T,DH,off", [
+    (2, 8, 4, 256, 32, 1), (1, 4, 2, 97, 40, 1), (16, 8, 8, 65, 64, 1), (1, 4, 1, 300, 64, 1), (3, 6, 2, 70, 12, 1),       # head dims of attn_f32.cu from buffers that it does not take
+    (1, 4, 2, 150, 63, 0), (24, 8, 8, 65, 50, 0), (2, 8, 4, 120, 34, 0), (20, 16, 16, 64, 72, 0)])                         # head dims of none of it
+def test_fp32_attention_on_the_general_kernels(eng, B, H, KV, T, DH, off):
+    """Shared walks and blocks of their own ((16, 8, 8, 65, 64), (24, 8, 8, 65, 50) and the last fill the SMs) by the variant that ran, bounds as in the test above."""
+    rng = np.random.default_rng(T + DH)
+    q, k, v, do = make(rng, B, H, KV, T, DH, 0)
+    scale = 1.0 / np.sqrt(DH)
+
+    def placed(size, arr=None):                          # a buffer that starts `off` floats into its allocation
+        i = eng.view(eng.alloc(size + off), 4 * off, 4 * size)
+        if arr is not None:
+            eng.upload(i, np.ascontiguousarray(arr.transpose(0, 2, 1, 3)))
+        return i
+    iq, ik, iv, ido = (placed(x.size, x) for x in (q, k, v, do))
+    out = {n: (placed(a.size), a.shape[1]) for n, a in (("o", q), ("dq", q), ("dk", k), ("dv", k))}
+    ilse, iD = eng.alloc(B * H * T), eng.alloc(B * H * T)
+    runs = []
+    for _ in range(2):
+        eng.run([op(E.ATTN_FWD, a=iq, b=ik, d=iv, c=out["o"][0], sa=ilse, m=T, n=DH, k=KV, batch=B, tb=H, dt=0, alpha=scale)])
+        assert eng.last_variant() == 0x86
+        eng.run([op(E.ATTN_BWD, a=iq, b=ik, d=iv, c=ido, sa=ilse, sb=out["o"][0], tb=out["dq"][0], sc=out["dk"][0], oa=out["dv"][0], ob=H, oc=iD, m=T, n=DH, k=KV,
+                    batch=B, dt=0, alpha=scale)])
+        assert eng.last_variant() == 0x87
+        runs.append({n: eng.download(i, (B, T, heads, DH)).transpose(0, 2, 1, 3) for n, (i, heads) in out.items()})
+    for n, ref in attention_f64(q, k, v, do, scale).items():
+        assert np.array_equal(runs[0][n], runs[1][n]), n
+        assert np.abs(runs[0][n] - ref).max() <= 2e-5 * np.abs(ref).max(), n
+    assert np.abs(eng.download(ilse, (B, H, T)) - O.attention_fwd(q, k, v, scale)[1]).max() <= 2e-5
+    assert eng.device_status() == 0
+
+
+@pytest.mark.parametrize("B,H,KV,T,DH", [(3, 8, 8, 26, 12), (4, 1, 1, 27, 64), (2, 12, 12, 71, 12), (6, 3, 1, 12, 40)])
+def test_short_fp32_attention_takes_no_longer_than_on_the_general_kernels(eng, B, H, KV, T, DH):
+    """Backward from aligned buffers against the general kernels (from buffers that start one float later).  us on one B200, aligned and there / here whatever the shape / now: 8.9 / 20.2 / 8.9,
+    13.7 / 29.4 / 13.7, 17.7 / 25.6 / 17.5, 18.4 / 25.6 / 14.7."""
+    rng = np.random.default_rng(T)
+    q, k, v, do = make(rng, B, H, KV, T, DH, 0)
+    times = []
+    for off in (0, 1):
+        placed = lambda x: eng.view(eng.alloc(x.size + off), 4 * off, 4 * x.size)
+        ins = [placed(x) for x in (q, k, v, do)]
+        for i, x in zip(ins, (q, k, v, do)):
+            eng.upload(i, np.ascontiguousarray(x.transpose(0, 2, 1, 3)))
+        io, idq, idk, idv, ilse, iD = placed(q), placed(q), placed(k), placed(k), eng.alloc(B * H * T), eng.alloc(B * H * T)
+        eng.run([op(E.ATTN_FWD, a=ins[0], b=ins[1], d=ins[2], c=io, sa=ilse, m=T, n=DH, k=KV, batch=B, tb=H, dt=0, alpha=DH ** -0.5)])
+        plan = [op(E.ATTN_BWD, a=ins[0], b=ins[1], d=ins[2], c=ins[3], sa=ilse, sb=io, tb=idq, sc=idk, oa=idv, ob=H, oc=iD, m=T, n=DH, k=KV, batch=B, dt=0, alpha=DH ** -0.5)] * 20
+        eng.capture(plan)
+        ms = ctypes.c_float(0)
+        runs = []
+        for _ in range(6):
+            assert eng.lib.eng_time_replay(5, ctypes.byref(ms)) == 0
+            runs.append(ms.value)
+        times.append(min(runs))
+    assert times[0] <= 1.1 * times[1], times
 
 
 @pytest.mark.parametrize("B,H,KV,T,DH,gain", [
