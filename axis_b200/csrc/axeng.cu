@@ -988,7 +988,7 @@ static int exec_op(const EngOp* op) {
                 int rc = ax_attn_bwd_tc(BUFP(op->a), BUFP(op->b), BUFP(op->d), BUFP(op->sb), BUFP(op->c), (const float*)BUFP(op->sa),
                                         (float*)BUFP(op->oc), dq_acc, BUFP(op->tb), BUFP(op->sc), BUFP(op->oa), s, rc_, rs_, G.d_status, st);
                 if (rc == 0) { rotated = rc_ != nullptr; done = 1; }
-                else if (rc < 0 && rc_) {        // served without the fused rotary (head_dim 128)?
+                else if (rc < 0 && rc_) {        // tables that don't start on 16 bytes leave the rotary to an op of its own
                     rc = ax_attn_bwd_tc(BUFP(op->a), BUFP(op->b), BUFP(op->d), BUFP(op->sb), BUFP(op->c), (const float*)BUFP(op->sa),
                                         (float*)BUFP(op->oc), dq_acc, BUFP(op->tb), BUFP(op->sc), BUFP(op->oa), s, nullptr, nullptr, G.d_status, st);
                     if (rc == 0) done = 1;
@@ -1123,8 +1123,8 @@ static int exec_op(const EngOp* op) {
 //   GEMM_GROUP mode 1 of two outputs with a low-rank term each, then SILU_MUL of the two: the group runs as mode 4.
 //   SCALE of g in place (oa = 1: only the next op reads the result), then ADD of it: c = a + alpha * g in one pass; GNORM_FLAT of c behind them
 //   joins it.
-// The products are served by the paired-CTA kernel from 256 rows and columns (one tile) on: below, and in every form that it refuses, the ops
-// run one by one.  Returns 0 (done up to *last), -1 (nothing done) or an error.
+// bf16 products are served by the paired-CTA or the small-product kernel from 256 rows and columns on, fp32 ones (the first form only) at any size; below, and in every
+// form that they refuse, the ops run one by one.  Returns 0 (done up to *last), -1 (nothing done) or an error.
 static int run_fused(const EngOp* ops, int n_ops, int i, int* last) {
     const EngOp* op = &ops[i];
     if (op->kind == ENG_SCALE) {

@@ -238,7 +238,8 @@ static int g_pairs_avail = 0;      // co-resident CTA pairs of the paired kernel
 static int g_side = 0;
 static bool g_beside = false;
 void ax_gemm_side(int on) { g_side = on; g_beside = g_beside || on; }
-// A plan that has queued products on the side stream has them running beside the main chain from then on (until the next plan starts)
+// A plan that has switched to another stream, for products beside the main chain or for collectives, is taken to have work beside the chain from then on, until the next plan
+// starts: the width of a product's tiles, and with it whether its depth is shared and the last bits of its sums, depends on what its plan queued before it.
 void ax_gemm_plan_begin(void) { g_side = 0; g_beside = false; }
 bool ax_gemm_beside(void) { return g_beside; }
 int ax_gemm_pdl(void) {

@@ -1,6 +1,6 @@
 // bf16 GEMM with paired CTAs (tcgen05 cta_group::2): a cluster of two CTAs on
-// neighbouring SMs computes one output tile of 256 x 256 (or, by a rule at
-// ax_gemm_width, 192 or 128 columns).  Each CTA loads its own 128 rows of A and
+// neighbouring SMs computes one output tile of 256 x 256 (or, by the rule at
+// ax_gemm_tc2_width, 192 or 128 columns).  Each CTA loads its own 128 rows of A and
 // its own half of the columns of B (plain TMA tile loads — nothing is
 // multicast; the pair shares B through the MMA unit, which reads both CTAs'
 // shared memory), so a k-block costs 32 KB of L2->smem traffic per SM instead of
@@ -306,7 +306,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
     if (timing && threadIdx.x == 0) prof[2] = clock64();
 
     if (warp == 0) {
-        // ── TMA producer (both CTAs): own 128 rows of A, own 128 columns of B.  The whole warp runs the loop, one elected lane issues ──
+        // ── TMA producer (both CTAs): own 128 rows of A, own half of the tile's columns of B.  The whole warp runs the loop, one elected lane issues ──
         // This loop was the bound: as one thread of a divergent warp that chose its maps anew for each k-block it took 418 cycles and 61 for each
         // TMA instruction, 540 / 607 / 663 a k-block of 256 x 256 x 64 with both operands K-major / one / none (one pair alone, K 8192), where
         // the MMAs need 512.  Converged, with the choice made once for a run of k-blocks and one instruction for each operand, all three take 512 (that

@@ -1173,6 +1173,45 @@ def test_wide_tiles_where_the_epilogue_is_the_round(eng, m, n, k, tb, dt, width,
     assert eng.device_status() == 0
 
 
+@pytest.mark.parametrize("dt", [1, 2])
+@pytest.mark.parametrize("m,n,k,width", [(2000, 1501, 640, 192), (2000, 1411, 712, 192), (1304, 777, 1000, 128), (1288, 642, 1000, 128)])
+def test_narrow_tiles_whose_rows_are_no_whole_pieces(eng, dt, m, n, k, width):
+    """A B^T with any n: the threads of the epilogue store (and read the addend), the last tile holding 157, 67, 9 and 2 columns."""
+    for kw in (dict(alpha=0.5), dict(beta=-2.0, addend=True)):
+        got, ref = run_gemm(eng, np.random.default_rng(m + n), m, n, k, 1, dt, **kw)
+        assert (eng.last_variant(), eng.last_gemm_parts(), eng.last_gemm_width()) == (0x122, 1, width)
+        check(got, ref, dt == 1, k)
+    assert eng.device_status() == 0
+
+
+def test_tall_groups_walk_their_tiles_in_bands(eng):
+    """A above 52 MB as in `test_tall_products_walk_their_tiles_in_bands`, in groups: several outputs of one input, a sum whose segments are above it together, a SwiGLU pair."""
+    rng = np.random.default_rng(52)
+    mk = lambda *sh: bf(rng.standard_normal(sh, dtype=np.float32))
+    m, k, ns = 3336, 7816, (264, 136, 72)
+    assert 2 * m * k > 52000000
+    x, ws = mk(m, k), [mk(k, n) for n in ns]
+    ix, iw, ic = put(eng, x, 1), [put(eng, w, 1) for w in ws], [eng.alloc(m * n, 2) for n in ns]
+    eng.run([op(E.GEMM_GROUP, a=ix, b=iw[0], sa=iw[1], sb=iw[2], c=ic[0], d=ic[1], sc=ic[2], m=m, k=k, n=ns[0], oa=ns[1], ob=ns[2], batch=3, oc=1, tb=0, dt=1)])
+    assert eng.last_variant() == 0x23
+    for n, w, c in zip(ns, ws, ic):
+        check(eng.download_bf16(c, (m, n)), x @ w, True, k)
+    g, u = x @ ws[0], x @ (wu := mk(k, ns[0]))
+    og, ou, oh = (eng.alloc(m * ns[0], 2) for _ in range(3))
+    eng.run([op(E.GEMM_GROUP, a=ix, b=iw[0], sa=put(eng, wu, 1), c=og, d=ou, sc=oh, m=m, n=ns[0], k=k, batch=2, oc=4, dt=1)])
+    assert eng.last_variant() == 0x23
+    for o, ref in ((og, g), (ou, u), (oh, g / (1 + np.exp(-np.clip(g, -80, None))) * u)):
+        check(eng.download_bf16(o, (m, ns[0])), ref, True, k)
+    ks, n = (3904, 2600, 1352), 520
+    assert 2 * m * sum(ks) > 52000000
+    a, b = [mk(m, q) for q in ks], [mk(n, q) for q in ks]
+    ia, ib, io = [put(eng, v, 1) for v in a], [put(eng, v, 1) for v in b], eng.alloc(m * n, 2)
+    eng.run([op(E.GEMM_GROUP, c=io, a=ia[0], sa=ia[1], sb=ia[2], b=ib[0], d=ib[1], sc=ib[2], m=m, n=n, k=ks[0], oa=ks[1], ob=ks[2], batch=3, oc=2, tb=1, dt=1)])
+    assert eng.last_variant() == 0x23
+    check(eng.download_bf16(io, (m, n)), sum(p @ q.T for p, q in zip(a, b)), True, sum(ks))
+    assert eng.device_status() == 0
+
+
 @pytest.mark.parametrize("r", [0, 16])
 @pytest.mark.parametrize("m,k,ns,width", [(3000, 640, (768, 192, 192), 192), (2904, 264, (704, 192, 128), 192), (1800, 72, (576, 64, 72), 128)])
 def test_narrow_tiles_of_groups_have_the_bits_of_wide_ones(eng, m, k, ns, width, r):
@@ -1208,7 +1247,7 @@ def test_narrow_tiles_of_groups_have_the_bits_of_wide_ones(eng, m, k, ns, width,
 
 
 def test_narrow_tiles_only_while_nothing_runs_beside_the_chain(eng):
-    """Products on the side stream take the pairs that wide tiles leave idle: behind the first of them in a plan the tiles are wide, and a new plan starts over."""
+    """Products on the side stream take the pairs that wide tiles leave idle: behind the first switch of a plan to another stream the tiles are wide, and a new plan starts over."""
     rng = np.random.default_rng(3)
     mk = lambda *sh: put(eng, bf(rng.standard_normal(sh).astype(np.float32)), 1)
     m, n, k = 2000, 1504, 640
