@@ -837,6 +837,8 @@ static int band_of(int m, long long k) {
 // 256 (33, 45, 66) 6.5 / 6.2 / 6.2.  Over 232 shapes the rule is 0.4 % behind the best of the three on average.
 // Only while a plan has queued nothing to another stream (see ax_gemm_plan_begin): products on the side stream fill the pairs that wide tiles leave, and
 // the step of 8 x 1024 tokens at D 768 takes 5114 us with narrow ones throughout, 5037 without.  Steps with adapters are 1 to 2 % shorter, small ones up to 5.
+// A shared or split depth stays one where the output is fp32, which narrow tiles would sum in one chain: the tensor core's accumulator loses with each step.  2-norm errors against float64 of
+// fp32 outputs, shared by two or four / in one chain: 1040 x 720 x 2016 4.7e-7 / 2.1e-6, 2440 x 696 x 1880 9.1e-7 / 1.9e-6, 2248 x 584 x 3496 1.8e-6 / 3.7e-6; rounded to bf16 all are 1.7e-3.
 // With three rounds or more the rounds even out and the wide tile, which moves the least, is the best under the power limit: 8192 x 1536 x 2560 (192, 256, 384)
 // 48.6 / 49.5 / 58.4.
 static int g_pairs = 0;                  // pairs that run at once
@@ -1106,7 +1108,7 @@ int ax_gemm_tc2_group(int out_bf16, int tb, int mode, int count, const void* con
         for (int g = 0; g < (mode == 2 ? count : 1); g++) kb += (k[g] + BK2 - 1) / BK2;
         for (int i = 0; i < 3; i++)
             for (int g = 0; g < (mode == 1 ? count : 1); g++) tiles[i] += (long long)((m[0] + 255) / 256) * ((n[g] + 255 - 64 * i) / (256 - 64 * i));
-        bn = ax_gemm_tc2_width(tiles, kb, !swb, true).width;
+        if (out_bf16 || ax_gemm_tc2_share((int)(tiles[0] < AX_SMS ? tiles[0] : AX_SMS), kb, nullptr) == 1) bn = ax_gemm_tc2_width(tiles, kb, !swb, true).width;
     }
     ax_gemm_width = mode == 4 ? 256 : bn;
 #define G2W(AM, BMj, T, EPI, W) gemm2_launch<AM, BMj, T, EPI, W>(mode, count, A, B, C, D, m, n, k, alpha, D ? beta : 0.f, status, 1, st, XA, XB, xk, swb)

@@ -1173,6 +1173,31 @@ def test_wide_tiles_where_the_epilogue_is_the_round(eng, m, n, k, tb, dt, width,
     assert eng.device_status() == 0
 
 
+@pytest.mark.parametrize("m,n,k,tb,parts", [(1040, 720, 2016, 0, 4), (1040, 720, 2016, 2, 4), (2440, 696, 1880, 1, 2), (2248, 584, 3496, 2, 2)])
+def test_fp32_outputs_keep_the_partial_sums_of_a_shared_depth(eng, m, n, k, tb, parts):
+    """The tensor core's accumulator loses with each step, so that one chain over the depth errs by as many times more as there are parts (2.1 and 4.4 times on one B200).  The default
+    route against the forced paired kernel, which shares these depths; a bound of 1.5 lies between no part lost and two made one.  Alone, and as a group of two outputs."""
+    rng = np.random.default_rng(m + k)
+    a, b = bf(rng.standard_normal((k, m) if tb == 2 else (m, k), dtype=np.float32)), bf(rng.standard_normal((n, k) if tb == 1 else (k, n), dtype=np.float32))
+    ref = (a.T if tb == 2 else a).astype(np.float64) @ (b.T if tb == 1 else b)
+    ia, ib, ic, idd = put(eng, a, 1), put(eng, b, 1), eng.alloc(m * n), eng.alloc(m * n)
+    alone = [op(E.GEMM_SB, a=ia, b=ib, c=ic, m=m, n=n, k=k, batch=1, tb=tb, dt=2)]
+    half = 256                                           # the group: columns of the same product, in as many tiles
+    hb = [np.ascontiguousarray(v) for v in ((b[:half], b[half:]) if tb == 1 else (b[:, :half], b[:, half:]))]
+    ih = [put(eng, v, 1) for v in hb]
+    group = [op(E.GEMM_GROUP, a=ia, b=ih[0], sa=ih[1], c=ic, d=idd, m=m, k=k, n=half, oa=n - half, batch=2, oc=1, tb=tb, dt=2)]
+    for plan in (alone, group):
+        errs = []
+        for mask in (0, 8):
+            eng.set_fallback(mask)
+            eng.run(plan)
+            eng.set_fallback(0)
+            errs.append(np.linalg.norm(eng.download(ic, (m, n) if plan is alone else (m, half)) - (ref if plan is alone else ref[:, :half])))
+            assert (eng.last_gemm_width(), eng.last_gemm_parts()) == (256, parts)
+        assert errs[0] <= 1.5 * errs[1], errs
+    assert eng.device_status() == 0
+
+
 @pytest.mark.parametrize("dt", [1, 2])
 @pytest.mark.parametrize("m,n,k,width", [(2000, 1501, 640, 192), (2000, 1411, 712, 192), (1304, 777, 1000, 128), (1288, 642, 1000, 128)])
 def test_narrow_tiles_whose_rows_are_no_whole_pieces(eng, dt, m, n, k, width):
