@@ -362,11 +362,19 @@ struct F32Cut { int rows, cols, sums, ctas; };
 static F32Cut f32_cut(int tb, bool plain, long long t128, long long t64, long long t64x32, long long t32, int steps, long long depth, bool vec) {
     // A 128 x 128 tile has the most FMAs per shared-memory read, but fewer than 148 of them leave SMs without work, and so does a last round that is mostly empty (one CTA
     // to an SM; us there / with 64 x 64 tiles: 171 tiles, 1072 x 2360 x 944 238 / 160, 189 tiles, 2688 x 1152 x 376 85 / 71; 210 tiles, 1760 x 1848 x 112 28.2 / 28.7).
-    if (t128 >= AX_SMS && 10 * t128 >= 7 * AX_SMS * ((t128 + AX_SMS - 1) / AX_SMS)) return {128, 128, 8, 1};
+    // Rows that are no whole 16-byte pieces are copied by 4 bytes, once for each tile that reads them, which is all there is to a product of one step (2111 x 2267 x 12 16.9 / 22.6) and counts
+    // most where both operands have short rows (A B^T: 1032 x 2085 x 13 11.5 / 16.4, 1675 x 1370 x 33 22.6 / 28.7, 2426 x 975 x 103 44.9 / 48.5, 1679 x 1771 x 237 87 / 94; but 1235 x 2108 x 701 234 / 219).
+    if (t128 >= AX_SMS && (10 * t128 >= 7 * AX_SMS * ((t128 + AX_SMS - 1) / AX_SMS) || (!vec && depth <= (tb == 1 ? 256 : 20)))) return {128, 128, 8, 1};
     // Shallow products of many tiles are set-up, one load and the stores: 64 x 64 tiles of 4 x 4 sums with 32-deep steps, which leave an SM room for more CTAs.  us there / with 64 x 64
     // tiles of 8 x 8 sums or 32 x 32: 2232 x 368 x 24 4.8 / 6.9, 680 x 2792 x 32 7.9 / 10.0, 1184 x 960 x 24 5.8 / 9.2, 1968 x 912 x 16 8.2 / 10.7; A B^T 1992 x 1072 x 136 25.8 / 31.5,
     // 1552 x 1176 x 104 21.2 / 25.5; but 1008 x 656 x 40 7.2 / 6.3.
     if (plain && t64 >= AX_SMS && (depth <= 32 || (tb == 1 && steps <= 3 && t64 >= 2 * AX_SMS))) return {64, 64, 4, 1};
+    // By 4-byte copies the 8 x 8 sums wait for their operands, 8 x 8 / 4 x 4: A B 1547 x 664 x 34 13.0 / 9.0, 1549 x 1025 x 73 26.9 / 18.6, 1453 x 1051 x 173 44.7 / 32.0; A B^T of 296 to 443 tiles
+    // 1.07 / 0.96 of the time with 4 x 4 sums and no second depth group, of more 0.87 / 0.96; A^T B of 222 to 443 0.77 / 0.96, of more, 1455 x 1377 x 37, 15.2 / 14.8, 1146 x 1651 x 112 33.0 / 25.8.
+    if (plain && !vec && (tb == 0 ? 2 * t64 >= 3 * AX_SMS : tb == 1 ? t64 >= 2 * AX_SMS && t64 < 3 * AX_SMS : t64 >= 3 * AX_SMS)) return {64, 64, 4, 1};
+    // With 4 x 4 sums four CTAs fit an SM, with 8 x 8 two, whose second round of 1.5 to 2 then takes longer than all at once while the depth is short, 8 x 8 / 4 x 4: A^T B 1740 x 1188 x 76 19.0 / 15.1,
+    // 2612 x 864 x 148 28.0 / 23.1, A B 2228 x 1012 x 140 27.5 / 24.4, A B^T 2636 x 856 x 328 61.7 / 50.7; but A^T B 2044 x 1004 x 764 93 / 97, and 364 tiles 12.2 / 14.9.
+    if (plain && vec && t64 >= 3 * AX_SMS && t64 <= 4 * AX_SMS && steps <= 5) return {64, 64, 4, 1};
     if (t64 >= 2 * AX_SMS) return {64, 64, 8, 1};
     // Below, a launch is the latency of its steps: 64 x 32 tiles (8 x 4 sums to a thread, 43 % of the FMA pipe with two CTAs on an SM, which is what
     // fits) with the depth cut over a cluster as far as two CTAs for each SM.  Where that leaves a third of the SMs idle or most with one CTA and some with two,
@@ -379,11 +387,13 @@ static F32Cut f32_cut(int tb, bool plain, long long t128, long long t64, long lo
     int ks = 1, ks32 = 1;
     while (ks < 8 && t64x32 * ks * 2 <= 2 * AX_SMS && steps >= 2 * ks) ks *= 2;
     while (ks32 < 8 && t32 * ks32 * 2 <= AX_SMS * 5 / 2 && steps >= 4 * ks32) ks32 *= 2;
+    // 70 clusters of four and 32 of eight run at once, a further one is a second round: 533 x 228 x 841, 72 of four, 27.7 us, 19.6 on 32 x 32; 220 x 258 x 958, 36 of eight, 18.1 and 13.1.
     const long long ctas = t64x32 * ks;
-    if (steps > 2 && 3 * ctas > 2 * AX_SMS && ctas <= 2 * AX_SMS && (ctas <= AX_SMS || 2 * ctas > 3 * AX_SMS) && 40 * t64x32 <= (ks > ks32 ? 28 : 23) * t32 &&
+    const bool fit = ks < 4 || t64x32 <= (ks == 4 ? 70 : 32);
+    if (fit && steps > 2 && 3 * ctas > 2 * AX_SMS && ctas <= 2 * AX_SMS && (ctas <= AX_SMS || 2 * ctas > 3 * AX_SMS) && 40 * t64x32 <= (ks > ks32 ? 28 : 23) * t32 &&
         (steps + ks - 1) / ks * ks * 100 <= steps * 127 && (vec || ks == 1 || tb)) return {64, 32, 8, ks};
-    // 4-byte copies count for each CTA that reads a tile of an operand: 64 x 64 tiles from one for each SM on (1964 x 456 x 3179 296 | 385 us, 2196 x 412 x 402 41 | 58, 270 x 2271 x 220 25.0 | 28.2).
-    if (plain && !vec && tb != 2 && depth > 64 && t64 >= AX_SMS) return {64, 64, 4, 1};
+    // 4-byte copies count for each CTA that reads a tile of an operand: 64 x 64 tiles from one for each SM on (1964 x 456 x 3179 296 | 385 us, 2196 x 412 x 402 41 | 58, 270 x 2271 x 220 25.0 | 28.2, 1115 x 687 x 51 9.4 | 11.0).
+    if (plain && !vec && tb != 2 && (depth > 64 || tb == 0) && t64 >= AX_SMS) return {64, 64, 4, 1};
     return {32, 32, 4, ks32};
 }
 static int cut_code(const F32Cut& c) { return c.rows << 20 | c.cols << 8 | c.sums << 4 | c.ctas; }

@@ -148,9 +148,14 @@ def test_cut_of_the_adapters_products(lib, count, one_x, N, F, R, members, token
     (1, 704, 192, 176, 1, 1, (32, 32, 4, 1)), (1, 144, 2488, 184, 1, 1, (32, 32, 4, 1)), (0, 1104, 40, 384, 1, 1, (32, 32, 4, 2)), (0, 64, 984, 1168, 1, 1, (64, 32, 8, 8)),
     # shallow products of many tiles
     (0, 1184, 960, 24, 1, 1, (64, 64, 4, 1)), (1, 1968, 912, 16, 1, 1, (64, 64, 4, 1)), (0, 680, 2792, 32, 1, 1, (64, 64, 4, 1)), (1, 1552, 1176, 104, 1, 1, (64, 64, 4, 1)),
-    (0, 1552, 1176, 104, 1, 1, (64, 64, 8, 1)), (2, 1008, 656, 40, 1, 1, (32, 32, 4, 1)),
+    (0, 1552, 1176, 104, 1, 1, (64, 64, 4, 1)), (0, 1264, 1108, 104, 1, 1, (64, 64, 8, 1)), (2, 1008, 656, 40, 1, 1, (32, 32, 4, 1)),
     # rows that are no whole 16-byte pieces
-    (0, 1964, 456, 3179, 1, 1, (64, 64, 4, 1)), (1, 270, 2271, 220, 1, 1, (64, 64, 4, 1)), (2, 270, 2271, 220, 1, 1, (32, 32, 4, 1)), (0, 2422, 201, 324, 1, 1, (64, 32, 8, 1)),
+    (0, 1964, 456, 3179, 1, 1, (64, 64, 4, 1)), (1, 270, 2271, 220, 1, 1, (64, 64, 4, 1)), (2, 270, 2271, 220, 1, 1, (32, 32, 4, 1)), (0, 2422, 201, 324, 1, 1, (64, 32, 8, 1)), (0, 1547, 664, 34, 1, 1, (64, 64, 4, 1)), (0, 1453, 1051, 173, 1, 1, (64, 64, 4, 1)),
+    (1, 1453, 1051, 173, 1, 1, (64, 64, 4, 1)), (1, 1613, 1101, 267, 1, 1, (64, 64, 8, 1)), (2, 1093, 1101, 267, 1, 1, (64, 64, 8, 1)), (2, 1146, 1651, 112, 1, 1, (64, 64, 4, 1)),
+    # clusters that run at once; rounds of 64 x 64 tiles
+    (1, 533, 228, 841, 1, 1, (32, 32, 4, 2)), (0, 560, 220, 612, 1, 1, (64, 32, 8, 4)), (1, 220, 258, 958, 1, 1, (32, 32, 4, 4)), (0, 128, 512, 1024, 1, 1, (64, 32, 8, 8)),
+    (2, 2612, 864, 148, 1, 1, (64, 64, 4, 1)), (2, 2044, 1004, 764, 1, 1, (64, 64, 8, 1)), (2, 1744, 784, 92, 1, 1, (64, 64, 8, 1)), (0, 1115, 687, 51, 1, 1, (64, 64, 4, 1)), (1, 1032, 2085, 13, 1, 1, (128, 128, 8, 1)), (2, 2111, 2267, 12, 1, 1, (128, 128, 8, 1)),
+    (1, 1679, 1771, 237, 1, 1, (128, 128, 8, 1)), (1, 1235, 2108, 701, 1, 1, (64, 64, 8, 1)), (0, 2111, 2267, 24, 1, 1, (64, 64, 4, 1)),
     (0, 215, 569, 2021, 1, 1, (32, 32, 4, 2)), (1, 202, 504, 677, 1, 1, (64, 32, 8, 4)), (0, 512, 256, 256, 1, 0, (32, 32, 4, 2)), (0, 1100, 1100, 100, 1, 1, (64, 64, 8, 1)),
     (0, 200, 200, 72, 19, 1, (64, 64, 8, 1)), (0, 1664, 1540, 96, 1, 1, (64, 64, 8, 1)), (0, 2000, 1700, 96, 1, 1, (128, 128, 8, 1)), (2, 2001, 1701, 40, 1, 1, (128, 128, 8, 1))])
 def test_tiles_of_the_fp32_products(lib, tb, m, n, k, batch, aligned, cut):

@@ -495,9 +495,9 @@ def test_fp32_gemm_tiles_and_splits(eng, m, n, k, batch, tb):
 
 
 @pytest.mark.parametrize("m,n,k,batch,cuts", [           # cuts of A B, A B^T, A^T B
-    (1100, 1100, 200, 1, [(64, 64, 8, 1)] * 3), (1093, 1101, 267, 1, [(64, 64, 8, 1)] * 3), (200, 200, 72, 19, [(64, 64, 8, 1), (64, 64, 4, 1), (64, 64, 8, 1)]),
+    (1100, 1100, 200, 1, [(64, 64, 8, 1)] * 3), (1093, 1101, 267, 1, [(64, 64, 4, 1)] * 2 + [(64, 64, 8, 1)]), (1613, 1101, 267, 1, [(64, 64, 4, 1), (64, 64, 8, 1), (64, 64, 4, 1)]), (1032, 2085, 13, 1, [(128, 128, 8, 1)] * 3), (200, 200, 72, 19, [(64, 64, 8, 1), (64, 64, 4, 1), (64, 64, 8, 1)]),
     (1100, 900, 24, 1, [(64, 64, 4, 1)] * 3), (1085, 907, 31, 1, [(64, 64, 4, 1)] * 3), (700, 1050, 451, 1, [(64, 64, 4, 1)] * 2 + [(32, 32, 4, 1)]),
-    (512, 256, 256, 1, [(64, 32, 8, 4)] * 3), (517, 250, 251, 1, [(32, 32, 4, 2)] + [(64, 32, 8, 4)] * 2), (523, 781, 300, 1, [(64, 32, 8, 1)] * 3), (120, 424, 1960, 1, [(64, 32, 8, 8)] * 3),
+    (512, 256, 256, 1, [(64, 32, 8, 4)] * 3), (517, 218, 251, 1, [(32, 32, 4, 2)] + [(64, 32, 8, 4)] * 2), (517, 250, 251, 1, [(32, 32, 4, 2)] * 3), (1528, 1404, 76, 1, [(64, 64, 4, 1)] * 3), (523, 781, 300, 1, [(64, 32, 8, 1)] * 3), (120, 424, 1960, 1, [(64, 32, 8, 8)] * 3),
     (31, 33, 65, 1, [(32, 32, 4, 1)] * 3), (90, 70, 1021, 1, [(32, 32, 4, 8)] * 3), (2000, 1700, 96, 1, [(128, 128, 8, 1)] * 3), (2001, 1701, 40, 1, [(128, 128, 8, 1)] * 3)])
 @pytest.mark.parametrize("tb", [0, 1, 2])
 def test_fp32_products_on_the_tiles_they_are_cut_into(eng, m, n, k, batch, cuts, tb):
