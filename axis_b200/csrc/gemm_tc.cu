@@ -375,7 +375,7 @@ int ax_gemm_tc(int out_bf16, int tb, const void* A, const void* B, void* C, cons
         int width = 256;
         if (g_pair_mode == 0 && !g_beside) {
             const long long rows = (m + 255) / 256, tiles[3] = {tiles2, rows * ((n + 191) / 192), rows * ((n + 127) / 128)};
-            const TileTimes t = ax_gemm_tc2_width(tiles, kblocks, S > 1, false);
+            const TileTimes t = ax_gemm_tc2_width(tiles, kblocks, S > 1, ((tb == 2 ? m : k) % 16 != 0) + ((tb == 1 ? k : n) % 16 != 0));
             // (not in place of partial sums that stay in 32 bits: see ax_gemm_tc2_width)
             if (t.width != 256 && (out_bf16 || (S == 1 && best2_s == 1)) && (best2_s == 1 || t.us < split_us)) {
                 width = t.width;

@@ -829,12 +829,14 @@ static int band_of(int m, long long k) {
     return 2ll * m * k > 52000000ll && tiles_m > 12 ? 12 : tiles_m;
 }
 
-// Columns of a tile.  A launch is a set-up, a first load and the last tile's epilogue (f), a round's k-blocks (t each; those of narrow tiles are bound by
-// shared memory and L2), and for each further round of tiles over the pairs its k-blocks or, where they are few, the epilogue that they run under (e).  us of 256 / 192 / 128
-// columns in chains of launches: 2000 x 1536 x 1536 (48, 64, 96 tiles) 12.8 / 11.3 / 13.6, x 4096 24.8 / 21.8 / 28.1, 8192 x 768 x 2304 (96, 128, 192) 26.6 / 23.2 / 27.9,
+// Columns of a tile.  A launch is a set-up, a first load and the last tile's epilogue (f, and c for each tile of a round), a round's k-blocks (t each, by how many of the operands have rows that
+// don't start on 32 bytes: every piece of 128 bytes is five sectors then), and for each further round of tiles over the pairs its k-blocks or, where they are few, the epilogue that they run under (e).
+// Constants are fitted to 1172 seeded products, groups and sums that narrow tiles take, with rms of 3 to 5 %; f of the wide tile is 0.4 us above its fit, as narrow ones are to win by less than that.
+// us of 256 / 192 / 128 columns in chains of launches: 2000 x 1536 x 1536 (48, 64, 96 tiles) 12.8 / 11.3 / 13.6, x 4096 24.8 / 21.8 / 28.1, 8192 x 768 x 2304 (96, 128, 192) 26.6 / 23.2 / 27.9,
 // 1536 x 1024 x 1024 (24 shared by two pairs, 36, 48) 9.5 / 8.2 / 7.7, x 2816 15.3 / 14.8 / 13.0, x 5632 20.7 / 24.6 / 22.7, 2000 x 4096 x 1536 (128, 176, 256) 21.3 / 22.9 / 25.4.
 // Few k-blocks: 2520 x 2920 x 104 (120, 160, 230) 9.9 / 11.5 / 12.9, 5720 x 816 x 128 (92, 115, 161) 7.9 / 8.2 / 9.2, 1544 x 2176 x 568 (63, 84, 119) 9.9 / 13.0 / 11.3, 768 x 2816 x
-// 256 (33, 45, 66) 6.5 / 6.2 / 6.2.  Over 232 shapes the rule is 0.4 % behind the best of the three on average.
+// 256 (33, 45, 66) 6.5 / 6.2 / 6.2.  Rows off 32 bytes, shared / 128: 1072 x 312 x (232 + 2456) 13.2 / 16.4, 1528 x (40, 168, 288) x 3304 17.7 / 21.2; 256 / 192: 888 x 2840 x 4360 31.2 / 33.5.
+// Where the rule takes a narrow tile, 1055 of other seeded shapes, it has 0.867 of the time of the wide one, in 15 of them more than 4 % longer (0.874, 39 of 1172, when t knew no alignment).
 // Only while a plan has queued nothing to another stream (see ax_gemm_plan_begin): products on the side stream fill the pairs that wide tiles leave, and
 // the step of 8 x 1024 tokens at D 768 takes 5114 us with narrow ones throughout, 5037 without.  Steps with adapters are 1 to 2 % shorter, small ones up to 5.
 // A shared or split depth stays one where the output is fp32, which narrow tiles would sum in one chain: the tensor core's accumulator loses with each step.  2-norm errors against float64 of
@@ -842,17 +844,18 @@ static int band_of(int m, long long k) {
 // With three rounds or more the rounds even out and the wide tile, which moves the least, is the best under the power limit: 8192 x 1536 x 2560 (192, 256, 384)
 // 48.6 / 49.5 / 58.4.
 static int g_pairs = 0;                  // pairs that run at once
-TileTimes ax_gemm_tc2_width(const long long* tiles /* of 256, 192, 128 columns */, int kb, bool may_share, bool group) {
+TileTimes ax_gemm_tc2_width(const long long* tiles /* of 256, 192, 128 columns */, int kb, bool may_share, int off32 /* operands, 0 to 2 */) {
     static const int width[3] = {256, 192, 128};
-    static const double f[3] = {5.6, 4.95, 4.5}, t[3] = {0.30, 0.263, 0.215}, e[3] = {3.4, 3.2, 2.5};
+    static const double f[3] = {5.1, 4.1, 3.5}, t[3][3] = {{0.282, 0.290, 0.369}, {0.223, 0.304, 0.322}, {0.194, 0.222, 0.275}}, c[3] = {0.0163, 0.0248, 0.0250}, e[3] = {3.4, 3.2, 2.5};
+    static const double t_shared[3] = {0.240, 0.255, 0.330};
     TileTimes best = {256, 0.0};
     for (int i = 0; i < 3; i++) {
         const long long rounds = g_pairs > 0 ? (tiles[i] + g_pairs - 1) / g_pairs : 1;
-        const double round = t[i] * kb;
-        double us = f[i] + round + (rounds - 1) * (round > e[i] ? round : e[i]), shared;
+        const double round = t[i][off32] * kb;
+        double us = f[i] + c[i] * (rounds > 1 ? g_pairs : tiles[i]) + round + (rounds - 1) * (round > e[i] ? round : e[i]);
         if (i == 0 && may_share && tiles[0] <= 33) {
-            const int S = ax_gemm_tc2_share((int)tiles[0], kb, &shared);
-            if (S > 1) us = group ? 8.2 + 0.36 * ((kb + S - 1) / S) + 0.04 * S * tiles[0] : f[0] + t[0] * shared;
+            const int S = ax_gemm_tc2_share((int)tiles[0], kb, nullptr);
+            if (S > 1) us = 7.7 + t_shared[off32] * ((kb + S - 1) / S) + 0.04 * S * tiles[0];
         }
         if (i == 0) best.us = us;
         else if (tiles[0] <= 2 * g_pairs && us < best.us) best = {width[i], us};
@@ -1108,7 +1111,12 @@ int ax_gemm_tc2_group(int out_bf16, int tb, int mode, int count, const void* con
         for (int g = 0; g < (mode == 2 ? count : 1); g++) kb += (k[g] + BK2 - 1) / BK2;
         for (int i = 0; i < 3; i++)
             for (int g = 0; g < (mode == 1 ? count : 1); g++) tiles[i] += (long long)((m[0] + 255) / 256) * ((n[g] + 255 - 64 * i) / (256 - 64 * i));
-        if (out_bf16 || ax_gemm_tc2_share((int)(tiles[0] < AX_SMS ? tiles[0] : AX_SMS), kb, nullptr) == 1) bn = ax_gemm_tc2_width(tiles, kb, !swb, true).width;
+        if (out_bf16 || ax_gemm_tc2_share((int)(tiles[0] < AX_SMS ? tiles[0] : AX_SMS), kb, nullptr) == 1) {
+            int kk = k[0], nn = 0;           // the deepest segment, any problem
+            for (int g = 1; mode == 2 && g < count; g++) kk = k[g] > kk ? k[g] : kk;
+            for (int g = 0; g < (mode == 1 ? count : 1); g++) nn |= n[g];
+            bn = ax_gemm_tc2_width(tiles, kb, !swb, ((tb == 2 ? m[0] : kk) % 16 != 0) + ((tb == 1 ? kk : nn) % 16 != 0)).width;
+        }
     }
     ax_gemm_width = mode == 4 ? 256 : bn;
 #define G2W(AM, BMj, T, EPI, W) gemm2_launch<AM, BMj, T, EPI, W>(mode, count, A, B, C, D, m, n, k, alpha, D ? beta : 0.f, status, 1, st, XA, XB, xk, swb)

@@ -105,7 +105,7 @@ int ax_gemm_tc2_init(void);
 int ax_gemm_tc2_share(int tiles, int kb, double* cost);
 bool ax_gemm_tc2_by_tma(const void* C, const void* D, long long n, int osz);
 struct TileTimes { int width; double us; };
-TileTimes ax_gemm_tc2_width(const long long* tiles, int kb, bool may_share, bool group);      // tiles of 256, 192 and 128 columns
+TileTimes ax_gemm_tc2_width(const long long* tiles, int kb, bool may_share, int off32);      // tiles of 256, 192 and 128 columns
 int ax_gemm_tc2(int out_bf16, int tb, const void* A, const void* B, void* C, const void* D,
                 int m, int n, int k, float alpha, float beta, int* status, int ksplit, int width, cudaStream_t st);
 void ax_gemm_set_mode(int mode);      // 0 auto, 1 single-CTA only, 2 paired whenever possible

@@ -1173,6 +1173,29 @@ def test_wide_tiles_where_the_epilogue_is_the_round(eng, m, n, k, tb, dt, width,
     assert eng.device_status() == 0
 
 
+@pytest.mark.parametrize("mode,m,dims,depth,tb,parts", [(2, 1072, (232, 2456), 312, 1, 4), (2, 264, (40, 1864, 184), 664, 1, 4), (1, 1528, (40, 168, 288), 3304, 0, 2), (1, 408, (136, 1312), 2696, 1, 4)])
+def test_wide_tiles_where_rows_do_not_start_on_32_bytes(eng, mode, m, dims, depth, tb, parts):
+    """Sums over segments (dims their depths, depth the columns) and outputs of one input (dims their columns): k-blocks of narrow tiles take longer there than the shared depth of wide ones."""
+    rng = np.random.default_rng(m)
+    mk = lambda *sh: bf(rng.standard_normal(sh, dtype=np.float32))
+    n, k = (depth, dims[0]) if mode == 2 else (dims[0], depth)
+    a = [mk(m, d) for d in dims] if mode == 2 else [mk(m, k)]
+    b = [mk(n, d) if mode == 2 else mk(d, k) if tb == 1 else mk(k, d) for d in dims]
+    ia, ib = [put(eng, v, 1) for v in a] + [0, 0], [put(eng, v, 1) for v in b] + [0]
+    ic = [eng.alloc(m * (n if mode == 2 else d), 2) for d in dims] + [0]
+    oa, ob = dims[1], dims[2] if len(dims) > 2 else 0
+    if mode == 2:
+        eng.run([op(E.GEMM_GROUP, c=ic[0], a=ia[0], sa=ia[1], sb=ia[2], b=ib[0], d=ib[1], sc=ib[2], m=m, n=n, k=k, oa=oa, ob=ob, batch=len(dims), oc=2, tb=1, dt=1)])
+        got = [(ic[0], n, sum(p.astype(np.float64) @ q.T for p, q in zip(a, b)), sum(dims))]
+    else:
+        eng.run([op(E.GEMM_GROUP, a=ia[0], b=ib[0], sa=ib[1], sb=ib[2], c=ic[0], d=ic[1], sc=ic[2], m=m, n=n, k=k, oa=oa, ob=ob, batch=len(dims), oc=1, tb=tb, dt=1)])
+        got = [(i, d, a[0].astype(np.float64) @ (q.T if tb == 1 else q), k) for i, d, q in zip(ic, dims, b)]
+    assert (eng.last_variant(), eng.last_gemm_width(), eng.last_gemm_parts()) == (0x23, 256, parts)
+    for i, w, ref, terms in got:
+        check(eng.download_bf16(i, (m, w)), ref, True, terms)
+    assert eng.device_status() == 0
+
+
 @pytest.mark.parametrize("m,n,k,tb,parts", [(1040, 720, 2016, 0, 4), (1040, 720, 2016, 2, 4), (2440, 696, 1880, 1, 2), (2248, 584, 3496, 2, 2)])
 def test_fp32_outputs_keep_the_partial_sums_of_a_shared_depth(eng, m, n, k, tb, parts):
     """The tensor core's accumulator loses with each step, so that one chain over the depth errs by as many times more as there are parts (2.1 and 4.4 times on one B200).  The default
