@@ -376,6 +376,8 @@ static F32Cut f32_cut(int tb, bool plain, long long t128, long long t64, long lo
     // 2612 x 864 x 148 28.0 / 23.1, A B 2228 x 1012 x 140 27.5 / 24.4, A B^T 2636 x 856 x 328 61.7 / 50.7; but A^T B 2044 x 1004 x 764 93 / 97, and 364 tiles 12.2 / 14.9.
     if (plain && vec && t64 >= 3 * AX_SMS && t64 <= 4 * AX_SMS && steps <= 5) return {64, 64, 4, 1};
     if (t64 >= 2 * AX_SMS) return {64, 64, 8, 1};
+    // Three steps of 32 are over before two of 64 where tiles are enough: A B 2732 x 316 x 88 8.9 / 10.6 on 32 x 32, A B^T 2392 x 444 x 92 12.2 / 14.6; but A B^T 300 x 1996 x 84, 160 tiles, 11.5 / 9.6.
+    if (plain && vec && tb != 2 && depth > 64 && depth <= 96 && 4 * t64 >= 5 * AX_SMS) return {64, 64, 4, 1};
     // Below, a launch is the latency of its steps: 64 x 32 tiles (8 x 4 sums to a thread, 43 % of the FMA pipe with two CTAs on an SM, which is what
     // fits) with the depth cut over a cluster as far as two CTAs for each SM.  Where that leaves a third of the SMs idle or most with one CTA and some with two,
     // or takes a second round, 32 x 32 tiles spread better; a product of two steps is over before a larger tile pays.  us, 64 x 32 with 1 / 2 / 4 CTAs to a tile |

@@ -154,7 +154,7 @@ def test_cut_of_the_adapters_products(lib, count, one_x, N, F, R, members, token
     (1, 1453, 1051, 173, 1, 1, (64, 64, 4, 1)), (1, 1613, 1101, 267, 1, 1, (64, 64, 8, 1)), (2, 1093, 1101, 267, 1, 1, (64, 64, 8, 1)), (2, 1146, 1651, 112, 1, 1, (64, 64, 4, 1)),
     # clusters that run at once; rounds of 64 x 64 tiles
     (1, 533, 228, 841, 1, 1, (32, 32, 4, 2)), (0, 560, 220, 612, 1, 1, (64, 32, 8, 4)), (1, 220, 258, 958, 1, 1, (32, 32, 4, 4)), (0, 128, 512, 1024, 1, 1, (64, 32, 8, 8)),
-    (2, 2612, 864, 148, 1, 1, (64, 64, 4, 1)), (2, 2044, 1004, 764, 1, 1, (64, 64, 8, 1)), (2, 1744, 784, 92, 1, 1, (64, 64, 8, 1)), (0, 1115, 687, 51, 1, 1, (64, 64, 4, 1)), (1, 1032, 2085, 13, 1, 1, (128, 128, 8, 1)), (2, 2111, 2267, 12, 1, 1, (128, 128, 8, 1)),
+    (2, 2612, 864, 148, 1, 1, (64, 64, 4, 1)), (2, 2044, 1004, 764, 1, 1, (64, 64, 8, 1)), (0, 2732, 316, 88, 1, 1, (64, 64, 4, 1)), (1, 300, 1996, 84, 1, 1, (32, 32, 4, 1)), (2, 748, 1408, 96, 1, 1, (32, 32, 4, 1)), (2, 1744, 784, 92, 1, 1, (64, 64, 8, 1)), (0, 1115, 687, 51, 1, 1, (64, 64, 4, 1)), (1, 1032, 2085, 13, 1, 1, (128, 128, 8, 1)), (2, 2111, 2267, 12, 1, 1, (128, 128, 8, 1)),
     (1, 1679, 1771, 237, 1, 1, (128, 128, 8, 1)), (1, 1235, 2108, 701, 1, 1, (64, 64, 8, 1)), (0, 2111, 2267, 24, 1, 1, (64, 64, 4, 1)),
     (0, 215, 569, 2021, 1, 1, (32, 32, 4, 2)), (1, 202, 504, 677, 1, 1, (64, 32, 8, 4)), (0, 512, 256, 256, 1, 0, (32, 32, 4, 2)), (0, 1100, 1100, 100, 1, 1, (64, 64, 8, 1)),
     (0, 200, 200, 72, 19, 1, (64, 64, 8, 1)), (0, 1664, 1540, 96, 1, 1, (64, 64, 8, 1)), (0, 2000, 1700, 96, 1, 1, (128, 128, 8, 1)), (2, 2001, 1701, 40, 1, 1, (128, 128, 8, 1))])
